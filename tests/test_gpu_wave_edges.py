@@ -1,0 +1,42 @@
+"""Batched growth against the one-split loop at the sizes where a wave kernel's tiling can go
+wrong: row counts at the edges of the partition's 2048-row tiles, one to a few hundred
+rows, ragged feature groups, few and many leaves.  Both loops sum exact integers, so the trees
+are equal bit for bit."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(n, nf, seed=0):
+    rng = np.random.default_rng([seed, n, nf])
+    X = rng.standard_normal((n, nf)).astype(np.float32)
+    X[:, 0] = np.round(X[:, 0] * 2)
+    X[rng.random((n, nf)) < 0.05] = np.nan
+    y = np.nan_to_num(X[:, 0]) - np.nan_to_num(X[:, -1]) + 0.3 * rng.standard_normal(n)
+    return X, y, np.arange(n) // 7
+
+
+def _same(a, b):
+    assert len(a) == len(b)
+    for t, (p, q) in enumerate(zip(a, b)):
+        for f in ("is_leaf", "feature", "threshold", "left", "right", "missing_left", "n_samples", "depth", "value",
+                  "gain", "values", "cover", "prefix"):
+            assert np.array_equal(getattr(p, f), getattr(q, f)), (t, f)
+
+
+@pytest.mark.parametrize("n,nf,leaves,extra", [
+    (65, 1, 4, {}), (2047, 3, 31, {}), (2048, 33, 31, {}), (2049, 16, 31, {}), (4097, 17, 255, {}),
+    (6144, 65, 8, {}), (20481, 31, 31, dict(goss=1)), (4096, 32, 2, {}),
+    (9001, 40, 31, dict(objective="pairwise")), (70001, 96, 31, dict(objective="pairwise", goss=1))])
+def test_waves_equal_one_split_loop(native, n, nf, leaves, extra):
+    X, y, ts = _case(n, nf)
+    p = dict(n_estimators=4, learning_rate=0.1, max_depth=8, max_leaves=leaves, horizon=1, random_state=3,
+             min_samples_leaf=2, pair_splits=False, goss=0)
+    p.update(extra)
+    trees = []
+    for grow in (0, 1):
+        b = native.Booster(**p, grow=grow)
+        b.fit(X, y, timestamps=ts)
+        trees.append(b.trees())
+    _same(trees[0], trees[1])

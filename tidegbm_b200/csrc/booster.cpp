@@ -738,7 +738,6 @@ WaveCtx FitRun::wave_ctx() const {
     w.cand_gain = D.cand_gain.p;
     w.cand_key = D.cand_key.p;
     w.tickets = D.tickets.p;
-    w.tile_counts = D.tile_counts.p;
     w.gp = gp;
     w.goss_scale = use_goss ? goss_scale : 1.0;
     w.n_slots = n_slots;
@@ -1226,7 +1225,7 @@ private:
         check(cudaStreamEndCapture(s_, &body_out), "body capture end");
         check(cudaGraphInstantiate(&exec_, graph_, 0), "graph instantiate");
         // launches counted per grow (the graph's kernels are this library's)
-        g_kernel_launches.fetch_sub(pair_ ? 12 : 8);
+        g_kernel_launches.fetch_sub(pair_ ? 11 : 7);
     }
 
     std::vector<FitRun*> runs_;

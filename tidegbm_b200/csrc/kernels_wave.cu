@@ -29,8 +29,8 @@
 //   q8 var       uint16 (qg + 128 | qh << 8): (1 << 20 | qg + 128) and qh: 2 reductions
 // Sums of quantised values are exact integers; the scan rescales them.
 //
-// Partition (split_indices, cpp/src/tree.cpp:68-91): stable, two launches over
-// 2048-row tiles of all planned leaves (count, then scatter with in-tile ballot ranks).
+// Partition (split_indices, cpp/src/tree.cpp:68-91): one launch over 2048-row tiles of all
+// planned leaves (in-tile ballot ranks; tiles reserve their places with one atomic).
 #include <atomic>
 #include <cstdint>
 #include <cstring>
@@ -798,19 +798,6 @@ constexpr int kPartThreads = 256;
 constexpr int kPartWarps = kPartThreads / 32;
 constexpr int kPartPer = kPartTile / kPartThreads;
 
-__device__ __forceinline__ int block_sum(int v, int* red) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    int t = 0;
-#pragma unroll
-    for (int w = 0; w < kPartWarps; ++w) t += red[w];
-    return t;
-}
-
 // A row's g payload (element i of the payload array), widened to 64 bits, and back.
 __device__ __forceinline__ long long load_payload(const WaveCtx& X, long long i) {
     if (X.pay_bytes == 8) return static_cast<const long long*>(X.gq)[i];
@@ -886,75 +873,33 @@ __device__ __forceinline__ void load_tile_prefix(const WaveCtx* ctxs, int n_ctx,
     __syncthreads();
 }
 
+// One launch moves the rows of every planned leaf into its children.  A tile of 2048 rows
+// ranks its rows by side with ballots, reserves its places in both children with one 64-bit
+// atomic add on the leaf's cursor (left rows in the low word, right rows in the high word)
+// and writes them: left rows upward from the leaf's start, right rows in blocks downward
+// from its end, so no tile needs the leaf's left total.  The tile whose reservation
+// completes the leaf knows that total and writes the children's ranges.
+//
+// Inside a tile the row order is kept, between tiles it depends on which reserves first.
+// Every use of a row list is an exact integer sum, so no result depends on the order, and a
+// child's list still runs over ascending row ids tile by tile, which is what the gathers of
+// codes need.  The reference's stable order took two launches (count, then scatter from the
+// tile prefixes): both are bound by their chain of dependent loads, and the second read the
+// rows and codes again.
 __global__ void __launch_bounds__(kPartThreads)
-    wave_part_count_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx) {
+    wave_part_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx) {
     pdl_wait();
     pdl_trigger();
     __shared__ int s_pref[kMaxWaveCtx + 1];
-    __shared__ int red[kPartWarps];
-    __shared__ int s_last;
+    __shared__ int wc[kPartPer * kPartWarps];
+    __shared__ unsigned long long s_old;
     load_tile_prefix(ctxs, n_ctx, s_pref);
     const int total = s_pref[n_ctx];
-    for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const TileRef tr = find_tile(ctxs, s_pref, n_ctx, t);
-        const WaveCtx& X = ctxs[tr.c];
-        WaveCtl* ctl = X.ctl;
-        const int L = ctl->exp_leaf[tr.e];
-        const DevNode& N = X.nodes[L];
-        const DevSplit& S = ctl->expanded[L] == 2 ? X.splits_pair[L] : X.splits[L];
-        const int32_t* in = (N.buf ? X.rows1 : X.rows0) + N.start;
-        const int base = tr.k * kPartTile, end = min(base + kPartTile, N.count);
-        int32_t row[kPartPer];
-        bool left[kPartPer];
-        load_tile(X, in, S, base, end, row, left);
-        int cnt = 0;
-#pragma unroll
-        for (int i = 0; i < kPartPer; ++i) cnt += left[i] ? 1 : 0;
-        cnt = block_sum(cnt, red);
-        const int t0 = ctl->exp_tile0[tr.e], t1 = ctl->exp_tile0[tr.e + 1];
-        if (threadIdx.x == 0) {
-            X.tile_counts[tr.lt] = cnt;
-            __threadfence();
-            s_last = atomicAdd(&ctl->part_ticket[tr.e], 1) == t1 - t0 - 1;
-        }
-        __syncthreads();
-        if (s_last) {
-            // the leaf's last tile: its tiles' counts -> exclusive prefixes (in place), and the
-            // leaf's left total, for the scatter
-            __threadfence();
-            volatile int* tc = X.tile_counts;
-            const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-            int run = 0;
-            for (int k0 = t0; k0 < t1; k0 += kPartThreads) {
-                const int k = k0 + static_cast<int>(threadIdx.x);
-                const int v = k < t1 ? tc[k] : 0;
-                int incl = v;
-#pragma unroll
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int u = __shfl_up_sync(0xffffffffu, incl, o);
-                    if (lane >= o) incl += u;
-                }
-                if (lane == 31) red[warp] = incl;
-                __syncthreads();
-                int wb = 0, all = 0;
-#pragma unroll
-                for (int w = 0; w < kPartWarps; ++w) {
-                    if (w < warp) wb += red[w];
-                    all += red[w];
-                }
-                if (k < t1) tc[k] = run + wb + incl - v;
-                run += all;
-                __syncthreads();  // red reuse
-            }
-            if (threadIdx.x == 0) {
-                ctl->exp_left[tr.e] = run;
-                ctl->part_ticket[tr.e] = 0;  // ready for the next wave
-            }
-        }
-        __syncthreads();  // s_last reuse
-    }
-    // Clear the histogram slots of this wave's children (2 per expansion, consecutive):
-    // the smaller child's is accumulated into by the histogram launch.
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const unsigned lt_mask = (1u << lane) - 1u;
+    // Clear the histogram slots of this wave's children (2 per expansion, consecutive): the
+    // smaller child's is accumulated into by the histogram launch.  First, so that the stores
+    // drain while the tiles wait for their loads.
     for (int c = 0; c < n_ctx; ++c) {
         const WaveCtx& X = ctxs[c];
         const int ns = 2 * X.ctl->n_exp;
@@ -973,38 +918,17 @@ __global__ void __launch_bounds__(kPartThreads)
             if (k < n16_4) c4[k] = make_uint4(0, 0, 0, 0);
         }
     }
-}
-
-__global__ void __launch_bounds__(kPartThreads)
-    wave_part_scatter_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ int s_pref[kMaxWaveCtx + 1];
-    __shared__ int wc[kPartPer * kPartWarps];
-    load_tile_prefix(ctxs, n_ctx, s_pref);
-    const int total = s_pref[n_ctx];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const unsigned lt_mask = (1u << lane) - 1u;
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
         const TileRef tr = find_tile(ctxs, s_pref, n_ctx, t);
         const WaveCtx& X = ctxs[tr.c];
-        const WaveCtl* ctl = X.ctl;
+        WaveCtl* ctl = X.ctl;
         const int L = ctl->exp_leaf[tr.e];
         const DevNode& N = X.nodes[L];
-        const DevSplit& S = X.ctl->expanded[L] == 2 ? X.splits_pair[L] : X.splits[L];
-        const int n_left = ctl->exp_left[tr.e];   // the leaf's left rows (count launch)
-        const int left0 = X.tile_counts[tr.lt];  // left rows of the leaf's earlier tiles
-        if (tr.k == 0 && threadIdx.x == 0) {
-            DevNode& A = X.spec[2 * L];
-            DevNode& B = X.spec[2 * L + 1];
-            A.start = N.start;
-            A.count = n_left;
-            B.start = N.start + n_left;
-            B.count = N.count - n_left;
-        }
+        const DevSplit& S = ctl->expanded[L] == 2 ? X.splits_pair[L] : X.splits[L];
         const int32_t* in = (N.buf ? X.rows1 : X.rows0) + N.start;
         int32_t* out = (N.buf ? X.rows0 : X.rows1) + N.start;
-        const int base = tr.k * kPartTile, end = min(base + kPartTile, N.count);
+        const int count = N.count;
+        const int base = tr.k * kPartTile, end = min(base + kPartTile, count);
         int32_t row[kPartPer];
         bool left[kPartPer];
         load_tile(X, in, S, base, end, row, left);
@@ -1031,6 +955,7 @@ __global__ void __launch_bounds__(kPartThreads)
 #pragma unroll
         for (int i = 0; i < kPartPer; ++i) {
             int e = run;
+#pragma unroll
             for (int w = 0; w < kPartWarps; ++w) {
                 const int cw = wc[i * kPartWarps + w];
                 if (w < warp) e += cw;
@@ -1038,17 +963,36 @@ __global__ void __launch_bounds__(kPartThreads)
             }
             excl[i] = e;
         }
+        const int n_right = end - base - run;  // run: the tile's left rows
+        if (threadIdx.x == 0) {
+            const unsigned long long old =
+                atomicAdd(&ctl->part_cur[tr.e],
+                          (static_cast<unsigned long long>(n_right) << 32) | static_cast<unsigned int>(run));
+            s_old = old;
+            const int l0 = static_cast<int>(old & 0xffffffffu), r0 = static_cast<int>(old >> 32);
+            if (l0 + r0 + (end - base) == count) {
+                DevNode& A = X.spec[2 * L];
+                DevNode& B = X.spec[2 * L + 1];
+                A.start = N.start;
+                A.count = l0 + run;
+                B.start = N.start + l0 + run;
+                B.count = count - l0 - run;
+            }
+        }
+        __syncthreads();
+        const int left0 = static_cast<int>(s_old & 0xffffffffu);
+        const int right0 = count - static_cast<int>(s_old >> 32) - n_right;
 #pragma unroll
         for (int i = 0; i < kPartPer; ++i) {
             if (row[i] < 0) continue;
             const int kk = base + i * kPartThreads + threadIdx.x;
             const int lrank = excl[i] + __popc(bal[i] & lt_mask);
-            const int dst = left[i] ? left0 + lrank : n_left + (base - left0) + (kk - base - lrank);
+            const int dst = left[i] ? left0 + lrank : right0 + (kk - base - lrank);
             out[dst] = row[i];
             store_payload(X, to0 + dst, pg[i]);
             if (X.hq != nullptr) static_cast<long long*>(X.hq)[to0 + dst] = ph[i];
         }
-        __syncthreads();  // wc reuse
+        __syncthreads();  // wc and s_old reuse
     }
 }
 
@@ -1344,9 +1288,7 @@ void launch_rows_max(const int32_t* rows, int n_rows, const double* g, const dou
 }
 
 void launch_wave_partition(const WaveCtx* ctxs, int n_ctx, int grid, cudaStream_t s) {
-    launch_pdl(wave_part_count_kernel, dim3(grid), dim3(kPartThreads), 0, s, "wave_part_count launch", ctxs, n_ctx);
-    launch_pdl(wave_part_scatter_kernel, dim3(grid), dim3(kPartThreads), 0, s, "wave_part_scatter launch", ctxs,
-               n_ctx);
+    launch_pdl(wave_part_kernel, dim3(grid), dim3(kPartThreads), 0, s, "wave_part launch", ctxs, n_ctx);
 }
 
 void launch_wave_tree_init(DevNode* nodes, DevSplit* splits, DevTreeState* st, WaveCtl* ctl, int n_sample_host,

@@ -458,6 +458,7 @@ __global__ void __launch_bounds__(kSelectThreads)
                     const DevNode& N = nodes[L];
                     tiles = (N.count + kPartTile - 1) / kPartTile;
                     ctl->exp_leaf[e] = L;
+                    ctl->part_cur[e] = 0ull;
                     // 2: the children are partitioned by L's with-pairs split, 1: by its axis split
                     ctl->expanded[L] = (X.pair_on && pair_used < X.max_pair) ? 2 : 1;
                     for (int sd = 0; sd < 2; ++sd) {

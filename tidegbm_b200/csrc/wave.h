@@ -15,9 +15,10 @@
 //             outside the top B can ever be chosen (the B better ones exhaust the
 //             budget first), and the best one is always expanded, so every wave commits
 //             at least one split and the result is the reference's tree.
-//   partition the planned leaves' rows into their children (stable, tree.cpp:68-91),
-//             into the other ping-pong buffer at the leaf's own row range: a leaf whose
-//             expansion is never committed keeps its rows untouched.
+//   partition the planned leaves' rows into their children (tree.cpp:68-91), into the
+//             other ping-pong buffer at the leaf's own row range: a leaf whose expansion
+//             is never committed keeps its rows untouched.  The order of the rows inside a
+//             child is free: everything computed from a row list is an exact integer sum.
 //   histogram the smaller child of every planned leaf, one persistent cluster launch
 //             over all (context, leaf) jobs: rows x feature groups cut into one
 //             contiguous range per cluster.
@@ -76,8 +77,9 @@ struct WaveCtl {
     int pad[2];
     int exp_leaf[kMaxLeavesCap];
     int exp_tile0[kMaxLeavesCap + 1];
-    int exp_left[kMaxLeavesCap];     // rows of the planned leaf going left (partition count)
-    int part_ticket[kMaxLeavesCap];  // count tiles done per planned leaf (zero between launches)
+    // rows of the planned leaf placed so far by its partition tiles: left in the low word,
+    // right in the high word (zeroed by the select that plans the expansion)
+    unsigned long long part_cur[kMaxLeavesCap];
     int expanded[kMaxNodes];  // 0 not expanded; 1, 2: children planned by the axis, with-pairs split
 };
 
@@ -112,7 +114,6 @@ struct WaveCtx {
     double* cand_gain;  // scan candidates [(2 * kMaxNodes + 1)][F]
     int* cand_key;
     int* tickets;      // [2 * kMaxNodes + 1], zero between launches
-    int* tile_counts;  // [max tiles of a wave]
     GrowParams gp;
     double goss_scale;
     int n_slots;
