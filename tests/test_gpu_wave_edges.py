@@ -27,6 +27,7 @@ def _same(a, b):
 
 @pytest.mark.parametrize("n,nf,leaves,extra", [
     (65, 1, 4, {}), (2047, 3, 31, {}), (2048, 33, 31, {}), (2049, 16, 31, {}), (4097, 17, 255, {}),
+    (30011, 40, 255, dict(wave_expand=0)), (12289, 70, 255, dict(wave_expand=0, objective="pairwise")),
     (6144, 65, 8, {}), (20481, 31, 31, dict(goss=1)), (4096, 32, 2, {}),
     (9001, 40, 31, dict(objective="pairwise")), (70001, 96, 31, dict(objective="pairwise", goss=1))])
 def test_waves_equal_one_split_loop(native, n, nf, leaves, extra):
@@ -36,7 +37,7 @@ def test_waves_equal_one_split_loop(native, n, nf, leaves, extra):
     p.update(extra)
     trees = []
     for grow in (0, 1):
-        b = native.Booster(**p, grow=grow)
+        b = native.Booster(**dict(p, grow=grow))
         b.fit(X, y, timestamps=ts)
         trees.append(b.trees())
     _same(trees[0], trees[1])

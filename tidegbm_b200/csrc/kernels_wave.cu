@@ -5,8 +5,8 @@
 // planned leaf; subtract_hist_inplace's larger child is derived in the scan).  One
 // persistent launch of clusters of 1, 2 or 4 CTAs (the autotuned privatisation depth:
 // how many CTA-private histograms a flush merges).  The work (rows x groups of 32
-// features, summed over the jobs) is cut into one contiguous range per cluster, walked as
-// pieces (job, feature group, rows) whose rows the cluster's CTAs split.  Inside a CTA the
+// features, summed over the jobs) is cut into one range per cluster, walked as pieces
+// (job, feature group, rows) whose rows the cluster's CTAs split.  Inside a CTA the
 // accumulation is the lane-per-row scheme:
 // a warp takes 32 rows, lane l holds its row's 32 code bytes of the group (staged in shared
 // memory by TMA gathers in the constant-hessian modes, else loaded from global memory) and
@@ -107,27 +107,21 @@ struct JobRows {
     int slot;
 };
 
+__device__ __forceinline__ int job_count(const WaveCtx& X, int src, int e) {
+    return src == 0 ? X.st->n_sample : X.ctl->job[e].count;
+}
+
 __device__ __forceinline__ JobRows job_rows(const WaveCtx& X, int src, int e) {
+    WaveJob j{0, 0, 0, 0};
+    if (src == 0) j.count = X.st->n_sample;
+    else j = X.ctl->job[e];
     JobRows r;
-    if (src == 0) {
-        r.rows = X.rows0;
-        r.gq = X.gq;
-        r.hq = X.hq;
-        r.count = X.st->n_sample;
-        r.slot = 0;
-        return r;
-    }
-    const int L = X.ctl->exp_leaf[e];
-    const DevNode& a = X.spec[2 * L];
-    const DevNode& b = X.spec[2 * L + 1];
-    const bool left_small = a.count <= b.count;  // cpp/src/tree.cpp:423
-    const DevNode& c = left_small ? a : b;
-    r.rows = (c.buf ? X.rows1 : X.rows0) + c.start;
-    const long long pos = static_cast<long long>(c.buf) * X.pay_pitch + c.start;
+    r.rows = (j.buf ? X.rows1 : X.rows0) + j.start;
+    const long long pos = static_cast<long long>(j.buf) * X.pay_pitch + j.start;
     r.gq = static_cast<const unsigned char*>(X.gq) + pos * X.pay_bytes;
     r.hq = X.hq != nullptr ? static_cast<const long long*>(X.hq) + pos : nullptr;
-    r.count = c.count;
-    r.slot = c.slot;
+    r.count = j.count;
+    r.slot = j.slot;
     return r;
 }
 
@@ -250,6 +244,11 @@ __device__ __noinline__ void accumulate_const(unsigned int* __restrict__ P, unsi
     const bool two_chunks = stride - fg0 >= 32;
     const bool v8 = two_chunks && (stride & 31) == 0;
     constexpr int kStep = kWarps * 32;
+    for (int k = threadIdx.x; k < kTot; k += kThreads) {
+        Gt[k] = 0ull;
+        Ct[k] = 0u;
+    }
+    __syncthreads();
     for (int s0 = r0; s0 < r1; s0 += T::sub) {
         const int s1 = min(r1, s0 + T::sub);
         const int k0 = s0 + warp * 32 + lane;
@@ -383,10 +382,9 @@ __device__ __noinline__ unsigned int accumulate_const_tma(unsigned int* __restri
     long long accG[kCells];
 #pragma unroll
     for (int cc = 0; cc < kCells; ++cc) accG[cc] = 0;
-    // the staging area's generic writes (zeroing, the previous piece's totals) before the
-    // gathers' asynchronous ones; the descriptor was written by a host copy
+    // the staging area's generic writes (the previous piece's totals) before the gathers'
+    // asynchronous ones
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    if (lane < 8) asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(map) : "memory");
     __syncthreads();
     bool ok = true;
     unsigned int pending = 0u;  // slots with gathers in flight
@@ -416,9 +414,11 @@ __device__ __noinline__ unsigned int accumulate_const_tma(unsigned int* __restri
         return p;
     };
     const int n_rounds = r1 > r0 ? (r1 - r0 + kStep - 1) / kStep : 0;
-    PT p0 = issue(0, 0, row_of(0));
-    PT p1 = issue(1, 1, row_of(1));
+    const int ra = row_of(0), rb = row_of(1);  // all three loads before the first use
     int rq = row_of(2);
+    PT p0 = issue(0, 0, ra);
+    PT p1 = issue(1, 1, rb);
+    bool first = true;  // the first fold writes Ct, later ones add
     const int h = (lane >> 2) & 1;  // lanes 4-7 of each 8 read their second half first
     for (int i = 0; i < n_rounds; ++i) {
         const int s = i & 1;
@@ -468,10 +468,11 @@ __device__ __noinline__ unsigned int accumulate_const_tma(unsigned int* __restri
                     dc = n1 | (n2 << 16);
                 }
                 accG[cc] += dg;
-                Ct[ti] += dc;
+                Ct[ti] = first ? dc : Ct[ti] + dc;
 #pragma unroll
                 for (int pl = 0; pl < T::planes; ++pl) P[pl * kPlane + cell] = 0u;
             }
+            first = false;
             __syncthreads();
         }
     }
@@ -483,7 +484,9 @@ __device__ __noinline__ unsigned int accumulate_const_tma(unsigned int* __restri
 #pragma unroll
     for (int cc = 0; cc < kCells; ++cc) {
         const int cell = threadIdx.x + cc * kThreads;
-        Gt[(cell & 31) * kTotPitch + (cell >> 5)] = static_cast<unsigned long long>(accG[cc]);
+        const int ti = (cell & 31) * kTotPitch + (cell >> 5);
+        Gt[ti] = static_cast<unsigned long long>(accG[cc]);
+        if (first) Ct[ti] = 0u;  // no rows
     }
     return phase;
 }
@@ -601,13 +604,101 @@ __device__ __noinline__ void accumulate_var(unsigned int* __restrict__ P, unsign
     }
 }
 
+// A cell's totals summed over the cluster, and its hessian and count in the output's form.
+template <bool kVar>
+struct CellSum {
+    unsigned long long g = 0, h = 0;
+    unsigned int c = 0, c2 = 0;
+};
+
+// The end of a piece: every rank of a cluster of CS CTAs takes a share of the group's cells,
+// adds it over the CTAs' shared totals (all loads before the first use) and writes it out.
+// The CTAs may reuse their totals after the second barrier; its arrival comes before the
+// global writes, so that nothing waits for those.
+template <bool kVar, int CS>
+__device__ __forceinline__ void flush_piece(const WaveCtx& X, const unsigned long long* Gt, const unsigned long long* Ht,
+                                            const unsigned int* Ct, unsigned int rank, int nf_here, size_t out0, bool whole,
+                                            unsigned long long hq1, unsigned long long hq2) {
+    constexpr int kIter = kPlane / CS / kThreads;  // cells a thread writes (8, 4 or 2)
+    const int share = nf_here * kBins / CS;
+    const int i0 = static_cast<int>(rank) * share + static_cast<int>(threadIdx.x);
+    const int i1 = static_cast<int>(rank + 1) * share;
+    CellSum<kVar> v[kIter];
+    if constexpr (CS > 1) cg::this_cluster().sync();
+#pragma unroll
+    for (int kk = 0; kk < CS; ++kk) {
+        const unsigned long long* rG = CS > 1 ? cg::this_cluster().map_shared_rank(Gt, kk) : Gt;
+        const unsigned long long* rH = CS > 1 ? cg::this_cluster().map_shared_rank(Ht, kk) : Ht;
+        const unsigned int* rC = CS > 1 ? cg::this_cluster().map_shared_rank(Ct, kk) : Ct;
+#pragma unroll
+        for (int q = 0; q < kIter; ++q) {
+            const int i = i0 + q * kThreads;
+            if (i >= i1) continue;
+            const int ti = i + (i >> 8);  // (feature i >> 8, bin i & 255) in the padded layout
+            const unsigned int pc = rC[ti];
+            v[q].g += rG[ti];
+            if constexpr (kVar) {
+                v[q].h += rH[ti];
+                v[q].c += pc;
+            } else {
+                v[q].c += pc & 0xffffu;
+                v[q].c2 += pc >> 16;
+            }
+        }
+    }
+    if constexpr (CS > 1) asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+#pragma unroll
+    for (int q = 0; q < kIter; ++q) {
+        const int i = i0 + q * kThreads;
+        if (i >= i1) continue;
+        unsigned long long h = v[q].h;
+        unsigned int cn = v[q].c;
+        if constexpr (!kVar) {
+            h = static_cast<unsigned long long>(v[q].c) * hq1 + static_cast<unsigned long long>(v[q].c2) * hq2;
+            cn += v[q].c2;
+        }
+        if (cn == 0u) continue;
+        const size_t o = out0 + i;
+        if (whole) {
+            reinterpret_cast<unsigned long long*>(X.G)[o] = v[q].g;
+            reinterpret_cast<unsigned long long*>(X.H)[o] = h;
+            X.C[o] = static_cast<int>(cn);
+        } else {
+            atomicAdd(reinterpret_cast<unsigned long long*>(X.G) + o, v[q].g);
+            atomicAdd(reinterpret_cast<unsigned long long*>(X.H) + o, h);
+            atomicAdd(X.C + o, static_cast<int>(cn));
+        }
+    }
+    if constexpr (CS > 1) asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+    else __syncthreads();
+}
+
 // One launch histograms every job (context, planned leaf's smaller child; or each
 // context's root) of the wave.  The work, rows x feature groups summed over the jobs, is
-// cut into equal contiguous ranges, one per cluster; a cluster walks its range as pieces
+// cut into one contiguous range per cluster; a cluster walks its range as pieces
 // (job, feature group, row range), its CTAs split each piece's rows, and after a piece the
 // cluster adds its CTAs' totals through distributed shared memory and writes them out:
 // plain stores when the piece is the whole (job, feature group), 64-bit atomics when
 // other clusters share it.  A job's slot is clear before the launch.
+//
+// The ranges: equal ones balance the rows but let a cluster straddle two (job, group)
+// pairs, which costs it a second set-up, fold and flush.  Where there are at most 32 jobs
+// and no more pairs than clusters, every pair gets clusters of its own in proportion to its
+// rows, if the largest share then exceeds the equal one by less than that cost
+// (kPieceRows rows a CTA).
+//
+// A child wave has a few hundred to a few thousand rows a CTA, so its launch is mostly fixed
+// cost.  In cycles of one CTA at 100k x 32 the start took: plan 7,300 and piece set-up 5,500
+// (chains of loads through the contexts and the node table: now one record a job, the
+// contexts staged before the wait), flush 10,000 and the barrier and clearing after it 4,500
+// (loads of one CTA's totals after another, global writes before the barrier: now all loads,
+// the barrier, then the writes; nothing to clear).  Together with the pairs' own clusters:
+// fits of 0.85M x 64 pairwise 92.2 -> 83.5 ms, 1.2M x 96 int8 97.0 -> 84.3 ms, 10M x 128
+// 435 -> 416 ms.
+constexpr int kPieceRows = 1500;
+constexpr int kMinCtaRows = 128;  // no finer split of a pair: a CTA's fold and flush cost more
+constexpr int kWarpJobs = 32;
+
 template <int kMode>
 __global__ void __launch_bounds__(kThreads, 1)
     wave_hist_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx, int src, unsigned long long* rows_counter) {
@@ -622,40 +713,139 @@ __global__ void __launch_bounds__(kThreads, 1)
     // TMA staging (constant-hessian modes): slots over Gt from its first 128-byte boundary,
     // two mbarriers per warp, their parities
     __shared__ __align__(8) unsigned long long s_bars[2 * kWarps];
+    __shared__ WaveCtx s_ctx;  // the first context's constants
     unsigned char* stage = smem_raw + Lay::tot_off;
     stage += (128u - (smem_u32(stage) & 127u)) & 127u;
     unsigned int phase = 0u;
-    {  // private state first: it overlaps the previous kernel's tail
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    // What does not depend on the previous kernel first, so that it overlaps its tail: the
+    // private state, the barriers, and the context's constants (written by a host copy before
+    // the fit's first tree), its TMA descriptor included.
+    {
         uint4* z = reinterpret_cast<uint4*>(smem_raw);
-        for (int k = threadIdx.x; k < static_cast<int>(Lay::region / 16); k += blockDim.x) z[k] = make_uint4(0, 0, 0, 0);
+        for (int k = threadIdx.x; k < static_cast<int>(Lay::work / 16); k += blockDim.x) z[k] = make_uint4(0, 0, 0, 0);
     }
-    if (!T::var && (threadIdx.x & 31) == 0) {
-        mbar_init(smem_u32(&s_bars[2 * (threadIdx.x >> 5)]));
-        mbar_init(smem_u32(&s_bars[2 * (threadIdx.x >> 5) + 1]));
+    stage_ctx(s_ctx, ctxs);
+    if (!T::var && lane == 0) {
+        mbar_init(smem_u32(&s_bars[2 * warp]));
+        mbar_init(smem_u32(&s_bars[2 * warp + 1]));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (!T::var && lane < 8)
+        for (int c = 0; c < n_ctx; ++c)
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(&ctxs[c].codes_map) : "memory");
+    __syncthreads();
     pdl_wait();
     pdl_trigger();
+    auto ctx_of = [&](int c) -> const WaveCtx& { return c == 0 ? s_ctx : ctxs[c]; };
 
     // ---- work plan (the same in every CTA) ----
     __shared__ int s_cpref[kMaxWaveCtx + 1];
     __shared__ unsigned long long s_red[kWarps], s_rsum[kWarps];
-    if (static_cast<int>(threadIdx.x) < n_ctx)
-        s_cpref[threadIdx.x] = src == 0 ? (ctxs[threadIdx.x].ctl->active ? 1 : 0) : ctxs[threadIdx.x].ctl->n_exp;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int c = 0; c < n_ctx; ++c) {
-            const int v = s_cpref[c];
-            s_cpref[c] = acc;
-            acc += v;
+    __shared__ int s_cstart[kWarpJobs + 1], s_cper[kWarpJobs], s_aligned;
+    __shared__ unsigned long long s_hq[2];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int csize = static_cast<int>(cluster.dim_blocks().y);  // CTAs per cluster: 1, 2 or 4
+    const int cl = static_cast<int>(blockIdx.y) / csize;
+    const int n_cl = static_cast<int>(gridDim.y) / csize;
+    const unsigned int rank = csize > 1 ? cluster.block_rank() : 0u;
+    if (warp == 0) {
+        int all = 0;
+        for (int c0 = 0; c0 < n_ctx; c0 += 32) {
+            const int c = c0 + lane;
+            int v = 0;
+            if (c < n_ctx) v = src == 0 ? (ctx_of(c).ctl->active ? 1 : 0) : ctx_of(c).ctl->n_exp;
+            int incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (c < n_ctx) s_cpref[c] = all + incl - v;
+            all += __shfl_sync(0xffffffffu, incl, 31);
         }
-        s_cpref[n_ctx] = min(acc, kMaxWaveJobs);
+        const int nj = min(all, kMaxWaveJobs);
+        if (lane == 0) {
+            s_cpref[n_ctx] = nj;
+            s_aligned = 0;
+        }
+        __syncwarp();
+        if (nj <= kWarpJobs) {
+            // a lane per job: the work prefix, and the clusters of each of the job's pairs
+            int count = 0, groups = 0;
+            if (lane < nj) {
+                int c = 0;
+                while (c + 1 < n_ctx && s_cpref[c + 1] <= lane) ++c;
+                count = job_count(ctx_of(c), src, lane - s_cpref[c]);
+                groups = (ctx_of(c).gp.n_features + kFG - 1) / kFG;
+            }
+            const unsigned long long w = static_cast<unsigned long long>(count) * groups;
+            unsigned long long incl = w;
+            unsigned int rows = static_cast<unsigned int>(count);
+            int pairs = groups;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const unsigned long long t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+                pairs += __shfl_xor_sync(0xffffffffu, pairs, o);
+            }
+            const unsigned long long w_all = __shfl_sync(0xffffffffu, incl, 31);
+            if (lane < nj) s_wstart[lane] = incl - w;
+            if (lane == 0) s_wstart[nj] = w_all;
+            if (rows_counter != nullptr && blockIdx.y == 0) {
+                unsigned long long r = rows;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+                if (lane == 0) atomicAdd(rows_counter, r);
+            }
+            if (pairs <= n_cl && w_all > 0) {
+                // one cluster a pair, the others in proportion to the rows (rounded down), then
+                // what is left one by one to the largest share
+                const float spare = static_cast<float>(n_cl - pairs) / static_cast<float>(w_all) * 0.9999f;
+                const int cap = max(1, (count + kMinCtaRows * csize - 1) / (kMinCtaRows * csize));
+                int per = min(1 + static_cast<int>(spare * static_cast<float>(count)), cap);
+                int used = groups * per;
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1) used += __shfl_xor_sync(0xffffffffu, used, o);
+                for (int it = 0; it < 8; ++it) {
+                    const bool can = groups > 0 && per < cap && groups <= n_cl - used;
+                    float share = can ? static_cast<float>(count) / static_cast<float>(per) : -1.f;
+                    int who = lane;
+#pragma unroll
+                    for (int o = 16; o > 0; o >>= 1) {
+                        const float os = __shfl_xor_sync(0xffffffffu, share, o);
+                        const int ow = __shfl_xor_sync(0xffffffffu, who, o);
+                        if (os > share || (os == share && ow < who)) {
+                            share = os;
+                            who = ow;
+                        }
+                    }
+                    if (share < 0.f) break;
+                    if (lane == who) ++per;
+                    used += __shfl_sync(0xffffffffu, groups, who);
+                }
+                float most = groups > 0 ? static_cast<float>(count) / static_cast<float>(per) : 0.f;
+                int cs = groups * per;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    most = fmaxf(most, __shfl_xor_sync(0xffffffffu, most, o));
+                    const int t = __shfl_up_sync(0xffffffffu, cs, o);
+                    if (lane >= o) cs += t;
+                }
+                if (most <= static_cast<float>(w_all) / static_cast<float>(n_cl) + static_cast<float>(kPieceRows * csize)) {
+                    if (lane < nj) {
+                        s_cstart[lane] = cs - groups * per;
+                        s_cper[lane] = per;
+                    }
+                    if (lane == 31) s_cstart[nj] = cs;
+                    if (lane == 0) s_aligned = 1;
+                }
+            }
+        }
     }
     __syncthreads();
     const int n_jobs = s_cpref[n_ctx];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    {
+    if (n_jobs > kWarpJobs) {
         // work of each job (rows x feature groups), exclusive prefix over a contiguous run
         // of jobs per thread
         const int per = (n_jobs + kThreads - 1) / kThreads;
@@ -664,13 +854,12 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int j = j0; j < j1; ++j) {
             int c = 0;
             while (c + 1 < n_ctx && s_cpref[c + 1] <= j) ++c;
-            const WaveCtx& X = ctxs[c];
-            const JobRows jr = job_rows(X, src, src == 0 ? 0 : j - s_cpref[c]);
+            const int count = job_count(ctx_of(c), src, j - s_cpref[c]);
             const unsigned long long w =
-                static_cast<unsigned long long>(jr.count) * ((X.gp.n_features + kFG - 1) / kFG);
+                static_cast<unsigned long long>(count) * ((ctx_of(c).gp.n_features + kFG - 1) / kFG);
             s_wstart[j] = w;
             local += w;
-            lrows += static_cast<unsigned long long>(jr.count);
+            lrows += static_cast<unsigned long long>(count);
         }
         unsigned long long incl = local, rs = lrows;
 #pragma unroll
@@ -698,18 +887,30 @@ __global__ void __launch_bounds__(kThreads, 1)
             s_wstart[n_jobs] = all;
             if (rows_counter != nullptr && blockIdx.y == 0) atomicAdd(rows_counter, rows_all);
         }
+        __syncthreads();
     }
-    __syncthreads();
-    cg::cluster_group cluster = cg::this_cluster();
-    const int csize = static_cast<int>(cluster.dim_blocks().y);  // CTAs per cluster: 1, 2 or 4
-    const int cl = static_cast<int>(blockIdx.y) / csize;
-    const int n_cl = static_cast<int>(gridDim.y) / csize;
-    const unsigned int rank = cluster.block_rank();
-    const unsigned long long w_all = s_wstart[n_jobs];
-    const unsigned long long w_end = w_all * static_cast<unsigned long long>(cl + 1) / static_cast<unsigned long long>(n_cl);
+    unsigned long long w, w_end;
+    if (s_aligned) {
+        if (cl >= s_cstart[n_jobs]) return;  // no pair for this cluster
+        int lo = 0, hi = n_jobs - 1;
+        while (lo < hi) {
+            const int mid = (lo + hi + 1) >> 1;
+            if (s_cstart[mid] <= cl) lo = mid;
+            else hi = mid - 1;
+        }
+        const int q = cl - s_cstart[lo], per = s_cper[lo], fg = q / per, k = q - fg * per;
+        const unsigned int groups = static_cast<unsigned int>((s_cstart[lo + 1] - s_cstart[lo]) / per);
+        const unsigned long long R = (s_wstart[lo + 1] - s_wstart[lo]) / groups;
+        const unsigned long long w0 = s_wstart[lo] + R * fg;
+        w = w0 + R * k / per;
+        w_end = w0 + R * (k + 1) / per;
+    } else {
+        const unsigned long long w_all = s_wstart[n_jobs];
+        w = w_all * static_cast<unsigned long long>(cl) / static_cast<unsigned long long>(n_cl);
+        w_end = w_all * static_cast<unsigned long long>(cl + 1) / static_cast<unsigned long long>(n_cl);
+    }
     const unsigned long long max_piece = static_cast<unsigned long long>(kMaxShareRows) * csize;
-    for (unsigned long long w = w_all * static_cast<unsigned long long>(cl) / static_cast<unsigned long long>(n_cl);
-         w < w_end;) {
+    while (w < w_end) {
         // the job holding w: the last j with s_wstart[j] <= w (a non-empty job)
         int lo = 0, hi = n_jobs - 1;
         while (lo < hi) {
@@ -720,7 +921,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int j = lo;
         int c = 0;
         while (c + 1 < n_ctx && s_cpref[c + 1] <= j) ++c;
-        const WaveCtx& X = ctxs[c];
+        const WaveCtx& X = ctx_of(c);
         const int n_f = X.gp.n_features;
         const JobRows jr = job_rows(X, src, src == 0 ? 0 : j - s_cpref[c]);
         const unsigned long long R = static_cast<unsigned long long>(jr.count);
@@ -732,64 +933,31 @@ __global__ void __launch_bounds__(kThreads, 1)
         const int qrows = (piece1 - piece0 + csize - 1) / csize;
         const int r0 = min(piece1, piece0 + static_cast<int>(rank) * qrows), r1 = min(piece1, r0 + qrows);
         const int fg0 = fg * kFG;
+        if (!T::var && threadIdx.x == 0) {  // the fixed-point hessians of the two row classes, for the flush
+            const double hscale = X.st->hscale;
+            s_hq[0] = static_cast<unsigned long long>(__double2ll_rn(1.0 * hscale));
+            s_hq[1] = static_cast<unsigned long long>(__double2ll_rn(1.0 * X.goss_scale * hscale));
+        }
         if constexpr (T::var)
             accumulate_var<kMode>(P, Gt, Ht, Ct, jr.rows, r0, r1, X.codes, X.gp.stride, fg0, jr.gq, jr.hq);
-        else if (X.codes_map_ok && (reinterpret_cast<uintptr_t>(&X.codes_map) & 63u) == 0)  // TMA wants 64 B
-            phase = accumulate_const_tma<kMode>(P, Gt, Ct, stage, s_bars, phase, jr.rows, r0, r1, &X.codes_map, fg0,
+        else if (X.codes_map_ok && (reinterpret_cast<uintptr_t>(&ctxs[c].codes_map) & 63u) == 0)  // TMA wants 64 B
+            phase = accumulate_const_tma<kMode>(P, Gt, Ct, stage, s_bars, phase, jr.rows, r0, r1, &ctxs[c].codes_map, fg0,
                                                 jr.gq, &X.ctl->error);
         else
             accumulate_const<kMode>(P, Gt, Ct, jr.rows, r0, r1, X.codes, X.gp.stride, fg0, jr.gq);
         __syncthreads();
-        cluster.sync();
-        // rank k adds its share of the cells over the cluster and writes them out
         const bool whole = piece0 == 0 && static_cast<unsigned long long>(piece1) == R;
         const int nf_here = min(kFG, n_f - fg0);
-        const size_t slot_off = static_cast<size_t>(jr.slot) * static_cast<size_t>(n_f) * kBins;
-        const double hscale = X.st->hscale;
-        const unsigned long long hq1 = static_cast<unsigned long long>(__double2ll_rn(1.0 * hscale));
-        const unsigned long long hq2 = static_cast<unsigned long long>(__double2ll_rn(1.0 * X.goss_scale * hscale));
-        const int share = (kTot + csize - 1) / csize;
-        const int i1 = min(kTot, static_cast<int>(rank + 1) * share);
-        for (int ti = static_cast<int>(rank) * share + threadIdx.x; ti < i1; ti += kThreads) {
-            const int f = ti / kTotPitch, b = ti - f * kTotPitch;
-            if (b >= kBins || f >= nf_here) continue;
-            unsigned long long g = 0, hs = 0;
-            unsigned int cn = 0, c1 = 0, c2 = 0;
-            for (int kk = 0; kk < csize; ++kk) {
-                g += cluster.map_shared_rank(Gt, kk)[ti];
-                const unsigned int pc = cluster.map_shared_rank(Ct, kk)[ti];
-                if constexpr (T::var) {
-                    hs += cluster.map_shared_rank(Ht, kk)[ti];
-                    cn += pc;
-                } else {
-                    c1 += pc & 0xffffu;
-                    c2 += pc >> 16;
-                }
-            }
-            if constexpr (!T::var) {
-                hs = static_cast<unsigned long long>(c1) * hq1 + static_cast<unsigned long long>(c2) * hq2;
-                cn = c1 + c2;
-            }
-            if (cn == 0u) continue;
-            const size_t o = slot_off + static_cast<size_t>(fg0 + f) * kBins + b;
-            if (whole) {
-                reinterpret_cast<unsigned long long*>(X.G)[o] = g;
-                reinterpret_cast<unsigned long long*>(X.H)[o] = hs;
-                X.C[o] = static_cast<int>(cn);
-            } else {
-                atomicAdd(reinterpret_cast<unsigned long long*>(X.G) + o, g);
-                atomicAdd(reinterpret_cast<unsigned long long*>(X.H) + o, hs);
-                atomicAdd(X.C + o, static_cast<int>(cn));
-            }
-        }
-        cluster.sync();  // no CTA clears its totals while others read them
-        {
-            uint4* z = reinterpret_cast<uint4*>(smem_raw + Lay::tot_off);
-            for (int k = threadIdx.x; k < static_cast<int>(Lay::tot_bytes / 16); k += kThreads)
-                z[k] = make_uint4(0, 0, 0, 0);
-        }
-        __syncthreads();
+        const size_t out0 = (static_cast<size_t>(jr.slot) * static_cast<size_t>(n_f) + fg0) * kBins;
+        if (csize == 1) flush_piece<T::var, 1>(X, Gt, Ht, Ct, rank, nf_here, out0, whole, s_hq[0], s_hq[1]);
+        else if (csize == 2) flush_piece<T::var, 2>(X, Gt, Ht, Ct, rank, nf_here, out0, whole, s_hq[0], s_hq[1]);
+        else flush_piece<T::var, 4>(X, Gt, Ht, Ct, rank, nf_here, out0, whole, s_hq[0], s_hq[1]);
         w += len;
+        if (T::var && w < w_end) {  // the totals lie over the planes: clear for the next piece
+            uint4* z = reinterpret_cast<uint4*>(smem_raw);
+            for (int k = threadIdx.x; k < static_cast<int>(Lay::region / 16); k += kThreads) z[k] = make_uint4(0, 0, 0, 0);
+            __syncthreads();
+        }
     }
 }
 
@@ -973,10 +1141,17 @@ __global__ void __launch_bounds__(kPartThreads)
             if (l0 + r0 + (end - base) == count) {
                 DevNode& A = X.spec[2 * L];
                 DevNode& B = X.spec[2 * L + 1];
-                A.start = N.start;
-                A.count = l0 + run;
-                B.start = N.start + l0 + run;
-                B.count = count - l0 - run;
+                const int nl = l0 + run, nr = count - nl, slot = A.slot, start = N.start;
+                A.start = start;
+                A.count = nl;
+                B.start = start + nl;
+                B.count = nr;
+                const bool ls = nl <= nr;  // the left child is the smaller one (cpp/src/tree.cpp:423)
+                ctl->job[tr.e] = WaveJob{ls ? start : start + nl, ls ? nl : nr, 1 - N.buf, ls ? slot : slot + 1};
+                const bool deep = N.depth + 1 < X.gp.max_depth;
+                const int need = 2 * X.gp.min_samples_leaf;
+                ctl->child[2 * tr.e] = WaveChild{2 * L, slot, N.slot, slot + 1, !ls, deep && nl >= need, {0, 0}};
+                ctl->child[2 * tr.e + 1] = WaveChild{2 * L + 1, slot + 1, N.slot, slot, ls, deep && nr >= need, {0, 0}};
             }
         }
         __syncthreads();

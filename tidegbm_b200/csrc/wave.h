@@ -62,6 +62,19 @@ inline int hist_mode(int hist_bits, bool const_h) {
 // an 8-byte h payload).
 inline int hist_pay_bytes(int mode) { return mode <= kHistExactVar ? 8 : mode <= kHistQ16Var ? 4 : 2; }
 
+// What the histogram and the scan read of a planned expansion, written whole by the
+// partition tile that completes the leaf: one load instead of a chain through the node
+// table.  WaveJob: the smaller child's rows (cpp/src/tree.cpp:423) and slot.  WaveChild:
+// candidate index, slot, and the parent and small-sibling slots the larger child's
+// histogram is derived from.
+struct alignas(16) WaveJob {
+    int start, count, buf, slot;
+};
+struct alignas(16) WaveChild {
+    int ci, slot, pslot, sslot;
+    int derive, eligible, pad[2];
+};
+
 // Per-tree control of one context, device resident.
 struct WaveCtl {
     int splits_done;  // splits committed so far
@@ -80,6 +93,8 @@ struct WaveCtl {
     // rows of the planned leaf placed so far by its partition tiles: left in the low word,
     // right in the high word (zeroed by the select that plans the expansion)
     unsigned long long part_cur[kMaxLeavesCap];
+    WaveJob job[kMaxLeavesCap];            // per planned expansion
+    WaveChild child[2 * kMaxLeavesCap];    // per planned expansion and side
     int expanded[kMaxNodes];  // 0 not expanded; 1, 2: children planned by the axis, with-pairs split
 };
 
@@ -146,6 +161,19 @@ struct WaveCtx {
     int* pair_tickets;           // [2 * kMaxNodes + 1], zero between launches
 };
 constexpr int kMaxPairs = 15;  // pairs of the top pair_top_k <= 6 features
+
+#if defined(__CUDACC__)
+// Copies the first context into shared memory (the caller synchronises the CTA).  The
+// contexts are written before the fit's first tree and do not change, so a wave kernel does
+// this before pdl_wait: its later reads of pointers and parameters then cost no memory
+// round trip of their own.
+__device__ __forceinline__ void stage_ctx(WaveCtx& to, const WaveCtx* ctxs) {
+    static_assert(sizeof(WaveCtx) % 16 == 0, "copied in 16-byte words");
+    const uint4* src = reinterpret_cast<const uint4*>(ctxs);
+    uint4* dst = reinterpret_cast<uint4*>(&to);
+    for (int k = threadIdx.x; k < static_cast<int>(sizeof(WaveCtx) / 16); k += blockDim.x) dst[k] = __ldg(src + k);
+}
+#endif
 
 // Per-tree set-up of one context: root node (all sampled rows, slot 0), control reset.
 // use_dev_count: the sample size is st->n_sample (GOSS), else n_sample_host.
