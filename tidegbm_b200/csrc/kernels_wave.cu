@@ -978,67 +978,24 @@ __device__ __forceinline__ void store_payload(const WaveCtx& X, long long i, lon
     else static_cast<short*>(X.gq)[i] = static_cast<short>(v);
 }
 
-// Global tile t -> (context, expansion, tile within the expansion).
-struct TileRef {
-    int c, e, k, lt;
-};
-
-__device__ __forceinline__ TileRef find_tile(const WaveCtx* ctxs, const int* s_pref, int n_ctx, int t) {
-    TileRef r;
-    int c = 0;
-    while (c + 1 < n_ctx && s_pref[c + 1] <= t) ++c;
-    const int lt = t - s_pref[c];
-    const WaveCtl* ctl = ctxs[c].ctl;
-    int lo = 0, hi = ctl->n_exp - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (ctl->exp_tile0[mid] <= lt) lo = mid;
-        else hi = mid - 1;
-    }
-    r.c = c;
-    r.e = lo;
-    r.k = lt - ctl->exp_tile0[lo];
-    r.lt = lt;
-    return r;
-}
-
-__device__ __forceinline__ void load_tile(const WaveCtx& X, const int32_t* in, const DevSplit& S, int base, int end,
+__device__ __forceinline__ void load_tile(const WaveCtx& X, const int32_t* in, const WaveExp& S, int base, int end,
                                           int32_t (&row)[kPartPer], bool (&left)[kPartPer]) {
-    const int feature = S.feature, threshold = S.threshold, ml = S.missing_left, type = S.type;
-    unsigned long long cat[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) cat[k] = S.cat[k];
 #pragma unroll
     for (int i = 0; i < kPartPer; ++i) {
         const int k = base + i * kPartThreads + threadIdx.x;
         row[i] = k < end ? in[k] : -1;
     }
     unsigned int b[kPartPer], b2[kPartPer];
-    const uint8_t* col = X.codes_col + static_cast<size_t>(feature) * X.col_pitch;
-    const uint8_t* col2 = type == 1 ? X.codes_col + static_cast<size_t>(S.feature2) * X.col_pitch : col;
+    const uint8_t* col = X.codes_col + static_cast<size_t>(S.feature) * X.col_pitch;
+    const uint8_t* col2 = S.type == 1 ? X.codes_col + static_cast<size_t>(S.feature2) * X.col_pitch : col;
 #pragma unroll
     for (int i = 0; i < kPartPer; ++i) {
         b[i] = row[i] >= 0 ? col[row[i]] : 0u;
-        b2[i] = row[i] >= 0 && type == 1 ? col2[row[i]] : 0u;
+        b2[i] = row[i] >= 0 && S.type == 1 ? col2[row[i]] : 0u;
     }
 #pragma unroll
     for (int i = 0; i < kPartPer; ++i)
-        left[i] = row[i] >= 0 && goes_left(type, cat, threshold, ml, b[i], b2[i], X.gp.n_bins);
-}
-
-__device__ __forceinline__ void load_tile_prefix(const WaveCtx* ctxs, int n_ctx, int* s_pref) {
-    if (static_cast<int>(threadIdx.x) < n_ctx) s_pref[threadIdx.x] = ctxs[threadIdx.x].ctl->tiles_total;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int c = 0; c < n_ctx; ++c) {
-            const int v = s_pref[c];
-            s_pref[c] = acc;
-            acc += v;
-        }
-        s_pref[n_ctx] = acc;
-    }
-    __syncthreads();
+        left[i] = row[i] >= 0 && goes_left(S.type, S.cat, S.threshold, S.missing_left, b[i], b2[i], X.gp.n_bins);
 }
 
 // One launch moves the rows of every planned leaf into its children.  A tile of 2048 rows
@@ -1056,20 +1013,40 @@ __device__ __forceinline__ void load_tile_prefix(const WaveCtx* ctxs, int n_ctx,
 // rows and codes again.
 __global__ void __launch_bounds__(kPartThreads)
     wave_part_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx) {
-    pdl_wait();
-    pdl_trigger();
+    __shared__ WaveCtx s_ctx;  // the first context's constants
     __shared__ int s_pref[kMaxWaveCtx + 1];
     __shared__ int wc[kPartPer * kPartWarps];
     __shared__ unsigned long long s_old;
-    load_tile_prefix(ctxs, n_ctx, s_pref);
-    const int total = s_pref[n_ctx];
+    stage_ctx(s_ctx, ctxs);
+    __syncthreads();
+    pdl_wait();
+    pdl_trigger();
+    auto ctx_of = [&](int c) -> const WaveCtx& { return c == 0 ? s_ctx : ctxs[c]; };
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
+    if (warp == 0) {
+        int all = 0;
+        for (int c0 = 0; c0 < n_ctx; c0 += 32) {
+            const int c = c0 + lane;
+            const int v = c < n_ctx ? ctx_of(c).ctl->tiles_total : 0;
+            int incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (c < n_ctx) s_pref[c] = all + incl - v;
+            all += __shfl_sync(0xffffffffu, incl, 31);
+        }
+        if (lane == 0) s_pref[n_ctx] = all;
+    }
+    __syncthreads();
+    const int total = s_pref[n_ctx];
     // Clear the histogram slots of this wave's children (2 per expansion, consecutive): the
     // smaller child's is accumulated into by the histogram launch.  First, so that the stores
     // drain while the tiles wait for their loads.
     for (int c = 0; c < n_ctx; ++c) {
-        const WaveCtx& X = ctxs[c];
+        const WaveCtx& X = ctx_of(c);
         const int ns = 2 * X.ctl->n_exp;
         if (ns == 0) continue;
         const size_t elems = static_cast<size_t>(X.gp.n_features) * kBins;
@@ -1087,23 +1064,30 @@ __global__ void __launch_bounds__(kPartThreads)
         }
     }
     for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        const TileRef tr = find_tile(ctxs, s_pref, n_ctx, t);
-        const WaveCtx& X = ctxs[tr.c];
+        int c = 0;
+        while (c + 1 < n_ctx && s_pref[c + 1] <= t) ++c;
+        const WaveCtx& X = ctx_of(c);
         WaveCtl* ctl = X.ctl;
-        const int L = ctl->exp_leaf[tr.e];
-        const DevNode& N = X.nodes[L];
-        const DevSplit& S = ctl->expanded[L] == 2 ? X.splits_pair[L] : X.splits[L];
-        const int32_t* in = (N.buf ? X.rows1 : X.rows0) + N.start;
-        int32_t* out = (N.buf ? X.rows0 : X.rows1) + N.start;
-        const int count = N.count;
-        const int base = tr.k * kPartTile, end = min(base + kPartTile, count);
+        // the expansion of tile t: the last one that starts at or before it (every warp counts
+        // the starts, 32 at a time)
+        const int lt = t - s_pref[c], n_exp = ctl->n_exp;
+        int e = -1;
+        for (int e0 = 0; e0 < n_exp; e0 += 32) {
+            const int first = ctl->exp_tile0[e0 + lane];  // the array is longer than its use
+            e += __popc(__ballot_sync(0xffffffffu, e0 + lane < n_exp && first <= lt));
+        }
+        const WaveExp S = ctl->exp[e];
+        const int L = S.leaf, count = S.count;
+        const int32_t* in = (S.buf ? X.rows1 : X.rows0) + S.start;
+        int32_t* out = (S.buf ? X.rows0 : X.rows1) + S.start;
+        const int base = (lt - ctl->exp_tile0[e]) * kPartTile, end = min(base + kPartTile, count);
         int32_t row[kPartPer];
         bool left[kPartPer];
         load_tile(X, in, S, base, end, row, left);
         // the rows' payloads move with them (same positions in the other buffer); loaded
         // here so that their latency overlaps the ranks below
-        const long long from0 = static_cast<long long>(N.buf) * X.pay_pitch + N.start;
-        const long long to0 = static_cast<long long>(1 - N.buf) * X.pay_pitch + N.start;
+        const long long from0 = static_cast<long long>(S.buf) * X.pay_pitch + S.start;
+        const long long to0 = static_cast<long long>(1 - S.buf) * X.pay_pitch + S.start;
         long long pg[kPartPer], ph[kPartPer];
 #pragma unroll
         for (int i = 0; i < kPartPer; ++i) {
@@ -1134,24 +1118,24 @@ __global__ void __launch_bounds__(kPartThreads)
         const int n_right = end - base - run;  // run: the tile's left rows
         if (threadIdx.x == 0) {
             const unsigned long long old =
-                atomicAdd(&ctl->part_cur[tr.e],
+                atomicAdd(&ctl->part_cur[e],
                           (static_cast<unsigned long long>(n_right) << 32) | static_cast<unsigned int>(run));
             s_old = old;
             const int l0 = static_cast<int>(old & 0xffffffffu), r0 = static_cast<int>(old >> 32);
             if (l0 + r0 + (end - base) == count) {
                 DevNode& A = X.spec[2 * L];
                 DevNode& B = X.spec[2 * L + 1];
-                const int nl = l0 + run, nr = count - nl, slot = A.slot, start = N.start;
-                A.start = start;
+                const int nl = l0 + run, nr = count - nl, slot = S.child_slot;
+                A.start = S.start;
                 A.count = nl;
-                B.start = start + nl;
+                B.start = S.start + nl;
                 B.count = nr;
                 const bool ls = nl <= nr;  // the left child is the smaller one (cpp/src/tree.cpp:423)
-                ctl->job[tr.e] = WaveJob{ls ? start : start + nl, ls ? nl : nr, 1 - N.buf, ls ? slot : slot + 1};
-                const bool deep = N.depth + 1 < X.gp.max_depth;
+                ctl->job[e] = WaveJob{ls ? S.start : S.start + nl, ls ? nl : nr, 1 - S.buf, ls ? slot : slot + 1};
+                const bool deep = S.depth + 1 < X.gp.max_depth;
                 const int need = 2 * X.gp.min_samples_leaf;
-                ctl->child[2 * tr.e] = WaveChild{2 * L, slot, N.slot, slot + 1, !ls, deep && nl >= need, {0, 0}};
-                ctl->child[2 * tr.e + 1] = WaveChild{2 * L + 1, slot + 1, N.slot, slot, ls, deep && nr >= need, {0, 0}};
+                ctl->child[2 * e] = WaveChild{2 * L, slot, S.slot, slot + 1, !ls, deep && nl >= need, {0, 0}};
+                ctl->child[2 * e + 1] = WaveChild{2 * L + 1, slot + 1, S.slot, slot, ls, deep && nr >= need, {0, 0}};
             }
         }
         __syncthreads();

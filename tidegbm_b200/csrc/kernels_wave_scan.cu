@@ -41,39 +41,18 @@ __device__ __forceinline__ void children_prefix(const WaveCtx* ctxs, int n_ctx, 
     __syncthreads();
 }
 
-// The histogram job of one child: its node and split outputs, its candidate index, its
-// slot, and (the larger child) the parent and small-sibling slots it is derived from.
-struct ScanTarget {
-    DevNode* N;
-    DevSplit* out;
-    int ci, slot, pslot, sslot;
-    bool derive;
-};
-
-__device__ __forceinline__ ScanTarget scan_target(const WaveCtx& X, int src, int k) {
-    ScanTarget t;
-    t.pslot = t.sslot = 0;
-    t.derive = false;
-    if (src == 0) {
-        t.N = X.nodes;
-        t.out = X.splits;
-        t.ci = kRootCand;
-        t.slot = 0;
-        return t;
-    }
-    const int L = X.ctl->exp_leaf[k >> 1];
-    const int side = k & 1;
-    t.ci = 2 * L + side;
-    t.N = X.spec + t.ci;
-    t.out = X.spec_split + t.ci;
-    t.slot = t.N->slot;
-    const DevNode& A = X.spec[2 * L];
-    const DevNode& B = X.spec[2 * L + 1];
-    const int small = A.count <= B.count ? 0 : 1;  // cpp/src/tree.cpp:423
-    t.derive = side != small;
-    t.pslot = X.nodes[L].slot;
-    t.sslot = X.spec[2 * L + small].slot;
-    return t;
+// The histogram job of one child (child k of the context's wave, or the root): its
+// candidate index, its slot, and (the larger child) the parent and small-sibling slots it is
+// derived from.
+__device__ __forceinline__ WaveChild scan_child(const WaveCtx& X, int src, int k) {
+    if (src != 0) return X.ctl->child[k];
+    return WaveChild{kRootCand, 0, 0, 0, 0, 0 < X.gp.max_depth && X.st->n_sample >= 2 * X.gp.min_samples_leaf, {0, 0}};
+}
+__device__ __forceinline__ DevNode* child_node(const WaveCtx& X, int src, int ci) {
+    return src == 0 ? X.nodes : X.spec + ci;
+}
+__device__ __forceinline__ DevSplit* child_split(const WaveCtx& X, int src, int ci) {
+    return src == 0 ? X.splits : X.spec_split + ci;
 }
 
 // The last feature job of a child (one warp): the best candidate over its features
@@ -124,49 +103,63 @@ __device__ __forceinline__ void set_totals(DevNode* N, long long Gt, long long H
 // scan_feature_warp (the larger child first derived as parent - smaller), the per-feature
 // bests kept as candidates, and the child's last job picks its split.  Categorical
 // features are left to wave_scan_cat_kernel; the children's tickets count both.
-constexpr int kScanWarpThreads = 256;
+constexpr int kScanWarpThreads = 128;
+constexpr int kScanWarpCtas = 4;  // per SM
 
-__global__ void __launch_bounds__(kScanWarpThreads, 2)
+__global__ void __launch_bounds__(kScanWarpThreads, kScanWarpCtas)
     wave_scan_warp_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx, int src) {
+    __shared__ WaveCtx s_ctx;  // the first context's constants
+    __shared__ int s_jpref[kMaxWaveCtx + 1];
+    stage_ctx(s_ctx, ctxs);
+    __syncthreads();
     pdl_wait();
     pdl_trigger();
-    __shared__ int s_pref[kMaxWaveCtx + 1];
-    __shared__ int s_jpref[kMaxWaveCtx + 1];
-    children_prefix(ctxs, n_ctx, src, s_pref);
-    if (threadIdx.x == 0) {
-        int acc = 0;
-        for (int c = 0; c < n_ctx; ++c) {
-            s_jpref[c] = acc;
-            acc += (s_pref[c + 1] - s_pref[c]) * ctxs[c].gp.n_features;
+    auto ctx_of = [&](int c) -> const WaveCtx& { return c == 0 ? s_ctx : ctxs[c]; };
+    const int lane = threadIdx.x & 31;
+    if (threadIdx.x < 32) {
+        int all = 0;
+        for (int c0 = 0; c0 < n_ctx; c0 += 32) {
+            const int c = c0 + lane;
+            int v = 0;
+            if (c < n_ctx) {
+                const WaveCtl* ctl = ctx_of(c).ctl;
+                v = (src == 0 ? (ctl->active ? 1 : 0) : 2 * ctl->n_exp) * ctx_of(c).gp.n_features;
+            }
+            int incl = v;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int t = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += t;
+            }
+            if (c < n_ctx) s_jpref[c] = all + incl - v;
+            all += __shfl_sync(0xffffffffu, incl, 31);
         }
-        s_jpref[n_ctx] = acc;
+        if (lane == 0) s_jpref[n_ctx] = all;
     }
     __syncthreads();
-    const int lane = threadIdx.x & 31;
     const int wpb = kScanWarpThreads / 32;
     const int total = s_jpref[n_ctx];
     for (int jw = blockIdx.x * wpb + (threadIdx.x >> 5); jw < total; jw += gridDim.x * wpb) {
         int c = 0;
         while (c + 1 < n_ctx && s_jpref[c + 1] <= jw) ++c;
-        const WaveCtx& X = ctxs[c];
+        const WaveCtx& X = ctx_of(c);
         const GrowParams& p = X.gp;
         const int rem = jw - s_jpref[c];
         const int k = rem / p.n_features, f = rem - k * p.n_features;
         if (X.is_cat != nullptr && X.is_cat[f]) continue;
-        const ScanTarget t = scan_target(X, src, k);
+        const WaveChild t = scan_child(X, src, k);
         const size_t e = static_cast<size_t>(p.n_features) * kBins;
-        const bool eligible = t.N->depth < p.max_depth && t.N->count >= 2 * p.min_samples_leaf;
         const double inv_gs = X.st->inv_gscale, inv_hs = X.st->inv_hscale;
         Cand best{-1e300, 0x7fffffff};
-        if (eligible || f == 0) {
+        if (t.eligible || f == 0) {
             const size_t fo = static_cast<size_t>(f) * kBins;
             const size_t so = static_cast<size_t>(t.slot) * e + fo, po = static_cast<size_t>(t.pslot) * e + fo,
                          qo = static_cast<size_t>(t.sslot) * e + fo;
             long long Gt, Ht, Ct;
             best = scan_feature_warp(X.G + so, X.H + so, X.C + so, X.G + po, X.H + po, X.C + po, X.G + qo, X.H + qo,
-                                     X.C + qo, t.derive, eligible, f, p.n_bins, inv_gs, inv_hs, p.l2, p.min_split_gain,
+                                     X.C + qo, t.derive, t.eligible, f, p.n_bins, inv_gs, inv_hs, p.l2, p.min_split_gain,
                                      p.min_samples_leaf, p.min_child_weight, Gt, Ht, Ct);
-            if (f == 0 && lane == 0) set_totals(t.N, Gt, Ht, Ct, inv_gs, inv_hs, p.l2);
+            if (f == 0 && lane == 0) set_totals(child_node(X, src, t.ci), Gt, Ht, Ct, inv_gs, inv_hs, p.l2);
         }
         int last = 0;
         if (lane == 0) {
@@ -177,7 +170,7 @@ __global__ void __launch_bounds__(kScanWarpThreads, 2)
             last = atomicAdd(&X.tickets[t.ci], 1) == p.n_features - 1;
         }
         last = __shfl_sync(0xffffffffu, last, 0);
-        if (last) finish_child(X, t.ci, t.out, lane);
+        if (last) finish_child(X, t.ci, child_split(X, src, t.ci), lane);
     }
 }
 
@@ -200,9 +193,9 @@ __global__ void __launch_bounds__(kScanThreads)
         const WaveCtx& X = ctxs[c];
         const GrowParams& p = X.gp;
         if (f >= p.n_features || X.is_cat == nullptr || !X.is_cat[f]) continue;  // uniform over the CTA
-        const ScanTarget t = scan_target(X, src, j - s_pref[c]);
+        const WaveChild t = scan_child(X, src, j - s_pref[c]);
         const size_t e = static_cast<size_t>(p.n_features) * kBins;
-        const bool eligible = t.N->depth < p.max_depth && t.N->count >= 2 * p.min_samples_leaf;
+        const bool eligible = t.eligible != 0;
         const double inv_gs = X.st->inv_gscale, inv_hs = X.st->inv_hscale;
         Cand best{-1e300, 0x7fffffff};
         if (eligible || f == 0) {
@@ -220,7 +213,7 @@ __global__ void __launch_bounds__(kScanThreads)
                                         p.min_samples_leaf, p.min_child_weight, X.cat_smooth, Gt, Ht, Ct, csm,
                                         X.cand_cat + (static_cast<size_t>(t.ci) * p.n_features + f) * 4);
             }
-            if (f == 0 && threadIdx.x == 0) set_totals(t.N, Gt, Ht, Ct, inv_gs, inv_hs, p.l2);
+            if (f == 0 && threadIdx.x == 0) set_totals(child_node(X, src, t.ci), Gt, Ht, Ct, inv_gs, inv_hs, p.l2);
         }
         if (threadIdx.x == 0) {
             const size_t cs = static_cast<size_t>(t.ci) * p.n_features + f;
@@ -230,7 +223,8 @@ __global__ void __launch_bounds__(kScanThreads)
             last = atomicAdd(&X.tickets[t.ci], 1) == p.n_features - 1;
         }
         __syncthreads();
-        if (last && threadIdx.x < 32) finish_child(X, t.ci, t.out, static_cast<int>(threadIdx.x));
+        if (last && threadIdx.x < 32)
+            finish_child(X, t.ci, child_split(X, src, t.ci), static_cast<int>(threadIdx.x));
         __syncthreads();  // shared state reuse
     }
 }
@@ -238,8 +232,9 @@ __global__ void __launch_bounds__(kScanThreads)
 // A leaf the reference's selection may pick: depth and size limits, a valid split of gain
 // above min_split_gain (tree.cpp:343-383; the strict '>' against min_split_gain).
 __device__ __forceinline__ bool candidate(const GrowParams& p, const DevNode& N, const DevSplit& S) {
-    return N.is_leaf && N.depth < p.max_depth && N.count >= 2 * p.min_samples_leaf && S.valid &&
-           S.gain > p.min_split_gain;
+    // no short circuit: the loads go out together
+    return (N.is_leaf != 0) & (N.depth < p.max_depth) & (N.count >= 2 * p.min_samples_leaf) & (S.valid != 0) &
+           (S.gain > p.min_split_gain);
 }
 
 // better leaf: larger gain, lower id on ties
@@ -247,14 +242,22 @@ __device__ __forceinline__ bool better_leaf(double ga, int ia, double gb, int ib
     return ga > gb || (ga == gb && ia < ib);
 }
 
+// A gain as an unsigned integer of the same order (both zeros alike); never 0 for a number.
+__device__ __forceinline__ unsigned long long ordered(double g) {
+    const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(g + 0.0));
+    return (b >> 63) ? ~b : b | 0x8000000000000000ull;
+}
+
 constexpr int kSelectThreads = 256;  // all stage the selection state; warp 0 then selects
 
 __global__ void __launch_bounds__(kSelectThreads)
     wave_select_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx, int* gsync, unsigned* host_flag,
                        cudaGraphConditionalHandle cond, int use_cond) {
+    __shared__ WaveCtx X;  // this context's constants
+    stage_ctx(X, ctxs + blockIdx.x);
+    __syncthreads();
     pdl_wait();
     pdl_trigger();
-    const WaveCtx& X = ctxs[blockIdx.x];
     const GrowParams& p = X.gp;
     WaveCtl* ctl = X.ctl;
     DevTreeState* st = X.st;
@@ -284,26 +287,29 @@ __global__ void __launch_bounds__(kSelectThreads)
         // the split a leaf takes: with the PAIR candidates while the tree's pair budget lasts
         // (tree.cpp:214-218, re-scored after every pair split, tree.cpp:393-396)
         auto pairs_on = [&]() { return X.pair_on && pair_used < X.max_pair; };
+        // every load of a node before the first use, whether or not it is expanded
         auto stage_all = [&](int t, int step) {
             const bool pr = pairs_on();
             for (int k = t; k < nn; k += step) {
-                const DevSplit S = pr ? X.splits_pair[k] : splits[k];
-                s_nc[k] = candidate(p, nodes[k], S) ? 1 : 0;
-                s_ng[k] = S.gain;
-                s_ty[k] = static_cast<unsigned char>(S.type);
-                s_pty[k] = X.pair_on ? static_cast<unsigned char>(X.splits_pair[k].type) : 0;
-                const int ex = ctl->expanded[k];
+                const DevSplit* Sp = (pr ? X.splits_pair : splits) + k;
+                const DevSplit* Cp = (pr ? X.spec_split_pair : X.spec_split) + 2 * k;
+                const DevNode &N = nodes[k], &A = X.spec[2 * k], &B = X.spec[2 * k + 1];
+                const double g = Sp->gain, g0 = Cp[0].gain, g1 = Cp[1].gain;
+                const int ty = Sp->type, ty0 = Cp[0].type, ty1 = Cp[1].type, ex = ctl->expanded[k];
+                const bool c = candidate(p, N, *Sp), c0 = candidate(p, A, Cp[0]), c1 = candidate(p, B, Cp[1]);
+                s_nc[k] = c ? 1 : 0;
+                s_ng[k] = g;
+                s_ty[k] = static_cast<unsigned char>(ty);
                 s_ex[k] = static_cast<unsigned char>(ex);
-                if (ex) {
-                    for (int sd = 0; sd < 2; ++sd) {
-                        const int ci = 2 * k + sd;
-                        const DevSplit C = pr ? X.spec_split_pair[ci] : X.spec_split[ci];
-                        s_cc[ci] = candidate(p, X.spec[ci], C) ? 1 : 0;
-                        s_cg[ci] = C.gain;
-                        s_cty[ci] = static_cast<unsigned char>(C.type);
-                        s_cpty[ci] = X.pair_on ? static_cast<unsigned char>(X.spec_split_pair[ci].type) : 0;
-                    }
-                }
+                s_cc[2 * k] = c0 ? 1 : 0;
+                s_cc[2 * k + 1] = c1 ? 1 : 0;
+                s_cg[2 * k] = g0;
+                s_cg[2 * k + 1] = g1;
+                s_cty[2 * k] = static_cast<unsigned char>(ty0);
+                s_cty[2 * k + 1] = static_cast<unsigned char>(ty1);
+                s_pty[k] = X.pair_on ? static_cast<unsigned char>(X.splits_pair[k].type) : 0;
+                s_cpty[2 * k] = X.pair_on ? static_cast<unsigned char>(X.spec_split_pair[2 * k].type) : 0;
+                s_cpty[2 * k + 1] = X.pair_on ? static_cast<unsigned char>(X.spec_split_pair[2 * k + 1].type) : 0;
             }
         };
         // the node-table writes of the pending commits (children ids nn_first + 2i, + 1 for
@@ -350,24 +356,24 @@ __global__ void __launch_bounds__(kSelectThreads)
                 finished = true;
                 break;
             }
-            double bg = 0.0;
+            // the best candidate: the largest ordered gain (two 32-bit warp maxima), lowest id
+            unsigned long long bk = 0ull;
             int bi = 0x7fffffff;
             for (int k = lane; k < nn; k += 32) {
                 if (!s_nc[k]) continue;
-                if (bi == 0x7fffffff || better_leaf(s_ng[k], k, bg, bi)) {
-                    bg = s_ng[k];
+                const unsigned long long key = ordered(s_ng[k]);
+                if (bi == 0x7fffffff || key > bk) {
+                    bk = key;
                     bi = k;
                 }
             }
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) {
-                const double og = __shfl_xor_sync(0xffffffffu, bg, o);
-                const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-                if (oi != 0x7fffffff && (bi == 0x7fffffff || better_leaf(og, oi, bg, bi))) {
-                    bg = og;
-                    bi = oi;
-                }
-            }
+            const bool has = bi != 0x7fffffff;
+            const unsigned hi = has ? static_cast<unsigned>(bk >> 32) : 0u;
+            const unsigned top = __reduce_max_sync(0xffffffffu, hi);
+            const unsigned lo = has && hi == top ? static_cast<unsigned>(bk) : 0u;
+            const unsigned topl = __reduce_max_sync(0xffffffffu, lo);
+            bi = static_cast<int>(
+                __reduce_min_sync(0xffffffffu, has && hi == top && lo == topl ? static_cast<unsigned>(bi) : 0x7fffffffu));
             if (bi == 0x7fffffff) {
                 finished = true;
                 break;
@@ -448,7 +454,7 @@ __global__ void __launch_bounds__(kSelectThreads)
                     int rank = 0;
                     for (int q = 0; q < nc; ++q)
                         if (q != i && better_leaf(s_gain[q], s_id[q], s_gain[i], s_id[i])) ++rank;
-                    take = rank < B && (X.max_expand <= 0 || rank < X.max_expand) && !ctl->expanded[s_id[i]];
+                    take = rank < B && (X.max_expand <= 0 || rank < X.max_expand) && !s_ex[s_id[i]];
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, take);
                 int tiles = 0;
@@ -456,11 +462,16 @@ __global__ void __launch_bounds__(kSelectThreads)
                 if (take) {
                     const int L = s_id[i];
                     const DevNode& N = nodes[L];
+                    // 2: the children are partitioned by L's with-pairs split, 1: by its axis split
+                    const bool pr = X.pair_on && pair_used < X.max_pair;
+                    const DevSplit S = pr ? X.splits_pair[L] : splits[L];
                     tiles = (N.count + kPartTile - 1) / kPartTile;
                     ctl->exp_leaf[e] = L;
                     ctl->part_cur[e] = 0ull;
-                    // 2: the children are partitioned by L's with-pairs split, 1: by its axis split
-                    ctl->expanded[L] = (X.pair_on && pair_used < X.max_pair) ? 2 : 1;
+                    ctl->expanded[L] = pr ? 2 : 1;
+                    ctl->exp[e] = WaveExp{L, N.start, N.count, N.buf, S.feature, S.threshold, S.missing_left, S.type,
+                                          S.feature2, N.depth, N.slot, slot_first + 2 * e,
+                                          {S.cat[0], S.cat[1], S.cat[2], S.cat[3]}};
                     for (int sd = 0; sd < 2; ++sd) {
                         DevNode ch{};
                         ch.start = N.start;
@@ -515,13 +526,19 @@ __global__ void __launch_bounds__(kSelectThreads)
     }
     // launch-loop condition: any context still growing (the last context to finish sets it)
     if (threadIdx.x == 0) {
-        if (active) atomicOr(&gsync[0], 1);
-        __threadfence();
-        const int t = atomicAdd(&gsync[1], 1);
-        if (t == n_ctx - 1) {
+        unsigned v = active ? 1u : 0u;
+        bool last = true;
+        if (n_ctx > 1) {
+            if (active) atomicOr(&gsync[0], 1);
             __threadfence();
-            const unsigned v = static_cast<unsigned>(atomicExch(&gsync[0], 0));
-            gsync[1] = 0;
+            last = atomicAdd(&gsync[1], 1) == n_ctx - 1;
+            if (last) {
+                __threadfence();
+                v = static_cast<unsigned>(atomicExch(&gsync[0], 0));
+                gsync[1] = 0;
+            }
+        }
+        if (last) {
             gsync[2] += 1;  // selects run (for the count of launched kernels)
             if (host_flag != nullptr) {
                 *reinterpret_cast<volatile unsigned*>(host_flag) = v;
@@ -531,7 +548,6 @@ __global__ void __launch_bounds__(kSelectThreads)
         }
     }
 }
-
 
 // ---- PAIR stage (tree.cpp:214-281) --------------------------------------------------------
 //
@@ -747,7 +763,7 @@ void launch_wave_pair(const WaveCtx* ctxs, int n_ctx, int src, cudaStream_t s) {
 }
 
 void launch_wave_scan(const WaveCtx* ctxs, int n_ctx, int src, int max_f, int ys, bool any_cat, cudaStream_t s) {
-    launch_pdl(wave_scan_warp_kernel, dim3(148 * 2), dim3(kScanWarpThreads), 0, s, "wave_scan launch", ctxs, n_ctx,
+    launch_pdl(wave_scan_warp_kernel, dim3(148 * kScanWarpCtas), dim3(kScanWarpThreads), 0, s, "wave_scan launch", ctxs, n_ctx,
                src);
     if (any_cat)
         launch_pdl(wave_scan_cat_kernel, dim3(max_f, ys), dim3(kScanThreads), 0, s, "wave_scan_cat launch", ctxs, n_ctx,

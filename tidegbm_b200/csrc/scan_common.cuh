@@ -221,6 +221,7 @@ __device__ __forceinline__ Cand scan_feature_warp(long long* __restrict__ Gf, lo
             const long long GL = rg - G0, HL = rh - H0, CL = rc - C0;  // bins 1..b
 #pragma unroll
             for (int ml = 0; ml <= 1; ++ml) {
+                if (ml && C0 == 0) continue;  // no missing rows: the same sums as ml = 0, which wins the tie
                 const long long gL = GL + (ml ? G0 : 0), hL = HL + (ml ? H0 : 0), cL = CL + (ml ? C0 : 0);
                 const long long cR = Ct - cL;
                 if (cL < min_leaf || cR < min_leaf) continue;

@@ -62,6 +62,15 @@ inline int hist_mode(int hist_bits, bool const_h) {
 // an 8-byte h payload).
 inline int hist_pay_bytes(int mode) { return mode <= kHistExactVar ? 8 : mode <= kHistQ16Var ? 4 : 2; }
 
+// What the partition reads of a planned expansion, written whole by the select that plans
+// it: the leaf's rows and slot, its children's first slot, and the split.
+struct alignas(16) WaveExp {
+    int leaf, start, count, buf;
+    int feature, threshold, missing_left, type;
+    int feature2, depth, slot, child_slot;
+    unsigned long long cat[4];
+};
+
 // What the histogram and the scan read of a planned expansion, written whole by the
 // partition tile that completes the leaf: one load instead of a chain through the node
 // table.  WaveJob: the smaller child's rows (cpp/src/tree.cpp:423) and slot.  WaveChild:
@@ -93,7 +102,8 @@ struct WaveCtl {
     // rows of the planned leaf placed so far by its partition tiles: left in the low word,
     // right in the high word (zeroed by the select that plans the expansion)
     unsigned long long part_cur[kMaxLeavesCap];
-    WaveJob job[kMaxLeavesCap];            // per planned expansion
+    WaveExp exp[kMaxLeavesCap];            // per planned expansion
+    WaveJob job[kMaxLeavesCap];
     WaveChild child[2 * kMaxLeavesCap];    // per planned expansion and side
     int expanded[kMaxNodes];  // 0 not expanded; 1, 2: children planned by the axis, with-pairs split
 };
