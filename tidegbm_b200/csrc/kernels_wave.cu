@@ -978,26 +978,6 @@ __device__ __forceinline__ void store_payload(const WaveCtx& X, long long i, lon
     else static_cast<short*>(X.gq)[i] = static_cast<short>(v);
 }
 
-__device__ __forceinline__ void load_tile(const WaveCtx& X, const int32_t* in, const WaveExp& S, int base, int end,
-                                          int32_t (&row)[kPartPer], bool (&left)[kPartPer]) {
-#pragma unroll
-    for (int i = 0; i < kPartPer; ++i) {
-        const int k = base + i * kPartThreads + threadIdx.x;
-        row[i] = k < end ? in[k] : -1;
-    }
-    unsigned int b[kPartPer], b2[kPartPer];
-    const uint8_t* col = X.codes_col + static_cast<size_t>(S.feature) * X.col_pitch;
-    const uint8_t* col2 = S.type == 1 ? X.codes_col + static_cast<size_t>(S.feature2) * X.col_pitch : col;
-#pragma unroll
-    for (int i = 0; i < kPartPer; ++i) {
-        b[i] = row[i] >= 0 ? col[row[i]] : 0u;
-        b2[i] = row[i] >= 0 && S.type == 1 ? col2[row[i]] : 0u;
-    }
-#pragma unroll
-    for (int i = 0; i < kPartPer; ++i)
-        left[i] = row[i] >= 0 && goes_left(S.type, S.cat, S.threshold, S.missing_left, b[i], b2[i], X.gp.n_bins);
-}
-
 // One launch moves the rows of every planned leaf into its children.  A tile of 2048 rows
 // ranks its rows by side with ballots, reserves its places in both children with one 64-bit
 // atomic add on the leaf's cursor (left rows in the low word, right rows in the high word)
@@ -1015,7 +995,7 @@ __global__ void __launch_bounds__(kPartThreads)
     wave_part_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx) {
     __shared__ WaveCtx s_ctx;  // the first context's constants
     __shared__ int s_pref[kMaxWaveCtx + 1];
-    __shared__ int wc[kPartPer * kPartWarps];
+    __shared__ int wc[kPartWarps];
     __shared__ unsigned long long s_old;
     stage_ctx(s_ctx, ctxs);
     __syncthreads();
@@ -1081,41 +1061,51 @@ __global__ void __launch_bounds__(kPartThreads)
         const int32_t* in = (S.buf ? X.rows1 : X.rows0) + S.start;
         int32_t* out = (S.buf ? X.rows0 : X.rows1) + S.start;
         const int base = (lt - ctl->exp_tile0[e]) * kPartTile, end = min(base + kPartTile, count);
-        int32_t row[kPartPer];
-        bool left[kPartPer];
-        load_tile(X, in, S, base, end, row, left);
-        // the rows' payloads move with them (same positions in the other buffer); loaded
-        // here so that their latency overlaps the ranks below
+        // a warp takes 256 consecutive rows, 32 at a time; the rows' payloads move with them
+        // (same positions in the other buffer), so their loads go out with the row ids'
         const long long from0 = static_cast<long long>(S.buf) * X.pay_pitch + S.start;
         const long long to0 = static_cast<long long>(1 - S.buf) * X.pay_pitch + S.start;
+        const int k0 = base + warp * (32 * kPartPer) + lane;
+        int32_t row[kPartPer];
         long long pg[kPartPer], ph[kPartPer];
 #pragma unroll
+        for (int i = 0; i < kPartPer; ++i) row[i] = k0 + 32 * i < end ? in[k0 + 32 * i] : -1;
+#pragma unroll
         for (int i = 0; i < kPartPer; ++i) {
-            const int kk = base + i * kPartThreads + threadIdx.x;
-            pg[i] = row[i] >= 0 ? load_payload(X, from0 + kk) : 0;
-            ph[i] = row[i] >= 0 && X.hq != nullptr ? static_cast<const long long*>(X.hq)[from0 + kk] : 0;
+            const int kk = k0 + 32 * i;
+            pg[i] = kk < end ? load_payload(X, from0 + kk) : 0;
+            ph[i] = kk < end && X.hq != nullptr ? static_cast<const long long*>(X.hq)[from0 + kk] : 0;
+        }
+        unsigned int b[kPartPer], b2[kPartPer];
+        const uint8_t* col = X.codes_col + static_cast<size_t>(S.feature) * X.col_pitch;
+        const uint8_t* col2 = S.type == 1 ? X.codes_col + static_cast<size_t>(S.feature2) * X.col_pitch : col;
+#pragma unroll
+        for (int i = 0; i < kPartPer; ++i) {
+            b[i] = row[i] >= 0 ? col[row[i]] : 0u;
+            b2[i] = row[i] >= 0 && S.type == 1 ? col2[row[i]] : 0u;
         }
         unsigned bal[kPartPer];
+        int excl[kPartPer];  // left rows of the warp's earlier 32s, then of the tile's earlier rows
+        int mine = 0;
 #pragma unroll
         for (int i = 0; i < kPartPer; ++i) {
-            bal[i] = __ballot_sync(0xffffffffu, left[i]);
-            if (lane == 0) wc[i * kPartWarps + warp] = __popc(bal[i]);
+            const bool l =
+                row[i] >= 0 && goes_left(S.type, S.cat, S.threshold, S.missing_left, b[i], b2[i], X.gp.n_bins);
+            bal[i] = __ballot_sync(0xffffffffu, l);
+            excl[i] = mine;
+            mine += __popc(bal[i]);
         }
+        if (lane == 0) wc[warp] = mine;
         __syncthreads();
-        int run = 0;
-        int excl[kPartPer];
+        int run = 0;  // the tile's left rows
+        int before = 0;
 #pragma unroll
-        for (int i = 0; i < kPartPer; ++i) {
-            int e = run;
-#pragma unroll
-            for (int w = 0; w < kPartWarps; ++w) {
-                const int cw = wc[i * kPartWarps + w];
-                if (w < warp) e += cw;
-                run += cw;
-            }
-            excl[i] = e;
+        for (int w = 0; w < kPartWarps; ++w) {
+            const int cw = wc[w];
+            if (w < warp) before += cw;
+            run += cw;
         }
-        const int n_right = end - base - run;  // run: the tile's left rows
+        const int n_right = end - base - run;
         if (threadIdx.x == 0) {
             const unsigned long long old =
                 atomicAdd(&ctl->part_cur[e],
@@ -1144,9 +1134,10 @@ __global__ void __launch_bounds__(kPartThreads)
 #pragma unroll
         for (int i = 0; i < kPartPer; ++i) {
             if (row[i] < 0) continue;
-            const int kk = base + i * kPartThreads + threadIdx.x;
-            const int lrank = excl[i] + __popc(bal[i] & lt_mask);
-            const int dst = left[i] ? left0 + lrank : right0 + (kk - base - lrank);
+            const int kk = k0 + 32 * i;
+            const int lrank = before + excl[i] + __popc(bal[i] & lt_mask);
+            const bool l = (bal[i] >> lane) & 1u;
+            const int dst = l ? left0 + lrank : right0 + (kk - base - lrank);
             out[dst] = row[i];
             store_payload(X, to0 + dst, pg[i]);
             if (X.hq != nullptr) static_cast<long long*>(X.hq)[to0 + dst] = ph[i];

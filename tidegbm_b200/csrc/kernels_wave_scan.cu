@@ -237,11 +237,6 @@ __device__ __forceinline__ bool candidate(const GrowParams& p, const DevNode& N,
            (S.gain > p.min_split_gain);
 }
 
-// better leaf: larger gain, lower id on ties
-__device__ __forceinline__ bool better_leaf(double ga, int ia, double gb, int ib) {
-    return ga > gb || (ga == gb && ia < ib);
-}
-
 // A gain as an unsigned integer of the same order (both zeros alike); never 0 for a number.
 __device__ __forceinline__ unsigned long long ordered(double g) {
     const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(g + 0.0));
@@ -264,16 +259,16 @@ __global__ void __launch_bounds__(kSelectThreads)
     DevNode* nodes = X.nodes;
     DevSplit* splits = X.splits;
     const int lane = threadIdx.x & 31;
-    __shared__ double s_gain[kMaxLeavesCap + 1];
+    __shared__ unsigned long long s_gain[kMaxLeavesCap + 1];
     __shared__ int s_id[kMaxLeavesCap + 1];
     // Selection state staged once, so that the commit loop reads no global memory: per
     // node its current split's gain, candidacy, type and with-pairs type, and whether it
     // is expanded; per expanded node the same for its two planned children.  Restaged
     // from the node table when the pair budget runs out (the splits change).
-    __shared__ double s_ng[kMaxNodes];
-    __shared__ unsigned char s_nc[kMaxNodes], s_ex[kMaxNodes], s_ty[kMaxNodes], s_pty[kMaxNodes];
-    __shared__ double s_cg[2 * kMaxNodes];
-    __shared__ unsigned char s_cc[2 * kMaxNodes], s_cty[2 * kMaxNodes], s_cpty[2 * kMaxNodes];
+    __shared__ unsigned long long s_key[kMaxNodes];  // ordered gain of a candidate, else 0
+    __shared__ unsigned char s_ex[kMaxNodes], s_ty[kMaxNodes], s_pty[kMaxNodes];
+    __shared__ unsigned long long s_ckey[2 * kMaxNodes];
+    __shared__ unsigned char s_cty[2 * kMaxNodes], s_cpty[2 * kMaxNodes];
     __shared__ int s_commit[kMaxLeavesCap];
     int active = 0;
     if (ctl->active) {
@@ -297,14 +292,11 @@ __global__ void __launch_bounds__(kSelectThreads)
                 const double g = Sp->gain, g0 = Cp[0].gain, g1 = Cp[1].gain;
                 const int ty = Sp->type, ty0 = Cp[0].type, ty1 = Cp[1].type, ex = ctl->expanded[k];
                 const bool c = candidate(p, N, *Sp), c0 = candidate(p, A, Cp[0]), c1 = candidate(p, B, Cp[1]);
-                s_nc[k] = c ? 1 : 0;
-                s_ng[k] = g;
+                s_key[k] = c ? ordered(g) : 0ull;
                 s_ty[k] = static_cast<unsigned char>(ty);
                 s_ex[k] = static_cast<unsigned char>(ex);
-                s_cc[2 * k] = c0 ? 1 : 0;
-                s_cc[2 * k + 1] = c1 ? 1 : 0;
-                s_cg[2 * k] = g0;
-                s_cg[2 * k + 1] = g1;
+                s_ckey[2 * k] = c0 ? ordered(g0) : 0ull;
+                s_ckey[2 * k + 1] = c1 ? ordered(g1) : 0ull;
                 s_cty[2 * k] = static_cast<unsigned char>(ty0);
                 s_cty[2 * k + 1] = static_cast<unsigned char>(ty1);
                 s_pty[k] = X.pair_on ? static_cast<unsigned char>(X.splits_pair[k].type) : 0;
@@ -360,20 +352,18 @@ __global__ void __launch_bounds__(kSelectThreads)
             unsigned long long bk = 0ull;
             int bi = 0x7fffffff;
             for (int k = lane; k < nn; k += 32) {
-                if (!s_nc[k]) continue;
-                const unsigned long long key = ordered(s_ng[k]);
-                if (bi == 0x7fffffff || key > bk) {
+                const unsigned long long key = s_key[k];
+                if (key > bk) {
                     bk = key;
                     bi = k;
                 }
             }
-            const bool has = bi != 0x7fffffff;
-            const unsigned hi = has ? static_cast<unsigned>(bk >> 32) : 0u;
+            const unsigned hi = static_cast<unsigned>(bk >> 32);
             const unsigned top = __reduce_max_sync(0xffffffffu, hi);
-            const unsigned lo = has && hi == top ? static_cast<unsigned>(bk) : 0u;
+            const unsigned lo = hi == top ? static_cast<unsigned>(bk) : 0u;
             const unsigned topl = __reduce_max_sync(0xffffffffu, lo);
             bi = static_cast<int>(
-                __reduce_min_sync(0xffffffffu, has && hi == top && lo == topl ? static_cast<unsigned>(bi) : 0x7fffffffu));
+                __reduce_min_sync(0xffffffffu, hi == top && lo == topl ? static_cast<unsigned>(bi) : 0x7fffffffu));
             if (bi == 0x7fffffff) {
                 finished = true;
                 break;
@@ -396,12 +386,11 @@ __global__ void __launch_bounds__(kSelectThreads)
             const int ty = s_ty[bi];
             if (lane == 0) {
                 s_commit[n_commit] = bi;
-                s_nc[bi] = 0;
+                s_key[bi] = 0ull;
             }
             if (lane < 2) {
                 const int k = nn + lane, ci = 2 * bi + lane;
-                s_nc[k] = s_cc[ci];
-                s_ng[k] = s_cg[ci];
+                s_key[k] = s_ckey[ci];
                 s_ex[k] = 0;
                 s_ty[k] = s_cty[ci];
                 s_pty[k] = s_cpty[ci];
@@ -425,12 +414,8 @@ __global__ void __launch_bounds__(kSelectThreads)
             int nc = 0;
             for (int k0 = 0; k0 < nn; k0 += 32) {
                 const int k = k0 + lane;
-                bool is_c = false;
-                double gk = 0.0;
-                if (k < nn) {
-                    is_c = s_nc[k] != 0;
-                    gk = s_ng[k];
-                }
+                const unsigned long long gk = k < nn ? s_key[k] : 0ull;
+                const bool is_c = gk != 0ull;
                 const unsigned m = __ballot_sync(0xffffffffu, is_c);
                 if (is_c) {
                     const int pos = nc + __popc(m & ((1u << lane) - 1u));
@@ -451,9 +436,11 @@ __global__ void __launch_bounds__(kSelectThreads)
                 const int i = i0 + lane;
                 bool take = false;
                 if (i < nc) {
+                    // ids ascend with the position, so a tie ranks the earlier one first
                     int rank = 0;
-                    for (int q = 0; q < nc; ++q)
-                        if (q != i && better_leaf(s_gain[q], s_id[q], s_gain[i], s_id[i])) ++rank;
+                    const unsigned long long mine = s_gain[i];
+#pragma unroll 8
+                    for (int q = 0; q < nc; ++q) rank += (s_gain[q] > mine) | ((s_gain[q] == mine) & (q < i));
                     take = rank < B && (X.max_expand <= 0 || rank < X.max_expand) && !s_ex[s_id[i]];
                 }
                 const unsigned m = __ballot_sync(0xffffffffu, take);

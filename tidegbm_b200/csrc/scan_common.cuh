@@ -126,9 +126,28 @@ __device__ __forceinline__ Cand scan_feature(long long* __restrict__ Gf, long lo
     return best;
 }
 
-// One warp scans one feature: lane l owns bins [8l, 8l + 8) (the same arithmetic, in the
-// same order, as scan_feature, without block barriers).  Returns the warp's best candidate
-// and the feature's totals in every lane.
+// 1 / d to about 2^-39 for d in [1e-30, 1e30]: the hardware's approximate reciprocal
+// (rcp.approx.ftz.f64, good to about 2^-20) and one Newton-Raphson step.
+__device__ __forceinline__ double near_rcp(double d) {
+    double r;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(d));
+    return fma(r, fma(-d, r, 1.0), r);
+}
+
+// One warp scans one feature without block barriers; the candidates' gains are those of
+// scan_feature.  Lane l owns bins 64 i + 2 l + {0, 1}, i < 4, so that the 16-byte loads of a
+// warp are whole lines.  Returns the warp's best candidate and the feature's totals in every
+// lane.
+//
+// Choosing the best of a lane's 16 candidates (8 bins x missing left or right) takes two
+// passes.  A gain needs two FP64 divisions, and 32 of them in a row were most of the scan's
+// time (10,000 to 20,000 cycles of a warp).  The first pass only estimates
+// GL^2/(HL+l2) + GR^2/(HR+l2), up to a constant factor, with reciprocals good to 2^-39, all
+// candidates side by side; the second evaluates the reference's expression for those within
+// 2^-34 of the warp's best estimate, usually one.  The others cannot win or tie: the gain is
+// a monotone function of that sum, the parent's term is at most twice it (hessian sums are
+// not negative), and where a gamma could absorb the difference, or a denominator lies
+// outside the range of the reciprocal, every candidate is evaluated.
 __device__ __forceinline__ Cand scan_feature_warp(long long* __restrict__ Gf, long long* __restrict__ Hf,
                                                   int* __restrict__ Cf, const long long* __restrict__ PGf,
                                                   const long long* __restrict__ PHf, const int* __restrict__ PCf,
@@ -136,106 +155,154 @@ __device__ __forceinline__ Cand scan_feature_warp(long long* __restrict__ Gf, lo
                                                   const int* __restrict__ SCf, bool derive, bool scan, int f, int n_bins,
                                                   double inv_gs, double inv_hs, double lam, double gamma, int min_leaf,
                                                   double min_hess, long long& Gt, long long& Ht, long long& Ct) {
-    constexpr int kPer = kBins / 32;
-    const int lane = threadIdx.x & 31, b0 = lane * kPer;
-    long long g[kPer], hh[kPer], c[kPer];
+    constexpr int kChunks = kBins / 64;
+    const int lane = threadIdx.x & 31;
+    long long g[2 * kChunks], hh[2 * kChunks];
+    int c[2 * kChunks];
     {
-        const longlong2* g2 = reinterpret_cast<const longlong2*>((derive ? PGf : Gf) + b0);
-        const longlong2* h2 = reinterpret_cast<const longlong2*>((derive ? PHf : Hf) + b0);
-        const int4* c4 = reinterpret_cast<const int4*>((derive ? PCf : Cf) + b0);
+        const longlong2* g2 = reinterpret_cast<const longlong2*>(derive ? PGf : Gf) + lane;
+        const longlong2* h2 = reinterpret_cast<const longlong2*>(derive ? PHf : Hf) + lane;
+        const int2* c2 = reinterpret_cast<const int2*>(derive ? PCf : Cf) + lane;
 #pragma unroll
-        for (int i = 0; i < kPer / 2; ++i) {
-            const longlong2 a = g2[i], b = h2[i];
+        for (int i = 0; i < kChunks; ++i) {
+            const longlong2 a = g2[32 * i], b = h2[32 * i];
+            const int2 d = c2[32 * i];
             g[2 * i] = a.x;
             g[2 * i + 1] = a.y;
             hh[2 * i] = b.x;
             hh[2 * i + 1] = b.y;
-        }
-#pragma unroll
-        for (int i = 0; i < kPer / 4; ++i) {
-            const int4 a = c4[i];
-            c[4 * i] = a.x;
-            c[4 * i + 1] = a.y;
-            c[4 * i + 2] = a.z;
-            c[4 * i + 3] = a.w;
+            c[2 * i] = d.x;
+            c[2 * i + 1] = d.y;
         }
     }
     if (derive) {
-        const longlong2* g2 = reinterpret_cast<const longlong2*>(SGf + b0);
-        const longlong2* h2 = reinterpret_cast<const longlong2*>(SHf + b0);
-        const int4* c4 = reinterpret_cast<const int4*>(SCf + b0);
+        const longlong2* g2 = reinterpret_cast<const longlong2*>(SGf) + lane;
+        const longlong2* h2 = reinterpret_cast<const longlong2*>(SHf) + lane;
+        const int2* c2 = reinterpret_cast<const int2*>(SCf) + lane;
 #pragma unroll
-        for (int i = 0; i < kPer / 2; ++i) {
-            const longlong2 a = g2[i], b = h2[i];
+        for (int i = 0; i < kChunks; ++i) {
+            const longlong2 a = g2[32 * i], b = h2[32 * i];
+            const int2 d = c2[32 * i];
             g[2 * i] -= a.x;
             g[2 * i + 1] -= a.y;
             hh[2 * i] -= b.x;
             hh[2 * i + 1] -= b.y;
+            c[2 * i] -= d.x;
+            c[2 * i + 1] -= d.y;
         }
 #pragma unroll
-        for (int i = 0; i < kPer / 4; ++i) {
-            const int4 a = c4[i];
-            c[4 * i] -= a.x;
-            c[4 * i + 1] -= a.y;
-            c[4 * i + 2] -= a.z;
-            c[4 * i + 3] -= a.w;
+        for (int i = 0; i < kChunks; ++i) {
+            reinterpret_cast<longlong2*>(Gf)[lane + 32 * i] = make_longlong2(g[2 * i], g[2 * i + 1]);
+            reinterpret_cast<longlong2*>(Hf)[lane + 32 * i] = make_longlong2(hh[2 * i], hh[2 * i + 1]);
+            reinterpret_cast<int2*>(Cf)[lane + 32 * i] = make_int2(c[2 * i], c[2 * i + 1]);
         }
-        longlong2* go = reinterpret_cast<longlong2*>(Gf + b0);
-        longlong2* ho = reinterpret_cast<longlong2*>(Hf + b0);
-        int4* co = reinterpret_cast<int4*>(Cf + b0);
-#pragma unroll
-        for (int i = 0; i < kPer / 2; ++i) {
-            go[i] = make_longlong2(g[2 * i], g[2 * i + 1]);
-            ho[i] = make_longlong2(hh[2 * i], hh[2 * i + 1]);
-        }
-#pragma unroll
-        for (int i = 0; i < kPer / 4; ++i)
-            co[i] = make_int4(static_cast<int>(c[4 * i]), static_cast<int>(c[4 * i + 1]), static_cast<int>(c[4 * i + 2]),
-                              static_cast<int>(c[4 * i + 3]));
     }
-    long long tg = 0, th = 0, tc = 0;
+    const long long G0 = __shfl_sync(0xffffffffu, g[0], 0), H0 = __shfl_sync(0xffffffffu, hh[0], 0);
+    const int C0 = __shfl_sync(0xffffffffu, c[0], 0);
+    // sums through each bin, in place
+    long long bg = 0, bh = 0;
+    int bc = 0;
+    unsigned present = 0u;  // bins that hold rows
 #pragma unroll
-    for (int i = 0; i < kPer; ++i) {
-        tg += g[i];
-        th += hh[i];
-        tc += c[i];
-    }
-    const long long ig = warp_incl_scan(tg, lane), ih = warp_incl_scan(th, lane), ic = warp_incl_scan(tc, lane);
-    Gt = __shfl_sync(0xffffffffu, ig, 31);
-    Ht = __shfl_sync(0xffffffffu, ih, 31);
-    Ct = __shfl_sync(0xffffffffu, ic, 31);
-    const long long G0 = __shfl_sync(0xffffffffu, g[0], 0), H0 = __shfl_sync(0xffffffffu, hh[0], 0),
-                    C0 = __shfl_sync(0xffffffffu, c[0], 0);
-    Cand best{-1e300, 0x7fffffff};
-    if (scan) {
-        const double dGt = static_cast<double>(Gt) * inv_gs, dHt = static_cast<double>(Ht) * inv_hs;
-        const double parent = (dGt * dGt) / (dHt + lam);
-        long long rg = ig - tg, rh = ih - th, rc = ic - tc;  // bins before this lane's
+    for (int i = 0; i < kChunks; ++i) {
+        present |= (c[2 * i] != 0 ? 1u : 0u) << (2 * i) | (c[2 * i + 1] != 0 ? 2u : 0u) << (2 * i);
+        long long ig = g[2 * i] + g[2 * i + 1], ih = hh[2 * i] + hh[2 * i + 1];
+        int ic = c[2 * i] + c[2 * i + 1];
 #pragma unroll
-        for (int i = 0; i < kPer; ++i) {
-            rg += g[i];
-            rh += hh[i];
-            rc += c[i];
-            const int b = b0 + i;
-            if (b < 1 || b > n_bins - 2 || c[i] == 0) continue;
-            const long long GL = rg - G0, HL = rh - H0, CL = rc - C0;  // bins 1..b
-#pragma unroll
-            for (int ml = 0; ml <= 1; ++ml) {
-                if (ml && C0 == 0) continue;  // no missing rows: the same sums as ml = 0, which wins the tie
-                const long long gL = GL + (ml ? G0 : 0), hL = HL + (ml ? H0 : 0), cL = CL + (ml ? C0 : 0);
-                const long long cR = Ct - cL;
-                if (cL < min_leaf || cR < min_leaf) continue;
-                const double dgL = static_cast<double>(gL) * inv_gs, dhL = static_cast<double>(hL) * inv_hs;
-                const double dgR = static_cast<double>(Gt - gL) * inv_gs, dhR = static_cast<double>(Ht - hL) * inv_hs;
-                if (dhL < min_hess || dhR < min_hess) continue;
-                const double gain = 0.5 * ((dgL * dgL) / (dhL + lam) + (dgR * dgR) / (dhR + lam) - parent) - gamma;
-                const Cand cand{gain, f * 512 + b * 2 + ml};
-                if (better(cand, best)) best = cand;
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long tg = __shfl_up_sync(0xffffffffu, ig, o), th = __shfl_up_sync(0xffffffffu, ih, o);
+            const int tc = __shfl_up_sync(0xffffffffu, ic, o);
+            if (lane >= o) {
+                ig += tg;
+                ih += th;
+                ic += tc;
             }
         }
-        best = warp_best(best);
+        const long long g1 = g[2 * i + 1], h1 = hh[2 * i + 1];
+        const int c1 = c[2 * i + 1];
+        g[2 * i + 1] = bg + ig;
+        hh[2 * i + 1] = bh + ih;
+        c[2 * i + 1] = bc + ic;
+        g[2 * i] = bg + ig - g1;
+        hh[2 * i] = bh + ih - h1;
+        c[2 * i] = bc + ic - c1;
+        bg += __shfl_sync(0xffffffffu, ig, 31);
+        bh += __shfl_sync(0xffffffffu, ih, 31);
+        bc += __shfl_sync(0xffffffffu, ic, 31);
     }
-    return best;
+    Gt = bg;
+    Ht = bh;
+    Ct = bc;
+    Cand best{-1e300, 0x7fffffff};
+    if (!scan) return best;
+    const double dGt = static_cast<double>(Gt) * inv_gs, dHt = static_cast<double>(Ht) * inv_hs;
+    const double parent = (dGt * dGt) / (dHt + lam);
+    // no missing rows: missing left has the same sums as missing right, which wins the tie
+    const int n_ml = C0 == 0 ? 1 : 2;
+    double est[4 * kChunks];
+    double top = 0.0;
+    unsigned ok = 0u;  // candidates within the leaf limits: bit q for bin q, bit 8 + q missing left
+#pragma unroll
+    for (int q = 0; q < 4 * kChunks; ++q) est[q] = -1.0;
+#pragma unroll
+    for (int ml = 0; ml < 2; ++ml) {
+        if (ml == n_ml) break;  // the same for the whole warp
+#pragma unroll
+        for (int q = 0; q < 2 * kChunks; ++q) {
+            const int b = 64 * (q >> 1) + 2 * lane + (q & 1);
+            const long long gL = ml ? g[q] : g[q] - G0, hL = ml ? hh[q] : hh[q] - H0;
+            const int cL = ml ? c[q] : c[q] - C0;
+            const double vL = static_cast<double>(gL), vR = static_cast<double>(Gt - gL);
+            const double dhL = static_cast<double>(hL) * inv_hs, dhR = static_cast<double>(Ht - hL) * inv_hs;
+            const bool use = (b >= 1) & (b <= n_bins - 2) & ((present >> q & 1u) != 0u) & (cL >= min_leaf) &
+                             (static_cast<int>(Ct) - cL >= min_leaf) & !(dhL < min_hess) & !(dhR < min_hess);
+            const double e = fma(vL * vL, near_rcp(dhL + lam), vR * vR * near_rcp(dhR + lam));
+            est[8 * ml + q] = use ? e : -1.0;
+            ok |= (use ? 1u : 0u) << (8 * ml + q);
+        }
+    }
+#pragma unroll
+    for (int q = 0; q < 4 * kChunks; ++q) top = fmax(top, est[q]);
+    {
+        // the warp's best estimate: non-negative doubles order like their bits
+        const unsigned long long tb = static_cast<unsigned long long>(__double_as_longlong(top));
+        const unsigned hi = __reduce_max_sync(0xffffffffu, static_cast<unsigned>(tb >> 32));
+        const unsigned lo =
+            __reduce_max_sync(0xffffffffu, static_cast<unsigned>(tb >> 32) == hi ? static_cast<unsigned>(tb) : 0u);
+        top = __longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo));
+    }
+    // every denominator lies in [l2 + min_child_weight, H + l2]
+    const bool exact_all = !(lam + fmax(min_hess, 0.0) >= 1e-30) || !(dHt + lam < 1e30) || !(top > 0.0) ||
+                           !(fabs(gamma) <= top * inv_gs * inv_gs * 1048576.0);
+    if (!exact_all) {
+        const double least = top * (1.0 - 0x1p-34);
+#pragma unroll
+        for (int q = 0; q < 4 * kChunks; ++q)
+            if (!(est[q] >= least)) ok &= ~(1u << q);
+    }
+    while (__any_sync(0xffffffffu, ok != 0u)) {
+        if (ok != 0u) {
+            const int q = __ffs(ok) - 1, bin = q & 7, ml = q >> 3;
+            ok &= ok - 1u;
+            long long gL = 0, hL = 0;
+#pragma unroll
+            for (int i = 0; i < 2 * kChunks; ++i)
+                if (i == bin) {
+                    gL = g[i];
+                    hL = hh[i];
+                }
+            if (!ml) {
+                gL -= G0;
+                hL -= H0;
+            }
+            const double dgL = static_cast<double>(gL) * inv_gs, dhL = static_cast<double>(hL) * inv_hs;
+            const double dgR = static_cast<double>(Gt - gL) * inv_gs, dhR = static_cast<double>(Ht - hL) * inv_hs;
+            const double gain = 0.5 * ((dgL * dgL) / (dhL + lam) + (dgR * dgR) / (dhR + lam) - parent) - gamma;
+            const Cand cand{gain, f * 512 + (64 * (bin >> 1) + 2 * lane + (bin & 1)) * 2 + ml};
+            if (better(cand, best)) best = cand;
+        }
+    }
+    return warp_best(best);
 }
 
 // ---- categorical features ---------------------------------------------------------------
