@@ -197,9 +197,9 @@ struct DeviceState {
     DBuf<WaveCtx> wctx;
     DBuf<uint8_t> is_cat;                 // categorical flags per feature (fit and predict)
     DBuf<unsigned long long> cand_cat;    // scan candidates' left masks
-    DBuf<DevSplit> splits_pair, spec_split_pair, pair_cand;  // PAIR search (wave.h)
-    DBuf<unsigned long long> energy;
-    DBuf<int> pair_tickets;
+    DBuf<DevSplit> splits_pair, spec_split_pair;  // PAIR search (wave.h)
+    DBuf<unsigned long long> energy, pair_G, pair_H;
+    DBuf<int> pair_C, pair_tickets;
     // predict
     DBuf<uint8_t> pcodes;
     DBuf<int16_t> t_feat, t_left, t_right, t_feat2;
@@ -223,7 +223,8 @@ struct DeviceState {
         loss_valid.release(); run_start.release(); run_len.release(); order.release();
         gqw.release(); hqw.release(); spec.release(); spec_split.release(); ctl.release(); cand_gain.release();
         cand_key.release(); tickets.release(); wctx.release(); cand_cat.release(); splits_pair.release();
-        spec_split_pair.release(); pair_cand.release(); energy.release(); pair_tickets.release();
+        spec_split_pair.release(); energy.release(); pair_G.release(); pair_H.release(); pair_C.release();
+        pair_tickets.release();
     }
 
 };
@@ -514,7 +515,13 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
             D.splits_pair.alloc(kMaxNodes, s);
             D.spec_split_pair.alloc(2 * kMaxNodes, s);
             D.energy.alloc(2 * kMaxNodes + 1, s);
-            D.pair_cand.alloc(static_cast<size_t>(2 * kMaxNodes + 1) * kMaxPairs, s);
+            const size_t cells = static_cast<size_t>(wave_children(c.max_leaves, c.wave_expand)) * kMaxPairs * kBins;
+            D.pair_G.alloc(cells, s);
+            D.pair_H.alloc(cells, s);
+            D.pair_C.alloc(cells, s);
+            check(cudaMemsetAsync(D.pair_G.p, 0, 8 * cells, s), "pair histogram reset");
+            check(cudaMemsetAsync(D.pair_H.p, 0, 8 * cells, s), "pair histogram reset");
+            check(cudaMemsetAsync(D.pair_C.p, 0, 4 * cells, s), "pair histogram reset");
             D.pair_tickets.alloc(2 * kMaxNodes + 1, s);
             check(cudaMemsetAsync(D.pair_tickets.p, 0, sizeof(int) * (2 * kMaxNodes + 1), s), "pair ticket reset");
         }
@@ -757,7 +764,9 @@ WaveCtx FitRun::wave_ctx() const {
     w.splits_pair = D.splits_pair.p;
     w.spec_split_pair = D.spec_split_pair.p;
     w.energy = D.energy.p;
-    w.pair_cand = D.pair_cand.p;
+    w.pair_G = D.pair_G.p;
+    w.pair_H = D.pair_H.p;
+    w.pair_C = D.pair_C.p;
     w.pair_tickets = D.pair_tickets.p;
     return w;
 }
@@ -810,9 +819,10 @@ void FitRun::tree_begin(int t) {
     const uint64_t seed = z ^ (z >> 31);
     const size_t slot = static_cast<size_t>(n_f) * kBins;
     if (wave) {
-        launch_wave_quantize(mode, D.rows0.p, D.g.p, h_rows, flag, goss_scale, D.st.p, seed, D.gqw.p, D.hqw.p, n, s);
-        if (c.pair_splits)
-            check(cudaMemsetAsync(D.energy.p + 2 * kMaxNodes, 0, sizeof(unsigned long long), s), "energy reset");
+        unsigned long long* root_energy = c.pair_splits ? D.energy.p + 2 * kMaxNodes : nullptr;
+        if (root_energy) check(cudaMemsetAsync(root_energy, 0, sizeof(unsigned long long), s), "energy reset");
+        launch_wave_quantize(mode, D.rows0.p, D.g.p, h_rows, flag, goss_scale, D.st.p, seed, D.gqw.p, D.hqw.p,
+                             root_energy, n, s);
         // the root's slot; the children's slots are cleared by the partition of their wave
         check(cudaMemsetAsync(D.histG.p, 0, sizeof(long long) * slot, s), "hist reset");
         check(cudaMemsetAsync(D.histH.p, 0, sizeof(long long) * slot, s), "hist reset");
@@ -1017,6 +1027,7 @@ public:
         }
         if (leaves > kMaxWaveJobs) throw TideError("wave: too many leaves over the contexts of one launch");
         mode_ = runs_[0]->mode;
+        if (pair_) prepare_wave_pair();
         tune_.cluster = 4;
         tune_.clusters = wave_hist_clusters(4);
         ctx_.alloc(n_ctx_, s_);
@@ -1149,7 +1160,7 @@ public:
         }
         hist(0);
         launch_wave_scan(ctx_.p, n_ctx_, 0, max_f_, scan_ys_, cat_, s_);
-        if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 0, s_);
+        if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 0, (mode_ & 1) != 0, s_);
         launch_wave_select(ctx_.p, n_ctx_, gsync_.p, dflag_, 0ull, 0, s_);
         // waves, enqueued ahead; the flag written by wave w's select is read once wave w
         // has completed (its event), two waves behind the host
@@ -1166,10 +1177,10 @@ public:
                 check(cudaEventSynchronize(ev_[w - 2]), "wave event");
                 if (*reinterpret_cast<volatile unsigned*>(hflag_) == 0u) break;
             }
-            launch_wave_partition(ctx_.p, n_ctx_, part_grid_, s_);
+            launch_wave_partition(ctx_.p, n_ctx_, part_grid_, pair_, s_);
             hist(1);
             launch_wave_scan(ctx_.p, n_ctx_, 1, max_f_, scan_ys_, cat_, s_);
-            if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 1, s_);
+            if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 1, (mode_ & 1) != 0, s_);
             launch_wave_select(ctx_.p, n_ctx_, gsync_.p, dflag_, 0ull, 0, s_);
             check(cudaEventRecord(ev_[w], s_), "event record");
         }
@@ -1195,7 +1206,7 @@ private:
               "graph capture");
         launch_wave_hist(mode_, ctx_.p, n_ctx_, 0, tune_, rows_counter_, s_);
         launch_wave_scan(ctx_.p, n_ctx_, 0, max_f_, scan_ys_, cat_, s_);
-        if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 0, s_);
+        if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 0, (mode_ & 1) != 0, s_);
         launch_wave_select(ctx_.p, n_ctx_, gsync_.p, nullptr, handle, 1, s_);
         cudaStreamCaptureStatus cs;
         const cudaGraphNode_t* deps = nullptr;
@@ -1216,16 +1227,16 @@ private:
         // the body: one wave
         check(cudaStreamBeginCaptureToGraph(s_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
               "body capture");
-        launch_wave_partition(ctx_.p, n_ctx_, part_grid_, s_);
+        launch_wave_partition(ctx_.p, n_ctx_, part_grid_, pair_, s_);
         launch_wave_hist(mode_, ctx_.p, n_ctx_, 1, tune_, rows_counter_, s_);
         launch_wave_scan(ctx_.p, n_ctx_, 1, max_f_, scan_ys_, cat_, s_);
-        if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 1, s_);
+        if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 1, (mode_ & 1) != 0, s_);
         launch_wave_select(ctx_.p, n_ctx_, gsync_.p, nullptr, handle, 1, s_);
         cudaGraph_t body_out = nullptr;
         check(cudaStreamEndCapture(s_, &body_out), "body capture end");
         check(cudaGraphInstantiate(&exec_, graph_, 0), "graph instantiate");
         // launches counted per grow (the graph's kernels are this library's)
-        g_kernel_launches.fetch_sub(pair_ ? 11 : 7);
+        g_kernel_launches.fetch_sub(pair_ ? 9 : 7);
     }
 
     std::vector<FitRun*> runs_;

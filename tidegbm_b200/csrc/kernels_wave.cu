@@ -991,12 +991,15 @@ __device__ __forceinline__ void store_payload(const WaveCtx& X, long long i, lon
 // codes need.  The reference's stable order took two launches (count, then scatter from the
 // tile prefixes): both are bound by their chain of dependent loads, and the second read the
 // rows and codes again.
+// kPair: some context searches PAIR splits, so the children's gradient energies (sums of g^2,
+// exact in fixed point) are made on the way.
+template <bool kPair>
 __global__ void __launch_bounds__(kPartThreads)
     wave_part_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx) {
     __shared__ WaveCtx s_ctx;  // the first context's constants
     __shared__ int s_pref[kMaxWaveCtx + 1];
     __shared__ int wc[kPartWarps];
-    __shared__ unsigned long long s_old;
+    __shared__ unsigned long long s_old, s_en[2];
     stage_ctx(s_ctx, ctxs);
     __syncthreads();
     pdl_wait();
@@ -1084,6 +1087,18 @@ __global__ void __launch_bounds__(kPartThreads)
             b[i] = row[i] >= 0 ? col[row[i]] : 0u;
             b2[i] = row[i] >= 0 && S.type == 1 ? col2[row[i]] : 0u;
         }
+        // PAIR: the rows' g^2 as the tree sees them (GOSS-scaled), in fixed point
+        unsigned long long en[kPair ? kPartPer : 1];
+        if (kPair && X.pair_on) {
+            const double scale = ldexp(1.0, energy_shift(X.st));
+#pragma unroll
+            for (int i = 0; i < (kPair ? kPartPer : 0); ++i) {
+                double gv = row[i] >= 0 ? X.g[row[i]] : 0.0;
+                if (row[i] >= 0 && X.goss_flag != nullptr && X.goss_flag[row[i]] == 2) gv *= X.goss_scale;
+                en[i] = static_cast<unsigned long long>(__double2ll_rn(gv * gv * scale));
+            }
+            if (threadIdx.x < 2) s_en[threadIdx.x] = 0ull;
+        }
         unsigned bal[kPartPer];
         int excl[kPartPer];  // left rows of the warp's earlier 32s, then of the tile's earlier rows
         int mine = 0;
@@ -1097,6 +1112,23 @@ __global__ void __launch_bounds__(kPartThreads)
         }
         if (lane == 0) wc[warp] = mine;
         __syncthreads();
+        if (kPair && X.pair_on) {
+            unsigned long long el = 0, er = 0;
+#pragma unroll
+            for (int i = 0; i < (kPair ? kPartPer : 0); ++i) {
+                if ((bal[i] >> lane) & 1u) el += en[i];
+                else er += en[i];
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                el += __shfl_xor_sync(0xffffffffu, el, o);
+                er += __shfl_xor_sync(0xffffffffu, er, o);
+            }
+            if (lane == 0) {
+                atomicAdd(&s_en[0], el);
+                atomicAdd(&s_en[1], er);
+            }
+        }
         int run = 0;  // the tile's left rows
         int before = 0;
 #pragma unroll
@@ -1129,6 +1161,7 @@ __global__ void __launch_bounds__(kPartThreads)
             }
         }
         __syncthreads();
+        if (kPair && X.pair_on && threadIdx.x < 2) atomicAdd(&X.energy[2 * L + threadIdx.x], s_en[threadIdx.x]);
         const int left0 = static_cast<int>(s_old & 0xffffffffu);
         const int right0 = count - static_cast<int>(s_old >> 32) - n_right;
 #pragma unroll
@@ -1249,8 +1282,11 @@ template <int kMode>
 __global__ void wave_quantize_kernel(const int32_t* __restrict__ rows, const double* __restrict__ g,
                                      const double* __restrict__ h, const uint8_t* __restrict__ goss_flag,
                                      double goss_scale, const DevTreeState* __restrict__ st,
-                                     unsigned long long seed, void* __restrict__ gq, void* __restrict__ hq) {
+                                     unsigned long long seed, void* __restrict__ gq, void* __restrict__ hq,
+                                     unsigned long long* __restrict__ energy) {
     const int count = st->n_sample;
+    const double escale = energy != nullptr ? ldexp(1.0, energy_shift(st)) : 0.0;
+    unsigned long long en = 0;
     const double gscale = st->gscale, hscale = st->hscale;
     for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < count; k += gridDim.x * blockDim.x) {
         const int r = rows[k];
@@ -1261,6 +1297,7 @@ __global__ void wave_quantize_kernel(const int32_t* __restrict__ rows, const dou
             gv *= goss_scale;
             hv *= goss_scale;
         }
+        if (energy != nullptr) en += static_cast<unsigned long long>(__double2ll_rn(gv * gv * escale));
         if constexpr (kMode == kHistExactConst) {
             const long long v = __double2ll_rn(gv * gscale);
             static_cast<long long*>(gq)[k] = static_cast<long long>((static_cast<unsigned long long>(v) << 1) | (sc ? 1ull : 0ull));
@@ -1282,6 +1319,11 @@ __global__ void wave_quantize_kernel(const int32_t* __restrict__ rows, const dou
             const int qh = sround(hv * hscale, uniform01(seed, r, 1), 0, 255);
             static_cast<unsigned short*>(gq)[k] = static_cast<unsigned short>((qg + 128) | (qh << 8));
         }
+    }
+    if (energy != nullptr) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) en += __shfl_xor_sync(0xffffffffu, en, o);
+        if ((threadIdx.x & 31) == 0 && en != 0ull) atomicAdd(energy, en);
     }
 }
 
@@ -1346,8 +1388,9 @@ void hist_launch(const WaveCtx* ctxs, int n_ctx, int src, HistTune tune, unsigne
 
 template <int kMode>
 void quantize_launch(const int32_t* rows, const double* g, const double* h, const uint8_t* flag, double gs,
-                     const DevTreeState* st, unsigned long long seed, void* gq, void* hq, int blocks, cudaStream_t s) {
-    wave_quantize_kernel<kMode><<<blocks, 256, 0, s>>>(rows, g, h, flag, gs, st, seed, gq, hq);
+                     const DevTreeState* st, unsigned long long seed, void* gq, void* hq, unsigned long long* energy,
+                     int blocks, cudaStream_t s) {
+    wave_quantize_kernel<kMode><<<blocks, 256, 0, s>>>(rows, g, h, flag, gs, st, seed, gq, hq, energy);
 }
 
 }  // namespace
@@ -1437,8 +1480,8 @@ void launch_rows_max(const int32_t* rows, int n_rows, const double* g, const dou
     check(cudaGetLastError(), "rows_max launch");
 }
 
-void launch_wave_partition(const WaveCtx* ctxs, int n_ctx, int grid, cudaStream_t s) {
-    launch_pdl(wave_part_kernel, dim3(grid), dim3(kPartThreads), 0, s, "wave_part launch", ctxs, n_ctx);
+void launch_wave_partition(const WaveCtx* ctxs, int n_ctx, int grid, bool pair, cudaStream_t s) {
+    launch_pdl(pair ? wave_part_kernel<true> : wave_part_kernel<false>, dim3(grid), dim3(kPartThreads), 0, s, "wave_part launch", ctxs, n_ctx);
 }
 
 void launch_wave_tree_init(DevNode* nodes, DevSplit* splits, DevTreeState* st, WaveCtl* ctl, int n_sample_host,
@@ -1454,15 +1497,15 @@ void launch_wave_scales(DevTreeState* st, const AllScale* all, int mode, cudaStr
 
 void launch_wave_quantize(int mode, const int32_t* rows, const double* g, const double* h, const uint8_t* goss_flag,
                           double goss_scale, const DevTreeState* st, unsigned long long seed, void* gq, void* hq,
-                          int max_rows, cudaStream_t s) {
+                          unsigned long long* energy, int max_rows, cudaStream_t s) {
     const int blocks = std::max(1, std::min(1184, (max_rows + 255) / 256));
     switch (mode) {
-        case kHistExactConst: quantize_launch<kHistExactConst>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, blocks, s); break;
-        case kHistExactVar: quantize_launch<kHistExactVar>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, blocks, s); break;
-        case kHistQ16Const: quantize_launch<kHistQ16Const>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, blocks, s); break;
-        case kHistQ16Var: quantize_launch<kHistQ16Var>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, blocks, s); break;
-        case kHistQ8Const: quantize_launch<kHistQ8Const>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, blocks, s); break;
-        default: quantize_launch<kHistQ8Var>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, blocks, s); break;
+        case kHistExactConst: quantize_launch<kHistExactConst>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
+        case kHistExactVar: quantize_launch<kHistExactVar>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
+        case kHistQ16Const: quantize_launch<kHistQ16Const>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
+        case kHistQ16Var: quantize_launch<kHistQ16Var>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
+        case kHistQ8Const: quantize_launch<kHistQ8Const>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
+        default: quantize_launch<kHistQ8Var>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
     }
     check(cudaGetLastError(), "wave_quantize launch");
 }

@@ -538,215 +538,315 @@ __global__ void __launch_bounds__(kSelectThreads)
 
 // ---- PAIR stage (tree.cpp:214-281) --------------------------------------------------------
 //
-// energy: the rows' sum of g^2 (g as the tree sees it: GOSS-scaled for sampled others), one
-// fixed-point sum per candidate index (exact integer adds: the same total in any order).
-// pair: one CTA per (child, pair of its top features) when the child's best axis gain is
-// weak against that energy: the histogram of pair_bin(code1, code2) over the child's rows
-// (exact fixed-point sums of the same per-row values the main histogram adds), scanned as
-// one numeric feature with pair_l2; the child's last pair CTA to finish merges the pairs'
-// best splits with the axis split (strict '>' in pair order) into the with-pairs split.
+// A child whose best axis gain is weak against its gradient energy (the rows' sum of g^2, an
+// exact fixed-point sum that the partition makes while it moves the rows) also tries the
+// pairs of its top features: the histogram of pair_bin(code1, code2) over its rows (exact
+// fixed-point sums of the values the main histogram adds), scanned as one numeric feature
+// with pair_l2, merged with the axis split (strict '>' in pair order).
+//
+// The rows of all weak children are cut into chunks of at most kPairChunk rows, spread over
+// the grid.  A CTA adds its chunk's rows into every pair's histogram at once: a row's six
+// codes and its payload are read once for 15 pairs, and each pair costs three (per-row
+// hessians: five) 32-bit shared reductions with the 19-bit split of the main histogram.
+// Chunks are added up in global memory; the child's last chunk to finish scans the pairs, a
+// warp each, merges them and clears the sums.  Before, one CTA per (child, pair) walked all
+// of the child's rows with 64-bit shared atomics (compare-and-swap loops), after a kernel of
+// its own for the energies: 66 us of a 141 us wave at 100k x 32 rows.  The 80-tree fit there
+// went from 120.9 to 70.5 ms.
+constexpr int kPairThreads = 256;
+constexpr int kPairWarps = kPairThreads / 32;
+constexpr int kPairChunk = 8192;   // the 19-bit low sums stay below 2^32, the counts in 16 bits
+constexpr int kPairMinChunk = 512;
+constexpr int kPairLo = 19;
+constexpr int kPairTop = 6;        // pair_top_k (host-checked)
 
-struct ChildRef {
-    int ci;
-    const DevNode* N;
-    const int32_t* rows;
-    DevSplit* axis;
-    DevSplit* with_pairs;
-};
-
-__device__ __forceinline__ ChildRef child_ref(const WaveCtx& X, int src, int k) {
-    ChildRef r;
-    if (src == 0) {
-        r.ci = kRootCand;
-        r.N = X.nodes;
-        r.axis = X.splits;
-        r.with_pairs = X.splits_pair;
-    } else {
-        const int L = X.ctl->exp_leaf[k >> 1];
-        r.ci = 2 * L + (k & 1);
-        r.N = X.spec + r.ci;
-        r.axis = X.spec_split + r.ci;
-        r.with_pairs = X.spec_split_pair + r.ci;
+// The k features of largest gain in the order std::sort leaves them (tree.cpp:223-225).  When
+// each of the k largest gains is unlike all others any sort agrees; otherwise (ties, NaN)
+// libstdc++'s own order is replayed.  One warp; gains in shared memory.
+__device__ __forceinline__ void top_features(const double* gains, int n_f, int k, short* scratch, int* top) {
+    const int lane = threadIdx.x & 31;
+    bool plain = true;
+    for (int f = lane; f < n_f; f += 32) plain &= gains[f] == gains[f];
+    int chosen[kPairTop];
+#pragma unroll
+    for (int r = 0; r < kPairTop; ++r) chosen[r] = -1;
+#pragma unroll
+    for (int r = 0; r < kPairTop; ++r) {
+        if (r >= k) break;
+        unsigned long long bk = 0ull;
+        int bi = 0x7fffffff;
+        bool twice = false;  // the lane's largest gain occurs twice
+        for (int f = lane; f < n_f; f += 32) {
+            bool used = false;
+#pragma unroll
+            for (int q = 0; q < r; ++q) used |= chosen[q] == f;
+            const unsigned long long key = used ? 0ull : ordered(gains[f]);
+            twice |= key != 0ull && key == bk;
+            if (key > bk) {
+                bk = key;
+                bi = f;
+                twice = false;
+            }
+        }
+        const unsigned hi = static_cast<unsigned>(bk >> 32);
+        const unsigned th = __reduce_max_sync(0xffffffffu, hi);
+        const unsigned lo = hi == th ? static_cast<unsigned>(bk) : 0u;
+        const unsigned tl = __reduce_max_sync(0xffffffffu, lo);
+        const bool best = hi == th && lo == tl && bi != 0x7fffffff;
+        const unsigned at = __ballot_sync(0xffffffffu, best);
+        plain &= __popc(at) == 1 && !(best && twice);
+        chosen[r] = __shfl_sync(0xffffffffu, bi, at ? __ffs(at) - 1 : 0);
+        if (lane == 0) top[r] = chosen[r];
     }
-    r.rows = (r.N->buf ? X.rows1 : X.rows0) + r.N->start;
-    return r;
+    if (!__all_sync(0xffffffffu, plain)) {
+        if (lane == 0) {
+            for (int f = 0; f < n_f; ++f) scratch[f] = static_cast<short>(f);
+            libstdcxx_sort(scratch, n_f, [&](short a, short b) { return gains[a] > gains[b]; });
+            for (int r = 0; r < k; ++r) top[r] = scratch[r];
+        }
+    }
+    __syncwarp();
 }
 
-__device__ __forceinline__ int energy_shift(const DevTreeState* st) {
-    const double mg = __longlong_as_double(static_cast<long long>(st->max_abs_g_bits));
-    const double e2 = mg * mg;
-    if (!(e2 > 0.0) || st->n_sample <= 0) return 0;
-    int clog = 0;
-    while ((1ll << clog) < static_cast<long long>(st->n_sample)) ++clog;
-    return max(-1000, min(1000, 61 - (ilogb(e2) + 1) - clog));
-}
-
-constexpr int kEnergyRows = 8192;
-
-__global__ void __launch_bounds__(256) wave_energy_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx, int src) {
+template <bool kVar>
+__global__ void __launch_bounds__(kPairThreads, 2)
+    wave_pair_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx, int src) {
+    constexpr int kPlanes = kVar ? 5 : 3;  // g low, g high, (h low, h high,) counts
+    constexpr int kCells = kMaxPairs * kBins;
+    extern __shared__ __align__(16) unsigned int s_pl[];  // [kPlanes][kCells]
+    __shared__ WaveCtx s_ctx;
+    __shared__ int s_pref[kMaxWaveCtx + 1];
+    __shared__ int s_count[kPairThreads], s_chunk0[kPairThreads + 1], s_wsum[kPairWarps];
+    __shared__ double s_gains[kMaxPairFeatures];
+    __shared__ short s_sort[kMaxPairFeatures];
+    __shared__ int s_top[kPairTop], s_last;
+    __shared__ Cand s_best[kMaxPairs];
+    stage_ctx(s_ctx, ctxs);
+    for (int q = threadIdx.x; q < kPlanes * kCells / 4; q += kPairThreads)
+        reinterpret_cast<uint4*>(s_pl)[q] = make_uint4(0, 0, 0, 0);
+    __syncthreads();
     pdl_wait();
     pdl_trigger();
-    __shared__ int s_pref[kMaxWaveCtx + 1];
-    __shared__ unsigned long long s_red[8];
+    auto ctx_of = [&](int c) -> const WaveCtx& { return c == 0 ? s_ctx : ctxs[c]; };
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     children_prefix(ctxs, n_ctx, src, s_pref);
     const int total = s_pref[n_ctx];
-    for (int j = blockIdx.y; j < total; j += gridDim.y) {
-        int c = 0;
-        while (c + 1 < n_ctx && s_pref[c + 1] <= j) ++c;
-        const WaveCtx& X = ctxs[c];
-        if (!X.pair_on) continue;
-        const ChildRef cr = child_ref(X, src, j - s_pref[c]);
-        const GrowParams& p = X.gp;
-        if (cr.N->depth >= p.max_depth || cr.N->count < 2 * p.min_samples_leaf) continue;
-        const double scale = ldexp(1.0, energy_shift(X.st));
-        const int count = cr.N->count;
-        for (int r0 = blockIdx.x * kEnergyRows; r0 < count; r0 += gridDim.x * kEnergyRows) {
-            unsigned long long acc = 0;
-            const int r1 = min(count, r0 + kEnergyRows);
-            for (int i = r0 + threadIdx.x; i < r1; i += blockDim.x) {
-                const int r = cr.rows[i];
-                double gv = X.g[r];
-                if (X.goss_flag != nullptr && X.goss_flag[r] == 2) gv *= X.goss_scale;
-                acc += static_cast<unsigned long long>(__double2ll_rn(gv * gv * scale));
+    for (int j0 = 0; j0 < total; j0 += kPairThreads) {
+        // a thread per child: its rows when it is weak
+        int c = 0, cnt = 0;
+        const int j = j0 + static_cast<int>(threadIdx.x);
+        if (j < total) {
+            while (c + 1 < n_ctx && s_pref[c + 1] <= j) ++c;
+            const WaveCtx& X = ctx_of(c);
+            if (X.pair_on) {
+                const WaveChild t = scan_child(X, src, j - s_pref[c]);
+                const DevNode* N = child_node(X, src, t.ci);
+                const DevSplit* axis = child_split(X, src, t.ci);
+                const double axis_gain = axis->valid ? axis->gain : -1e300;
+                const double energy = static_cast<double>(X.energy[t.ci]) * ldexp(1.0, -energy_shift(X.st));
+                const bool weak = t.eligible && X.gp.n_features >= 2 && X.pair_top_k >= 2 &&
+                                  ((axis_gain < X.pair_trigger * fmax(energy * 0.01, 1e-12)) || axis_gain <= 0);
+                if (weak) cnt = N->count;
+                else if (j % static_cast<int>(gridDim.x) == static_cast<int>(blockIdx.x))
+                    *(src == 0 ? X.splits_pair : X.spec_split_pair + t.ci) = *axis;  // no pair search
             }
+        }
+        // chunks of the batch's weak children
+        int sum = cnt;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = acc;
+        for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+        __syncthreads();  // the previous batch is done
+        if (lane == 0) s_wsum[warp] = sum;
+        s_count[threadIdx.x] = cnt;
+        __syncthreads();
+        long long all = 0;
+#pragma unroll
+        for (int w = 0; w < kPairWarps; ++w) all += s_wsum[w];
+        if (all == 0) continue;
+        const long long per = (all + gridDim.x - 1) / gridDim.x;
+        const int chunk = static_cast<int>(
+            min(static_cast<long long>(kPairChunk), max(static_cast<long long>(kPairMinChunk), (per + 255) / 256 * 256)));
+        const int nch = (cnt + chunk - 1) / chunk;
+        int incl = nch;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+        }
+        __syncthreads();  // every thread has read s_wsum
+        if (lane == 31) s_wsum[warp] = incl;
+        __syncthreads();
+        int before = 0, tasks = 0;
+#pragma unroll
+        for (int w = 0; w < kPairWarps; ++w) {
+            if (w < warp) before += s_wsum[w];
+            tasks += s_wsum[w];
+        }
+        s_chunk0[threadIdx.x] = before + incl - nch;
+        if (threadIdx.x == 0) s_chunk0[kPairThreads] = tasks;
+        __syncthreads();
+        for (int task = blockIdx.x; task < tasks; task += gridDim.x) {
+            int lo = 0, hi = kPairThreads - 1;  // the last child that starts at or before the task
+            while (lo < hi) {
+                const int mid = (lo + hi + 1) >> 1;
+                if (s_chunk0[mid] <= task) lo = mid;
+                else hi = mid - 1;
+            }
+            const int jj = j0 + lo, n_chunks = s_chunk0[lo + 1] - s_chunk0[lo];
+            int cc = 0;
+            while (cc + 1 < n_ctx && s_pref[cc + 1] <= jj) ++cc;
+            const WaveCtx& X = ctx_of(cc);
+            const GrowParams& p = X.gp;
+            const int k_child = jj - s_pref[cc], n_f = p.n_features;
+            const WaveChild t = scan_child(X, src, k_child);
+            const DevNode* N = child_node(X, src, t.ci);
+            const int buf = N->buf, start = N->start;
+            const int k = min(min(X.pair_top_k, kPairTop), n_f), n_pairs = k * (k - 1) / 2;
+            for (int f = threadIdx.x; f < n_f; f += kPairThreads)
+                s_gains[f] = X.cand_gain[static_cast<size_t>(t.ci) * n_f + f];
+            __syncthreads();
+            if (warp == 0) top_features(s_gains, n_f, k, s_sort, s_top);
+            __syncthreads();
+            const uint8_t* col[kPairTop];
+#pragma unroll
+            for (int a = 0; a < kPairTop; ++a)
+                col[a] = X.codes_col + static_cast<size_t>(s_top[a < k ? a : 0]) * X.col_pitch;
+            const int32_t* rows = (buf ? X.rows1 : X.rows0) + start;
+            const long long pos0 = static_cast<long long>(buf) * X.pay_pitch + start;
+            const long long* gpay = static_cast<const long long*>(X.gq) + pos0;
+            const long long* hpay = kVar ? static_cast<const long long*>(X.hq) + pos0 : nullptr;
+            // x mod n_bins for 32-bit x: the quotient by floor(2^32 / n_bins) is at most one short
+            const unsigned nb = static_cast<unsigned>(p.n_bins);
+            const unsigned inv = nb > 1u ? static_cast<unsigned>(0x100000000ull / nb) : 0u;
+            const int r0 = (task - s_chunk0[lo]) * chunk, r1 = min(s_count[lo], r0 + chunk);
+            for (int i = r0 + static_cast<int>(threadIdx.x); i < r1; i += kPairThreads) {
+                const int r = rows[i];
+                const long long gv = gpay[i];
+                const long long hv = kVar ? hpay[i] : 0;
+                unsigned cd[kPairTop];
+#pragma unroll
+                for (int a = 0; a < kPairTop; ++a) cd[a] = a < k ? col[a][r] : 0u;
+                const long long v = kVar ? gv : gv >> 1;
+                const unsigned g_lo = static_cast<unsigned>(v) & ((1u << kPairLo) - 1u);
+                const unsigned g_hi = static_cast<unsigned>(static_cast<int>(v >> kPairLo));
+                const unsigned h_lo = static_cast<unsigned>(hv) & ((1u << kPairLo) - 1u);
+                const unsigned h_hi = static_cast<unsigned>(static_cast<int>(hv >> kPairLo));
+                const unsigned one = kVar ? 1u : (gv & 1) ? 0x10000u : 1u;
+                unsigned* P = s_pl;
+#pragma unroll
+                for (int a = 0; a < kPairTop; ++a)
+#pragma unroll
+                    for (int b = a + 1; b < kPairTop; ++b) {
+                        if (b >= k) continue;
+                        const unsigned x = cd[a] * 2654435761u + cd[b] * 40503u;  // pair_bin
+                        unsigned z = x - __umulhi(x, inv) * nb;
+                        if (z >= nb) z -= nb;
+                        if (nb == 1u) z = 0u;
+                        atomicAdd(&P[z], g_lo);
+                        atomicAdd(&P[kCells + z], g_hi);
+                        if constexpr (kVar) {
+                            atomicAdd(&P[2 * kCells + z], h_lo);
+                            atomicAdd(&P[3 * kCells + z], h_hi);
+                        }
+                        atomicAdd(&P[(kPlanes - 1) * kCells + z], one);
+                        P += kBins;
+                    }
+            }
+            __syncthreads();
+            // add the chunk to the child's sums and clear the planes
+            const unsigned long long hq1 = static_cast<unsigned long long>(__double2ll_rn(1.0 * X.st->hscale));
+            const unsigned long long hq2 =
+                static_cast<unsigned long long>(__double2ll_rn(1.0 * X.goss_scale * X.st->hscale));
+            const size_t base = static_cast<size_t>(k_child) * kCells;
+            for (int q = threadIdx.x; q < n_pairs * kBins; q += kPairThreads) {
+                const unsigned cn = s_pl[(kPlanes - 1) * kCells + q];
+                if (cn == 0u) continue;
+                const long long gs = static_cast<long long>(static_cast<int>(s_pl[kCells + q])) * (1ll << kPairLo) + s_pl[q];
+                unsigned long long hs;
+                unsigned n = cn;
+                if constexpr (kVar) {
+                    hs = static_cast<unsigned long long>(
+                        static_cast<long long>(static_cast<int>(s_pl[3 * kCells + q])) * (1ll << kPairLo) + s_pl[2 * kCells + q]);
+                } else {
+                    hs = static_cast<unsigned long long>(cn & 0xffffu) * hq1 + static_cast<unsigned long long>(cn >> 16) * hq2;
+                    n = (cn & 0xffffu) + (cn >> 16);
+                }
+                atomicAdd(&X.pair_G[base + q], static_cast<unsigned long long>(gs));
+                atomicAdd(&X.pair_H[base + q], hs);
+                atomicAdd(&X.pair_C[base + q], static_cast<int>(n));
+#pragma unroll
+                for (int pl = 0; pl < kPlanes; ++pl) s_pl[pl * kCells + q] = 0u;
+            }
+            __threadfence();
             __syncthreads();
             if (threadIdx.x == 0) {
-                unsigned long long t = 0;
-                for (int w = 0; w < 8; ++w) t += s_red[w];
-                atomicAdd(&X.energy[cr.ci], t);
+                s_last = atomicAdd(&X.pair_tickets[t.ci], 1) == n_chunks - 1;
+                __threadfence();
             }
             __syncthreads();
+            if (!s_last) continue;
+            // the child's last chunk: scan the pairs, a warp each
+            for (int q = warp; q < n_pairs; q += kPairWarps) {
+                const size_t o = base + static_cast<size_t>(q) * kBins;
+                long long Gt, Ht, Ct;
+                const Cand cd =
+                    scan_feature_warp(reinterpret_cast<long long*>(X.pair_G) + o, reinterpret_cast<long long*>(X.pair_H) + o,
+                                      X.pair_C + o, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, false, true, 0,
+                                      p.n_bins, X.st->inv_gscale, X.st->inv_hscale, X.pair_l2, p.min_split_gain,
+                                      p.min_samples_leaf, p.min_child_weight, Gt, Ht, Ct);
+                if (lane == 0) s_best[q] = cd;
+            }
+            __syncthreads();
+            for (int q = threadIdx.x; q < n_pairs * kBins; q += kPairThreads) {
+                X.pair_G[base + q] = 0ull;
+                X.pair_H[base + q] = 0ull;
+                X.pair_C[base + q] = 0;
+            }
+            if (threadIdx.x == 0) {
+                const DevSplit axis = *child_split(X, src, t.ci);
+                DevSplit best = axis;
+                double bg = axis.valid ? axis.gain : -1e300;
+                int q = 0;
+                for (int a = 0; a < k; ++a)
+                    for (int b = a + 1; b < k; ++b, ++q) {
+                        const Cand cd = s_best[q];
+                        if (cd.key == 0x7fffffff || !(cd.gain > bg)) continue;
+                        bg = cd.gain;
+                        best = DevSplit{};
+                        best.gain = cd.gain;
+                        best.valid = cd.gain >= p.min_split_gain;
+                        best.feature = s_top[a];
+                        best.feature2 = s_top[b];
+                        best.type = 1;
+                        best.threshold = (cd.key % 512) / 2;
+                        best.missing_left = cd.key & 1;
+                    }
+                *(src == 0 ? X.splits_pair : X.spec_split_pair + t.ci) = best;
+                X.pair_tickets[t.ci] = 0;
+            }
+            __syncthreads();  // shared state reuse
         }
     }
 }
 
-__global__ void __launch_bounds__(kScanThreads) wave_pair_kernel(const WaveCtx* __restrict__ ctxs, int n_ctx, int src) {
-    pdl_wait();
-    pdl_trigger();
-    __shared__ int s_pref[kMaxWaveCtx + 1];
-    __shared__ ScanShared sm;
-    __shared__ unsigned long long sG[kBins], sH[kBins];
-    __shared__ int sC[kBins];
-    __shared__ short s_top[kMaxPairFeatures];
-    __shared__ int last;
-    children_prefix(ctxs, n_ctx, src, s_pref);
-    const int total = s_pref[n_ctx];
-    const int pi = blockIdx.x;
-    for (int j = blockIdx.y; j < total; j += gridDim.y) {
-        int c = 0;
-        while (c + 1 < n_ctx && s_pref[c + 1] <= j) ++c;
-        const WaveCtx& X = ctxs[c];
-        if (!X.pair_on) continue;
-        const ChildRef cr = child_ref(X, src, j - s_pref[c]);
-        const GrowParams& p = X.gp;
-        const int n_f = p.n_features;
-        const bool eligible = cr.N->depth < p.max_depth && cr.N->count >= 2 * p.min_samples_leaf;
-        const DevSplit axis = *cr.axis;
-        const double axis_gain = axis.valid ? axis.gain : -1e300;
-        const double energy = static_cast<double>(X.energy[cr.ci]) * ldexp(1.0, -energy_shift(X.st));
-        const bool weak = eligible && n_f >= 2 &&
-                          ((axis_gain < X.pair_trigger * fmax(energy * 0.01, 1e-12)) || axis_gain <= 0);
-        const int k = min(X.pair_top_k, n_f);
-        const int n_pairs = weak ? k * (k - 1) / 2 : 0;
-        if (n_pairs == 0) {
-            if (pi == 0 && threadIdx.x == 0) *cr.with_pairs = axis;  // no pair search for this child
-            continue;
-        }
-        if (pi >= n_pairs) continue;
-        // top-k features by their best gain, std::sort's order (tree.cpp:223-225)
-        if (threadIdx.x == 0) {
-            for (int f = 0; f < n_f; ++f) s_top[f] = static_cast<short>(f);
-            const double* gains = X.cand_gain + static_cast<size_t>(cr.ci) * n_f;
-            libstdcxx_sort(s_top, n_f, [&](short a, short b) { return gains[a] > gains[b]; });
-        }
-        for (int q = threadIdx.x; q < kBins; q += blockDim.x) {
-            sG[q] = sH[q] = 0ull;
-            sC[q] = 0;
-        }
-        __syncthreads();
-        int a = 0, rem = pi;
-        while (rem >= k - 1 - a) {
-            rem -= k - 1 - a;
-            ++a;
-        }
-        const int f1 = s_top[a], f2 = s_top[a + 1 + rem];
-        const uint8_t* c1 = X.codes_col + static_cast<size_t>(f1) * X.col_pitch;
-        const uint8_t* c2 = X.codes_col + static_cast<size_t>(f2) * X.col_pitch;
-        const bool var = X.hq != nullptr;
-        // payloads by position (exact modes: 8-byte words), like the child's rows
-        const long long pos0 = static_cast<long long>(cr.N->buf) * X.pay_pitch + cr.N->start;
-        const long long* gpay = static_cast<const long long*>(X.gq) + pos0;
-        const long long* hpay = var ? static_cast<const long long*>(X.hq) + pos0 : nullptr;
-        const unsigned long long hq1 = static_cast<unsigned long long>(__double2ll_rn(1.0 * X.st->hscale));
-        const unsigned long long hq2 = static_cast<unsigned long long>(__double2ll_rn(1.0 * X.goss_scale * X.st->hscale));
-        const int count = cr.N->count;
-        for (int i = threadIdx.x; i < count; i += blockDim.x) {
-            const int r = cr.rows[i];
-            const unsigned z = pair_bin(c1[r], c2[r], p.n_bins);
-            unsigned long long gv, hv;
-            if (var) {
-                gv = static_cast<unsigned long long>(gpay[i]);
-                hv = static_cast<unsigned long long>(hpay[i]);
-            } else {
-                const long long pk = gpay[i];
-                gv = static_cast<unsigned long long>(pk >> 1);
-                hv = (pk & 1) ? hq2 : hq1;
-            }
-            atomicAdd(&sG[z], gv);
-            atomicAdd(&sH[z], hv);
-            atomicAdd(&sC[z], 1);
-        }
-        __syncthreads();
-        long long Gt, Ht, Ct;
-        const Cand cd = scan_feature(reinterpret_cast<long long*>(sG), reinterpret_cast<long long*>(sH), sC, nullptr,
-                                     nullptr, nullptr, nullptr, nullptr, nullptr, false, true, 0, p.n_bins,
-                                     X.st->inv_gscale, X.st->inv_hscale, X.pair_l2, p.min_split_gain,
-                                     p.min_samples_leaf, p.min_child_weight, sm, Gt, Ht, Ct);
-        if (threadIdx.x == 0) {
-            DevSplit ps{};
-            ps.gain = cd.gain;
-            ps.valid = cd.key != 0x7fffffff;  // found; min_split_gain is applied at the merge
-            ps.feature = f1;
-            ps.feature2 = f2;
-            ps.type = 1;
-            ps.threshold = ps.valid ? (cd.key % 512) / 2 : -1;
-            ps.missing_left = ps.valid ? (cd.key & 1) : 1;
-            X.pair_cand[static_cast<size_t>(cr.ci) * kMaxPairs + pi] = ps;
-            __threadfence();
-            last = atomicAdd(&X.pair_tickets[cr.ci], 1) == n_pairs - 1;
-        }
-        __syncthreads();
-        if (last && threadIdx.x == 0) {
-            __threadfence();
-            DevSplit best = axis;
-            double bg = axis_gain;
-            for (int q = 0; q < n_pairs; ++q) {
-                DevSplit pc;
-                const volatile int* src_w =
-                    reinterpret_cast<const volatile int*>(X.pair_cand + static_cast<size_t>(cr.ci) * kMaxPairs + q);
-                int* dst_w = reinterpret_cast<int*>(&pc);
-                for (int w = 0; w < static_cast<int>(sizeof(DevSplit) / 4); ++w) dst_w[w] = src_w[w];
-                if (pc.valid && pc.gain > bg) {
-                    bg = pc.gain;
-                    best = pc;
-                    best.valid = pc.gain >= p.min_split_gain;
-                }
-            }
-            *cr.with_pairs = best;
-            X.pair_tickets[cr.ci] = 0;
-        }
-        __syncthreads();
-    }
-}
+constexpr size_t pair_smem(bool var) { return static_cast<size_t>(var ? 5 : 3) * kMaxPairs * kBins * 4; }
 
 }  // namespace
 
-void launch_wave_pair(const WaveCtx* ctxs, int n_ctx, int src, cudaStream_t s) {
-    launch_pdl(wave_energy_kernel, dim3(16, 32), dim3(256), 0, s, "wave_energy launch", ctxs, n_ctx, src);
-    launch_pdl(wave_pair_kernel, dim3(kMaxPairs, 32), dim3(kScanThreads), 0, s, "wave_pair launch", ctxs, n_ctx, src);
+void prepare_wave_pair() {
+    check(cudaFuncSetAttribute(wave_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(pair_smem(false))), "wave_pair smem attr");
+    check(cudaFuncSetAttribute(wave_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(pair_smem(true))), "wave_pair smem attr");
+}
+
+void launch_wave_pair(const WaveCtx* ctxs, int n_ctx, int src, bool var, cudaStream_t s) {
+    const dim3 grid(148 * 2);  // co-resident by registers
+    if (var)
+        launch_pdl(wave_pair_kernel<true>, grid, dim3(kPairThreads), pair_smem(true), s, "wave_pair launch", ctxs, n_ctx, src);
+    else
+        launch_pdl(wave_pair_kernel<false>, grid, dim3(kPairThreads), pair_smem(false), s, "wave_pair launch", ctxs, n_ctx,
+                   src);
 }
 
 void launch_wave_scan(const WaveCtx* ctxs, int n_ctx, int src, int max_f, int ys, bool any_cat, cudaStream_t s) {

@@ -155,7 +155,7 @@ struct WaveCtx {
     // histogram of the hashed code pair; splits_pair / spec_split_pair hold the best split
     // with those pairs (the split a leaf takes while the tree's pair budget lasts), splits /
     // spec_split the one without.  energy: per candidate index, fixed point (2^-energy_shift
-    // of the rows' sum of g^2); pair_cand: per candidate index and pair, the pair's best.
+    // of the rows' sum of g^2).
     int pair_on;
     int pair_top_k;
     int max_pair;
@@ -167,12 +167,26 @@ struct WaveCtx {
     DevSplit* splits_pair;
     DevSplit* spec_split_pair;
     unsigned long long* energy;  // [2 * kMaxNodes + 1]
-    DevSplit* pair_cand;         // [(2 * kMaxNodes + 1)][kMaxPairs]
-    int* pair_tickets;           // [2 * kMaxNodes + 1], zero between launches
+    // pair histograms of the wave's children, [pair_children][kMaxPairs][kBins] each, and the
+    // chunks done per candidate index [2 * kMaxNodes + 1]; all zero between launches
+    unsigned long long* pair_G;
+    unsigned long long* pair_H;
+    int* pair_C;
+    int* pair_tickets;
 };
 constexpr int kMaxPairs = 15;  // pairs of the top pair_top_k <= 6 features
 
 #if defined(__CUDACC__)
+// The fixed-point shift of the gradient energies: no sum over the sample reaches 2^62.
+__device__ __forceinline__ int energy_shift(const DevTreeState* st) {
+    const double mg = __longlong_as_double(static_cast<long long>(st->max_abs_g_bits));
+    const double e2 = mg * mg;
+    const int n = st->n_sample;
+    if (!(e2 > 0.0) || n <= 0) return 0;
+    const int clog = n > 1 ? 32 - __clz(n - 1) : 0;
+    return max(-1000, min(1000, 61 - (ilogb(e2) + 1) - clog));
+}
+
 // Copies the first context into shared memory (the caller synchronises the CTA).  The
 // contexts are written before the fit's first tree and do not change, so a wave kernel does
 // this before pdl_wait: its later reads of pointers and parameters then cost no memory
@@ -185,6 +199,12 @@ __device__ __forceinline__ void stage_ctx(WaveCtx& to, const WaveCtx* ctxs) {
 }
 #endif
 
+// Children a wave may hold (two per planned expansion; at least the root).
+inline int wave_children(int max_leaves, int max_expand) {
+    const int e = max_leaves - 1;
+    return 2 * (max_expand > 0 && max_expand < e ? max_expand : e);
+}
+
 // Per-tree set-up of one context: root node (all sampled rows, slot 0), control reset.
 // use_dev_count: the sample size is st->n_sample (GOSS), else n_sample_host.
 void launch_wave_tree_init(DevNode* nodes, DevSplit* splits, DevTreeState* st, WaveCtl* ctl, int n_sample_host,
@@ -193,9 +213,10 @@ void launch_wave_tree_init(DevNode* nodes, DevSplit* splits, DevTreeState* st, W
 // sample is every row, the all-row maxima (all).
 void launch_wave_scales(DevTreeState* st, const AllScale* all, int mode, cudaStream_t s);
 // Payload of the sampled rows for `mode` (rows0[0 .. st->n_sample)), by position in rows0.
+// energy (PAIR, else nullptr; zeroed by the caller): the root's gradient energy.
 void launch_wave_quantize(int mode, const int32_t* rows, const double* g, const double* h, const uint8_t* goss_flag,
                           double goss_scale, const DevTreeState* st, unsigned long long seed, void* gq, void* hq,
-                          int max_rows, cudaStream_t s);
+                          unsigned long long* energy, int max_rows, cudaStream_t s);
 
 // Wave launches over n_ctx contexts (ctxs: device array).  src 0: the roots, src 1: the
 // expansions planned by the last select.
@@ -218,11 +239,12 @@ void launch_wave_scan(const WaveCtx* ctxs, int n_ctx, int src, int max_f, int ys
 // cond / use_cond: the graph's loop condition (set to "any context still growing").
 void launch_wave_select(const WaveCtx* ctxs, int n_ctx, int* gsync, unsigned* host_flag,
                         unsigned long long cond, int use_cond, cudaStream_t s);
-void launch_wave_partition(const WaveCtx* ctxs, int n_ctx, int grid, cudaStream_t s);
-// PAIR stage after a scan (contexts with pair_on): the children's (or roots') gradient
-// energy, then for the weak ones the pair histograms and their best splits, merged into
-// spec_split_pair (roots: splits_pair[0]).
-void launch_wave_pair(const WaveCtx* ctxs, int n_ctx, int src, cudaStream_t s);
+void launch_wave_partition(const WaveCtx* ctxs, int n_ctx, int grid, bool pair, cudaStream_t s);
+// PAIR stage after a scan (contexts with pair_on): for the children (or roots) whose best
+// axis gain is weak against their gradient energy the pair histograms and their best
+// splits, merged into spec_split_pair (roots: splits_pair[0]).  var: per-row hessians.
+void launch_wave_pair(const WaveCtx* ctxs, int n_ctx, int src, bool var, cudaStream_t s);
+void prepare_wave_pair();  // its shared-memory opt-in, once per device (not inside a capture)
 // sc->maxg_bits / maxh_bits <- max |g[rows]| and max h[rows] (h == nullptr: 1); sc zeroed.
 void launch_rows_max(const int32_t* rows, int n_rows, const double* g, const double* h, AllScale* sc,
                      cudaStream_t s);
