@@ -8,12 +8,19 @@
 // compare gives the reference's f64 upper_bound exactly.  f64 input compares against f64
 // edges.
 //
-// Launch shape: one CTA = 8 warps x a group of 32 features; lane = feature, so a
-// warp reads one row's 32 consecutive values (coalesced) and writes 32 code bytes.
-// Edges of the group sit in shared memory with a 257-element feature stride so the
-// first probes of the 32 lanes fall in 32 different banks.
+// Launch shape: one CTA = 8 warps x a group of at most 32 features, and as many CTAs as the
+// chip holds at once, each over one contiguous share of the rows (the group's edges are
+// staged once per CTA).  A lane owns a feature; a group of fewer features gives a warp
+// several rows at a time.  The group's edges sit in shared memory as [edge][lane], so a
+// lane only ever reads its own bank: the bisection's probes of a warp are one wavefront each
+// whatever the values are.  (With [feature][edge] rows the 32 probes of a step fell on random
+// banks, 3.4 deep on average, one row at a time: 2,513 us for 4M x 128 float32.)  Eight rows
+// are searched together while the next eight load, and the first two of the eight steps
+// compare with edges held in registers, so a value costs six shared loads, compares and
+// predicated adds: 805 us there, bound by instruction issue (its bytes take 396 us).
 #include "tgb_internal.h"
 
+#include <atomic>
 #include <cmath>
 
 namespace tgb {
@@ -21,79 +28,177 @@ namespace tgb {
 namespace {
 
 constexpr int kBinWarps = 8;
-constexpr int kEdgeStride = 257;
+constexpr int kBinThreads = kBinWarps * 32;
+constexpr int kBinRows = 8;  // rows a lane searches together
+// CTAs per SM: 64 registers a thread, or 64 KB of double edges
+constexpr int kBinCtas32 = 4, kBinCtas64 = 3;
+
+// std::upper_bound's own bisection (libstdc++ __upper_bound) over edge k at e[32 k]: the same
+// probes and the same answer as the reference, also when NaN edges break the order.
+template <typename T>
+__device__ __forceinline__ int upper_bound_exact(const T* e, int ne, T v) {
+    int first = 0, len = ne;
+    while (len > 0) {
+        const int half = len >> 1;
+        const int mid = first + half;
+        if (v < e[32 * mid]) {
+            len = half;
+        } else {
+            first = mid + 1;
+            len = len - half - 1;
+        }
+    }
+    return first;
+}
+
+// Categorical (binning.cpp:112-117): 1 + the value's index in the sorted vocabulary
+// (std::lower_bound's bisection), 0 when it is not in it.
+template <typename T>
+__device__ __forceinline__ int vocabulary_code(const T* e, int ne, T v) {
+    int first = 0, len = ne;
+    while (len > 0) {
+        const int half = len >> 1;
+        const int mid = first + half;
+        if (e[32 * mid] < v) {
+            first = mid + 1;
+            len = len - half - 1;
+        } else {
+            len = half;
+        }
+    }
+    return (first < ne && e[32 * first] == v) ? first + 1 : 0;
+}
+
+// The edge at shared address p + k rows of 32 (the offset is an immediate of the load).
+template <int k>
+__device__ __forceinline__ float edge_at(unsigned p, float) {
+    float v;
+    asm volatile("ld.shared.f32 %0, [%1 + %2];" : "=f"(v) : "r"(p), "n"(k * 128));
+    return v;
+}
+template <int k>
+__device__ __forceinline__ double edge_at(unsigned p, double) {
+    double v;
+    asm volatile("ld.shared.f64 %0, [%1 + %2];" : "=d"(v) : "r"(p), "n"(k * 256));
+    return v;
+}
+// p += k unless v < e, as one compare and one predicated add.
+template <unsigned k>
+__device__ __forceinline__ void advance(unsigned& p, float v, float e) {
+    asm("{ .reg .pred t; setp.geu.f32 t, %1, %2; @t add.u32 %0, %0, %3; }" : "+r"(p) : "f"(v), "f"(e), "n"(k));
+}
+template <unsigned k>
+__device__ __forceinline__ void advance(unsigned& p, double v, double e) {
+    asm("{ .reg .pred t; setp.geu.f64 t, %1, %2; @t add.u32 %0, %0, %3; }" : "+r"(p) : "d"(v), "d"(e), "n"(k));
+}
+// One halving step of kBinRows searches: p is the shared address of the first edge not yet
+// known to be <= v.
+template <int h, typename T>
+__device__ __forceinline__ void halve(unsigned (&p)[kBinRows], const T (&v)[kBinRows]) {
+    T e[kBinRows];
+#pragma unroll
+    for (int q = 0; q < kBinRows; ++q) e[q] = edge_at<h - 1>(p[q], v[q]);
+#pragma unroll
+    for (int q = 0; q < kBinRows; ++q) advance<h * 32 * sizeof(T)>(p[q], v[q], e[q]);
+}
 
 template <typename T>
-__global__ void __launch_bounds__(kBinWarps * 32)
+__global__ void __launch_bounds__(kBinThreads, sizeof(T) == 4 ? kBinCtas32 : kBinCtas64)
     bin_transform_kernel(const T* __restrict__ X, int n, int n_f, const T* __restrict__ edges,
                          const int* __restrict__ n_edges, uint8_t* __restrict__ codes, int stride,
                          int rows_per_cta, const uint8_t* __restrict__ is_cat) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* se = reinterpret_cast<T*>(smem_raw);
-    __shared__ int sne[32];
+    T* se = reinterpret_cast<T*>(smem_raw);  // [256][32]
+    __shared__ int s_plain[32];
     const int f0 = blockIdx.y * 32;
-    const int nf_here = min(32, n_f - f0);
-    for (int k = threadIdx.x; k < 32 * 256; k += blockDim.x) {
-        const int ff = k >> 8, b = k & 255;
-        T v = T(INFINITY);
-        if (ff < nf_here) v = edges[static_cast<size_t>(f0 + ff) * 256 + b];
-        se[ff * kEdgeStride + b] = v;
-    }
-    if (threadIdx.x < 32) sne[threadIdx.x] = threadIdx.x < nf_here ? n_edges[f0 + threadIdx.x] : 0;
-    __syncthreads();
+    const int nf = min(32, n_f - f0);
+    const int rpw = 32 / nf;  // rows of a warp's step
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (lane >= nf_here) return;
-    const T* e = se + lane * kEdgeStride;
-    const int ne = sne[lane];
-    const bool cat = is_cat != nullptr && is_cat[f0 + lane] != 0;
+    const int sub = lane / nf, ff = lane - sub * nf;
+    const bool active = sub < rpw;
+    const int f = f0 + ff;
+    const int ne = n_edges[f];
+    {
+        const T* ef = edges + static_cast<size_t>(f) * 256;
+#pragma unroll 1
+        for (int b0 = warp; b0 < 256; b0 += 16 * kBinWarps) {
+            T v[16];
+#pragma unroll
+            for (int q = 0; q < 16; ++q) v[q] = b0 + q * kBinWarps < ne ? ef[b0 + q * kBinWarps] : T(INFINITY);
+#pragma unroll
+            for (int q = 0; q < 16; ++q) se[(b0 + q * kBinWarps) * 32 + lane] = v[q];
+        }
+    }
+    if (threadIdx.x < 32) s_plain[threadIdx.x] = ne <= 255 ? 1 : 0;
+    __syncthreads();
+    const T* e = se + lane;
+    // ascending edges without NaN: counting the edges <= v by halving steps is upper_bound
+    bool plain = true;
+#pragma unroll 8
+    for (int b = warp; b < 255; b += kBinWarps) {  // past ne the staged edges are infinite
+        const T lo = e[32 * b], hi = e[32 * (b + 1)];
+        plain &= b >= ne || (b + 1 < ne ? lo <= hi : lo == lo);
+    }
+    if (!plain) s_plain[lane] = 0;
+    __syncthreads();
+    plain = s_plain[lane] != 0;
+    const bool cat = is_cat != nullptr && is_cat[f] != 0;
     const int r0 = blockIdx.x * rows_per_cta;
     const int r1 = min(n, r0 + rows_per_cta);
-    for (int r = r0 + warp; r < r1; r += kBinWarps) {
-        const T v = X[static_cast<size_t>(r) * n_f + f0 + lane];
-        int code = 0;
-        if (cat && !(v != v)) {
-            // categorical (binning.cpp:112-117): 1 + the value's index in the sorted
-            // vocabulary (std::lower_bound's bisection), 0 when it is not in it
-            int first = 0, len = ne;
-            while (len > 0) {
-                const int half = len >> 1;
-                const int mid = first + half;
-                if (e[mid] < v) {
-                    first = mid + 1;
-                    len = len - half - 1;
-                } else {
-                    len = half;
-                }
+    const T e127 = e[32 * 127], e63 = e[32 * 63], e191 = e[32 * 191];
+    const int step = kBinWarps * rpw;
+    int r = r0 + warp * rpw + sub;
+    constexpr unsigned kRow = 32 * sizeof(T);  // bytes from one edge to the next
+    const unsigned base = static_cast<unsigned>(__cvta_generic_to_shared(e));
+    const size_t x_step = static_cast<size_t>(step) * n_f, c_step = static_cast<size_t>(step) * stride;
+    const T* x = X + static_cast<size_t>(r) * n_f + f;
+    uint8_t* out = codes + static_cast<size_t>(r) * stride + f;
+    if (active && plain && !cat) {
+        T nv[kBinRows];  // the next rows' values, loaded while these are searched
+        const bool any = r + (kBinRows - 1) * step < r1;
+#pragma unroll
+        for (int q = 0; q < kBinRows; ++q) nv[q] = any ? __ldcs(x + q * x_step) : T(0);
+        for (; r + (kBinRows - 1) * step < r1; r += kBinRows * step, out += kBinRows * c_step) {
+            T v[kBinRows];
+            unsigned p[kBinRows];
+#pragma unroll
+            for (int q = 0; q < kBinRows; ++q) v[q] = nv[q];
+            x += kBinRows * x_step;
+            const bool more = r + (2 * kBinRows - 1) * step < r1;
+#pragma unroll
+            for (int q = 0; q < kBinRows; ++q) nv[q] = more ? __ldcs(x + q * x_step) : T(0);
+#pragma unroll
+            for (int q = 0; q < kBinRows; ++q) {
+                p[q] = base;
+                advance<128 * kRow>(p[q], v[q], e127);
+                advance<64 * kRow>(p[q], v[q], v[q] < e127 ? e63 : e191);
             }
-            code = (first < ne && e[first] == v) ? first + 1 : 0;
-        } else if (!(v != v)) {
-            // std::upper_bound's own bisection (libstdc++ __upper_bound): the same probes
-            // and the same answer as the reference, also when NaN edges break the order
-            int first = 0, len = ne;
-            while (len > 0) {
-                const int half = len >> 1;
-                const int mid = first + half;
-                if (v < e[mid]) {
-                    len = half;
-                } else {
-                    first = mid + 1;
-                    len = len - half - 1;
-                }
+            halve<32>(p, v);
+            halve<16>(p, v);
+            halve<8>(p, v);
+            halve<4>(p, v);
+            halve<2>(p, v);
+            halve<1>(p, v);
+#pragma unroll
+            for (int q = 0; q < kBinRows; ++q) {
+                const int code = min(static_cast<int>((p[q] - base) / kRow), ne) + 1;
+                out[q * c_step] = static_cast<uint8_t>(v[q] != v[q] ? 0 : code);  // NaN -> 0
             }
-            code = first + 1;
         }
-        codes[static_cast<size_t>(r) * stride + f0 + lane] = static_cast<uint8_t>(code);
     }
-}
-
-// Zero the padding bytes [n_f, stride) of every row so gathers of whole rows see 0.
-__global__ void zero_pad_kernel(uint8_t* codes, int n, int n_f, int stride) {
+    if (active) {  // the last rows of a plain feature, all rows of the others
+        for (; r < r1; r += step, x += x_step, out += c_step) {
+            const T v = *x;
+            const int code = cat ? vocabulary_code(e, ne, v) : upper_bound_exact(e, ne, v) + 1;
+            *out = static_cast<uint8_t>(v != v ? 0 : code);
+        }
+    }
+    // Zero the padding bytes [n_f, stride) so gathers of whole rows see 0.
     const int pad = stride - n_f;
-    const size_t total = static_cast<size_t>(n) * pad;
-    for (size_t k = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x; k < total;
-         k += static_cast<size_t>(gridDim.x) * blockDim.x) {
-        const size_t r = k / pad;
-        codes[r * stride + n_f + (k % pad)] = 0;
+    if (pad > 0 && blockIdx.y == gridDim.y - 1) {
+        const long long total = static_cast<long long>(r1 - r0) * pad;
+        for (long long k = threadIdx.x; k < total; k += kBinThreads)
+            codes[static_cast<size_t>(r0 + k / pad) * stride + n_f + k % pad] = 0;
     }
 }
 
@@ -136,18 +241,26 @@ template <typename T>
 void launch_bin(const T* X, int n, int n_f, const T* edges, const int* n_edges, uint8_t* codes,
                 int stride, cudaStream_t s, const uint8_t* is_cat) {
     if (n <= 0 || n_f <= 0) return;
-    const int rows_per_cta = 512;
-    dim3 grid((n + rows_per_cta - 1) / rows_per_cta, (n_f + 31) / 32);
-    const size_t smem = sizeof(T) * 32 * kEdgeStride;
+    const int groups = (n_f + 31) / 32;
+    const size_t smem = sizeof(T) * 32 * 256;
     auto kern = bin_transform_kernel<T>;
-    check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-          "bin smem attr");
-    kern<<<grid, kBinWarps * 32, smem, s>>>(X, n, n_f, edges, n_edges, codes, stride, rows_per_cta, is_cat);
-    check(cudaGetLastError(), "bin_transform launch");
-    if (stride > n_f) {
-        zero_pad_kernel<<<1184, 256, 0, s>>>(codes, n, n_f, stride);
-        check(cudaGetLastError(), "zero_pad launch");
+    // every CTA resident at once, of at least one step of all warps
+    const int ctas = std::max(1, 148 * (sizeof(T) == 4 ? kBinCtas32 : kBinCtas64) / groups);
+    const int min_rows = kBinWarps * kBinRows;
+    const int rows_per_cta = std::max(min_rows, (n + ctas - 1) / ctas);
+    {
+        static std::atomic<bool> done[64] = {};
+        int dev = 0;
+        check(cudaGetDevice(&dev), "cudaGetDevice");
+        if (dev < 0 || dev >= 64 || !done[dev]) {
+            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
+                  "bin smem attr");
+            if (dev >= 0 && dev < 64) done[dev] = true;
+        }
     }
+    dim3 grid((n + rows_per_cta - 1) / rows_per_cta, groups);
+    kern<<<grid, kBinThreads, smem, s>>>(X, n, n_f, edges, n_edges, codes, stride, rows_per_cta, is_cat);
+    check(cudaGetLastError(), "bin_transform launch");
 }
 
 }  // namespace
