@@ -158,6 +158,17 @@ struct OwnedStream {
     }
 };
 
+struct OwnedEvent {
+    cudaEvent_t e = nullptr;
+    cudaEvent_t get() {
+        if (!e) check(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "event");
+        return e;
+    }
+    ~OwnedEvent() {
+        if (e) cudaEventDestroy(e);
+    }
+};
+
 struct DeviceState {
     OwnedStream owned;
     cudaStream_t stream = nullptr;
@@ -200,17 +211,21 @@ struct DeviceState {
     DBuf<DevSplit> splits_pair, spec_split_pair;  // PAIR search (wave.h)
     DBuf<unsigned long long> energy, pair_G, pair_H;
     DBuf<int> pair_C, pair_tickets;
-    // predict
-    DBuf<uint8_t> pcodes;
-    DBuf<int16_t> t_feat, t_left, t_right, t_feat2;
-    DBuf<uint8_t> t_type;
-    DBuf<unsigned long long> t_cat;
-    DBuf<uint8_t> t_thr, t_ml;
-    DBuf<double> t_val, pout;
-    DBuf<int> t_off;
+    // predict: the fitted model's layout (tgb_internal.h, PredictTrees), its edges in the dtype
+    // of the last prediction's X (edges_dtype; -1: none), and the copy stream of long ones
+    DBuf<unsigned long long> t_word, t_cat;
+    DBuf<double> t_val;
+    DBuf<int4> t_trees;
+    DBuf<int> t_batches, t_ne;
+    DBuf<int16_t> t_feat2;
+    DBuf<unsigned char> t_edges;
+    int n_batches = 0, edges_dtype = -1;
+    bool any_kind = false;
+    OwnedStream copy;
+    OwnedEvent ev_ready, ev_in[2], ev_used[2], ev_out[2];
     size_t trees_flat = 0;
 
-    // Everything a fit allocates; predict's buffers (pcodes, t_*, pout) stay.
+    // Everything a fit allocates; the model's layout for predict (t_*) stays.
     void release_fit_buffers() {
         codes.release(); codes_col.release(); y.release(); pred.release(); g.release(); h.release();
         gq.release(); gq8.release(); rows0.release(); rows1.release(); histG.release(); histH.release();
@@ -554,6 +569,8 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
         check(cudaStreamSynchronize(s), "X upload");
         st.t_h2d = now() - tb - st.t_alloc;
         // ---- quantile edges: Binner::fit (binning.cpp:34-102) on the uploaded X ----
+        D.trees_flat = 0;  // what predict laid out of an earlier fit no longer holds
+        D.edges_dtype = -1;
         const double tbf = now();
         BinFitTimes bt;
         if (any_cat) {
@@ -958,6 +975,7 @@ bool FitRun::finish() {
     B.cfg = c;
     B.fitted = true;
     D.trees_flat = 0;
+    D.edges_dtype = -1;
     // The fit's working buffers go back to the pool (ordered on the stream); a fitted model
     // keeps only its host-side trees and edges, and predict allocates what it needs.
     const double trl = now();
@@ -1408,6 +1426,115 @@ void GpuBooster::fit_batch(const std::vector<GpuBooster*>& bs, const std::vector
     }
 }
 
+// Lays the fitted trees out for the predict kernel (booster.cpp:744-773 uses tree.values, not
+// the TORB prefixes), once per fitted model.
+void GpuBooster::upload_model() {
+    DeviceState& D = *ds_;
+    cudaStream_t s = D.stream;
+    std::vector<unsigned long long> word, cat;
+    std::vector<double> val;
+    std::vector<int4> tr;
+    std::vector<int> batches;
+    std::vector<int16_t> f2;
+    D.any_kind = false;
+    int batch_nodes = 0, batch_trees = 0;
+    for (const auto& t : trees) {
+        const int nn = static_cast<int>(t.nodes.size());
+        if (batches.empty() || batch_nodes + nn > predict_batch_nodes() || batch_trees + 1 > predict_batch_trees()) {
+            batches.push_back(static_cast<int>(tr.size()));
+            batch_nodes = batch_trees = 0;
+        }
+        batch_nodes += nn;
+        batch_trees += 1;
+        int depth = 0;
+        const int first = static_cast<int>(word.size());
+        for (int k = 0; k < nn; ++k) {
+            const HostNode& d = t.nodes[k];
+            const bool leaf = d.is_leaf != 0;
+            const unsigned long long l = static_cast<unsigned long long>(leaf ? k : d.left);
+            const unsigned long long r = static_cast<unsigned long long>(leaf ? k : d.right);
+            const unsigned long long thr = static_cast<unsigned long long>(leaf || d.threshold < 0 ? 0 : d.threshold & 0xff);
+            const unsigned long long f = static_cast<unsigned long long>(leaf ? 0 : d.feature);
+            const unsigned long long type = static_cast<unsigned long long>(leaf ? 0 : d.type);
+            word.push_back((l & 0xffff) | (r & 0xffff) << 16 | thr << 32 | (f & 0xffff) << 40 |
+                           static_cast<unsigned long long>(d.missing_left & 1) << 56 | type << 57);
+            val.push_back(t.values[k]);
+            f2.push_back(static_cast<int16_t>(type == 1 ? d.feature2 : 0));
+            for (int q = 0; q < 4; ++q) cat.push_back(d.cat[q]);
+            D.any_kind = D.any_kind || type != 0;
+            depth = std::max(depth, d.depth);
+        }
+        tr.push_back(make_int4(first, nn, depth, 0));
+    }
+    D.n_batches = static_cast<int>(batches.size());
+    batches.push_back(static_cast<int>(tr.size()));
+    D.t_word.alloc(std::max<size_t>(1, word.size()), s);
+    D.t_cat.alloc(std::max<size_t>(4, cat.size()), s);
+    D.t_val.alloc(std::max<size_t>(1, val.size()), s);
+    D.t_trees.alloc(std::max<size_t>(1, tr.size()), s);
+    D.t_batches.alloc(batches.size(), s);
+    D.t_feat2.alloc(std::max<size_t>(1, f2.size()), s);
+    D.t_ne.alloc(n_edges.size(), s);
+    check(cudaMemcpyAsync(D.t_word.p, word.data(), 8 * word.size(), cudaMemcpyHostToDevice, s), "trees");
+    check(cudaMemcpyAsync(D.t_cat.p, cat.data(), 8 * cat.size(), cudaMemcpyHostToDevice, s), "trees");
+    check(cudaMemcpyAsync(D.t_val.p, val.data(), 8 * val.size(), cudaMemcpyHostToDevice, s), "trees");
+    check(cudaMemcpyAsync(D.t_trees.p, tr.data(), sizeof(int4) * tr.size(), cudaMemcpyHostToDevice, s), "trees");
+    check(cudaMemcpyAsync(D.t_batches.p, batches.data(), 4 * batches.size(), cudaMemcpyHostToDevice, s), "trees");
+    check(cudaMemcpyAsync(D.t_feat2.p, f2.data(), 2 * f2.size(), cudaMemcpyHostToDevice, s), "trees");
+    check(cudaMemcpyAsync(D.t_ne.p, n_edges.data(), 4 * n_edges.size(), cudaMemcpyHostToDevice, s), "trees");
+    check(cudaStreamSynchronize(s), "trees");
+    D.trees_flat = trees.size();
+}
+
+// The model's edges as the transform reads them for X of this dtype (kept until another
+// dtype or another fit).
+void GpuBooster::upload_edges(int x_dtype) {
+    DeviceState& D = *ds_;
+    cudaStream_t s = D.stream;
+    const size_t cells = static_cast<size_t>(n_features) * 256, xsz = x_dtype == 0 ? 4 : 8;
+    std::vector<float> ef(x_dtype == 0 ? cells : 0, INFINITY);
+    std::vector<double> ed(x_dtype == 0 ? 0 : cells, INFINITY);
+    for (int f = 0; f < n_features; ++f)
+        for (int k = 0; k < n_edges[f]; ++k) {
+            const size_t o = static_cast<size_t>(f) * 256 + k;
+            if (x_dtype == 0) ef[o] = ceil_f32(edges[o]);
+            else ed[o] = edges[o];
+        }
+    D.edges_dtype = -1;
+    D.t_edges.alloc(cells * xsz, s);
+    const void* src = x_dtype == 0 ? static_cast<const void*>(ef.data()) : static_cast<const void*>(ed.data());
+    check(cudaMemcpyAsync(D.t_edges.p, src, cells * xsz, cudaMemcpyHostToDevice, s), "edges");
+    check(cudaStreamSynchronize(s), "edges");
+    D.edges_dtype = x_dtype;
+}
+
+namespace {
+// Waits for a stream's copies when a prediction ends early, before its buffers go back.
+struct StreamGuard {
+    cudaStream_t s;
+    bool armed = true;
+    ~StreamGuard() {
+        if (armed && s) cudaStreamSynchronize(s);
+    }
+};
+// A pinned block of the process's bounded cache.
+struct PinnedBlock {
+    size_t bytes;
+    void* p;
+    explicit PinnedBlock(size_t b) : bytes(b), p(pinned_take(b)) {}
+    ~PinnedBlock() { pinned_give(bytes, p); }
+};
+// Bytes of X in one chunk of a long prediction: its copy hides the chunk before it, and the
+// last chunk's kernels and result copy are what remains after the upload.  Narrow rows stop at
+// a number of rows, which bounds the pinned block of the results (2 MB).
+constexpr size_t kPredictChunkBytes = 16u << 20;
+constexpr size_t kPredictChunkRows = 131072;
+}  // namespace
+
+// X in chunks: the copy stream brings chunk c + 1 while the booster's stream transforms and
+// walks chunk c, and the host moves the results of chunk c - 1 from pinned memory to `out`.
+// The call is then as long as the upload.  (One copy of everything, the two kernels and a
+// pageable result copy in a row: 9.7 ms for 1M x 64 float32, of which the upload is 4.6.)
 void GpuBooster::predict_raw(const void* X, int x_dtype, int n, int n_f, double* out) {
     if (!fitted) throw TideError("not fitted");
     if (n_f != n_features) throw TideError("n_features mismatch");
@@ -1416,89 +1543,71 @@ void GpuBooster::predict_raw(const void* X, int x_dtype, int n, int n_f, double*
     DeviceState& D = *ds_;
     cudaStream_t s = D.stream;
     const int stride = (n_f + 15) / 16 * 16;
-    const size_t xsz = x_dtype == 0 ? 4 : 8;
-    // Flattened trees (booster.cpp:744-773 uses tree.values, not the TORB prefixes).
-    if (D.trees_flat != trees.size()) {
-        std::vector<int16_t> f, l, r, f2;
-        std::vector<uint8_t> th, ml, ty;
-        std::vector<unsigned long long> cm;
-        std::vector<double> v;
-        std::vector<int> off;
-        for (const auto& t : trees) {
-            off.push_back(static_cast<int>(f.size()));
-            for (size_t k = 0; k < t.nodes.size(); ++k) {
-                const HostNode& d = t.nodes[k];
-                f.push_back(static_cast<int16_t>(d.is_leaf ? -1 : d.feature));
-                l.push_back(static_cast<int16_t>(d.left));
-                r.push_back(static_cast<int16_t>(d.right));
-                th.push_back(static_cast<uint8_t>(d.threshold < 0 ? 0 : d.threshold));
-                ml.push_back(static_cast<uint8_t>(d.missing_left));
-                ty.push_back(static_cast<uint8_t>(d.is_leaf ? 0 : d.type));
-                f2.push_back(static_cast<int16_t>(!d.is_leaf && d.type == 1 ? d.feature2 : 0));
-                for (int q = 0; q < 4; ++q) cm.push_back(d.cat[q]);
-                v.push_back(t.values[k]);
-            }
-        }
-        D.t_feat2.alloc(std::max<size_t>(1, f2.size()), s);
-        if (!f2.empty()) check(cudaMemcpyAsync(D.t_feat2.p, f2.data(), 2 * f2.size(), cudaMemcpyHostToDevice, s), "trees");
-        D.t_type.alloc(std::max<size_t>(1, ty.size()), s);
-        D.t_cat.alloc(std::max<size_t>(4, cm.size()), s);
-        if (!ty.empty()) {
-            check(cudaMemcpyAsync(D.t_type.p, ty.data(), ty.size(), cudaMemcpyHostToDevice, s), "trees");
-            check(cudaMemcpyAsync(D.t_cat.p, cm.data(), 8 * cm.size(), cudaMemcpyHostToDevice, s), "trees");
-        }
-        D.t_feat.alloc(f.size(), s);
-        D.t_left.alloc(l.size(), s);
-        D.t_right.alloc(r.size(), s);
-        D.t_thr.alloc(th.size(), s);
-        D.t_ml.alloc(ml.size(), s);
-        D.t_val.alloc(v.size(), s);
-        D.t_off.alloc(std::max<size_t>(1, off.size()), s);
-        check(cudaMemcpyAsync(D.t_feat.p, f.data(), 2 * f.size(), cudaMemcpyHostToDevice, s), "trees");
-        check(cudaMemcpyAsync(D.t_left.p, l.data(), 2 * l.size(), cudaMemcpyHostToDevice, s), "trees");
-        check(cudaMemcpyAsync(D.t_right.p, r.data(), 2 * r.size(), cudaMemcpyHostToDevice, s), "trees");
-        check(cudaMemcpyAsync(D.t_thr.p, th.data(), th.size(), cudaMemcpyHostToDevice, s), "trees");
-        check(cudaMemcpyAsync(D.t_ml.p, ml.data(), ml.size(), cudaMemcpyHostToDevice, s), "trees");
-        check(cudaMemcpyAsync(D.t_val.p, v.data(), 8 * v.size(), cudaMemcpyHostToDevice, s), "trees");
-        if (!off.empty())
-            check(cudaMemcpyAsync(D.t_off.p, off.data(), 4 * off.size(), cudaMemcpyHostToDevice, s), "trees");
-        check(cudaStreamSynchronize(s), "trees");
-        D.trees_flat = trees.size();
-    }
+    const int dtype = x_dtype == 0 ? 0 : 1;
+    const size_t row_bytes = static_cast<size_t>(n_f) * (dtype == 0 ? 4 : 8);
+    if (D.trees_flat != trees.size()) upload_model();
+    if (D.edges_dtype != dtype) upload_edges(dtype);
+    const PredictTrees m{D.t_word.p,    D.t_val.p, D.t_trees.p, D.t_batches.p, D.n_batches, D.t_cat.p,
+                         D.t_feat2.p, n_bins,    D.any_kind};
+    const int chunk = static_cast<int>(
+        std::min({static_cast<size_t>(n), kPredictChunkRows,
+                  std::max<size_t>(1024, kPredictChunkBytes / row_bytes / 1024 * 1024)}));
+    const int n_chunks = (n + chunk - 1) / chunk, slots = std::min(2, n_chunks);
     DBuf<unsigned char> Xd;
-    Xd.alloc(static_cast<size_t>(n) * n_f * xsz, s);
-    D.pcodes.alloc(static_cast<size_t>(n) * stride, s);
-    D.pout.alloc(n, s);
-    check(cudaMemcpyAsync(Xd.p, X, static_cast<size_t>(n) * n_f * xsz, cudaMemcpyHostToDevice, s), "X upload");
-    DBuf<int> ne;
-    ne.alloc(n_f, s);
-    check(cudaMemcpyAsync(ne.p, n_edges.data(), sizeof(int) * n_f, cudaMemcpyHostToDevice, s), "edges");
-    if (x_dtype == 0) {
-        std::vector<float> ef(static_cast<size_t>(n_f) * 256, INFINITY);
-        for (int ff = 0; ff < n_f; ++ff)
-            for (int k = 0; k < n_edges[ff]; ++k) ef[static_cast<size_t>(ff) * 256 + k] = ceil_f32(edges[static_cast<size_t>(ff) * 256 + k]);
-        DBuf<float> ed;
-        ed.alloc(ef.size(), s);
-        check(cudaMemcpyAsync(ed.p, ef.data(), 4 * ef.size(), cudaMemcpyHostToDevice, s), "edges");
-        launch_bin_transform_f32(reinterpret_cast<const float*>(Xd.p), n, n_f, ed.p, ne.p, D.pcodes.p, stride, s,
-                                 D.is_cat.p);
-        check(cudaStreamSynchronize(s), "transform");
-    } else {
-        std::vector<double> eh(static_cast<size_t>(n_f) * 256, INFINITY);
-        for (int ff = 0; ff < n_f; ++ff)
-            for (int k = 0; k < n_edges[ff]; ++k) eh[static_cast<size_t>(ff) * 256 + k] = edges[static_cast<size_t>(ff) * 256 + k];
-        DBuf<double> ed;
-        ed.alloc(eh.size(), s);
-        check(cudaMemcpyAsync(ed.p, eh.data(), 8 * eh.size(), cudaMemcpyHostToDevice, s), "edges");
-        launch_bin_transform_f64(reinterpret_cast<const double*>(Xd.p), n, n_f, ed.p, ne.p, D.pcodes.p, stride, s,
-                                 D.is_cat.p);
-        check(cudaStreamSynchronize(s), "transform");
+    DBuf<uint8_t> codes;
+    DBuf<double> outd;
+    Xd.alloc(static_cast<size_t>(chunk) * row_bytes * slots, s);
+    codes.alloc(static_cast<size_t>(chunk) * stride, s);
+    outd.alloc(static_cast<size_t>(chunk) * slots, s);
+    // pinned slots of a power of two bytes: few sizes in the process's cache
+    size_t slot_bytes = 4096;
+    while (slot_bytes < static_cast<size_t>(chunk) * 8) slot_bytes *= 2;
+    PinnedBlock pinned(slot_bytes * slots);
+    auto host_slot = [&](int c) { return reinterpret_cast<double*>(static_cast<unsigned char*>(pinned.p) + slot_bytes * (c & 1)); };
+    const bool overlap = n_chunks > 1;
+    cudaStream_t in = s;
+    if (overlap) {
+        if (!D.copy.s) check(cudaStreamCreateWithFlags(&D.copy.s, cudaStreamNonBlocking), "cudaStreamCreate");
+        in = D.copy.s;
+        check(cudaEventRecord(D.ev_ready.get(), s), "event record");  // the buffers exist
+        check(cudaStreamWaitEvent(in, D.ev_ready.get(), 0), "event wait");
     }
-    launch_predict_trees(D.pcodes.p, stride, n, D.t_feat.p, D.t_left.p, D.t_right.p, D.t_thr.p, D.t_ml.p, D.t_val.p,
-                         D.t_off.p, static_cast<int>(trees.size()), init_score, cfg.learning_rate, D.t_type.p, D.t_cat.p, D.t_feat2.p,
-                         n_bins, D.pout.p, s);
-    check(cudaMemcpyAsync(out, D.pout.p, sizeof(double) * n, cudaMemcpyDeviceToHost, s), "predict D2H");
-    check(cudaStreamSynchronize(s), "predict");
+    StreamGuard guard_s{s}, guard_in{overlap ? in : nullptr};  // before the pinned block goes back
+    auto collect = [&](int c) {
+        if (overlap) check(cudaEventSynchronize(D.ev_out[c & 1].get()), "predict");
+        else check(cudaStreamSynchronize(s), "predict");
+        const size_t r0 = static_cast<size_t>(c) * chunk, rows = std::min<size_t>(chunk, n - r0);
+        std::memcpy(out + r0, host_slot(c), rows * sizeof(double));
+    };
+    for (int c = 0; c < n_chunks; ++c) {
+        const int k = c & 1;
+        const size_t r0 = static_cast<size_t>(c) * chunk;
+        const int rows = static_cast<int>(std::min<size_t>(chunk, n - r0));
+        unsigned char* xb = Xd.p + static_cast<size_t>(overlap ? k : 0) * chunk * row_bytes;
+        double* ob = outd.p + static_cast<size_t>(overlap ? k : 0) * chunk;
+        if (c >= 2) {
+            check(cudaStreamWaitEvent(in, D.ev_used[k].get(), 0), "event wait");
+            collect(c - 2);  // its pinned slot and result buffer are free again
+        }
+        check(cudaMemcpyAsync(xb, static_cast<const unsigned char*>(X) + r0 * row_bytes, rows * row_bytes,
+                              cudaMemcpyHostToDevice, in), "X upload");
+        if (overlap) {
+            check(cudaEventRecord(D.ev_in[k].get(), in), "event record");
+            check(cudaStreamWaitEvent(s, D.ev_in[k].get(), 0), "event wait");
+        }
+        if (dtype == 0)
+            launch_bin_transform_f32(reinterpret_cast<const float*>(xb), rows, n_f,
+                                     reinterpret_cast<const float*>(D.t_edges.p), D.t_ne.p, codes.p, stride, s, D.is_cat.p);
+        else
+            launch_bin_transform_f64(reinterpret_cast<const double*>(xb), rows, n_f,
+                                     reinterpret_cast<const double*>(D.t_edges.p), D.t_ne.p, codes.p, stride, s, D.is_cat.p);
+        if (overlap) check(cudaEventRecord(D.ev_used[k].get(), s), "event record");
+        launch_predict_trees(codes.p, stride, rows, m, init_score, cfg.learning_rate, ob, s);
+        check(cudaMemcpyAsync(host_slot(c), ob, sizeof(double) * rows, cudaMemcpyDeviceToHost, s), "predict D2H");
+        if (overlap) check(cudaEventRecord(D.ev_out[k].get(), s), "event record");
+    }
+    for (int c = std::max(0, n_chunks - 2); c < n_chunks; ++c) collect(c);
+    guard_s.armed = guard_in.armed = false;
 }
 
 }  // namespace tgb

@@ -173,6 +173,8 @@ public:
     void fit(const void* X, int x_dtype, const double* y, int n, int n_f, const int64_t* ts,
              const int64_t* entity);
     void predict_raw(const void* X, int x_dtype, int n, int n_f, double* out);
+    void upload_model();
+    void upload_edges(int x_dtype);
     // Fits every booster on its input in lockstep on one device: each tree of all of them
     // grows in the same wave launches (batched growth; boosters[0]'s stream and timing
     // hooks).  Each result equals the booster's own fit.

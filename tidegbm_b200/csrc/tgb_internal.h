@@ -344,10 +344,25 @@ void launch_pred_update(const PostParams& pp, const int16_t* nid, const double* 
                         double* pred, cudaStream_t s);
 void launch_fill_pred(const double* init_prefix, int n, int n_buckets, int iid_mode, double* pred,
                       cudaStream_t s);
-void launch_predict_trees(const uint8_t* codes, int stride, int n, const int16_t* tree_feat,
-                          const int16_t* tree_left, const int16_t* tree_right, const uint8_t* tree_thr,
-                          const uint8_t* tree_ml, const double* tree_val, const int* tree_off, int n_trees,
-                          double base, double lr, const uint8_t* tree_type, const unsigned long long* tree_cat,
-                          const int16_t* tree_feat2, int n_bins, double* out, cudaStream_t s);
+// A model laid out for prediction.  word[node]: left child 0-15, right child 16-31 (a leaf:
+// itself twice), threshold 32-39, feature 40-55, missing_left 56, split type 57-58; val[node]:
+// the leaf value; trees[t]: {first node, nodes, depth, 0}; batches[0 .. n_batches]: first trees
+// of runs of at most predict_batch_trees() trees and predict_batch_nodes() nodes; cat[4 node]
+// and feat2[node] as in the tree export (read where any_kind).
+struct PredictTrees {
+    const unsigned long long* word;
+    const double* val;
+    const int4* trees;
+    const int* batches;
+    int n_batches;
+    const unsigned long long* cat;
+    const int16_t* feat2;
+    int n_bins;
+    bool any_kind;
+};
+int predict_batch_nodes();
+int predict_batch_trees();
+void launch_predict_trees(const uint8_t* codes, int stride, int n, const PredictTrees& m, double base, double lr,
+                          double* out, cudaStream_t s);
 
 }  // namespace tgb
