@@ -5,12 +5,11 @@
 //
 // RankPairwise restates objective.cpp:179-219.  Per date group of m rows (group_runs,
 // objective.cpp:18-39): step = m > 48 ? max(1, m/24) : 1 and pairs (a, a + k*step).
-// A row's partners are exactly the positions a -/+ k*step, so each thread owns one
-// row and sums its own pair terms (gather, no atomics).  Visiting the partners in
-// ascending position order reproduces the reference's accumulation order for that
-// row (contributions as the later element of a pair arrive first, for smaller a),
-// so g and h follow the same FP64 addition sequence; this file is compiled with
-// -fmad=false to keep the statement-order rounding.
+// A row's partners are exactly the positions a -/+ k*step, so a row sums its own pair terms
+// (gather, no atomics).  Visiting the partners in ascending position order reproduces the
+// reference's accumulation order for that row (contributions as the later element of a pair
+// arrive first, for smaller a), so g and h follow the same FP64 addition sequence; this
+// file is compiled with -fmad=false to keep the statement-order rounding.
 //
 // Losses restate Objective::loss (objective.cpp:262-329): mean squared error, and
 // for ranking the negative mean within-group Pearson correlation.
@@ -48,39 +47,119 @@ __global__ void grad_mse_fused_kernel(const double* __restrict__ y, const double
 
 __device__ __forceinline__ int row_at(const int* order, int p) { return order ? order[p] : p; }
 
-__global__ void grad_pairwise_kernel(const double* __restrict__ y, const double* __restrict__ pred,
-                                     const int* __restrict__ run_start, const int* __restrict__ run_len,
-                                     const int* __restrict__ order, double* __restrict__ g,
-                                     double* __restrict__ h) {
+// One pair of rows of unlike targets (objective.cpp:196-212): the lambda added to the row of
+// the larger target and subtracted from the other, and the hessian both get.
+__device__ __forceinline__ void pair_terms(double phi, double plo, double dy, double& lam, double& d2) {
+    const double s = phi - plo;
+    const double e = exp(fmin(fmax(1.0 * s, -30.0), 30.0));
+    const double dyw = fmax(fabs(dy), 1e-6);
+    lam = -1.0 / (1.0 + e) * dyw;
+    d2 = 1.0 * 1.0 * e / ((1 + e) * (1 + e)) * dyw;
+}
+
+// A row's partners are the rows of its residue class modulo step, so a class of K rows is a
+// clique of K (K - 1) / 2 pairs (K <= 48; at most 36 where m > 48, 24 to 29 from m = 120 on).
+// A warp takes a class: lanes evaluate its pairs once each and leave the signed lambda of the
+// pair's first row and the hessian in shared memory; then a lane per row adds its row's terms
+// in ascending partner order, the order and the terms of the reference, so the sums are the
+// same to the last bit (a pair of equal targets leaves zeros, which change no sum).  The
+// kernel is bound by instruction issue, most of it the exponential and two FP64 divisions of
+// a pair, which are evaluated once instead of once for each row (8,000 dates of 50 to 800
+// rows: 442 -> 347 us; FP64 alone is about 160).  kGradRoom pairs of room a warp keep seven
+// CTAs on an SM; a run of larger classes gives a warp the room of several.
+constexpr int kClassRows = 48;
+constexpr int kGradRoom = 29 * 28 / 2;
+constexpr int kGradWarps = 4;
+static_assert(kGradWarps * kGradRoom >= kClassRows * (kClassRows - 1) / 2, "room for the largest class");
+
+__global__ void __launch_bounds__(kGradWarps * 32)
+    grad_pairwise_kernel(const double* __restrict__ y, const double* __restrict__ pred,
+                         const int* __restrict__ run_start, const int* __restrict__ run_len,
+                         const int* __restrict__ order, double* __restrict__ g,
+                         double* __restrict__ h) {
+    __shared__ double2 s_terms[kGradWarps * kGradRoom];  // {lambda, hessian} of pair b (b - 1) / 2 + a, a < b
+    __shared__ double2 s_rows[kGradWarps][kClassRows];   // {y, pred}
+    __shared__ unsigned short s_ab[kClassRows * (kClassRows - 1) / 2];  // a | b << 8
     const int r = blockIdx.x;
     const int s0 = run_start[r], m = run_len[r];
-    for (int a = threadIdx.x; a < m; a += blockDim.x) {
-        const int i = row_at(order, s0 + a);
-        double ga = 0.0, ha = 1e-6;
-        if (m >= 2) {
-            const int step = m > 48 ? max(1, m / 24) : 1;
-            const double yi = y[i], pi = pred[i];
-            // Partners in ascending position: a%step, a%step+step, ..., a-step, then a+step, ...
-            for (int p = a % step; p < m; p += step) {
-                if (p == a) continue;
-                const int j = row_at(order, s0 + p);
-                const double yj = y[j];
-                if (yi == yj) continue;
-                const bool i_hi = yi > yj;
-                const double phi = i_hi ? pi : pred[j];
-                const double plo = i_hi ? pred[j] : pi;
-                const double s = phi - plo;
-                const double e = exp(fmin(fmax(1.0 * s, -30.0), 30.0));
-                const double dyw = fmax(fabs(i_hi ? yi - yj : yj - yi), 1e-6);
-                const double lam = -1.0 / (1.0 + e) * dyw;
-                const double d2 = 1.0 * 1.0 * e / ((1 + e) * (1 + e)) * dyw;
-                if (i_hi) ga += 1.0 * lam;
-                else ga -= 1.0 * lam;
-                ha += 1.0 * d2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int step = m > 48 ? max(1, m / 24) : 1;
+    const int most = (m + step - 1) / step;  // rows of class 0, the largest
+    for (int b = threadIdx.x; b < most; b += kGradWarps * 32)
+        for (int a = 0; a < b; ++a) s_ab[b * (b - 1) / 2 + a] = static_cast<unsigned short>(a | b << 8);
+    __syncthreads();
+    const int span = max(1, (most * (most - 1) / 2 + kGradRoom - 1) / kGradRoom);  // warps' room a class takes
+    const int warps = kGradWarps / span;
+    if (warp >= warps) return;
+    double2 *terms = s_terms + warp * span * kGradRoom, *cls = s_rows[warp];
+    for (int c = warp; c < step && c < m; c += warps) {
+        const int K = (m - c + step - 1) / step, n_pairs = K * (K - 1) / 2;
+        int row[2];
+        bool nan = false;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int a = lane + 32 * q;
+            row[q] = a < K ? row_at(order, s0 + c + a * step) : -1;
+            if (row[q] >= 0) {
+                const double ya = y[row[q]];
+                cls[a] = make_double2(ya, pred[row[q]]);
+                nan |= ya != ya;
             }
         }
-        g[i] = ga;
-        h[i] = ha;
+        __syncwarp();
+        if (__any_sync(0xffffffffu, nan)) {
+            // a NaN target is the lower one of its pair for both rows: no shared terms
+#pragma unroll
+            for (int q = 0; q < 2; ++q) {
+                const int a = lane + 32 * q;
+                if (row[q] < 0) continue;
+                const double2 A = cls[a];
+                double ga = 0.0, ha = 1e-6, l, d;
+                for (int b = 0; b < K; ++b) {
+                    const double2 B = cls[b];
+                    if (b == a || A.x == B.x) continue;
+                    const bool a_hi = A.x > B.x;
+                    pair_terms(a_hi ? A.y : B.y, a_hi ? B.y : A.y, a_hi ? A.x - B.x : B.x - A.x, l, d);
+                    ga += a_hi ? l : -l;
+                    ha += d;
+                }
+                g[row[q]] = ga;
+                h[row[q]] = ha;
+            }
+            __syncwarp();
+            continue;
+        }
+        for (int q = lane; q < n_pairs; q += 32) {
+            const unsigned ab = s_ab[q];
+            const double2 A = cls[ab & 0xffu], B = cls[ab >> 8];
+            const bool a_hi = A.x > B.x;
+            double l, d;
+            pair_terms(a_hi ? A.y : B.y, a_hi ? B.y : A.y, a_hi ? A.x - B.x : B.x - A.x, l, d);
+            if (!a_hi) l = -l;  // row a is the lower one
+            if (A.x == B.x) l = d = 0.0;
+            terms[q] = make_double2(l, d);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int a = lane + 32 * q;
+            if (row[q] < 0) continue;
+            double ga = 0.0, ha = 1e-6;
+            // partners below a: a is the pair's second row; above: its first
+            int at = a * (a - 1) / 2;
+            for (int b = 0; b < K; ++b) {
+                if (b == a) at = a * (a + 1) / 2 + a;  // the pair (a, a + 1)
+                else {
+                    const double2 t = terms[at];
+                    ga += b < a ? -t.x : t.x;
+                    ha += t.y;
+                    at += b < a ? 1 : b;
+                }
+            }
+            g[row[q]] = ga;
+            h[row[q]] = ha;
+        }
+        __syncwarp();
     }
 }
 
@@ -232,7 +311,7 @@ void launch_grad_pairwise(const double* y, const double* pred, const int* run_st
                           const int* order, int n_runs, int n, double* g, double* h, cudaStream_t s) {
     (void)n;
     if (n_runs <= 0) return;
-    grad_pairwise_kernel<<<n_runs, 128, 0, s>>>(y, pred, run_start, run_len, order, g, h);
+    grad_pairwise_kernel<<<n_runs, kGradWarps * 32, 0, s>>>(y, pred, run_start, run_len, order, g, h);
     check(cudaGetLastError(), "grad_pairwise launch");
 }
 
