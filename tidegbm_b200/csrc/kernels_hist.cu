@@ -9,23 +9,22 @@
 // subtraction is exact.  The error against an FP64 sum is at most
 // rows * 2^-(shift+1) (about 1e-12 relative at 10M rows).
 //
-// Launch shape: CTA = (group of 32 features) x (contiguous chunk of the node's row
-// list), one CTA per SM.  A warp takes one row at a time and lane l owns feature l of
-// the group: the warp reads the row's 32 code bytes with one coalesced 32-byte access,
-// g and h are warp-uniform broadcasts, and each lane adds into bin (code_l, l) of the
-// CTA-private shared histogram, stored at b*32 + l: every lane of a warp access owns its
-// own bank whatever the codes are, and the features being distinct there are no
-// same-address collisions either.
+// Launch shape: CTA = (group of 32 features) x (contiguous chunk of the row list), one CTA
+// per SM, lane = row: a warp takes 32 rows, a lane holds its row's 32 code bytes of the group
+// rotated by its lane number, so that at each of 32 steps the 32 lanes touch 32 different
+// features, hence 32 banks of the [bin][feature] layout whatever the codes.
 //
-// Shared atomics are 32-bit only (the 64-bit shared add is not a single instruction):
-// a 64-bit fixed-point value is added as two words, the low word with atomicAdd, whose
-// returned old value tells whether this addition wrapped, then (high + carry) to the
-// high word.  The words end up holding the exact 64-bit sum modulo 2^64.  For objectives
-// with a constant hessian (mse with unit weights: h = 1, or 1 * goss_scale for sampled
-// GOSS rows) the hessian and count sums are two 32-bit row counters, c1 (unscaled rows)
-// and c2 (scaled rows): H = c1 * rint(2^hs) + c2 * rint(goss_scale * 2^hs), C = c1 + c2,
-// the same integers the per-row sums give.  The private histogram is flushed to the
-// node's global slot with one 64-bit global atomic per non-empty bin and value.
+// Shared reductions are 32-bit only (the 64-bit shared add is a compare-and-swap loop), so a
+// 64-bit value is split: r = v - top * 2^40 in [-2^39, 2^39) into 20 low bits and a signed
+// 20-bit rest, whose sums over a sub-chunk of 4,096 rows fit 32 bits, and top, which only
+// matters modulo 2^24 and is 0 for all but the largest values.  A code then costs five
+// fire-and-forget reductions (g low, g rest, h low, h rest, count), where the former
+// (low, high + carry) pairs cost as many with two whose returned value was waited for
+// (1.2M of 4M rows x 128 features: 381 -> 249 us; the reductions alone are about 170 at two
+// clocks a warp-wide one).  Rows with a top go through the same steps with two more, or, where
+// a warp has few of them, one by one with a lane per feature.  For objectives with a constant
+// hessian (mse with unit weights: h = 1, or 1 * goss_scale for sampled GOSS rows) the hessian
+// and count sums are two row counters (below): H = c1 * rint(2^hs) + c2 * rint(goss_scale * 2^hs), C = c1 + c2.
 #include "tgb_internal.h"
 
 #include <cmath>
@@ -41,19 +40,80 @@ constexpr int kHistThreads = 1024;
 constexpr int kHistWarps = kHistThreads / 32;
 constexpr int kMinRowsPerCta = 2048;
 constexpr int kFG = 32;      // features per CTA (one per lane)
-constexpr int kUnroll = 8;   // code loads in flight per warp
 constexpr int kPlane = kFG * kBins;  // 32-bit words per plane
+constexpr int kCells = kPlane / kHistThreads;  // cells owned per thread (8)
 
-// Exact 64-bit add into a (low, high) pair of 32-bit shared words.
-__device__ __forceinline__ void add64(unsigned int* lo, unsigned int* hi, int slot, unsigned long long v) {
-    const unsigned int vlo = static_cast<unsigned int>(v);
-    const unsigned int vhi = static_cast<unsigned int>(v >> 32);
-    const unsigned int old = atomicAdd(&lo[slot], vlo);
-    const unsigned int up = vhi + (old + vlo < old ? 1u : 0u);
-    if (up != 0u) atomicAdd(&hi[slot], up);
+// out[t] = in[(t + k) & 7] for a lane-dependent k in [0, 8): three conditional rotations.
+__device__ __forceinline__ void rotate_words(unsigned int (&w)[8], int k) {
+    unsigned int t[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = (k & 1) ? w[(i + 1) & 7] : w[i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = (k & 2) ? t[(i + 2) & 7] : t[i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) t[i] = (k & 4) ? w[(i + 4) & 7] : w[i];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = t[i];
 }
 
-template <bool kConstH>
+constexpr int kVarMinRows = 512;  // rows of a CTA: fewer cost more in flushes than they save
+constexpr int kVarSub = 4096;  // rows of a sub-chunk
+constexpr int kVarLo = 20;     // low bits; the rest of r is 20 bits, signed
+constexpr int kVarTop = 40;
+constexpr int kVarPlanes = 7;  // g low, g rest, h low, h rest, count, g top, h top
+constexpr int kFewTops = 6;    // rows of a warp step whose tops go one by one
+constexpr int kTotPitch = kBins + 1;
+constexpr int kTot = kFG * kTotPitch;
+constexpr size_t kVarSmem = static_cast<size_t>(kVarPlanes) * kPlane * 4;
+static_assert(static_cast<size_t>(kTot) * 20 <= kVarSmem, "the totals lie over the planes");
+
+// 16 code bytes; a caller's matrix may start at any byte.
+__device__ __forceinline__ uint4 load_codes16(const uint8_t* p, bool aligned) {
+    if (aligned) return __ldg(reinterpret_cast<const uint4*>(p));
+    unsigned int w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+        w[i] = static_cast<unsigned int>(p[4 * i]) | static_cast<unsigned int>(p[4 * i + 1]) << 8 |
+               static_cast<unsigned int>(p[4 * i + 2]) << 16 | static_cast<unsigned int>(p[4 * i + 3]) << 24;
+    return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+struct SplitValue {
+    unsigned int lo, rest;
+    int top;
+};
+__device__ __forceinline__ SplitValue split_value(long long v) {
+    SplitValue s;
+    // wrapping arithmetic: a saturated v keeps its value modulo 2^64
+    const unsigned long long u = static_cast<unsigned long long>(v);
+    const long long top = static_cast<long long>(u + (1ull << (kVarTop - 1))) >> kVarTop;
+    const long long r = static_cast<long long>(u - (static_cast<unsigned long long>(top) << kVarTop));
+    s.lo = static_cast<unsigned int>(r) & ((1u << kVarLo) - 1u);
+    s.rest = static_cast<unsigned int>(static_cast<int>(r >> kVarLo));
+    s.top = static_cast<int>(top);
+    return s;
+}
+
+template <bool kTops>
+__device__ __forceinline__ void add_steps(unsigned int* __restrict__ P, const unsigned int (&R)[8], int lane,
+                                          const SplitValue& gs, const SplitValue& hs) {
+#pragma unroll
+    for (int j = 0; j < 32; ++j) {
+        const int f = (j + lane) & 31;
+        const int cell = static_cast<int>((R[j >> 2] >> ((j & 3) * 8)) & 0xffu) * 32 + f;
+        atomicAdd(&P[cell], gs.lo);
+        atomicAdd(&P[kPlane + cell], gs.rest);
+        atomicAdd(&P[2 * kPlane + cell], hs.lo);
+        atomicAdd(&P[3 * kPlane + cell], hs.rest);
+        atomicAdd(&P[4 * kPlane + cell], 1u);
+        if (kTops) {
+            atomicAdd(&P[5 * kPlane + cell], static_cast<unsigned int>(gs.top));
+            atomicAdd(&P[6 * kPlane + cell], static_cast<unsigned int>(hs.top));
+        }
+    }
+}
+
+// Histogram of rows[0 .. count) with per-row hessians, added to G, H, C.
 __device__ __forceinline__ void hist_body(const uint8_t* __restrict__ codes, int stride, int n_f,
                                           const int32_t* __restrict__ rows, int count,
                                           const double* __restrict__ g, const double* __restrict__ h,
@@ -61,16 +121,10 @@ __device__ __forceinline__ void hist_body(const uint8_t* __restrict__ codes, int
                                           double gscale, double hscale, long long* G, long long* H,
                                           int* C) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    unsigned int* gLo = reinterpret_cast<unsigned int*>(smem_raw);
-    unsigned int* gHi = gLo + kPlane;
-    // kConstH: c1, c2 row counters; otherwise hLo, hHi, count.
-    unsigned int* p2 = gHi + kPlane;
-    unsigned int* p3 = p2 + kPlane;
-    unsigned int* p4 = p3 + kPlane;
-    constexpr int n_planes = kConstH ? 4 : 5;
+    unsigned int* P = reinterpret_cast<unsigned int*>(smem_raw);
 
     // Row chunk of this CTA.
-    const int need = (count + kMinRowsPerCta - 1) / kMinRowsPerCta;
+    const int need = (count + kVarMinRows - 1) / kVarMinRows;
     const int n_chunks = max(1, min(static_cast<int>(gridDim.y), need));
     if (static_cast<int>(blockIdx.y) >= n_chunks) return;
     const int chunk = (count + n_chunks - 1) / n_chunks;
@@ -80,86 +134,123 @@ __device__ __forceinline__ void hist_body(const uint8_t* __restrict__ codes, int
 
     {
         uint4* z = reinterpret_cast<uint4*>(smem_raw);
-        for (int k = threadIdx.x; k < n_planes * kPlane / 4; k += blockDim.x) z[k] = make_uint4(0, 0, 0, 0);
+        for (int k = threadIdx.x; k < static_cast<int>(kVarSmem / 16); k += blockDim.x) z[k] = make_uint4(0, 0, 0, 0);
     }
     __syncthreads();
 
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    const int f = blockIdx.x * kFG + lane;
-    const bool active = f < n_f;
-    const int fo = active ? f : 0;  // in-bounds byte for idle lanes
-    // A warp takes 32 rows at a time: lane j loads row j's index, g and h (one gather each),
-    // then the warp walks the 32 rows, kBatch code loads in flight, with the row's index
-    // and fixed-point values broadcast by shuffles.
-    for (int base = r0 + warp * 32; base < r1; base += kHistWarps * 32) {
-        const int nrow = min(32, r1 - base);
-        const bool own = lane < nrow;
-        const int rid = own ? rows[base + lane] : 0;
-        unsigned long long gq = 0ull, hq = 0ull;
+    const int q = lane >> 2, sh = (lane & 3) * 8;
+    const int fg0 = blockIdx.x * kFG;
+    const bool two_chunks = stride - fg0 >= 32;
+    const bool aligned = (reinterpret_cast<uintptr_t>(codes) & 15u) == 0;  // strides are multiples of 16
+    constexpr int kStep = kHistWarps * 32;
+    long long accG[kCells], accH[kCells];
+    unsigned int accC[kCells];
+#pragma unroll
+    for (int c = 0; c < kCells; ++c) {
+        accG[c] = accH[c] = 0;
+        accC[c] = 0u;
+    }
+    for (int s0 = r0; s0 < r1; s0 += kVarSub) {
+        const int s1 = min(r1, s0 + kVarSub);
+        // a row's id is loaded two steps ahead of its use, its values and codes one step ahead
+        const int k0 = s0 + warp * 32 + lane;
+        int r_cur = k0 < s1 ? rows[k0] : -1;
+        int r_nxt = k0 + kStep < s1 ? rows[k0 + kStep] : -1;
+        double gv = 0.0, hv = 0.0;
         int sc = 0;
-        if (own) {
-            double gv = g[rid];
-            sc = goss_flag != nullptr && goss_flag[rid] == 2;
-            if (sc) gv *= goss_scale;
-            gq = static_cast<unsigned long long>(__double2ll_rn(gv * gscale));
-            if (!kConstH) {
-                double hv = h[rid];
-                if (sc) hv *= goss_scale;
-                hq = static_cast<unsigned long long>(__double2ll_rn(hv * hscale));
+        uint4 ca = make_uint4(0, 0, 0, 0), cb = make_uint4(0, 0, 0, 0);
+        auto fetch = [&](int r) {
+            const uint8_t* src = codes + static_cast<size_t>(r) * stride + fg0;
+            gv = g[r];
+            hv = h[r];
+            sc = goss_flag != nullptr && goss_flag[r] == 2;
+            ca = load_codes16(src, aligned);
+            cb = two_chunks ? load_codes16(src + 16, aligned) : make_uint4(0, 0, 0, 0);
+        };
+        if (r_cur >= 0) fetch(r_cur);
+        for (int base = s0 + warp * 32; base < s1; base += kStep) {
+            const bool own = r_cur >= 0;
+            if (sc) {
+                gv *= goss_scale;
+                hv *= goss_scale;
             }
-        }
-        for (int j0 = 0; j0 < nrow; j0 += kUnroll) {
-            unsigned int cc[kUnroll];
+            const SplitValue gs = split_value(__double2ll_rn(gv * gscale)), hs = split_value(__double2ll_rn(hv * hscale));
+            unsigned int wd[8] = {ca.x, ca.y, ca.z, ca.w, cb.x, cb.y, cb.z, cb.w};
+            r_cur = r_nxt;
+            const int kn = base + 2 * kStep + lane;
+            r_nxt = kn < s1 ? rows[kn] : -1;
+            if (r_cur >= 0) fetch(r_cur);
+            const bool big = own && ((gs.top | hs.top) != 0);
+            const unsigned int bigs = __ballot_sync(0xffffffffu, big);
+            const bool few = __popc(bigs) <= kFewTops;
+            if (few) {  // the tops of the few rows that have one: a lane per feature
+                for (unsigned int left = bigs; left != 0u; left &= left - 1u) {
+                    const int L = __ffs(left) - 1;
+                    unsigned int w = 0u;
 #pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                const int j = j0 + u;
-                const int rj = __shfl_sync(0xffffffffu, rid, j & 31);
-                cc[u] = j < nrow ? codes[static_cast<size_t>(rj) * stride + fo] : 0u;
-            }
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                const int j = j0 + u;
-                const unsigned long long gj = __shfl_sync(0xffffffffu, gq, j & 31);
-                const int sj = __shfl_sync(0xffffffffu, sc, j & 31);
-                const unsigned long long hj = kConstH ? 0ull : __shfl_sync(0xffffffffu, hq, j & 31);
-                if (j >= nrow || !active) continue;
-                const int slot = static_cast<int>(cc[u]) * 32 + lane;
-                add64(gLo, gHi, slot, gj);
-                if (kConstH) {
-                    atomicAdd(sj ? &p3[slot] : &p2[slot], 1u);
-                } else {
-                    add64(p2, p3, slot, hj);
-                    atomicAdd(&p4[slot], 1u);
+                    for (int i = 0; i < 8; ++i) {
+                        const unsigned int t = __shfl_sync(0xffffffffu, wd[i], L);
+                        if (q == i) w = t;
+                    }
+                    const int gt = __shfl_sync(0xffffffffu, gs.top, L), ht = __shfl_sync(0xffffffffu, hs.top, L);
+                    const int cell = static_cast<int>((w >> sh) & 0xffu) * 32 + lane;
+                    if (gt != 0) atomicAdd(&P[5 * kPlane + cell], static_cast<unsigned int>(gt));
+                    if (ht != 0) atomicAdd(&P[6 * kPlane + cell], static_cast<unsigned int>(ht));
                 }
             }
+            rotate_words(wd, q);
+            unsigned int R[8];
+#pragma unroll
+            for (int t = 0; t < 8; ++t) R[t] = __funnelshift_r(wd[t], wd[(t + 1) & 7], sh);
+            if (own) {
+                if (few) add_steps<false>(P, R, lane, gs, hs);
+                else add_steps<true>(P, R, lane, gs, hs);
+            }
         }
+        __syncthreads();
+        // fold the sub-chunk into 64-bit registers and clear the planes
+#pragma unroll
+        for (int c = 0; c < kCells; ++c) {
+            const int cell = threadIdx.x + c * kHistThreads;
+            auto value = [&](int lo, int rest, int top) {
+                return static_cast<long long>(
+                    (static_cast<unsigned long long>(P[top * kPlane + cell]) << kVarTop) +
+                    static_cast<unsigned long long>(static_cast<long long>(static_cast<int>(P[rest * kPlane + cell])) *
+                                                    (1ll << kVarLo)) +
+                    P[lo * kPlane + cell]);
+            };
+            accG[c] += value(0, 1, 5);
+            accH[c] += value(2, 3, 6);
+            accC[c] += P[4 * kPlane + cell];
+#pragma unroll
+            for (int pl = 0; pl < kVarPlanes; ++pl) P[pl * kPlane + cell] = 0u;
+        }
+        __syncthreads();
+    }
+    // Totals over the planes in a padded [feature][bin] layout, so that the flush's global
+    // atomics are consecutive bins of a feature.
+    unsigned long long* Gt = reinterpret_cast<unsigned long long*>(smem_raw);
+    unsigned long long* Ht = Gt + kTot;
+    unsigned int* Ct = reinterpret_cast<unsigned int*>(Ht + kTot);
+#pragma unroll
+    for (int c = 0; c < kCells; ++c) {
+        const int cell = threadIdx.x + c * kHistThreads;
+        const int ti = (cell & 31) * kTotPitch + (cell >> 5);
+        Gt[ti] = static_cast<unsigned long long>(accG[c]);
+        Ht[ti] = static_cast<unsigned long long>(accH[c]);
+        Ct[ti] = accC[c];
     }
     __syncthreads();
-
-    // Flush: warp w takes bins w, w + 32, ...; lane l = feature l (conflict-free reads).
-    const int ff = blockIdx.x * kFG + lane;
-    if (ff >= n_f) return;
-    const unsigned long long hq1 = kConstH ? static_cast<unsigned long long>(__double2ll_rn(1.0 * hscale)) : 0ull;
-    const unsigned long long hq2 =
-        kConstH ? static_cast<unsigned long long>(__double2ll_rn(1.0 * goss_scale * hscale)) : 0ull;
-    for (int b = warp; b < kBins; b += kHistWarps) {
-        const int slot = b * 32 + lane;
-        unsigned long long hsum;
-        unsigned int c;
-        if (kConstH) {
-            const unsigned int c1 = p2[slot], c2 = p3[slot];
-            c = c1 + c2;
-            hsum = static_cast<unsigned long long>(c1) * hq1 + static_cast<unsigned long long>(c2) * hq2;
-        } else {
-            c = p4[slot];
-            hsum = (static_cast<unsigned long long>(p3[slot]) << 32) | p2[slot];
-        }
-        if (c == 0u) continue;
-        const unsigned long long gsum = (static_cast<unsigned long long>(gHi[slot]) << 32) | gLo[slot];
-        const size_t o = static_cast<size_t>(ff) * kBins + b;
-        atomicAdd(reinterpret_cast<unsigned long long*>(G) + o, gsum);
-        atomicAdd(reinterpret_cast<unsigned long long*>(H) + o, hsum);
-        atomicAdd(C + o, static_cast<int>(c));
+    const int nf = min(kFG, n_f - fg0);
+    for (int i = threadIdx.x; i < nf * kBins; i += kHistThreads) {
+        const int ti = i + (i >> 8);
+        const unsigned int cn = Ct[ti];
+        if (cn == 0u) continue;
+        const size_t o = static_cast<size_t>(fg0) * kBins + i;
+        atomicAdd(reinterpret_cast<unsigned long long*>(G) + o, Gt[ti]);
+        atomicAdd(reinterpret_cast<unsigned long long*>(H) + o, Ht[ti]);
+        atomicAdd(C + o, static_cast<int>(cn));
     }
 }
 
@@ -184,20 +275,6 @@ __device__ __forceinline__ void hist_body(const uint8_t* __restrict__ codes, int
 // accumulators (each thread owns 8 fixed cells) and clears them.
 constexpr int kSub = 8192;
 constexpr int kLoBits = 19;
-constexpr int kCells = kFG * kBins / kHistThreads;  // cells owned per thread (8)
-
-// out[t] = in[(t + k) & 7] for a lane-dependent k in [0, 8): three conditional rotations.
-__device__ __forceinline__ void rotate_words(unsigned int (&w)[8], int k) {
-    unsigned int t[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t[i] = (k & 1) ? w[(i + 1) & 7] : w[i];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) w[i] = (k & 2) ? t[(i + 2) & 7] : t[i];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) t[i] = (k & 4) ? w[(i + 4) & 7] : w[i];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) w[i] = t[i];
-}
 
 // The CTAs of a cluster (kCluster consecutive row chunks of one feature group) add
 // their partial histograms through distributed shared memory before the flush: each
@@ -428,7 +505,6 @@ __global__ void quantize_kernel(const int32_t* __restrict__ rows, const double* 
     }
 }
 
-template <bool kConstH>
 __global__ void __launch_bounds__(kHistThreads)
     hist_node_kernel(const uint8_t* __restrict__ codes, int stride, int n_f, int32_t* rows0,
                      int32_t* rows1, const DevNode* __restrict__ nodes,
@@ -442,7 +518,7 @@ __global__ void __launch_bounds__(kHistThreads)
     // Rows histogrammed, for the algorithmic-bytes figure of the benchmark.
     if (rows_counter != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0)
         atomicAdd(rows_counter, static_cast<unsigned long long>(N.count));
-    hist_body<kConstH>(codes, stride, n_f, rows, N.count, g, h, goss_flag, goss_scale, st->gscale, st->hscale,
+    hist_body(codes, stride, n_f, rows, N.count, g, h, goss_flag, goss_scale, st->gscale, st->hscale,
                        hs.G + nd * hs.slot_elems, hs.H + nd * hs.slot_elems, hs.C + nd * hs.slot_elems);
 }
 
@@ -450,7 +526,7 @@ __global__ void __launch_bounds__(kHistThreads)
     hist_rows_kernel(const uint8_t* __restrict__ codes, int stride, int n_f, const int32_t* __restrict__ rows,
                      int count, const double* __restrict__ g, const double* __restrict__ h, double gscale,
                      double hscale, long long* G, long long* H, int* C) {
-    hist_body<false>(codes, stride, n_f, rows, count, g, h, nullptr, 1.0, gscale, hscale, G, H, C);
+    hist_body(codes, stride, n_f, rows, count, g, h, nullptr, 1.0, gscale, hscale, G, H, C);
 }
 
 __global__ void tree_init_kernel(DevNode* nodes, DevSplit* splits, DevTreeState* st, int n_sample,
@@ -514,8 +590,6 @@ __global__ void scales_finalize_kernel(DevTreeState* st, const AllScale* __restr
     }
 }
 
-constexpr size_t hist_smem(bool const_h) { return static_cast<size_t>(kPlane) * 4 * (const_h ? 4 : 5); }
-
 template <typename K>
 void set_smem(K kern, size_t bytes) {
     check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)),
@@ -526,8 +600,8 @@ void set_smem(K kern, size_t bytes) {
 
 int hist_grid_rows(int n_f, int max_rows, bool const_h) {
     const int groups = (n_f + kFG - 1) / kFG;
+    if (!const_h) return std::max(1, std::min((max_rows + kVarMinRows - 1) / kVarMinRows, std::max(1, 148 / groups)));
     const int need = (max_rows + kMinRowsPerCta - 1) / kMinRowsPerCta;
-    if (!const_h) return std::max(1, std::min(need, (148 + groups - 1) / groups));
     // Clusters that fit on the device at once, shared among the feature groups.
     set_smem(hist_node_const_kernel<false>, kConstSmem);
     cudaLaunchConfig_t cfg{};
@@ -558,8 +632,8 @@ void launch_hist_node(const uint8_t* codes, int stride, int n_f, int32_t* const*
                    rows[1], nodes, st, node, gq, goss_scale, hs, rows_counter);
         return;
     } else {
-        set_smem(hist_node_kernel<false>, hist_smem(false));
-        hist_node_kernel<false><<<grid, kHistThreads, hist_smem(false), s>>>(
+        set_smem(hist_node_kernel, kVarSmem);
+        hist_node_kernel<<<grid, kHistThreads, kVarSmem, s>>>(
             codes, stride, n_f, rows[0], rows[1], nodes, st, node, g, h, goss_flag, goss_scale, hs, rows_counter);
     }
     check(cudaGetLastError(), "hist_node launch");
@@ -583,9 +657,9 @@ void launch_hist_rows(const uint8_t* codes, int stride, int n_f, const int32_t* 
                       const double* g, const double* h, int gshift, int hshift, long long* G,
                       long long* H, int* C, cudaStream_t s) {
     if (n_rows <= 0) return;
-    set_smem(hist_rows_kernel, hist_smem(false));
+    set_smem(hist_rows_kernel, kVarSmem);
     dim3 grid((n_f + kFG - 1) / kFG, hist_grid_rows(n_f, n_rows, false));
-    hist_rows_kernel<<<grid, kHistThreads, hist_smem(false), s>>>(codes, stride, n_f, rows, n_rows, g, h,
+    hist_rows_kernel<<<grid, kHistThreads, kVarSmem, s>>>(codes, stride, n_f, rows, n_rows, g, h,
                                                            std::ldexp(1.0, gshift), std::ldexp(1.0, hshift), G, H,
                                                            C);
     check(cudaGetLastError(), "hist_rows launch");
