@@ -396,7 +396,7 @@ void binner_refit_features(const std::vector<int>& fids, const void* X_host, con
 
 int binner_fit_device(const void* Xd, int x_dtype, int n, int n_f, int max_bin, int bin_sample, uint32_t seed,
                       std::vector<double>& edges, std::vector<int>& n_edges, int n_threads, void* stream,
-                      void* arena, size_t arena_bytes, BinFitTimes* tm, const void* X_host) {
+                      void* arena, size_t arena_bytes, BinFitTimes* tm, const void* X_host, const int* skip) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const double t0 = wall_now();
     const int n_chunks = (n + kFitChunk - 1) / kFitChunk;
@@ -416,6 +416,8 @@ int binner_fit_device(const void* Xd, int x_dtype, int n, int n_f, int max_bin, 
     std::vector<int> flagged;
     int nb = binner_fit_from_plan(plan, Xd, x_dtype, n, n_f, max_bin, bin_sample, edges, n_edges, stream, arena,
                                   arena_bytes, &flagged);
+    if (skip)
+        flagged.erase(std::remove_if(flagged.begin(), flagged.end(), [&](int f) { return skip[f] != 0; }), flagged.end());
     if (!flagged.empty()) {
         binner_refit_features(flagged, X_host, Xd, x_dtype, n, n_f, max_bin, bin_sample, seed, edges, n_edges,
                               n_threads, s);
@@ -434,25 +436,60 @@ int binner_fit_device(const void* Xd, int x_dtype, int n, int n_f, int max_bin, 
 
 namespace {
 
+// The distinct values of a categorical feature with their counts, ascending; false where that
+// takes the sorted column: too many distinct values for the table, or both zero signs (the
+// vocabulary holds the one std::sort leaves first).
+template <typename T>
+bool count_values(const T* X, int n, int n_f, int f, std::vector<std::pair<int, double>>& runs) {
+    constexpr size_t kSlots = 1 << 14;
+    constexpr size_t kMost = kSlots / 2;
+    std::vector<double> key(kSlots);
+    std::vector<int> count(kSlots, 0);
+    size_t distinct = 0;
+    bool pos_zero = false, neg_zero = false;
+    for (int i = 0; i < n; ++i) {
+        const double x = static_cast<double>(X[static_cast<size_t>(i) * n_f + f]);
+        if (is_nan(x)) continue;
+        uint64_t bits;
+        std::memcpy(&bits, &x, 8);
+        if (x == 0.0) (bits >> 63 ? neg_zero : pos_zero) = true;
+        size_t s = (bits * 0x9e3779b97f4a7c15ull) >> 50;  // 2^14 slots
+        while (count[s] != 0 && key[s] != x) s = (s + 1) & (kSlots - 1);
+        if (count[s] == 0) {
+            if (++distinct > kMost) return false;
+            key[s] = x;
+        }
+        ++count[s];
+    }
+    if (pos_zero && neg_zero) return false;
+    for (size_t s = 0; s < kSlots; ++s)
+        if (count[s] != 0) runs.emplace_back(count[s], key[s]);
+    std::sort(runs.begin(), runs.end(), [](const auto& a, const auto& b) { return a.second < b.second; });
+    return true;
+}
+
 // The vocabulary of one categorical feature (cpp/src/binning.cpp:47-84): the distinct
 // non-NaN values with at least cat_min_count occurrences (none: the most frequent one,
 // the smallest value on ties), cut to the max_bin - 1 most frequent ones when there are
 // more (std::partial_sort, so ties fall as in the reference), ascending.
 template <typename T>
 std::vector<double> cat_vocabulary(const T* X, int n, int n_f, int f, int max_bin, int cat_min_count) {
-    std::vector<double> v;
-    v.reserve(static_cast<size_t>(n));
-    for (int i = 0; i < n; ++i) {
-        const double x = static_cast<double>(X[static_cast<size_t>(i) * n_f + f]);
-        if (!is_nan(x)) v.push_back(x);
-    }
-    std::sort(v.begin(), v.end());
     std::vector<std::pair<int, double>> runs;  // (occurrences, value), ascending values
-    for (size_t a = 0; a < v.size();) {
-        size_t b = a + 1;
-        while (b < v.size() && v[b] == v[a]) ++b;
-        runs.emplace_back(static_cast<int>(b - a), v[a]);
-        a = b;
+    if (!count_values(X, n, n_f, f, runs)) {
+        runs.clear();
+        std::vector<double> v;
+        v.reserve(static_cast<size_t>(n));
+        for (int i = 0; i < n; ++i) {
+            const double x = static_cast<double>(X[static_cast<size_t>(i) * n_f + f]);
+            if (!is_nan(x)) v.push_back(x);
+        }
+        std::sort(v.begin(), v.end());
+        for (size_t a = 0; a < v.size();) {
+            size_t b = a + 1;
+            while (b < v.size() && v[b] == v[a]) ++b;
+            runs.emplace_back(static_cast<int>(b - a), v[a]);
+            a = b;
+        }
     }
     const int min_count = std::max(1, cat_min_count);
     std::vector<std::pair<int, double>> kept;
@@ -476,12 +513,13 @@ std::vector<double> cat_vocabulary(const T* X, int n, int n_f, int f, int max_bi
 
 }  // namespace
 
-int binner_fit_cat(const void* X, int x_dtype, int n, int n_f, const int* is_cat, int max_bin, int cat_min_count,
-                   int bin_sample, uint32_t seed, std::vector<double>& edges, std::vector<int>& n_edges,
-                   int n_threads) {
-    binner_fit(X, x_dtype, n, n_f, max_bin, bin_sample, seed, edges, n_edges, n_threads);
-    parallel_for(n_f, n_threads, [&](int f) {
-        if (!is_cat[f]) return;
+int binner_add_vocabularies(const void* X, int x_dtype, int n, int n_f, const int* is_cat, int max_bin,
+                            int cat_min_count, std::vector<double>& edges, std::vector<int>& n_edges, int n_threads) {
+    std::vector<int> cats;
+    for (int f = 0; f < n_f; ++f)
+        if (is_cat[f]) cats.push_back(f);
+    parallel_for(static_cast<int>(cats.size()), n_threads, [&](int k) {
+        const int f = cats[k];
         const std::vector<double> vocab =
             x_dtype == 0 ? cat_vocabulary(static_cast<const float*>(X), n, n_f, f, max_bin, cat_min_count)
                          : cat_vocabulary(static_cast<const double*>(X), n, n_f, f, max_bin, cat_min_count);
@@ -493,6 +531,13 @@ int binner_fit_cat(const void* X, int x_dtype, int n, int n_f, const int* is_cat
     int mx = 2;  // Binner::max_bins (binning.cpp:130-134): vocabulary + missing, or edges + 2
     for (int f = 0; f < n_f; ++f) mx = std::max(mx, n_edges[f] + (is_cat[f] ? 1 : 2));
     return std::max(mx, max_bin);
+}
+
+int binner_fit_cat(const void* X, int x_dtype, int n, int n_f, const int* is_cat, int max_bin, int cat_min_count,
+                   int bin_sample, uint32_t seed, std::vector<double>& edges, std::vector<int>& n_edges,
+                   int n_threads) {
+    binner_fit(X, x_dtype, n, n_f, max_bin, bin_sample, seed, edges, n_edges, n_threads);
+    return binner_add_vocabularies(X, x_dtype, n, n_f, is_cat, max_bin, cat_min_count, edges, n_edges, n_threads);
 }
 
 int binner_fit(const void* X, int x_dtype, int n, int n_f, int max_bin, int bin_sample, uint32_t seed,

@@ -573,18 +573,20 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
         D.edges_dtype = -1;
         const double tbf = now();
         BinFitTimes bt;
-        if (any_cat) {
-            // vocabularies of the categorical features (binning.cpp:47-84) on the host, the
-            // numeric features' edges with them (the host binner, bit-identical)
-            B.n_bins = binner_fit_cat(X, x_dtype, n, n_f, B.is_cat.data(), c.max_bin, c.cat_min_count, c.bin_sample,
-                                      static_cast<uint32_t>(c.random_state), B.edges, B.n_edges, n_threads);
-        } else if (binner_fits_device(n, n_f, c.bin_sample))
+        // With categorical features the numeric ones' edges come from the device all the same
+        // (bit-identical to the host binner's) and the vocabularies (binning.cpp:47-84) from the
+        // host's X.
+        const int* cats = any_cat ? B.is_cat.data() : nullptr;
+        if (binner_fits_device(n, n_f, c.bin_sample))
             B.n_bins = binner_fit_device(Xd.p, x_dtype, n, n_f, c.max_bin, c.bin_sample,
                                          static_cast<uint32_t>(c.random_state), B.edges, B.n_edges, n_threads, s,
-                                         D.codes_col.p, D.codes_col.n, &bt, X);  // scratch: codes_col, filled later
+                                         D.codes_col.p, D.codes_col.n, &bt, X, cats);  // scratch: codes_col, filled later
         else
             B.n_bins = binner_fit(X, x_dtype, n, n_f, c.max_bin, c.bin_sample, static_cast<uint32_t>(c.random_state),
                                   B.edges, B.n_edges, n_threads);
+        if (cats)
+            B.n_bins = binner_add_vocabularies(X, x_dtype, n, n_f, cats, c.max_bin, c.cat_min_count, B.edges, B.n_edges,
+                                               n_threads);
         B.n_features = n_f;
         st.t_binfit = now() - tbf;
         st.t_bin_counts = bt.counts;

@@ -198,6 +198,10 @@ int binner_fit(const void* X, int x_dtype, int n, int n_f, int max_bin, int bin_
 int binner_fit_cat(const void* X, int x_dtype, int n, int n_f, const int* is_cat, int max_bin, int cat_min_count,
                    int bin_sample, uint32_t seed, std::vector<double>& edges, std::vector<int>& n_edges,
                    int n_threads);
+// Its second half: the vocabularies of the features with is_cat[f] != 0 over the edges of all
+// features (X on the host).  Returns max_bins().
+int binner_add_vocabularies(const void* X, int x_dtype, int n, int n_f, const int* is_cat, int max_bin,
+                            int cat_min_count, std::vector<double>& edges, std::vector<int>& n_edges, int n_threads);
 // The same edges from X in device memory (row-major n x n_f, stream `stream`, a
 // cudaStream_t).  binner_fits_device says whether one feature-major sample buffer of
 // the sizes involved stays under 2^31 values (else use binner_fit).
@@ -235,6 +239,7 @@ int binner_fit_from_plan(const BinPlan& plan, const void* Xd, int x_dtype, int n
 // X_host (optional): the same X on the host, read when features are recomputed there.
 int binner_fit_device(const void* Xd, int x_dtype, int n, int n_f, int max_bin, int bin_sample, uint32_t seed,
                       std::vector<double>& edges, std::vector<int>& n_edges, int n_threads, void* stream,
-                      void* arena, size_t arena_bytes, BinFitTimes* tm, const void* X_host = nullptr);
+                      void* arena, size_t arena_bytes, BinFitTimes* tm, const void* X_host = nullptr,
+                      const int* skip = nullptr);
 
 }  // namespace tgb
