@@ -604,6 +604,16 @@ __device__ __noinline__ void accumulate_var(unsigned int* __restrict__ P, unsign
     }
 }
 
+// One piece of a cluster's work: a CTA's rows of a (job, feature group) and where its sums go.
+struct HistPiece {
+    const int32_t* rows;
+    const void* gq;
+    const void* hq;
+    unsigned long long hq1, hq2;  // fixed-point hessians of the two row classes
+    size_t out0;                  // first cell of the group in the job's slot
+    int c, r0, r1, fg0, nf, whole;
+};
+
 // A cell's totals summed over the cluster, and its hessian and count in the output's form.
 template <bool kVar>
 struct CellSum {
@@ -617,10 +627,12 @@ struct CellSum {
 // global writes, so that nothing waits for those.
 template <bool kVar, int CS>
 __device__ __forceinline__ void flush_piece(const WaveCtx& X, const unsigned long long* Gt, const unsigned long long* Ht,
-                                            const unsigned int* Ct, unsigned int rank, int nf_here, size_t out0, bool whole,
-                                            unsigned long long hq1, unsigned long long hq2) {
+                                            const unsigned int* Ct, unsigned int rank, const HistPiece& piece) {
+    const bool whole = piece.whole != 0;
+    const unsigned long long hq1 = piece.hq1, hq2 = piece.hq2;
+    const size_t out0 = piece.out0;
     constexpr int kIter = kPlane / CS / kThreads;  // cells a thread writes (8, 4 or 2)
-    const int share = nf_here * kBins / CS;
+    const int share = piece.nf * kBins / CS;
     const int i0 = static_cast<int>(rank) * share + static_cast<int>(threadIdx.x);
     const int i1 = static_cast<int>(rank + 1) * share;
     CellSum<kVar> v[kIter];
@@ -695,6 +707,9 @@ __device__ __forceinline__ void flush_piece(const WaveCtx& X, const unsigned lon
 // the barrier, then the writes; nothing to clear).  Together with the pairs' own clusters:
 // fits of 0.85M x 64 pairwise 92.2 -> 83.5 ms, 1.2M x 96 int8 97.0 -> 84.3 ms, 10M x 128
 // 435 -> 416 ms.
+//
+// The plan and each piece's parameters are worked out by one warp and left in shared memory:
+// 32 warps doing the same scalar work (64-bit divisions above all) took 8,000 cycles a piece.
 constexpr int kPieceRows = 1500;
 constexpr int kMinCtaRows = 128;  // no finer split of a pair: a CTA's fold and flush cost more
 constexpr int kWarpJobs = 32;
@@ -742,14 +757,20 @@ __global__ void __launch_bounds__(kThreads, 1)
     // ---- work plan (the same in every CTA) ----
     __shared__ int s_cpref[kMaxWaveCtx + 1];
     __shared__ unsigned long long s_red[kWarps], s_rsum[kWarps];
-    __shared__ int s_cstart[kWarpJobs + 1], s_cper[kWarpJobs], s_aligned;
-    __shared__ unsigned long long s_hq[2];
+    __shared__ HistPiece s_piece;
+    __shared__ int s_more, s_aligned;
     cg::cluster_group cluster = cg::this_cluster();
     const int csize = static_cast<int>(cluster.dim_blocks().y);  // CTAs per cluster: 1, 2 or 4
     const int cl = static_cast<int>(blockIdx.y) / csize;
     const int n_cl = static_cast<int>(gridDim.y) / csize;
     const unsigned int rank = csize > 1 ? cluster.block_rank() : 0u;
+    // warp 0 only: the cluster's own pair (aligned), and how far its rows are handed out
+    bool aligned = false;
+    int a_job = -1, a_fg = 0, a_rows = 0, a_row = 0, a_end = 0;
     if (warp == 0) {
+        // with one context the lane's job is read along with the number of jobs
+        int early = 0;
+        if (n_ctx == 1) early = job_count(s_ctx, src, lane);
         int all = 0;
         for (int c0 = 0; c0 < n_ctx; c0 += 32) {
             const int c = c0 + lane;
@@ -776,7 +797,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             if (lane < nj) {
                 int c = 0;
                 while (c + 1 < n_ctx && s_cpref[c + 1] <= lane) ++c;
-                count = job_count(ctx_of(c), src, lane - s_cpref[c]);
+                count = n_ctx == 1 ? early : job_count(ctx_of(c), src, lane - s_cpref[c]);
                 groups = (ctx_of(c).gp.n_features + kFG - 1) / kFG;
             }
             const unsigned long long w = static_cast<unsigned long long>(count) * groups;
@@ -809,18 +830,11 @@ __global__ void __launch_bounds__(kThreads, 1)
                 for (int o = 16; o > 0; o >>= 1) used += __shfl_xor_sync(0xffffffffu, used, o);
                 for (int it = 0; it < 8; ++it) {
                     const bool can = groups > 0 && per < cap && groups <= n_cl - used;
-                    float share = can ? static_cast<float>(count) / static_cast<float>(per) : -1.f;
-                    int who = lane;
-#pragma unroll
-                    for (int o = 16; o > 0; o >>= 1) {
-                        const float os = __shfl_xor_sync(0xffffffffu, share, o);
-                        const int ow = __shfl_xor_sync(0xffffffffu, who, o);
-                        if (os > share || (os == share && ow < who)) {
-                            share = os;
-                            who = ow;
-                        }
-                    }
-                    if (share < 0.f) break;
+                    // positive floats order like their bits; 0: no job can take another cluster
+                    const unsigned share = can ? __float_as_uint(__fdividef(static_cast<float>(count), static_cast<float>(per))) : 0u;
+                    const unsigned top = __reduce_max_sync(0xffffffffu, share);
+                    if (top == 0u) break;
+                    const int who = __ffs(__ballot_sync(0xffffffffu, share == top)) - 1;
                     if (lane == who) ++per;
                     used += __shfl_sync(0xffffffffu, groups, who);
                 }
@@ -833,11 +847,19 @@ __global__ void __launch_bounds__(kThreads, 1)
                     if (lane >= o) cs += t;
                 }
                 if (most <= static_cast<float>(w_all) / static_cast<float>(n_cl) + static_cast<float>(kPieceRows * csize)) {
-                    if (lane < nj) {
-                        s_cstart[lane] = cs - groups * per;
-                        s_cper[lane] = per;
-                    }
-                    if (lane == 31) s_cstart[nj] = cs;
+                    // this cluster's pair: the job whose clusters hold it, the pair's rows in
+                    // per equal parts (the first ones a row longer)
+                    aligned = true;
+                    const unsigned mine = __ballot_sync(0xffffffffu, cl >= cs - groups * per && cl < cs);
+                    const int src_lane = mine ? __ffs(mine) - 1 : 0;
+                    a_job = mine ? src_lane : -1;
+                    const int q = cl - __shfl_sync(0xffffffffu, cs - groups * per, src_lane);
+                    const int jper = __shfl_sync(0xffffffffu, per, src_lane), R = __shfl_sync(0xffffffffu, count, src_lane);
+                    a_fg = q / jper;
+                    const int k = q - a_fg * jper, part = R / jper, longer = R - part * jper;
+                    a_rows = R;
+                    a_row = part * k + min(k, longer);
+                    a_end = a_row + part + (k < longer ? 1 : 0);
                     if (lane == 0) s_aligned = 1;
                 }
             }
@@ -889,71 +911,95 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
         __syncthreads();
     }
-    unsigned long long w, w_end;
-    if (s_aligned) {
-        if (cl >= s_cstart[n_jobs]) return;  // no pair for this cluster
-        int lo = 0, hi = n_jobs - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (s_cstart[mid] <= cl) lo = mid;
-            else hi = mid - 1;
-        }
-        const int q = cl - s_cstart[lo], per = s_cper[lo], fg = q / per, k = q - fg * per;
-        const unsigned int groups = static_cast<unsigned int>((s_cstart[lo + 1] - s_cstart[lo]) / per);
-        const unsigned long long R = (s_wstart[lo + 1] - s_wstart[lo]) / groups;
-        const unsigned long long w0 = s_wstart[lo] + R * fg;
-        w = w0 + R * k / per;
-        w_end = w0 + R * (k + 1) / per;
-    } else {
+    unsigned long long w = 0, w_end = 0;  // warp 0, without pairs of their own: the range's work
+    if (warp == 0 && !s_aligned) {
         const unsigned long long w_all = s_wstart[n_jobs];
         w = w_all * static_cast<unsigned long long>(cl) / static_cast<unsigned long long>(n_cl);
         w_end = w_all * static_cast<unsigned long long>(cl + 1) / static_cast<unsigned long long>(n_cl);
     }
-    const unsigned long long max_piece = static_cast<unsigned long long>(kMaxShareRows) * csize;
-    while (w < w_end) {
-        // the job holding w: the last j with s_wstart[j] <= w (a non-empty job)
-        int lo = 0, hi = n_jobs - 1;
-        while (lo < hi) {
-            const int mid = (lo + hi + 1) >> 1;
-            if (s_wstart[mid] <= w) lo = mid;
-            else hi = mid - 1;
+    const int max_piece = kMaxShareRows * csize;
+    while (true) {
+        if (warp == 0) {
+            // the next piece: job, feature group and rows
+            int j = -1, fg = 0, R = 0, piece0 = 0, piece1 = 0;
+            if (aligned) {
+                if (a_row < a_end && a_job >= 0) {
+                    j = a_job;
+                    fg = a_fg;
+                    R = a_rows;
+                    piece0 = a_row;
+                    piece1 = min(a_end, a_row + max_piece);
+                    a_row = piece1;
+                }
+            } else if (w < w_end) {
+                // the job holding w: the last j with s_wstart[j] <= w (a non-empty job)
+                int lo = 0, hi = n_jobs - 1;
+                while (lo < hi) {
+                    const int mid = (lo + hi + 1) >> 1;
+                    if (s_wstart[mid] <= w) lo = mid;
+                    else hi = mid - 1;
+                }
+                j = lo;
+                int c = 0;
+                while (c + 1 < n_ctx && s_cpref[c + 1] <= j) ++c;
+                R = job_count(ctx_of(c), src, src == 0 ? 0 : j - s_cpref[c]);
+                const unsigned long long off = w - s_wstart[j];
+                fg = static_cast<int>(off / static_cast<unsigned long long>(R));
+                piece0 = static_cast<int>(off - static_cast<unsigned long long>(fg) * R);
+                const unsigned long long len =
+                    min(min(static_cast<unsigned long long>(R - piece0), w_end - w), static_cast<unsigned long long>(max_piece));
+                piece1 = piece0 + static_cast<int>(len);
+                w += len;
+            }
+            if (lane == 0) s_more = j >= 0;
+            if (j >= 0) {
+                int c = 0;
+                while (c + 1 < n_ctx && s_cpref[c + 1] <= j) ++c;
+                const WaveCtx& X = ctx_of(c);
+                if (lane == 0) {
+                    const JobRows jr = job_rows(X, src, src == 0 ? 0 : j - s_cpref[c]);
+                    const int q = (piece1 - piece0 + csize - 1) / csize;
+                    HistPiece p;
+                    p.rows = jr.rows;
+                    p.gq = jr.gq;
+                    p.hq = jr.hq;
+                    p.c = c;
+                    p.r0 = min(piece1, piece0 + static_cast<int>(rank) * q);
+                    p.r1 = min(piece1, p.r0 + q);
+                    p.fg0 = fg * kFG;
+                    p.nf = min(kFG, X.gp.n_features - p.fg0);
+                    p.whole = piece0 == 0 && piece1 == R;
+                    p.out0 = (static_cast<size_t>(jr.slot) * static_cast<size_t>(X.gp.n_features) + p.fg0) * kBins;
+                    p.hq1 = p.hq2 = 0ull;
+                    if (!T::var) {
+                        const double hscale = X.st->hscale;
+                        p.hq1 = static_cast<unsigned long long>(__double2ll_rn(1.0 * hscale));
+                        p.hq2 = static_cast<unsigned long long>(__double2ll_rn(1.0 * X.goss_scale * hscale));
+                    }
+                    s_piece = p;
+                }
+            }
         }
-        const int j = lo;
-        int c = 0;
-        while (c + 1 < n_ctx && s_cpref[c + 1] <= j) ++c;
-        const WaveCtx& X = ctx_of(c);
-        const int n_f = X.gp.n_features;
-        const JobRows jr = job_rows(X, src, src == 0 ? 0 : j - s_cpref[c]);
-        const unsigned long long R = static_cast<unsigned long long>(jr.count);
-        const unsigned long long off = w - s_wstart[j];
-        const int fg = static_cast<int>(off / R);
-        const unsigned long long ra = off - static_cast<unsigned long long>(fg) * R;
-        const unsigned long long len = min(min(R - ra, w_end - w), max_piece);
-        const int piece0 = static_cast<int>(ra), piece1 = static_cast<int>(ra + len);
-        const int qrows = (piece1 - piece0 + csize - 1) / csize;
-        const int r0 = min(piece1, piece0 + static_cast<int>(rank) * qrows), r1 = min(piece1, r0 + qrows);
-        const int fg0 = fg * kFG;
-        if (!T::var && threadIdx.x == 0) {  // the fixed-point hessians of the two row classes, for the flush
-            const double hscale = X.st->hscale;
-            s_hq[0] = static_cast<unsigned long long>(__double2ll_rn(1.0 * hscale));
-            s_hq[1] = static_cast<unsigned long long>(__double2ll_rn(1.0 * X.goss_scale * hscale));
-        }
-        if constexpr (T::var)
-            accumulate_var<kMode>(P, Gt, Ht, Ct, jr.rows, r0, r1, X.codes, X.gp.stride, fg0, jr.gq, jr.hq);
-        else if (X.codes_map_ok && (reinterpret_cast<uintptr_t>(&ctxs[c].codes_map) & 63u) == 0)  // TMA wants 64 B
-            phase = accumulate_const_tma<kMode>(P, Gt, Ct, stage, s_bars, phase, jr.rows, r0, r1, &ctxs[c].codes_map, fg0,
-                                                jr.gq, &X.ctl->error);
-        else
-            accumulate_const<kMode>(P, Gt, Ct, jr.rows, r0, r1, X.codes, X.gp.stride, fg0, jr.gq);
         __syncthreads();
-        const bool whole = piece0 == 0 && static_cast<unsigned long long>(piece1) == R;
-        const int nf_here = min(kFG, n_f - fg0);
-        const size_t out0 = (static_cast<size_t>(jr.slot) * static_cast<size_t>(n_f) + fg0) * kBins;
-        if (csize == 1) flush_piece<T::var, 1>(X, Gt, Ht, Ct, rank, nf_here, out0, whole, s_hq[0], s_hq[1]);
-        else if (csize == 2) flush_piece<T::var, 2>(X, Gt, Ht, Ct, rank, nf_here, out0, whole, s_hq[0], s_hq[1]);
-        else flush_piece<T::var, 4>(X, Gt, Ht, Ct, rank, nf_here, out0, whole, s_hq[0], s_hq[1]);
-        w += len;
-        if (T::var && w < w_end) {  // the totals lie over the planes: clear for the next piece
+        if (!s_more) break;
+        const WaveCtx& X = ctx_of(s_piece.c);
+        if constexpr (T::var)
+            accumulate_var<kMode>(P, Gt, Ht, Ct, s_piece.rows, s_piece.r0, s_piece.r1, X.codes, X.gp.stride, s_piece.fg0,
+                                  s_piece.gq, s_piece.hq);
+        else if (X.codes_map_ok && (reinterpret_cast<uintptr_t>(&ctxs[s_piece.c].codes_map) & 63u) == 0)  // TMA: 64 B
+            phase = accumulate_const_tma<kMode>(P, Gt, Ct, stage, s_bars, phase, s_piece.rows, s_piece.r0, s_piece.r1,
+                                                &ctxs[s_piece.c].codes_map, s_piece.fg0, s_piece.gq, &X.ctl->error);
+        else
+            accumulate_const<kMode>(P, Gt, Ct, s_piece.rows, s_piece.r0, s_piece.r1, X.codes, X.gp.stride, s_piece.fg0,
+                                    s_piece.gq);
+        __syncthreads();
+        if (csize == 1) flush_piece<T::var, 1>(X, Gt, Ht, Ct, rank, s_piece);
+        else if (csize == 2) flush_piece<T::var, 2>(X, Gt, Ht, Ct, rank, s_piece);
+        else flush_piece<T::var, 4>(X, Gt, Ht, Ct, rank, s_piece);
+        if (T::var) {  // the totals lie over the planes: clear for a next piece (rare: most take one)
+            if (warp == 0 && lane == 0) s_more = aligned ? a_row < a_end : w < w_end;
+            __syncthreads();
+            if (!s_more) break;
             uint4* z = reinterpret_cast<uint4*>(smem_raw);
             for (int k = threadIdx.x; k < static_cast<int>(Lay::region / 16); k += kThreads) z[k] = make_uint4(0, 0, 0, 0);
             __syncthreads();
