@@ -196,7 +196,7 @@ struct DeviceState {
     DBuf<int> bucket_seg_end, cuts;
     DBuf<AllScale> all_scale;
     DBuf<double> init_prefix, values_all, prefix_all, losses, loss_part;
-    DBuf<int> cover_all, loss_valid;
+    DBuf<int> cover_all, loss_valid, loss_ticket;
     DBuf<int> run_start, run_len, order;
     // batched growth (wave.h)
     DBuf<unsigned char> gqw, hqw;  // per-row histogram payloads (mode dependent, <= 8 B a row)
@@ -235,7 +235,7 @@ struct DeviceState {
         rest_pos.release(); cub_tmp.release(); goss_flag.release(); nid.release(); seg_sums.release();
         chunks.release(); bucket_seg_end.release(); cuts.release(); all_scale.release(); init_prefix.release();
         values_all.release(); prefix_all.release(); losses.release(); loss_part.release(); cover_all.release();
-        loss_valid.release(); run_start.release(); run_len.release(); order.release();
+        loss_valid.release(); loss_ticket.release(); run_start.release(); run_len.release(); order.release();
         gqw.release(); hqw.release(); spec.release(); spec_split.release(); ctl.release(); cand_gain.release();
         cand_key.release(); tickets.release(); wctx.release(); cand_cat.release(); splits_pair.release();
         spec_split_pair.release(); energy.release(); pair_G.release(); pair_H.release(); pair_C.release();
@@ -550,6 +550,10 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
     }
     D.nid.alloc(n, s);
     D.all_scale.alloc(1, s);
+    D.loss_ticket.alloc(1, s);
+    check(cudaMemsetAsync(D.all_scale.p, 0, sizeof(AllScale), s), "scale reset");
+    check(cudaMemsetAsync(D.st.p, 0, sizeof(DevTreeState), s), "state reset");
+    check(cudaMemsetAsync(D.loss_ticket.p, 0, sizeof(int), s), "ticket reset");
     D.init_prefix.alloc(nbk, s);
     D.nodes_all.alloc(static_cast<size_t>(T) * max_nodes, s);
     D.st_all.alloc(T, s);
@@ -647,7 +651,9 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
     std::vector<int> seg_end(nbk, 0);
     for (int b = 0; b < nbk && !c.iid_mode; ++b)
         seg_end[b] = cut[b] > 0 ? static_cast<int>(std::lower_bound(bounds.begin(), bounds.end(), cut[b]) - bounds.begin()) + 1 : 0;
-    const int kChunk = 8192;
+    // rows of a CTA's chunk in the post-tree sweep: enough chunks for three CTAs on every SM
+    // (100k rows in 8,192-row chunks ran on 32 CTAs: 20 us a tree)
+    const int kChunk = std::max(512, std::min(8192, (n / (148 * 3) + 511) / 512 * 512));
     chunks.clear();
     for (int k = 0, lo = 0; k < static_cast<int>(bounds.size()); lo = bounds[k], ++k)
         for (int a = lo; a < bounds[k]; a += kChunk) chunks.push_back(make_int4(k, a, std::min(bounds[k], a + kChunk), 0));
@@ -703,7 +709,7 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
         }
         check(cudaStreamSynchronize(s), "runs upload");
     } else {
-        D.loss_part.alloc(2368, s);
+        D.loss_part.alloc(pred_update_parts(n), s);
     }
 
     // GOSS device buffers (the sample itself is set up with the sampler, above).
@@ -794,15 +800,17 @@ WaveCtx FitRun::wave_ctx() const {
 // histogram scales, and the per-row histogram payload.
 void FitRun::tree_begin(int t) {
     const bool wave = c.grow != 0;
+    // the maxima of the gradients go to all_scale, reset at the fit's start and by tree_end
     if (const_h) {
         if (!g_ready) launch_grad_mse_fused(D.y.p, D.pred.p, n, D.g.p, D.all_scale.p, s);
         g_ready = false;
-        launch_all_scale_finalize(D.all_scale.p, n, s);
     } else {
-        launch_grad_pairwise(D.y.p, D.pred.p, D.run_start.p, D.run_len.p, order_d, n_runs, n, D.g.p, D.h.p, s);
-        launch_all_scale(D.g.p, D.h.p, n, D.all_scale.p, s);
+        launch_grad_pairwise(D.y.p, D.pred.p, D.run_start.p, D.run_len.p, order_d, n_runs, n, D.g.p, D.h.p,
+                             D.all_scale.p, s);
     }
     const double* h_rows = const_h ? nullptr : D.h.p;
+    const size_t slot = static_cast<size_t>(n_f) * kBins;
+    const size_t seg_words = static_cast<size_t>(n_segments) * kMaxNodes * 3;
     if (use_goss) {
         const double tr = now();
         const int32_t* pos = sampler->wait(t);  // host time spent waiting for the draw
@@ -812,22 +820,18 @@ void FitRun::tree_begin(int t) {
         sampler->release(t, s);
         launch_goss_select(D.g.p, h_rows, n, n_top, n_other, D.rest_pos.p, sampler->min_pos(t), gw, D.all_scale.p,
                            goss_scale, D.goss_flag.p, D.rows0.p, D.tile_counts.p, D.st.p, s);
-        if (wave) {
-            launch_wave_tree_init(D.nodes.p, D.splits.p, D.st.p, D.ctl.p, 0, 1, s);
-            launch_wave_scales(D.st.p, nullptr, mode, s);
-        } else {
-            launch_tree_init(D.nodes.p, D.splits.p, D.st.p, 0, 1, s);
-            launch_scales(D.st.p, nullptr, c.hist_bits == 8, s);
-        }
+    }
+    if (wave) {
+        launch_wave_begin(WaveBegin{D.nodes.p, D.splits.p, D.st.p, D.ctl.p, D.all_scale.p, D.histG.p, D.histH.p, D.histC.p,
+                                    slot, D.seg_sums.p, seg_words, c.pair_splits ? D.energy.p + 2 * kMaxNodes : nullptr,
+                                    D.rows0.p, n, use_goss ? 1 : 0, mode},
+                          s);
     } else {
-        launch_iota_rows(D.rows0.p, n, s);
-        if (wave) {
-            launch_wave_tree_init(D.nodes.p, D.splits.p, D.st.p, D.ctl.p, n, 0, s);
-            launch_wave_scales(D.st.p, D.all_scale.p, mode, s);
-        } else {
-            launch_tree_init(D.nodes.p, D.splits.p, D.st.p, n, 0, s);
-            launch_scales(D.st.p, D.all_scale.p, c.hist_bits == 8, s);
-        }
+        launch_all_scale_finalize(D.all_scale.p, n, s);
+        if (!use_goss) launch_iota_rows(D.rows0.p, n, s);
+        launch_tree_init(D.nodes.p, D.splits.p, D.st.p, use_goss ? 0 : n, use_goss ? 1 : 0, s);
+        launch_scales(D.st.p, use_goss ? nullptr : D.all_scale.p, c.hist_bits == 8, s);
+        check(cudaMemsetAsync(D.seg_sums.p, 0, sizeof(unsigned long long) * seg_words, s), "seg sums reset");
     }
     const uint8_t* flag = use_goss ? D.goss_flag.p : nullptr;
     // per-tree stream of the stochastic rounding (SplitMix64 of seed and tree)
@@ -836,16 +840,10 @@ void FitRun::tree_begin(int t) {
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
     const uint64_t seed = z ^ (z >> 31);
-    const size_t slot = static_cast<size_t>(n_f) * kBins;
     if (wave) {
-        unsigned long long* root_energy = c.pair_splits ? D.energy.p + 2 * kMaxNodes : nullptr;
-        if (root_energy) check(cudaMemsetAsync(root_energy, 0, sizeof(unsigned long long), s), "energy reset");
+        // (the children's histogram slots are cleared by the partition of their wave)
         launch_wave_quantize(mode, D.rows0.p, D.g.p, h_rows, flag, goss_scale, D.st.p, seed, D.gqw.p, D.hqw.p,
-                             root_energy, n, s);
-        // the root's slot; the children's slots are cleared by the partition of their wave
-        check(cudaMemsetAsync(D.histG.p, 0, sizeof(long long) * slot, s), "hist reset");
-        check(cudaMemsetAsync(D.histH.p, 0, sizeof(long long) * slot, s), "hist reset");
-        check(cudaMemsetAsync(D.histC.p, 0, sizeof(int) * slot, s), "hist reset");
+                             c.pair_splits ? D.energy.p + 2 * kMaxNodes : nullptr, n, s);
     } else {
         if (c.hist_bits == 8)
             launch_quantize8(D.rows0.p, D.g.p, flag, goss_scale, D.st.p, seed, D.gq8.p, n, s);
@@ -891,27 +889,22 @@ void FitRun::tree_end(int t) {
     double* prefix_t = D.prefix_all.p + static_cast<size_t>(t) * nbk * max_nodes;
     int* cover_t = D.cover_all.p + static_cast<size_t>(t) * max_nodes;
     launch_apply_accum(D.codes_col.p, codes_col_pitch(n), n_f, D.nodes.p, D.st.p, D.g.p, h_rows, D.chunks.p,
-                       static_cast<int>(chunks.size()), D.all_scale.p, D.nid.p, D.seg_sums.p, n_segments, B.n_bins,
+                       static_cast<int>(chunks.size()), D.all_scale.p, D.nid.p, D.seg_sums.p, B.n_bins,
                        (any_cat ? 1 : 0) | (c.pair_splits ? 2 : 0), s);
     launch_finalize_tree(pp, D.st.p, D.seg_sums.p, D.bucket_seg_end.p, D.cuts.p, D.all_scale.p, values_t, cover_t,
-                         prefix_t, s);
+                         prefix_t, D.nodes.p, D.nodes_all.p + static_cast<size_t>(t) * max_nodes, D.st_all.p + t,
+                         max_nodes, s);
     if (const_h) {
         // the next tree's gradient from the same pass (not after the last tree)
         g_ready = t + 1 < T;
-        launch_pred_update_loss(pp, D.nid.p, prefix_t, D.st.p, D.pred.p, D.y.p, D.loss_part.p, 2368,
-                                g_ready ? D.g.p : nullptr, g_ready ? D.all_scale.p : nullptr, s);
-        launch_loss_finalize(0, D.loss_part.p, nullptr, 2368, n, D.losses.p + t, s);
+        launch_pred_update_loss(pp, D.nid.p, prefix_t, D.st.p, D.pred.p, D.y.p, D.loss_part.p,
+                                g_ready ? D.g.p : nullptr, g_ready ? D.all_scale.p : nullptr, D.loss_ticket.p,
+                                D.losses.p + t, s);
     } else {
         launch_pred_update(pp, D.nid.p, prefix_t, D.st.p, D.pred.p, s);
         launch_loss_pairwise(D.y.p, D.pred.p, D.run_start.p, D.run_len.p, order_d, n_runs, D.loss_part.p,
-                             D.loss_valid.p, s);
-        launch_loss_finalize(5, D.loss_part.p, D.loss_valid.p, n_runs, n, D.losses.p + t, s);
+                             D.loss_valid.p, D.loss_ticket.p, D.losses.p + t, s);
     }
-    check(cudaMemcpyAsync(D.nodes_all.p + static_cast<size_t>(t) * max_nodes, D.nodes.p, sizeof(DevNode) * max_nodes,
-                          cudaMemcpyDeviceToDevice, s),
-          "nodes snapshot");
-    check(cudaMemcpyAsync(D.st_all.p + t, D.st.p, sizeof(DevTreeState), cudaMemcpyDeviceToDevice, s),
-          "state snapshot");
 }
 
 bool FitRun::finish() {

@@ -576,7 +576,7 @@ int tgb_grad_mse(const double* y, const double* pred, int n, double* g, double* 
 int tgb_grad_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len, const int* order,
                       int n_runs, int n, double* g, double* h, void* stream) {
     return guard([&] {
-        tgb::launch_grad_pairwise(y, pred, run_start, run_len, order, n_runs, n, g, h, as_stream(stream));
+        tgb::launch_grad_pairwise(y, pred, run_start, run_len, order, n_runs, n, g, h, nullptr, as_stream(stream));
     });
 }
 

@@ -119,14 +119,27 @@ __global__ void goss_mark_kernel(const int32_t* __restrict__ order, const unsign
             mh = fmax(mh, top ? 1.0 : fabs(1.0 * goss_scale));
         }
     }
+    // one atomic a CTA and maximum, where there is one
+    __shared__ double s_mg[8], s_mh[8];
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
         mh = fmax(mh, __shfl_xor_sync(0xffffffffu, mh, o));
     }
-    if ((threadIdx.x & 31) == 0 && (mg > 0.0 || mh > 0.0)) {
-        atomicMax(&st->max_abs_g_bits, static_cast<unsigned long long>(__double_as_longlong(mg)));
-        atomicMax(&st->max_h_bits, static_cast<unsigned long long>(__double_as_longlong(mh)));
+    if ((threadIdx.x & 31) == 0) {
+        s_mg[threadIdx.x >> 5] = mg;
+        s_mh[threadIdx.x >> 5] = mh;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
+            mg = fmax(mg, s_mg[w]);
+            mh = fmax(mh, s_mh[w]);
+        }
+        if (mg > 0.0 || mh > 0.0) {
+            atomicMax(&st->max_abs_g_bits, static_cast<unsigned long long>(__double_as_longlong(mg)));
+            atomicMax(&st->max_h_bits, static_cast<unsigned long long>(__double_as_longlong(mh)));
+        }
     }
 }
 
@@ -180,7 +193,6 @@ void launch_goss_select(const double* g, const double* h, int n, int n_top, int 
     const unsigned int* k32 = w.exact ? nullptr : static_cast<const unsigned int*>(w.keys_out);
     const int32_t* fixed = static_cast<const int32_t*>(w.keys_in);
     check(cudaMemsetAsync(goss_flag, 0, static_cast<size_t>(n), s), "goss flag reset");
-    check(cudaMemsetAsync(&st->max_abs_g_bits, 0, 2 * sizeof(unsigned long long), s), "sample max reset");
     goss_mark_kernel<<<std::max(1, std::min(2368, (n_top + n_other + 255) / 256)), 256, 0, s>>>(
         w.vals_out, k32, fixed, n, n_top, n_other, rest_pos, min_rest, g, h, goss_scale, goss_flag, st);
     check(cudaGetLastError(), "goss_mark launch");

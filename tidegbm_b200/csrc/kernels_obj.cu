@@ -37,12 +37,7 @@ __global__ void grad_mse_fused_kernel(const double* __restrict__ y, const double
         g[i] = gv;
         mg = fmax(mg, fabs(gv));
     }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-    // Non-negative doubles order like their bit patterns.
-    if ((threadIdx.x & 31) == 0) atomicMax(&sc->maxg_bits, static_cast<unsigned long long>(__double_as_longlong(mg)));
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-        atomicMax(&sc->maxh_bits, static_cast<unsigned long long>(__double_as_longlong(1.0)));
+    block_max_into(mg, 1.0, sc);
 }
 
 __device__ __forceinline__ int row_at(const int* order, int p) { return order ? order[p] : p; }
@@ -76,7 +71,8 @@ __global__ void __launch_bounds__(kGradWarps * 32)
     grad_pairwise_kernel(const double* __restrict__ y, const double* __restrict__ pred,
                          const int* __restrict__ run_start, const int* __restrict__ run_len,
                          const int* __restrict__ order, double* __restrict__ g,
-                         double* __restrict__ h) {
+                         double* __restrict__ h, AllScale* __restrict__ sc) {
+    double mg = 0.0, mh = 0.0;
     __shared__ double2 s_terms[kGradWarps * kGradRoom];  // {lambda, hessian} of pair b (b - 1) / 2 + a, a < b
     __shared__ double2 s_rows[kGradWarps][kClassRows];   // {y, pred}
     __shared__ unsigned short s_ab[kClassRows * (kClassRows - 1) / 2];  // a | b << 8
@@ -90,9 +86,8 @@ __global__ void __launch_bounds__(kGradWarps * 32)
     __syncthreads();
     const int span = max(1, (most * (most - 1) / 2 + kGradRoom - 1) / kGradRoom);  // warps' room a class takes
     const int warps = kGradWarps / span;
-    if (warp >= warps) return;
     double2 *terms = s_terms + warp * span * kGradRoom, *cls = s_rows[warp];
-    for (int c = warp; c < step && c < m; c += warps) {
+    for (int c = warp < warps ? warp : m; c < step && c < m; c += warps) {
         const int K = (m - c + step - 1) / step, n_pairs = K * (K - 1) / 2;
         int row[2];
         bool nan = false;
@@ -125,6 +120,8 @@ __global__ void __launch_bounds__(kGradWarps * 32)
                 }
                 g[row[q]] = ga;
                 h[row[q]] = ha;
+                mg = fmax(mg, fabs(ga));
+                mh = fmax(mh, fabs(ha));
             }
             __syncwarp();
             continue;
@@ -158,37 +155,23 @@ __global__ void __launch_bounds__(kGradWarps * 32)
             }
             g[row[q]] = ga;
             h[row[q]] = ha;
+            mg = fmax(mg, fabs(ga));
+            mh = fmax(mh, fabs(ha));
         }
         __syncwarp();
     }
-}
-
-__global__ void loss_mse_kernel(const double* __restrict__ y, const double* __restrict__ pred, int n,
-                                double* __restrict__ partials) {
-    double s = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const double d = pred[i] - y[i];
-        s += 1.0 * d * d;
-    }
-    __shared__ double ws[32];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double t = 0.0;
-        for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += ws[w];
-        partials[blockIdx.x] = t;
-    }
+    if (sc != nullptr) block_max_into(mg, mh, sc);
 }
 
 __global__ void loss_pairwise_kernel(const double* __restrict__ y, const double* __restrict__ pred,
                                      const int* __restrict__ run_start, const int* __restrict__ run_len,
                                      const int* __restrict__ order, double* __restrict__ corr,
-                                     int* __restrict__ valid) {
+                                     int* __restrict__ valid, int* __restrict__ ticket, double* __restrict__ loss) {
     const int r = blockIdx.x;
     const int s0 = run_start[r], m = run_len[r];
     __shared__ double red[3][32];
     __shared__ double mean[2];
+    __shared__ int s_last;
     double sy = 0, sp = 0;
     for (int k = threadIdx.x; k < m; k += blockDim.x) {
         const int i = row_at(order, s0 + k);
@@ -245,54 +228,41 @@ __global__ void loss_pairwise_kernel(const double* __restrict__ y, const double*
         const bool ok = m >= 3 && a > 1e-18 && b > 1e-18;
         corr[r] = ok ? cc / sqrt(a * b) : 0.0;
         valid[r] = ok ? 1 : 0;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
+        __threadfence();
     }
-}
-
-// kind 0: MSE = sum(partials) / n; kind 5: -mean(corr over valid runs).
-__global__ void loss_finalize_kernel(int kind, const double* __restrict__ partials, const int* __restrict__ valid,
-                                     int n_part, int n, double* __restrict__ out) {
-    __shared__ double ws[32];
-    __shared__ int wc[32];
-    double s = 0.0;
-    int c = 0;
-    for (int k = threadIdx.x; k < n_part; k += blockDim.x) {
-        if (kind == 5) {
-            if (valid[k]) {
-                s += partials[k];
-                c += 1;
-            }
-        } else {
-            s += partials[k];
+    __syncthreads();
+    if (!s_last) return;
+    // the last run to finish: minus the mean correlation over the valid runs, added in a fixed order
+    double t = 0.0;
+    int n_ok = 0;
+    for (int k = threadIdx.x; k < static_cast<int>(gridDim.x); k += blockDim.x)
+        if (__ldcg(valid + k)) {
+            t += __ldcg(corr + k);
+            n_ok += 1;
         }
-    }
     for (int o = 16; o > 0; o >>= 1) {
-        s += __shfl_xor_sync(0xffffffffu, s, o);
-        c += __shfl_xor_sync(0xffffffffu, c, o);
+        t += __shfl_xor_sync(0xffffffffu, t, o);
+        n_ok += __shfl_xor_sync(0xffffffffu, n_ok, o);
     }
     if ((threadIdx.x & 31) == 0) {
-        ws[threadIdx.x >> 5] = s;
-        wc[threadIdx.x >> 5] = c;
+        red[0][w] = t;
+        red[1][w] = static_cast<double>(n_ok);
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        double t = 0.0;
-        int tc = 0;
-        for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) {
-            t += ws[w];
-            tc += wc[w];
+        double a = 0, k_ok = 0;
+        for (int k = 0; k < nw; ++k) {
+            a += red[0][k];
+            k_ok += red[1][k];
         }
-        if (kind == 5) *out = tc > 0 ? -t / tc : 0.0;
-        else *out = n > 0 ? t / static_cast<double>(n) : 0.0;
+        *loss = k_ok > 0 ? -a / k_ok : 0.0;
+        *ticket = 0;
     }
 }
 
 }  // namespace
-
-void launch_loss_finalize(int kind, const double* partials, const int* valid, int n_part, int n, double* out,
-                          cudaStream_t s) {
-    loss_finalize_kernel<<<1, 1024, 0, s>>>(kind, partials, valid, n_part, n, out);
-    check(cudaGetLastError(), "loss_finalize launch");
-}
 
 void launch_grad_mse(const double* y, const double* pred, int n, double* g, double* h, cudaStream_t s) {
     if (n <= 0) return;
@@ -308,23 +278,18 @@ void launch_grad_mse_fused(const double* y, const double* pred, int n, double* g
 }
 
 void launch_grad_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len,
-                          const int* order, int n_runs, int n, double* g, double* h, cudaStream_t s) {
+                          const int* order, int n_runs, int n, double* g, double* h, AllScale* sc, cudaStream_t s) {
     (void)n;
     if (n_runs <= 0) return;
-    grad_pairwise_kernel<<<n_runs, kGradWarps * 32, 0, s>>>(y, pred, run_start, run_len, order, g, h);
+    grad_pairwise_kernel<<<n_runs, kGradWarps * 32, 0, s>>>(y, pred, run_start, run_len, order, g, h, sc);
     check(cudaGetLastError(), "grad_pairwise launch");
 }
 
-void launch_loss_mse(const double* y, const double* pred, int n, double* partials, int n_part,
-                     cudaStream_t s) {
-    loss_mse_kernel<<<n_part, 256, 0, s>>>(y, pred, n, partials);
-    check(cudaGetLastError(), "loss_mse launch");
-}
-
 void launch_loss_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len,
-                          const int* order, int n_runs, double* corr, int* valid, cudaStream_t s) {
+                          const int* order, int n_runs, double* corr, int* valid, int* ticket, double* loss,
+                          cudaStream_t s) {
     if (n_runs <= 0) return;
-    loss_pairwise_kernel<<<n_runs, 128, 0, s>>>(y, pred, run_start, run_len, order, corr, valid);
+    loss_pairwise_kernel<<<n_runs, 128, 0, s>>>(y, pred, run_start, run_len, order, corr, valid, ticket, loss);
     check(cudaGetLastError(), "loss_pairwise launch");
 }
 

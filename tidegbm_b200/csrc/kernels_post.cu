@@ -26,41 +26,7 @@ namespace {
 
 constexpr int kApplyThreads = 256;
 
-__device__ int shift_for_all(double max_abs, long long count) {
-    if (!(max_abs > 0.0) || count <= 0) return 0;
-    int clog = 0;
-    while ((1ll << clog) < count) ++clog;
-    const int e = ilogb(max_abs);
-    return max(-1000, min(1000, 61 - (e + 1) - clog));
-}
-
-__global__ void max_abs_kernel(const double* __restrict__ g, const double* __restrict__ h, int n,
-                               AllScale* __restrict__ sc) {
-    double mg = 0.0, mh = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        mg = fmax(mg, fabs(g[i]));
-        mh = fmax(mh, fabs(h[i]));
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-        mh = fmax(mh, __shfl_xor_sync(0xffffffffu, mh, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(&sc->maxg_bits, static_cast<unsigned long long>(__double_as_longlong(mg)));
-        atomicMax(&sc->maxh_bits, static_cast<unsigned long long>(__double_as_longlong(mh)));
-    }
-}
-
-__global__ void all_scale_finalize_kernel(AllScale* sc, int n) {
-    const double mg = __longlong_as_double(static_cast<long long>(sc->maxg_bits));
-    const double mh = __longlong_as_double(static_cast<long long>(sc->maxh_bits));
-    sc->gshift = shift_for_all(mg, n);
-    sc->hshift = shift_for_all(mh, n);
-    sc->gscale = ldexp(1.0, sc->gshift);
-    sc->hscale = ldexp(1.0, sc->hshift);
-    sc->inv_gscale = ldexp(1.0, -sc->gshift);
-    sc->inv_hscale = ldexp(1.0, -sc->hshift);
-}
+__global__ void all_scale_finalize_kernel(AllScale* sc, int n) { finalize_all_scale(sc, n); }
 
 // Exact 64-bit add into (low, high) 32-bit shared words: the low word's returned old
 // value says whether this addition wrapped; the carry goes to the high word.
@@ -302,25 +268,47 @@ __global__ void __launch_bounds__(kApplyThreads, 3)
 
 __device__ __forceinline__ double leaf_value(double G, double H, double l2) { return -G / (H + l2); }
 
-__global__ void finalize_tree_kernel(PostParams pp, const DevTreeState* __restrict__ st,
-                                     const unsigned long long* __restrict__ seg_sums,
-                                     const int* __restrict__ bucket_seg_end, const int* __restrict__ cuts,
-                                     const AllScale* __restrict__ sc, double* __restrict__ values,
-                                     int* __restrict__ cover, double* __restrict__ prefix) {
+// Leaf values, TORB prefixes and the tree's snapshot, one CTA.  A thread per node first runs over
+// the segments and leaves the node's sums through each of them (in place), so that a bucket's
+// prefix is one read; summing from the first segment for every (bucket, node) took 10 us at
+// 32 buckets.  Then the maxima that the next tree's gradients and sample reduce into are reset.
+__global__ void __launch_bounds__(1024)
+    finalize_tree_kernel(PostParams pp, DevTreeState* __restrict__ st, unsigned long long* __restrict__ seg_sums,
+                         const int* __restrict__ bucket_seg_end, const int* __restrict__ cuts, AllScale* __restrict__ sc,
+                         double* __restrict__ values, int* __restrict__ cover, double* __restrict__ prefix,
+                         const DevNode* __restrict__ nodes, DevNode* __restrict__ nodes_out,
+                         DevTreeState* __restrict__ st_out, int max_nodes) {
+    pdl_wait();
+    pdl_trigger();
     const int nn = st->n_nodes;
     const double ig = sc->inv_gscale, ih = sc->inv_hscale;
     for (int k = threadIdx.x; k < nn; k += blockDim.x) {
-        long long G = 0, H = 0, Cn = 0;
+        unsigned long long G = 0, H = 0, Cn = 0;
+#pragma unroll 8
         for (int s = 0; s < pp.n_segments; ++s) {
-            const unsigned long long* e = seg_sums + (static_cast<size_t>(s) * kMaxNodes + k) * 3;
-            G += static_cast<long long>(e[0]);
-            H += static_cast<long long>(e[1]);
-            Cn += static_cast<long long>(e[2]);
+            unsigned long long* e = seg_sums + (static_cast<size_t>(s) * kMaxNodes + k) * 3;
+            G += e[0];
+            H += e[1];
+            Cn += e[2];
+            e[0] = G;
+            e[1] = H;
         }
-        values[k] = leaf_value(static_cast<double>(G) * ig, static_cast<double>(H) * ih, pp.l2);
+        values[k] = leaf_value(static_cast<double>(static_cast<long long>(G)) * ig,
+                               static_cast<double>(static_cast<long long>(H)) * ih, pp.l2);
         cover[k] = static_cast<int>(Cn);
     }
+    {
+        // the tree as it was grown (16-byte words)
+        const uint4* from = reinterpret_cast<const uint4*>(nodes);
+        uint4* to = reinterpret_cast<uint4*>(nodes_out);
+        for (int k = threadIdx.x; k < max_nodes * static_cast<int>(sizeof(DevNode) / 16); k += blockDim.x) to[k] = from[k];
+    }
     __syncthreads();
+    if (threadIdx.x == 0) {
+        *st_out = *st;
+        sc->maxg_bits = sc->maxh_bits = 0ull;
+        st->max_abs_g_bits = st->max_h_bits = 0ull;
+    }
     const int nb = pp.n_buckets;
     for (int q = threadIdx.x; q < nb * nn; q += blockDim.x) {
         const int b = q / nn, k = q % nn;
@@ -330,10 +318,11 @@ __global__ void finalize_tree_kernel(PostParams pp, const DevTreeState* __restri
             v = full;
         } else {
             long long pG = 0, pH = 0;
-            for (int s = 0; s < bucket_seg_end[b]; ++s) {
-                const unsigned long long* e = seg_sums + (static_cast<size_t>(s) * kMaxNodes + k) * 3;
-                pG += static_cast<long long>(e[0]);
-                pH += static_cast<long long>(e[1]);
+            const int end = bucket_seg_end[b];
+            if (end > 0) {
+                const unsigned long long* e = seg_sums + (static_cast<size_t>(end - 1) * kMaxNodes + k) * 3;
+                pG = static_cast<long long>(e[0]);
+                pH = static_cast<long long>(e[1]);
             }
             const double cov = static_cast<double>(cuts[b]);
             const double alpha = cov <= 0.0 ? 0.0 : fmin(1.0, cov / fmax(pp.min_cover, 1.0));
@@ -348,6 +337,8 @@ __global__ void finalize_tree_kernel(PostParams pp, const DevTreeState* __restri
 __global__ void pred_update_kernel(PostParams pp, const int16_t* __restrict__ nid,
                                    const double* __restrict__ prefix, const DevTreeState* __restrict__ st,
                                    double* __restrict__ pred) {
+    pdl_wait();
+    pdl_trigger();
     const int nn = st->n_nodes;
     const int n = pp.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -364,13 +355,16 @@ __global__ void pred_update_kernel(PostParams pp, const int16_t* __restrict__ ni
 // pred update fused with the MSE training loss on the updated predictions
 // (booster.cpp:655-664 then 704-706): per-block partial sums of (pred - y)^2.
 // g != nullptr: also the next tree's mse gradient g = 1 * (pred - y) (objective.cpp:105-118,
-// the same double the gradient kernel computes) and its largest |g| into sc (reset by the
-// caller), so that the next tree needs no separate pass over pred and y.
+// the same double the gradient kernel computes) and its largest |g| into sc (reset by
+// finalize_tree), so that the next tree needs no separate pass over pred and y.  The last CTA to
+// finish adds the partial sums up, in a fixed order, and writes the loss.
 __global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict__ nid,
                                         const double* __restrict__ prefix, const DevTreeState* __restrict__ st,
                                         double* __restrict__ pred, const double* __restrict__ y,
                                         double* __restrict__ partials, double* __restrict__ g,
-                                        AllScale* __restrict__ sc) {
+                                        AllScale* __restrict__ sc, int* __restrict__ ticket, double* __restrict__ loss) {
+    pdl_wait();
+    pdl_trigger();
     const int nn = st->n_nodes;
     const int n = pp.n;
     double acc = 0.0, mg = 0.0;
@@ -390,22 +384,33 @@ __global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict
             mg = fmax(mg, fabs(gv));
         }
     }
-    if (g != nullptr) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
-        if ((threadIdx.x & 31) == 0)
-            atomicMax(&sc->maxg_bits, static_cast<unsigned long long>(__double_as_longlong(mg)));
-        if (blockIdx.x == 0 && threadIdx.x == 0)
-            atomicMax(&sc->maxh_bits, static_cast<unsigned long long>(__double_as_longlong(1.0)));
-    }
+    if (g != nullptr) block_max_into(mg, 1.0, sc);
     __shared__ double ws[32];
-    for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-    if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
+    __shared__ int s_last;
+    auto block_sum = [&](double v) {
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if ((threadIdx.x & 31) == 0) ws[threadIdx.x >> 5] = v;
+        __syncthreads();
         double t = 0.0;
         for (int w = 0; w < static_cast<int>(blockDim.x >> 5); ++w) t += ws[w];
-        partials[blockIdx.x] = t;
+        __syncthreads();
+        return t;
+    };
+    const double mine = block_sum(acc);
+    if (threadIdx.x == 0) {
+        partials[blockIdx.x] = mine;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
+        __threadfence();
+    }
+    __syncthreads();
+    if (!s_last) return;
+    double all = 0.0;
+    for (int k = threadIdx.x; k < static_cast<int>(gridDim.x); k += blockDim.x) all += __ldcg(partials + k);
+    all = block_sum(all);
+    if (threadIdx.x == 0) {
+        *loss = n > 0 ? all / static_cast<double>(n) : 0.0;
+        *ticket = 0;
     }
 }
 
@@ -589,12 +594,13 @@ void launch_predict_trees(const uint8_t* codes, int stride, int n, const Predict
     else predict_launch<1>(variant, bytes, codes, stride, n, m, base, lr, out, s);
 }
 
+int pred_update_parts(int n) { return std::max(1, std::min(2368, (n + 255) / 256)); }
+
 void launch_pred_update_loss(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
-                             double* pred, const double* y, double* partials, int n_part, double* g, AllScale* sc,
-                             cudaStream_t s) {
-    if (g != nullptr) check(cudaMemsetAsync(sc, 0, 2 * sizeof(unsigned long long), s), "all scale reset");
-    pred_update_loss_kernel<<<n_part, 256, 0, s>>>(pp, nid, prefix, st, pred, y, partials, g, sc);
-    check(cudaGetLastError(), "pred_update_loss launch");
+                             double* pred, const double* y, double* partials, double* g, AllScale* sc, int* ticket,
+                             double* loss, cudaStream_t s) {
+    launch_pdl(pred_update_loss_kernel, dim3(pred_update_parts(pp.n)), dim3(256), 0, s, "pred_update_loss launch", pp, nid,
+               prefix, st, pred, y, partials, g, sc, ticket, loss);
 }
 
 void launch_all_scale_finalize(AllScale* sc, int n, cudaStream_t s) {
@@ -602,20 +608,10 @@ void launch_all_scale_finalize(AllScale* sc, int n, cudaStream_t s) {
     check(cudaGetLastError(), "all_scale_finalize launch");
 }
 
-void launch_all_scale(const double* g, const double* h, int n, AllScale* sc, cudaStream_t s) {
-    check(cudaMemsetAsync(sc, 0, 2 * sizeof(unsigned long long), s), "all scale reset");
-    max_abs_kernel<<<std::max(1, std::min(1184, (n + 255) / 256)), 256, 0, s>>>(g, h, n, sc);
-    check(cudaGetLastError(), "max_abs launch");
-    all_scale_finalize_kernel<<<1, 1, 0, s>>>(sc, n);
-    check(cudaGetLastError(), "all_scale_finalize launch");
-}
-
 void launch_apply_accum(const uint8_t* col, long long pitch, int n_f, const DevNode* nodes, const DevTreeState* st,
                         const double* g, const double* h, const int4* chunks, int n_chunks,
-                        const AllScale* sc, int16_t* nid, unsigned long long* seg_sums, int n_segments,
-                        int n_bins, int kinds, cudaStream_t s) {
-    check(cudaMemsetAsync(seg_sums, 0, sizeof(unsigned long long) * 3 * kMaxNodes * n_segments, s),
-          "seg sums reset");
+                        const AllScale* sc, int16_t* nid, unsigned long long* seg_sums, int n_bins, int kinds,
+                        cudaStream_t s) {
     auto kern = kinds == 0 ? apply_accum_kernel<0> : kinds == 1 ? apply_accum_kernel<1>
                                                    : kinds == 2 ? apply_accum_kernel<2> : apply_accum_kernel<3>;
     {  // static + dynamic shared memory above 48 KB needs the opt-in, once per device
@@ -640,17 +636,18 @@ void launch_apply_accum(const uint8_t* col, long long pitch, int n_f, const DevN
     check(cudaGetLastError(), "apply_accum launch");
 }
 
-void launch_finalize_tree(const PostParams& pp, const DevTreeState* st, const unsigned long long* seg_sums,
-                          const int* bucket_seg_end, const int* cuts, const AllScale* sc, double* values,
-                          int* cover, double* prefix, cudaStream_t s) {
-    finalize_tree_kernel<<<1, 1024, 0, s>>>(pp, st, seg_sums, bucket_seg_end, cuts, sc, values, cover, prefix);
-    check(cudaGetLastError(), "finalize_tree launch");
+void launch_finalize_tree(const PostParams& pp, DevTreeState* st, unsigned long long* seg_sums,
+                          const int* bucket_seg_end, const int* cuts, AllScale* sc, double* values, int* cover,
+                          double* prefix, const DevNode* nodes, DevNode* nodes_out, DevTreeState* st_out, int max_nodes,
+                          cudaStream_t s) {
+    launch_pdl(finalize_tree_kernel, dim3(1), dim3(1024), 0, s, "finalize_tree launch", pp, st, seg_sums, bucket_seg_end,
+               cuts, sc, values, cover, prefix, nodes, nodes_out, st_out, max_nodes);
 }
 
 void launch_pred_update(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
                         double* pred, cudaStream_t s) {
-    pred_update_kernel<<<std::max(1, std::min(2368, (pp.n + 255) / 256)), 256, 0, s>>>(pp, nid, prefix, st, pred);
-    check(cudaGetLastError(), "pred_update launch");
+    launch_pdl(pred_update_kernel, dim3(pred_update_parts(pp.n)), dim3(256), 0, s, "pred_update launch", pp, nid, prefix,
+               st, pred);
 }
 
 }  // namespace tgb

@@ -1226,38 +1226,35 @@ __global__ void __launch_bounds__(kPartThreads)
 }
 
 // ---- per-tree set-up ------------------------------------------------------------------
-__global__ void wave_tree_init_kernel(DevNode* nodes, DevSplit* splits, DevTreeState* st, WaveCtl* ctl,
-                                      int n_sample, int use_dev_count) {
-    const int count = use_dev_count ? st->n_sample : n_sample;
-    if (threadIdx.x == 0) {
-        DevNode r{};
-        r.start = 0;
-        r.count = count;
-        r.buf = 0;
-        r.depth = 0;
-        r.is_leaf = 1;
-        r.feature = -1;
-        r.threshold = -1;
-        r.missing_left = 1;
-        r.left = r.right = r.parent = -1;
-        r.slot = 0;
-        nodes[0] = r;
-        splits[0].valid = 0;
-        st->n_nodes = 1;
-        st->done = 0;
-        st->parent = -1;
-        st->small_node = st->large_node = -1;
-        st->n_sample = count;
-        ctl->splits_done = 0;
-        ctl->n_exp = 0;
-        ctl->exp_counter = 0;
-        ctl->tiles_total = 0;
-        ctl->active = 1;
-        ctl->slot0 = 1;
-        ctl->error = 0;
-        ctl->waves = 0;
-        ctl->pair_used = 0;
-    }
+// The root node and the control of a new tree (one thread).
+__device__ __forceinline__ void init_tree(DevNode* nodes, DevSplit* splits, DevTreeState* st, WaveCtl* ctl, int count) {
+    DevNode r{};
+    r.start = 0;
+    r.count = count;
+    r.buf = 0;
+    r.depth = 0;
+    r.is_leaf = 1;
+    r.feature = -1;
+    r.threshold = -1;
+    r.missing_left = 1;
+    r.left = r.right = r.parent = -1;
+    r.slot = 0;
+    nodes[0] = r;
+    splits[0].valid = 0;
+    st->n_nodes = 1;
+    st->done = 0;
+    st->parent = -1;
+    st->small_node = st->large_node = -1;
+    st->n_sample = count;
+    ctl->splits_done = 0;
+    ctl->n_exp = 0;
+    ctl->exp_counter = 0;
+    ctl->tiles_total = 0;
+    ctl->active = 1;
+    ctl->slot0 = 1;
+    ctl->error = 0;
+    ctl->waves = 0;
+    ctl->pair_used = 0;
     ctl->expanded[0] = 0;
 }
 
@@ -1273,7 +1270,7 @@ __device__ int shift_for(double max_abs, int count) {
 // Exact modes: power-of-two shifts (no sum over the sample can reach 2^62, no row's value
 // 2^37).  Quantised modes: the largest |g| (and h) of the sample maps to the largest
 // code; constant-hessian modes keep the exact hessian shift (H is rebuilt from counts).
-__global__ void wave_scales_kernel(DevTreeState* st, const AllScale* __restrict__ all, int mode) {
+__device__ __forceinline__ void set_scales(DevTreeState* st, const AllScale* __restrict__ all, int mode) {
     if (all) {
         st->max_abs_g_bits = all->maxg_bits;
         st->max_h_bits = all->maxh_bits;
@@ -1302,6 +1299,33 @@ __global__ void wave_scales_kernel(DevTreeState* st, const AllScale* __restrict_
         st->hscale = mh > 0.0 ? hmax / mh : 1.0;
         st->inv_hscale = 1.0 / st->hscale;
     }
+}
+
+__global__ void wave_scales_kernel(DevTreeState* st, const AllScale* __restrict__ all, int mode) {
+    set_scales(st, all, mode);
+}
+
+// Everything between the gradients (and the GOSS sample) and the payloads of a new tree, in one
+// launch: the all-row scales, the root, the control and the histogram scales by one thread; the
+// root's histogram slot, the segment sums and the root's energy cleared and, without GOSS,
+// the row list written by the others.  (Nine launches of a few microseconds each before.)
+__global__ void __launch_bounds__(256) wave_begin_kernel(WaveBegin a) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        finalize_all_scale(a.all, a.n);
+        init_tree(a.nodes, a.splits, a.st, a.ctl, a.sampled ? a.st->n_sample : a.n);
+        set_scales(a.st, a.sampled ? nullptr : a.all, a.mode);
+        if (a.energy != nullptr) *a.energy = 0ull;
+    }
+    const size_t at = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x, step = static_cast<size_t>(gridDim.x) * blockDim.x;
+    const uint4 zero = make_uint4(0, 0, 0, 0);
+    for (size_t k = at; k < a.slot_elems / 2; k += step) {  // slot_elems is a multiple of 256
+        reinterpret_cast<uint4*>(a.G)[k] = zero;
+        reinterpret_cast<uint4*>(a.H)[k] = zero;
+        if (k < a.slot_elems / 4) reinterpret_cast<uint4*>(a.C)[k] = zero;
+    }
+    for (size_t k = at; k < a.seg_words; k += step) a.seg_sums[k] = 0ull;
+    if (!a.sampled)
+        for (size_t k = at; k < static_cast<size_t>(a.n); k += step) a.rows0[k] = static_cast<int32_t>(k);
 }
 
 // SplitMix64 output function (Steele, Lea and Flood, OOPSLA 2014): the stream of uniform
@@ -1530,10 +1554,9 @@ void launch_wave_partition(const WaveCtx* ctxs, int n_ctx, int grid, bool pair, 
     launch_pdl(pair ? wave_part_kernel<true> : wave_part_kernel<false>, dim3(grid), dim3(kPartThreads), 0, s, "wave_part launch", ctxs, n_ctx);
 }
 
-void launch_wave_tree_init(DevNode* nodes, DevSplit* splits, DevTreeState* st, WaveCtl* ctl, int n_sample_host,
-                           int use_dev_count, cudaStream_t s) {
-    wave_tree_init_kernel<<<1, 32, 0, s>>>(nodes, splits, st, ctl, n_sample_host, use_dev_count);
-    check(cudaGetLastError(), "wave_tree_init launch");
+void launch_wave_begin(const WaveBegin& a, cudaStream_t s) {
+    wave_begin_kernel<<<148 * 2, 256, 0, s>>>(a);
+    check(cudaGetLastError(), "wave_begin launch");
 }
 
 void launch_wave_scales(DevTreeState* st, const AllScale* all, int mode, cudaStream_t s) {

@@ -152,6 +152,50 @@ void check(cudaError_t e, const char* what);
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// The CTA's largest mg and mh (non-negative doubles, which order like their bits) into sc, one
+// atomic each: a warp's worth of atomics on the same two words took 10 us a pass.
+__device__ __forceinline__ void block_max_into(double mg, double mh, AllScale* sc) {
+    __shared__ double s_mg[32], s_mh[32];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        mg = fmax(mg, __shfl_xor_sync(0xffffffffu, mg, o));
+        mh = fmax(mh, __shfl_xor_sync(0xffffffffu, mh, o));
+    }
+    if ((threadIdx.x & 31) == 0) {
+        s_mg[threadIdx.x >> 5] = mg;
+        s_mh[threadIdx.x >> 5] = mh;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < static_cast<int>(blockDim.x >> 5); ++w) {
+            mg = fmax(mg, s_mg[w]);
+            mh = fmax(mh, s_mh[w]);
+        }
+        atomicMax(&sc->maxg_bits, static_cast<unsigned long long>(__double_as_longlong(mg)));
+        atomicMax(&sc->maxh_bits, static_cast<unsigned long long>(__double_as_longlong(mh)));
+    }
+}
+
+__device__ __forceinline__ int shift_for_all(double max_abs, long long count) {
+    if (!(max_abs > 0.0) || count <= 0) return 0;
+    int clog = 0;
+    while ((1ll << clog) < count) ++clog;
+    const int e = ilogb(max_abs);
+    return max(-1000, min(1000, 61 - (e + 1) - clog));
+}
+
+// The all-row scales from the maxima.
+__device__ __forceinline__ void finalize_all_scale(AllScale* sc, int n) {
+    const double mg = __longlong_as_double(static_cast<long long>(sc->maxg_bits));
+    const double mh = __longlong_as_double(static_cast<long long>(sc->maxh_bits));
+    sc->gshift = shift_for_all(mg, n);
+    sc->hshift = shift_for_all(mh, n);
+    sc->gscale = ldexp(1.0, sc->gshift);
+    sc->hscale = ldexp(1.0, sc->hshift);
+    sc->inv_gscale = ldexp(1.0, -sc->gshift);
+    sc->inv_hscale = ldexp(1.0, -sc->hshift);
+}
+
 template <typename... KArgs, typename... Args>
 inline void launch_pdl(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, const char* what,
                        Args... args) {
@@ -307,13 +351,13 @@ void launch_partition_rows_noalloc(const uint8_t* codes, int stride, const int32
 void launch_grad_mse(const double* y, const double* pred, int n, double* g, double* h, cudaStream_t s);
 // g = pred - y, sc <- max |g| and max h = 1 (reset first).
 void launch_grad_mse_fused(const double* y, const double* pred, int n, double* g, AllScale* sc, cudaStream_t s);
+// sc (may be null): the largest |g| and h are reduced into it (reset by the caller).
 void launch_grad_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len,
-                          const int* order, int n_runs, int n, double* g, double* h, cudaStream_t s);
-void launch_loss_mse(const double* y, const double* pred, int n, double* partials, int n_part, cudaStream_t s);
+                          const int* order, int n_runs, int n, double* g, double* h, AllScale* sc, cudaStream_t s);
+// The ranking loss: corr / valid are per-run scratch, ticket a zero that is left at zero.
 void launch_loss_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len,
-                          const int* order, int n_runs, double* corr, int* valid, cudaStream_t s);
-void launch_loss_finalize(int kind, const double* partials, const int* valid, int n_part, int n,
-                          double* out, cudaStream_t s);
+                          const int* order, int n_runs, double* corr, int* valid, int* ticket, double* loss,
+                          cudaStream_t s);
 
 // GOSS (kernels_goss.cu)
 size_t goss_cub_bytes(int n, bool exact);
@@ -325,21 +369,24 @@ void launch_goss_select(const double* g, const double* h, int n, int n_top, int 
                         int32_t* rows0, int* tile_counts, DevTreeState* st, cudaStream_t s);
 
 // post-tree sweep (kernels_post.cu)
-void launch_all_scale(const double* g, const double* h, int n, AllScale* sc, cudaStream_t s);
 void launch_all_scale_finalize(AllScale* sc, int n, cudaStream_t s);
-// pred += lr * prefix[bucket][leaf] and per-block sums of (pred - y)^2 into partials[n_part].
-// g, sc (mse only, may be null): the next tree's gradient and its maxima from the same pass.
+// pred += lr * prefix[bucket][leaf] and the mean of (pred - y)^2 into *loss (partials:
+// pred_update_parts(n) doubles of scratch, ticket: a zero that is left at zero).  g, sc (mse
+// only, may be null): the next tree's gradient and its maxima from the same pass.
+int pred_update_parts(int n);
 void launch_pred_update_loss(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
-                             double* pred, const double* y, double* partials, int n_part, double* g, AllScale* sc,
-                             cudaStream_t s);
-// col: column-major codes (col[f * pitch + r], launch_codes_transpose)
+                             double* pred, const double* y, double* partials, double* g, AllScale* sc, int* ticket,
+                             double* loss, cudaStream_t s);
+// col: column-major codes (col[f * pitch + r], launch_codes_transpose); seg_sums: zeroed by the caller
 void launch_apply_accum(const uint8_t* col, long long pitch, int n_f, const DevNode* nodes, const DevTreeState* st,
                         const double* g, const double* h, const int4* chunks, int n_chunks, const AllScale* sc,
-                        int16_t* nid, unsigned long long* seg_sums, int n_segments, int n_bins, int kinds,
-                        cudaStream_t s);
-void launch_finalize_tree(const PostParams& pp, const DevTreeState* st, const unsigned long long* seg_sums,
-                          const int* bucket_seg_end, const int* cuts, const AllScale* sc, double* values,
-                          int* cover, double* prefix, cudaStream_t s);
+                        int16_t* nid, unsigned long long* seg_sums, int n_bins, int kinds, cudaStream_t s);
+// seg_sums is used up (turned into prefixes); the maxima in sc and st are reset for the next
+// tree; nodes and st are copied to the tree's slots.
+void launch_finalize_tree(const PostParams& pp, DevTreeState* st, unsigned long long* seg_sums,
+                          const int* bucket_seg_end, const int* cuts, AllScale* sc, double* values, int* cover,
+                          double* prefix, const DevNode* nodes, DevNode* nodes_out, DevTreeState* st_out, int max_nodes,
+                          cudaStream_t s);
 void launch_pred_update(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
                         double* pred, cudaStream_t s);
 void launch_fill_pred(const double* init_prefix, int n, int n_buckets, int iid_mode, double* pred,

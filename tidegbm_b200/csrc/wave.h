@@ -205,10 +205,26 @@ inline int wave_children(int max_leaves, int max_expand) {
     return 2 * (max_expand > 0 && max_expand < e ? max_expand : e);
 }
 
-// Per-tree set-up of one context: root node (all sampled rows, slot 0), control reset.
-// use_dev_count: the sample size is st->n_sample (GOSS), else n_sample_host.
-void launch_wave_tree_init(DevNode* nodes, DevSplit* splits, DevTreeState* st, WaveCtl* ctl, int n_sample_host,
-                           int use_dev_count, cudaStream_t s);
+// Per-tree set-up of one context: all-row scales, root node, control reset, histogram scales; the
+// root's slot (slot 0 of G, H, C), seg_sums and energy (may be null) cleared; rows0 = 0 .. n - 1
+// unless `sampled` (GOSS: the sample is in rows0 and st->n_sample).
+struct WaveBegin {
+    DevNode* nodes;
+    DevSplit* splits;
+    DevTreeState* st;
+    WaveCtl* ctl;
+    AllScale* all;
+    long long* G;
+    long long* H;
+    int* C;
+    size_t slot_elems;
+    unsigned long long* seg_sums;
+    size_t seg_words;
+    unsigned long long* energy;
+    int32_t* rows0;
+    int n, sampled, mode;
+};
+void launch_wave_begin(const WaveBegin& a, cudaStream_t s);
 // Per-tree histogram scales of one context from the sample maxima (st) or, when the
 // sample is every row, the all-row maxima (all).
 void launch_wave_scales(DevTreeState* st, const AllScale* all, int mode, cudaStream_t s);
