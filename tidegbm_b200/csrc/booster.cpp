@@ -212,7 +212,8 @@ struct DeviceState {
     DBuf<unsigned long long> energy, pair_G, pair_H;
     DBuf<int> pair_C, pair_tickets;
     // predict: the fitted model's layout (tgb_internal.h, PredictTrees), its edges in the dtype
-    // of the last prediction's X (edges_dtype; -1: none), and the copy stream of long ones
+    // of the last prediction's X (edges_dtype; -1: none).  The copy stream and its events serve
+    // long predictions and a fit's GOSS positions (never both at once).
     DBuf<unsigned long long> t_word, t_cat;
     DBuf<double> t_val;
     DBuf<int4> t_trees;
@@ -274,6 +275,7 @@ struct FitRun {
     int n_top = 0, n_other = 0;
     double goss_scale = 1.0;
     std::unique_ptr<GossSampler> sampler;
+    bool copies = false;  // the booster's copy stream carries this fit's GOSS positions
     std::vector<int4> chunks;
     int n_segments = 0, n_runs = 0, max_tiles = 0, grid_rows = 0, mode = 0, n_slots = 0;
     const int* order_d = nullptr;
@@ -294,6 +296,7 @@ struct FitRun {
     FitRun(GpuBooster& b, const Config& cfg, DeviceState& d, cudaStream_t stream, bool exact)
         : B(b), c(cfg), D(d), s(stream), exact_goss(exact) {}
     ~FitRun() {
+        if (copies) cudaStreamSynchronize(D.copy.s);  // before the buffers and pinned slots it uses go back
         if (sampler) sampler->stop();
         for (auto& e : hist_ev) cudaEventDestroy(e);
     }
@@ -719,7 +722,11 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
         D.vals_in.alloc(n, s);
         D.vals_out.alloc(n, s);
         D.goss_flag.alloc(n, s);
-        D.rest_pos.alloc(std::max(1, n_other), s);
+        D.rest_pos.alloc(2 * static_cast<size_t>(std::max(1, n_other)), s);
+        if (!D.copy.s) check(cudaStreamCreateWithFlags(&D.copy.s, cudaStreamNonBlocking), "cudaStreamCreate");
+        copies = true;
+        check(cudaEventRecord(D.ev_ready.get(), s), "event record");  // the buffer exists
+        check(cudaStreamWaitEvent(D.copy.s, D.ev_ready.get(), 0), "event wait");
         const size_t cb = goss_cub_bytes(n, exact_goss);
         D.cub_tmp.alloc(cb, s);
         D.goss_overflow.alloc(1, s);
@@ -815,11 +822,20 @@ void FitRun::tree_begin(int t) {
         const double tr = now();
         const int32_t* pos = sampler->wait(t);  // host time spent waiting for the draw
         st.t_rng += now() - tr;
-        check(cudaMemcpyAsync(D.rest_pos.p, pos, sizeof(int32_t) * std::max(1, n_other), cudaMemcpyHostToDevice, s),
+        // The positions travel on the copy stream into one of two buffers, as soon as the select
+        // two trees back has read it, under the trees in between (75 us a tree of 10M rows when
+        // the copy was queued between the kernels).
+        const int k = t & 1;
+        int32_t* rest_d = D.rest_pos.p + static_cast<size_t>(k) * std::max(1, n_other);
+        if (t >= 2) check(cudaStreamWaitEvent(D.copy.s, D.ev_used[k].get(), 0), "event wait");
+        check(cudaMemcpyAsync(rest_d, pos, sizeof(int32_t) * std::max(1, n_other), cudaMemcpyHostToDevice, D.copy.s),
               "positions upload");
-        sampler->release(t, s);
-        launch_goss_select(D.g.p, h_rows, n, n_top, n_other, D.rest_pos.p, sampler->min_pos(t), gw, D.all_scale.p,
+        sampler->release(t, D.copy.s);
+        check(cudaEventRecord(D.ev_in[k].get(), D.copy.s), "event record");
+        check(cudaStreamWaitEvent(s, D.ev_in[k].get(), 0), "event wait");
+        launch_goss_select(D.g.p, h_rows, n, n_top, n_other, rest_d, sampler->min_pos(t), gw, D.all_scale.p,
                            goss_scale, D.goss_flag.p, D.rows0.p, D.tile_counts.p, D.st.p, s);
+        check(cudaEventRecord(D.ev_used[k].get(), s), "event record");
     }
     if (wave) {
         launch_wave_begin(WaveBegin{D.nodes.p, D.splits.p, D.st.p, D.ctl.p, D.all_scale.p, D.histG.p, D.histH.p, D.histC.p,
@@ -1586,9 +1602,7 @@ void GpuBooster::predict_raw(const void* X, int x_dtype, int n, int n_f, double*
     Xd.alloc(static_cast<size_t>(chunk) * row_bytes * slots, s);
     codes.alloc(static_cast<size_t>(chunk) * stride, s);
     outd.alloc(static_cast<size_t>(chunk) * slots, s);
-    // pinned slots of a power of two bytes: few sizes in the process's cache
-    size_t slot_bytes = 4096;
-    while (slot_bytes < static_cast<size_t>(chunk) * 8) slot_bytes *= 2;
+    const size_t slot_bytes = static_cast<size_t>(chunk) * 8;
     PinnedBlock pinned(slot_bytes * slots);
     auto host_slot = [&](int c) { return reinterpret_cast<double*>(static_cast<unsigned char*>(pinned.p) + slot_bytes * (c & 1)); };
     const bool overlap = n_chunks > 1;

@@ -27,21 +27,33 @@
 
 namespace tgb {
 
-// Pinned host blocks kept for reuse across fits of the process (cudaMallocHost and
-// cudaFreeHost cost milliseconds each).
+// Pinned host blocks kept for reuse across fits and predictions of the process (cudaMallocHost
+// and cudaFreeHost cost milliseconds each).  Sizes are rounded up to powers of two, so that
+// the folds of a walk-forward split and fits of similar sizes share blocks (by exact size, the
+// 48 blocks of six folds next to those of other fits went past the limit and were allocated and
+// freed on every call: 200 ms became 350 to 1,000).  At most kPinnedBlocks blocks and
+// kPinnedBytes bytes stay; the oldest goes first.
+constexpr size_t kPinnedBlocks = 128;
+constexpr size_t kPinnedBytes = 1ull << 30;
 inline std::mutex& pinned_cache_mutex() {
     static std::mutex mu;
     return mu;
 }
 inline std::vector<std::pair<size_t, void*>>& pinned_cache() {
-    static std::vector<std::pair<size_t, void*>> cache;
+    static std::vector<std::pair<size_t, void*>> cache;  // oldest first
     return cache;
 }
+inline size_t pinned_class(size_t bytes) {
+    size_t c = 4096;
+    while (c < bytes) c *= 2;
+    return c;
+}
 inline void* pinned_take(size_t bytes) {
+    bytes = pinned_class(bytes);
     {
         std::lock_guard<std::mutex> lk(pinned_cache_mutex());
         auto& c = pinned_cache();
-        for (size_t k = 0; k < c.size(); ++k)
+        for (size_t k = c.size(); k-- > 0;)
             if (c[k].first == bytes) {
                 void* p = c[k].second;
                 c.erase(c.begin() + static_cast<long>(k));
@@ -49,14 +61,25 @@ inline void* pinned_take(size_t bytes) {
             }
     }
     void* p = nullptr;
-    if (cudaMallocHost(&p, bytes) != cudaSuccess) throw std::runtime_error("cudaMallocHost (GOSS positions)");
+    if (cudaMallocHost(&p, bytes) != cudaSuccess) throw std::runtime_error("cudaMallocHost (pinned block)");
     return p;
 }
 inline void pinned_give(size_t bytes, void* p) {
-    std::lock_guard<std::mutex> lk(pinned_cache_mutex());
-    auto& c = pinned_cache();
-    if (c.size() < 64) c.emplace_back(bytes, p);
-    else cudaFreeHost(p);
+    bytes = pinned_class(bytes);
+    std::vector<void*> out;
+    {
+        std::lock_guard<std::mutex> lk(pinned_cache_mutex());
+        auto& c = pinned_cache();
+        c.emplace_back(bytes, p);
+        size_t total = 0;
+        for (const auto& e : c) total += e.first;
+        while (c.size() > kPinnedBlocks || total > kPinnedBytes) {
+            total -= c.front().first;
+            out.push_back(c.front().second);
+            c.erase(c.begin());
+        }
+    }
+    for (void* q : out) cudaFreeHost(q);
 }
 
 class GossSampler {
