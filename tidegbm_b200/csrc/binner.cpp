@@ -221,7 +221,7 @@ bool binner_fits_device(int n, int n_f, int bin_sample) {
 
 void binner_plan(const std::vector<int>& ch, int n, int n_f, int bin_sample, uint32_t seed, int n_threads,
                  BinPlan& plan) {
-    const int n_chunks = (n + kFitChunk - 1) / kFitChunk;
+    const int n_chunks = (n + fit_chunk(n) - 1) / fit_chunk(n);
     const size_t nc = static_cast<size_t>(n_chunks) * n_f;
     plan.n_chunks = n_chunks;
     // per-feature totals and the first non-NaN rank of every (chunk, feature)
@@ -399,7 +399,7 @@ int binner_fit_device(const void* Xd, int x_dtype, int n, int n_f, int max_bin, 
                       void* arena, size_t arena_bytes, BinFitTimes* tm, const void* X_host, const int* skip) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const double t0 = wall_now();
-    const int n_chunks = (n + kFitChunk - 1) / kFitChunk;
+    const int n_chunks = (n + fit_chunk(n) - 1) / fit_chunk(n);
     const size_t nc = static_cast<size_t>(n_chunks) * n_f;
     std::vector<int> ch(nc);
     {
