@@ -15,7 +15,9 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
+#include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <numeric>
 #include <thread>
@@ -266,7 +268,8 @@ struct FitRun {
     GpuBooster& B;
     Config c;
     DeviceState& D;
-    cudaStream_t s;
+    cudaStream_t s;   // the trees' stream (a batch: the first booster's)
+    cudaStream_t ps;  // prepare's stream and its buffers' (the booster's own)
     bool exact_goss;
     int n = 0, n_f = 0, stride = 0, T = 0, max_nodes = 0, nbk = 1;
     int n_threads = 1;
@@ -294,7 +297,7 @@ struct FitRun {
     DBuf<unsigned long long> rows_counter;
 
     FitRun(GpuBooster& b, const Config& cfg, DeviceState& d, cudaStream_t stream, bool exact)
-        : B(b), c(cfg), D(d), s(stream), exact_goss(exact) {}
+        : B(b), c(cfg), D(d), s(stream), ps(d.stream), exact_goss(exact) {}
     ~FitRun() {
         if (copies) cudaStreamSynchronize(D.copy.s);  // before the buffers and pinned slots it uses go back
         if (sampler) sampler->stop();
@@ -313,6 +316,7 @@ struct FitRun {
 
 void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in, int n_f_in, const int64_t* ts_in,
                      const int64_t* ent_in) {
+    cudaStream_t s = ps;  // everything here, until the last line waits for it
     t0 = now();
     launches0 = g_kernel_launches.load();
     n = n_in;
@@ -749,8 +753,8 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
         const WaveCtx wc = wave_ctx();
         D.wctx.alloc(1, s);
         check(cudaMemcpyAsync(D.wctx.p, &wc, sizeof(WaveCtx), cudaMemcpyHostToDevice, s), "wave context upload");
-        check(cudaStreamSynchronize(s), "wave context upload");
     }
+    check(cudaStreamSynchronize(s), "fit set-up");
     st.t_prep = now() - t_prep0;  // TORB segments, rank groups, GOSS buffers, initial predictions
 }
 
@@ -1442,6 +1446,12 @@ void GpuBooster::fit_batch(const std::vector<GpuBooster*>& bs, const std::vector
     for (auto* b : bs)
         if (b->device != b0.device) throw TideError("fit_batch: boosters must share one device");
     cudaStream_t s = b0.ds_->stream;
+    // The buffers belong to the boosters' own streams, the trees run on s: nothing goes back
+    // before s is done with it, however the call ends.
+    struct SyncOnExit {
+        cudaStream_t s;
+        ~SyncOnExit() { cudaStreamSynchronize(s); }
+    } sync_on_exit{s};
     std::vector<std::unique_ptr<FitRun>> own;
     std::vector<FitRun*> runs;
     for (size_t k = 0; k < bs.size(); ++k) {
@@ -1452,9 +1462,60 @@ void GpuBooster::fit_batch(const std::vector<GpuBooster*>& bs, const std::vector
             ck.profile_hist = false;
         }
         own.push_back(std::make_unique<FitRun>(*bs[k], ck, *bs[k]->ds_, s, false));
-        own.back()->prepare(in[k].X, in[k].x_dtype, in[k].y, in[k].n, in[k].n_f, in[k].ts, in[k].entity);
         runs.push_back(own.back().get());
     }
+    // Set-ups overlap, each on its booster's stream: one fit's upload runs under the binning
+    // of others, whose shuffles and sorts (a CTA per feature) leave most of the chip idle.  Three
+    // at a time, as long as their uploaded X together stay within kBatchUpload; a larger one goes
+    // alone, as when they ran one after another (6 folds of 0.4M to 0.85M x 64: 57 ms of 141).
+    constexpr size_t kBatchUpload = 8ull << 30;
+    constexpr int kBatchThreads = 3;
+    std::mutex mu;
+    std::condition_variable cv;
+    size_t next = 0, uploading = 0;
+    int running = 0;
+    std::vector<std::exception_ptr> failed(bs.size());
+    bool stop = false;
+    auto work = [&] {
+        while (true) {
+            size_t k, bytes;
+            {
+                std::unique_lock<std::mutex> lk(mu);
+                cv.wait(lk, [&] {
+                    if (stop || next >= bs.size()) return true;
+                    const size_t b = static_cast<size_t>(std::max(in[next].n, 0)) * std::max(in[next].n_f, 0) *
+                                     (in[next].x_dtype == 0 ? 4 : 8);
+                    return running == 0 || uploading + b <= kBatchUpload;
+                });
+                if (stop || next >= bs.size()) return;
+                k = next++;
+                bytes = static_cast<size_t>(std::max(in[k].n, 0)) * std::max(in[k].n_f, 0) * (in[k].x_dtype == 0 ? 4 : 8);
+                uploading += bytes;
+                ++running;
+            }
+            try {
+                runs[k]->prepare(in[k].X, in[k].x_dtype, in[k].y, in[k].n, in[k].n_f, in[k].ts, in[k].entity);
+            } catch (...) {
+                failed[k] = std::current_exception();
+            }
+            {
+                std::lock_guard<std::mutex> lk(mu);
+                uploading -= bytes;
+                --running;
+                if (failed[k]) stop = true;  // as when they ran in order: no later one starts
+            }
+            cv.notify_all();
+        }
+    };
+    {
+        std::vector<std::thread> th;
+        const size_t n_th = std::min<size_t>(kBatchThreads, bs.size());
+        for (size_t t = 1; t < n_th; ++t) th.emplace_back(work);
+        work();
+        for (auto& t : th) t.join();
+    }
+    for (auto& f : failed)
+        if (f) std::rethrow_exception(f);
     fit_runs(runs, s);
     std::vector<size_t> refit;
     for (size_t k = 0; k < bs.size(); ++k) {
