@@ -615,9 +615,9 @@ def run_ours(args) -> None:
     h2d = p.X.nbytes + p.y.nbytes
     kernels_per_tree = None
     if st.get("timed_selects"):
-        # per tree: gradients, GOSS (keys, 4+1 CUB passes, fix-up, mark, count, scatter), set-up,
-        # payload, post-tree sweep: 20 launches; waves: 3 + 4 x (selects - 1) kernels
-        kernels_per_tree = 20 + 3 + 4 * (st["timed_selects"] / K - 1)
+        # per tree: GOSS (keys, 4+1 CUB passes, fix-up, mark, count, scatter), set-up, payload,
+        # sweep, finalize, prediction update: 15 kernels; waves: 3 + 4 x (selects - 1)
+        kernels_per_tree = 15 + 3 + 4 * (st["timed_selects"] / K - 1)
     e2e = {"value": world * n_est / e2e_wall, "unit": "trees/s", "h2d_bytes_per_step": int(h2d / n_est),
            "d2h_bytes_per_step": int(d2h / n_est), "fit_wall_s": e2e_wall, "trees": n_est,
            "breakdown_s": {k: st[k] for k in ("total", "sort", "pre_upload", "bin_fit", "bin_counts", "bin_draws",
@@ -657,8 +657,8 @@ def run_ours(args) -> None:
             "hist_gbs": hp["gbs"], "roofline": roof, "e2e": e2e,
             "gpu_launches": int(round(kernels_per_tree * K)) if kernels_per_tree else int(st["timed_launches"]),
             "gpu_launches_note": "this library's kernels in the K timed trees (the CUB radix-sort passes of GOSS "
-                                 "included); the waves of a tree run as one graph launch of 3 + 4 x (selects - 1) "
-                                 "kernels, selects counted on the device",
+                                 "included); a tree is one graph launch, its waves 3 + 4 x (selects - 1) kernels, "
+                                 "selects counted on the device",
             "clocks": clk.summary()}
     extra_ok = rank == 0 and not args.quick
 

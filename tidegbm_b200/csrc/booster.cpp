@@ -32,11 +32,15 @@
 namespace tgb {
 
 std::atomic<long long> g_kernel_launches{0};
+static thread_local long long t_kernel_launches = 0;  // this thread's share of them
 
 void check(cudaError_t e, const char* what) {
     if (e != cudaSuccess) throw TideError(std::string("CUDA ") + what + ": " + cudaGetErrorString(e));
     const size_t L = std::strlen(what);
-    if (L > 7 && std::strcmp(what + L - 7, " launch") == 0) g_kernel_launches.fetch_add(1);
+    if (L > 7 && std::strcmp(what + L - 7, " launch") == 0) {
+        g_kernel_launches.fetch_add(1);
+        ++t_kernel_launches;
+    }
 }
 
 void* device_alloc(size_t bytes, cudaStream_t s) {
@@ -274,7 +278,6 @@ struct FitRun {
     int n = 0, n_f = 0, stride = 0, T = 0, max_nodes = 0, nbk = 1;
     int n_threads = 1;
     bool use_goss = false, const_h = true, any_cat = false;
-    bool g_ready = false;  // the previous tree's sweep wrote this tree's mse gradient
     int n_top = 0, n_other = 0;
     double goss_scale = 1.0;
     std::unique_ptr<GossSampler> sampler;
@@ -306,10 +309,13 @@ struct FitRun {
 
     void prepare(const void* X_in, int x_dtype, const double* y_in, int n_in, int n_f_in, const int64_t* ts_in,
                  const int64_t* ent_in);
-    void tree_begin(int t);
+    void first_gradient();
+    void feed(int t);
+    void fed(int t);
+    void tree_begin(int t, cudaStream_t q);
     void hist_leafwise(int node, bool in_timed);
     void grow_leafwise(bool in_timed);
-    void tree_end(int t);
+    void tree_end(cudaStream_t q);
     bool finish();  // reads the trees back; true when the 32-bit GOSS sort overflowed
     WaveCtx wave_ctx() const;
 };
@@ -726,7 +732,7 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
         D.vals_in.alloc(n, s);
         D.vals_out.alloc(n, s);
         D.goss_flag.alloc(n, s);
-        D.rest_pos.alloc(2 * static_cast<size_t>(std::max(1, n_other)), s);
+        D.rest_pos.alloc(2 * static_cast<size_t>(goss_rest_words(n_other)), s);
         if (!D.copy.s) check(cudaStreamCreateWithFlags(&D.copy.s, cudaStreamNonBlocking), "cudaStreamCreate");
         copies = true;
         check(cudaEventRecord(D.ev_ready.get(), s), "event record");  // the buffer exists
@@ -807,40 +813,52 @@ WaveCtx FitRun::wave_ctx() const {
     return w;
 }
 
+// The first tree's mse gradient; the later ones come from the prediction update (tree_end).
+void FitRun::first_gradient() {
+    if (const_h) launch_grad_mse_fused(D.y.p, D.pred.p, n, D.g.p, D.all_scale.p, s);
+}
+
+// What the host contributes to tree t, ahead of its kernels: the GOSS draw positions.  They
+// travel on the copy stream into one of two buffers, as soon as the tree two back is done with
+// it, under the trees in between (75 us a tree of 10M rows when the copy was queued between the
+// kernels).
+void FitRun::feed(int t) {
+    if (!use_goss) return;
+    const double tr = now();
+    const int32_t* pos = sampler->wait(t);  // host time spent waiting for the draw
+    st.t_rng += now() - tr;
+    const int k = t & 1;
+    const size_t words = static_cast<size_t>(goss_rest_words(n_other));
+    if (t >= 2) check(cudaStreamWaitEvent(D.copy.s, D.ev_used[k].get(), 0), "event wait");
+    check(cudaMemcpyAsync(D.rest_pos.p + k * words, pos, sizeof(int32_t) * words, cudaMemcpyHostToDevice, D.copy.s),
+          "positions upload");
+    sampler->release(t, D.copy.s);
+    check(cudaEventRecord(D.ev_in[k].get(), D.copy.s), "event record");
+    check(cudaStreamWaitEvent(s, D.ev_in[k].get(), 0), "event wait");
+}
+
+// After tree t's kernels have been enqueued on s.
+void FitRun::fed(int t) {
+    if (use_goss) check(cudaEventRecord(D.ev_used[t & 1].get(), s), "event record");
+}
+
 // Gradients (booster.cpp:701), the GOSS sample (booster.cpp:554-585), the tree's root and
-// histogram scales, and the per-row histogram payload.
-void FitRun::tree_begin(int t) {
+// histogram scales, and the per-row histogram payload, on stream q.  The kernels take the tree's
+// number from the device (st->tree), so that a captured graph serves every tree; t is read by
+// the one-split loop's int8 mode only.  Running it twice for a tree changes nothing.
+void FitRun::tree_begin(int t, cudaStream_t q) {
+    const cudaStream_t s = q;
     const bool wave = c.grow != 0;
     // the maxima of the gradients go to all_scale, reset at the fit's start and by tree_end
-    if (const_h) {
-        if (!g_ready) launch_grad_mse_fused(D.y.p, D.pred.p, n, D.g.p, D.all_scale.p, s);
-        g_ready = false;
-    } else {
+    if (!const_h)
         launch_grad_pairwise(D.y.p, D.pred.p, D.run_start.p, D.run_len.p, order_d, n_runs, n, D.g.p, D.h.p,
                              D.all_scale.p, s);
-    }
     const double* h_rows = const_h ? nullptr : D.h.p;
+    if (use_goss)
+        launch_goss_select(D.g.p, h_rows, n, n_top, n_other, D.rest_pos.p, gw, D.all_scale.p, goss_scale,
+                           D.goss_flag.p, D.rows0.p, D.tile_counts.p, D.st.p, s);
     const size_t slot = static_cast<size_t>(n_f) * kBins;
     const size_t seg_words = static_cast<size_t>(n_segments) * kMaxNodes * 3;
-    if (use_goss) {
-        const double tr = now();
-        const int32_t* pos = sampler->wait(t);  // host time spent waiting for the draw
-        st.t_rng += now() - tr;
-        // The positions travel on the copy stream into one of two buffers, as soon as the select
-        // two trees back has read it, under the trees in between (75 us a tree of 10M rows when
-        // the copy was queued between the kernels).
-        const int k = t & 1;
-        int32_t* rest_d = D.rest_pos.p + static_cast<size_t>(k) * std::max(1, n_other);
-        if (t >= 2) check(cudaStreamWaitEvent(D.copy.s, D.ev_used[k].get(), 0), "event wait");
-        check(cudaMemcpyAsync(rest_d, pos, sizeof(int32_t) * std::max(1, n_other), cudaMemcpyHostToDevice, D.copy.s),
-              "positions upload");
-        sampler->release(t, D.copy.s);
-        check(cudaEventRecord(D.ev_in[k].get(), D.copy.s), "event record");
-        check(cudaStreamWaitEvent(s, D.ev_in[k].get(), 0), "event wait");
-        launch_goss_select(D.g.p, h_rows, n, n_top, n_other, rest_d, sampler->min_pos(t), gw, D.all_scale.p,
-                           goss_scale, D.goss_flag.p, D.rows0.p, D.tile_counts.p, D.st.p, s);
-        check(cudaEventRecord(D.ev_used[k].get(), s), "event record");
-    }
     if (wave) {
         launch_wave_begin(WaveBegin{D.nodes.p, D.splits.p, D.st.p, D.ctl.p, D.all_scale.p, D.histG.p, D.histH.p, D.histC.p,
                                     slot, D.seg_sums.p, seg_words, c.pair_splits ? D.energy.p + 2 * kMaxNodes : nullptr,
@@ -854,15 +872,17 @@ void FitRun::tree_begin(int t) {
         check(cudaMemsetAsync(D.seg_sums.p, 0, sizeof(unsigned long long) * seg_words, s), "seg sums reset");
     }
     const uint8_t* flag = use_goss ? D.goss_flag.p : nullptr;
-    // per-tree stream of the stochastic rounding (SplitMix64 of seed and tree)
-    uint64_t z = (static_cast<uint64_t>(static_cast<uint32_t>(c.random_state)) << 32) + static_cast<uint64_t>(t);
+    // per-tree stream of the stochastic rounding: SplitMix64 of seed and tree (the waves' kernel
+    // does the same with the device's tree number)
+    const uint64_t base = static_cast<uint64_t>(static_cast<uint32_t>(c.random_state)) << 32;
+    uint64_t z = base + static_cast<uint64_t>(t);
     z += 0x9e3779b97f4a7c15ull;
     z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
     z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
     const uint64_t seed = z ^ (z >> 31);
     if (wave) {
         // (the children's histogram slots are cleared by the partition of their wave)
-        launch_wave_quantize(mode, D.rows0.p, D.g.p, h_rows, flag, goss_scale, D.st.p, seed, D.gqw.p, D.hqw.p,
+        launch_wave_quantize(mode, D.rows0.p, D.g.p, h_rows, flag, goss_scale, D.st.p, base, true, D.gqw.p, D.hqw.p,
                              c.pair_splits ? D.energy.p + 2 * kMaxNodes : nullptr, n, s);
     } else {
         if (c.hist_bits == 8)
@@ -901,29 +921,22 @@ void FitRun::grow_leafwise(bool in_timed) {
     }
 }
 
-// Post-tree sweep (booster.cpp:589-664), outputs straight into tree slot t, then the
-// prediction update and the training loss (booster.cpp:704-706).
-void FitRun::tree_end(int t) {
+// Post-tree sweep (booster.cpp:589-664), outputs straight into the tree's slots, then the
+// prediction update, the training loss (booster.cpp:704-706) and the next mse gradient.
+void FitRun::tree_end(cudaStream_t q) {
     const double* h_rows = const_h ? nullptr : D.h.p;
-    double* values_t = D.values_all.p + static_cast<size_t>(t) * max_nodes;
-    double* prefix_t = D.prefix_all.p + static_cast<size_t>(t) * nbk * max_nodes;
-    int* cover_t = D.cover_all.p + static_cast<size_t>(t) * max_nodes;
+    const TreeOut out{D.values_all.p, D.cover_all.p, D.prefix_all.p, D.nodes_all.p, D.st_all.p, D.losses.p, max_nodes, nbk};
     launch_apply_accum(D.codes_col.p, codes_col_pitch(n), n_f, D.nodes.p, D.st.p, D.g.p, h_rows, D.chunks.p,
                        static_cast<int>(chunks.size()), D.all_scale.p, D.nid.p, D.seg_sums.p, B.n_bins,
-                       (any_cat ? 1 : 0) | (c.pair_splits ? 2 : 0), s);
-    launch_finalize_tree(pp, D.st.p, D.seg_sums.p, D.bucket_seg_end.p, D.cuts.p, D.all_scale.p, values_t, cover_t,
-                         prefix_t, D.nodes.p, D.nodes_all.p + static_cast<size_t>(t) * max_nodes, D.st_all.p + t,
-                         max_nodes, s);
+                       (any_cat ? 1 : 0) | (c.pair_splits ? 2 : 0), q);
+    launch_finalize_tree(pp, D.st.p, D.seg_sums.p, D.bucket_seg_end.p, D.cuts.p, D.all_scale.p, D.nodes.p, out, q);
     if (const_h) {
-        // the next tree's gradient from the same pass (not after the last tree)
-        g_ready = t + 1 < T;
-        launch_pred_update_loss(pp, D.nid.p, prefix_t, D.st.p, D.pred.p, D.y.p, D.loss_part.p,
-                                g_ready ? D.g.p : nullptr, g_ready ? D.all_scale.p : nullptr, D.loss_ticket.p,
-                                D.losses.p + t, s);
+        launch_pred_update_loss(pp, D.nid.p, out, D.st.p, D.pred.p, D.y.p, D.loss_part.p, D.g.p, D.all_scale.p,
+                                D.loss_ticket.p, q);
     } else {
-        launch_pred_update(pp, D.nid.p, prefix_t, D.st.p, D.pred.p, s);
+        launch_pred_update(pp, D.nid.p, out, D.st.p, D.pred.p, q);
         launch_loss_pairwise(D.y.p, D.pred.p, D.run_start.p, D.run_len.p, order_d, n_runs, D.loss_part.p,
-                             D.loss_valid.p, D.loss_ticket.p, D.losses.p + t, s);
+                             D.loss_valid.p, D.loss_ticket.p, D.st.p, D.losses.p, q);
     }
 }
 
@@ -1080,22 +1093,33 @@ public:
     // builds the first tree's root histograms, timed with CUDA events (a warm-up run, then
     // the better of two), and the fastest is kept.  The root
     // slots are cleared before each run and after the last, so the tree starts afresh.
-    void autotune() {
+    long long tune_key() {
         int dev = 0;
         check(cudaGetDevice(&dev), "cudaGetDevice");
         int rb = 0;
         while ((1ll << rb) < rows_) ++rb;
-        const long long key = ((((static_cast<long long>(dev) * 8 + mode_) * 128 + n_ctx_) * 4096 + max_f_) * 64) + rb;
-        static std::mutex mu;
-        static std::vector<std::pair<long long, HistTune>> cache;
-        {
-            std::lock_guard<std::mutex> lk(mu);
-            for (auto& kv : cache)
-                if (kv.first == key) {
-                    tune_ = kv.second;
-                    return;
-                }
-        }
+        return ((((static_cast<long long>(dev) * 8 + mode_) * 128 + n_ctx_) * 4096 + max_f_) * 64) + rb;
+    }
+    struct TuneCache {
+        std::mutex mu;
+        std::vector<std::pair<long long, HistTune>> kept;
+    };
+    static TuneCache& tune_cache() {
+        static TuneCache c;
+        return c;
+    }
+    bool tuned() {
+        const long long key = tune_key();
+        TuneCache& c = tune_cache();
+        std::lock_guard<std::mutex> lk(c.mu);
+        for (auto& kv : c.kept)
+            if (kv.first == key) {
+                tune_ = kv.second;
+                return true;
+            }
+        return false;
+    }
+    void autotune() {
         cudaEvent_t a, b;
         check(cudaEventCreate(&a), "event");
         check(cudaEventCreate(&b), "event");
@@ -1125,16 +1149,19 @@ public:
         cudaEventDestroy(b);
         zero_roots();
         tune_ = best;
-        std::lock_guard<std::mutex> lk(mu);
-        cache.emplace_back(key, best);
+        TuneCache& c = tune_cache();
+        std::lock_guard<std::mutex> lk(c.mu);
+        c.kept.emplace_back(tune_key(), best);
     }
 
-    // The first tree's set-up has run (the roots' rows and payloads are on the device):
-    // tune, then capture the graph with the tuned launch shape.
+    // Tune on the first tree's roots, then capture the graph with the tuned launch shape.
     void first_tree() {
         if (ready_) return;
         ready_ = true;
-        if (autotune_) autotune();
+        if (autotune_ && !tuned()) {
+            for (auto* r : runs_) r->tree_begin(0, s_);  // the roots to tune on; run again with the tree
+            autotune();
+        }
         if (use_graph_) {
             try {
                 build_graph();
@@ -1168,15 +1195,24 @@ public:
         for (auto& e : ev_) cudaEventDestroy(e);
     }
 
-    // One tree of every context.  hist_ev: optional event pairs around each histogram launch
-    // (host-driven mode only); rows_counter: optional device counter of histogrammed rows.
-    void grow(std::vector<cudaEvent_t>* hist_ev, size_t* hist_used) {
+    // One tree of every context, its set-up and sweep included.  hist_ev: optional event pairs
+    // around each histogram launch (host-driven waves only).
+    void tree(int t, std::vector<cudaEvent_t>* hist_ev, size_t* hist_used) {
         first_tree();
-        unsigned long long* rows_counter = rows_counter_;
         if (exec_ && hist_ev == nullptr) {
-            check(cudaGraphLaunch(exec_, s_), "wave graph launch");
+            check(cudaGraphLaunch(exec_, s_), "tree graph");
+            g_kernel_launches.fetch_add(graph_kernels_);
             return;
         }
+        for (auto* r : runs_) r->tree_begin(t, s_);
+        grow(hist_ev, hist_used);
+        for (auto* r : runs_) r->tree_end(s_);
+    }
+
+private:
+    // The waves of one tree, enqueued by the host.
+    void grow(std::vector<cudaEvent_t>* hist_ev, size_t* hist_used) {
+        unsigned long long* rows_counter = rows_counter_;
         auto hist = [&](int src) {
             const bool prof = hist_ev && *hist_used + 2 <= hist_ev->size();
             if (prof) check(cudaEventRecord((*hist_ev)[*hist_used], s_), "event record");
@@ -1219,7 +1255,6 @@ public:
         }
     }
 
-private:
     void zero_roots() {
         for (auto* r : runs_) {
             const size_t slot = static_cast<size_t>(r->n_f) * kBins;
@@ -1250,19 +1285,28 @@ private:
     }
 
     void build_graph() {
-        // The root stage and the waves that every full tree takes are captured into the top
-        // graph, then a WHILE node whose body is one wave.  An iteration of the node costs about
-        // 4 us more than the next kernels of a stream; a straight wave after the tree's end
-        // costs its five empty kernels.  A full tree takes at least straight_waves() and, in
-        // best-first order, a third more (9 to 12 for 31 leaves): 8 straight waves there took
-        // fits of 100k x 32, 0.85M x 64 and 10M x 128 from 69.7, 74.6 and 391 ms to 67.4, 72.8
-        // and 386.
+        // A whole tree of every context: each context's set-up on a branch of its own, the root
+        // stage, the waves that every full tree takes, then a WHILE node whose body is one wave,
+        // and each context's sweep on its branch.  The host then makes one launch a tree (and
+        // the copies of the draw positions): enqueueing six folds' set-ups and sweeps took it
+        // 0.55 ms of a 2.66 ms tree, in which the device waited, and they ran one after another.
+        // An iteration of the node costs about 4 us more than the next kernels of a stream; a
+        // straight wave after the tree's end costs its five empty kernels.  A full tree takes at
+        // least straight_waves() and, in best-first order, a third more (9 to 12 for 31 leaves):
+        // 8 straight waves there took fits of 100k x 32, 0.85M x 64 and 10M x 128 from 69.7, 74.6
+        // and 391 ms to 67.4, 72.8 and 386.
         check(cudaGraphCreate(&graph_, 0), "graph create");
         cudaGraphConditionalHandle handle;
         check(cudaGraphConditionalHandleCreate(&handle, graph_, 1, cudaGraphCondAssignDefault),
               "graph conditional handle");
+        std::vector<OwnedStream>(n_ctx_ - 1).swap(side_);
+        for (auto& q : side_) check(cudaStreamCreateWithFlags(&q.s, cudaStreamNonBlocking), "cudaStreamCreate");
+        std::vector<OwnedEvent>(n_ctx_).swap(side_ev_);
+        for (auto& e : side_ev_) e.get();
+        const long long before = t_kernel_launches;
         check(cudaStreamBeginCaptureToGraph(s_, graph_, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
               "graph capture");
+        branch([](FitRun* r, cudaStream_t q) { r->tree_begin(0, q); });
         launch_wave_hist(mode_, ctx_.p, n_ctx_, 0, tune_, rows_counter_, s_);
         launch_wave_scan(ctx_.p, n_ctx_, 0, max_f_, scan_ys_, cat_, s_);
         if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 0, (mode_ & 1) != 0, s_);
@@ -1290,6 +1334,8 @@ private:
         cudaGraph_t body = cp.conditional.phGraph_out[0];
         check(cudaStreamUpdateCaptureDependencies(s_, &cond_node, 1, cudaStreamSetCaptureDependencies),
               "capture dependencies");
+        branch([](FitRun* r, cudaStream_t q) { r->tree_end(q); });
+        graph_kernels_ = t_kernel_launches - before;
         cudaGraph_t top = nullptr;
         check(cudaStreamEndCapture(s_, &top), "graph capture end");
         // the body: one wave
@@ -1299,9 +1345,21 @@ private:
         cudaGraph_t body_out = nullptr;
         check(cudaStreamEndCapture(s_, &body_out), "body capture end");
         check(cudaGraphInstantiate(&exec_, graph_, 0), "graph instantiate");
-        // launches counted per grow (the graph's kernels are this library's)
-        const int per_wave = 4 + (pair_ ? 1 : 0) + (cat_ ? 1 : 0);
-        g_kernel_launches.fetch_sub((per_wave - 1) + per_wave * (straight + 1));
+        // captured, not launched: tree() counts the kernels of the top graph
+        g_kernel_launches.fetch_sub(t_kernel_launches - before);
+    }
+
+    // f for every context, each on a stream of its own between s_ before and s_ after.
+    template <typename F>
+    void branch(F f) {
+        if (n_ctx_ > 1) check(cudaEventRecord(side_ev_[0].get(), s_), "event record");
+        for (int k = 1; k < n_ctx_; ++k) {
+            check(cudaStreamWaitEvent(side_[k - 1].s, side_ev_[0].get(), 0), "event wait");
+            f(runs_[k], side_[k - 1].s);
+            check(cudaEventRecord(side_ev_[k].get(), side_[k - 1].s), "event record");
+        }
+        f(runs_[0], s_);
+        for (int k = 1; k < n_ctx_; ++k) check(cudaStreamWaitEvent(s_, side_ev_[k].get(), 0), "event wait");
     }
 
     std::vector<FitRun*> runs_;
@@ -1316,6 +1374,9 @@ private:
     unsigned* hflag_ = nullptr;
     unsigned* dflag_ = nullptr;
     std::vector<cudaEvent_t> ev_;
+    std::vector<OwnedStream> side_;
+    std::vector<OwnedEvent> side_ev_;
+    long long graph_kernels_ = 0;
     cudaGraph_t graph_ = nullptr;
     cudaGraphExec_t exec_ = nullptr;
 };
@@ -1353,6 +1414,7 @@ void fit_runs(std::vector<FitRun*>& runs, cudaStream_t s) {
         for (auto* r : runs) r->st.t_driver = now() - td;
     }
     const double ttree = now();
+    for (auto* r : runs) r->first_gradient();
     for (int t = 0; t < T; ++t) {
         const bool in_timed = timing && t >= c.timing_from && t < timing_end;
         if (timing && t == c.timing_from) {
@@ -1367,14 +1429,18 @@ void fit_runs(std::vector<FitRun*>& runs, cudaStream_t s) {
             launches_end = g_kernel_launches.load();
             if (drv) selects_end = drv->selects();
         }
-        for (auto* r : runs) r->tree_begin(t);
+        for (auto* r : runs) r->feed(t);
         if (wave) {
             const bool prof = in_timed && c.profile_hist;
-            drv->grow(prof ? &r0.hist_ev : nullptr, prof ? &r0.hist_ev_used : nullptr);
+            drv->tree(t, prof ? &r0.hist_ev : nullptr, prof ? &r0.hist_ev_used : nullptr);
         } else {
-            for (auto* r : runs) r->grow_leafwise(in_timed);
+            for (auto* r : runs) {
+                r->tree_begin(t, s);
+                r->grow_leafwise(in_timed);
+                r->tree_end(s);
+            }
         }
-        for (auto* r : runs) r->tree_end(t);
+        for (auto* r : runs) r->fed(t);
     }
     if (timing && timing_end == T) {
         check(cudaEventRecord(ev_end, s), "event record");

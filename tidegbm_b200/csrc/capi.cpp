@@ -623,7 +623,7 @@ int tgb_hist_build_quantized(const unsigned char* codes, int stride, int n_featu
         tgb::check(cudaMemsetAsync(all.p, 0, sizeof(tgb::AllScale), s), "scale reset");
         tgb::launch_rows_max(rows, n_rows, g, h, all.p, s);
         tgb::launch_wave_scales(st.p, all.p, mode, s);
-        tgb::launch_wave_quantize(mode, rows, g, h, nullptr, 1.0, st.p, seed, gq.p, hq.p, nullptr,
+        tgb::launch_wave_quantize(mode, rows, g, h, nullptr, 1.0, st.p, seed, false, gq.p, hq.p, nullptr,
                                   std::max(1, n_rows), s);
         tgb::WaveCtx w{};
         w.codes = codes;

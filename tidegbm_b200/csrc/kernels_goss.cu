@@ -100,10 +100,12 @@ __global__ void goss_iota_kernel(int32_t* __restrict__ vals, int n) {
 // rank (min_rest, the largest |g| among them); only those two threads read g.
 __global__ void goss_mark_kernel(const int32_t* __restrict__ order, const unsigned int* __restrict__ k32,
                                  const int32_t* __restrict__ fixed, int n, int n_top, int n_other,
-                                 const int32_t* __restrict__ rest_pos, int min_rest, const double* __restrict__ g,
+                                 const int32_t* __restrict__ rest, int rest_words, const double* __restrict__ g,
                                  const double* __restrict__ h, double goss_scale, uint8_t* __restrict__ flag,
                                  DevTreeState* __restrict__ st) {
     const int total = n_top + n_other;
+    const int32_t* __restrict__ rest_pos = rest + static_cast<size_t>(st->tree & 1) * rest_words;
+    const int min_rest = rest_pos[rest_words - 1];
     double mg = 0.0, mh = 0.0;
     for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < total; p += gridDim.x * blockDim.x) {
         const bool top = p < n_top;
@@ -167,9 +169,9 @@ void launch_goss_iota(int32_t* vals, int n, cudaStream_t s) {
     check(cudaGetLastError(), "goss_iota launch");
 }
 
-void launch_goss_select(const double* g, const double* h, int n, int n_top, int n_other, const int32_t* rest_pos,
-                        int min_rest, GossWork& w, const AllScale* all, double goss_scale, uint8_t* goss_flag,
-                        int32_t* rows0, int* tile_counts, DevTreeState* st, cudaStream_t s) {
+void launch_goss_select(const double* g, const double* h, int n, int n_top, int n_other, const int32_t* rest,
+                        GossWork& w, const AllScale* all, double goss_scale, uint8_t* goss_flag, int32_t* rows0,
+                        int* tile_counts, DevTreeState* st, cudaStream_t s) {
     const int blocks = std::max(1, std::min(2368, (n + 255) / 256));
     if (w.exact) goss_keys_kernel<true><<<blocks, 256, 0, s>>>(g, n, all, w.keys_in);
     else goss_keys_kernel<false><<<blocks, 256, 0, s>>>(g, n, all, w.keys_in);
@@ -194,7 +196,8 @@ void launch_goss_select(const double* g, const double* h, int n, int n_top, int 
     const int32_t* fixed = static_cast<const int32_t*>(w.keys_in);
     check(cudaMemsetAsync(goss_flag, 0, static_cast<size_t>(n), s), "goss flag reset");
     goss_mark_kernel<<<std::max(1, std::min(2368, (n_top + n_other + 255) / 256)), 256, 0, s>>>(
-        w.vals_out, k32, fixed, n, n_top, n_other, rest_pos, min_rest, g, h, goss_scale, goss_flag, st);
+        w.vals_out, k32, fixed, n, n_top, n_other, rest, goss_rest_words(n_other), g, h, goss_scale, goss_flag,
+        st);
     check(cudaGetLastError(), "goss_mark launch");
     launch_compact_flagged(goss_flag, n, rows0, &st->n_sample, tile_counts, s);
 }

@@ -166,7 +166,8 @@ __global__ void __launch_bounds__(kGradWarps * 32)
 __global__ void loss_pairwise_kernel(const double* __restrict__ y, const double* __restrict__ pred,
                                      const int* __restrict__ run_start, const int* __restrict__ run_len,
                                      const int* __restrict__ order, double* __restrict__ corr,
-                                     int* __restrict__ valid, int* __restrict__ ticket, double* __restrict__ loss) {
+                                     int* __restrict__ valid, int* __restrict__ ticket, DevTreeState* __restrict__ st,
+                                     double* __restrict__ losses) {
     const int r = blockIdx.x;
     const int s0 = run_start[r], m = run_len[r];
     __shared__ double red[3][32];
@@ -257,8 +258,9 @@ __global__ void loss_pairwise_kernel(const double* __restrict__ y, const double*
             a += red[0][k];
             k_ok += red[1][k];
         }
-        *loss = k_ok > 0 ? -a / k_ok : 0.0;
+        losses[st->tree] = k_ok > 0 ? -a / k_ok : 0.0;
         *ticket = 0;
+        st->tree += 1;  // only this thread reads it here
     }
 }
 
@@ -286,10 +288,11 @@ void launch_grad_pairwise(const double* y, const double* pred, const int* run_st
 }
 
 void launch_loss_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len,
-                          const int* order, int n_runs, double* corr, int* valid, int* ticket, double* loss,
-                          cudaStream_t s) {
+                          const int* order, int n_runs, double* corr, int* valid, int* ticket, DevTreeState* st,
+                          double* losses, cudaStream_t s) {
     if (n_runs <= 0) return;
-    loss_pairwise_kernel<<<n_runs, 128, 0, s>>>(y, pred, run_start, run_len, order, corr, valid, ticket, loss);
+    loss_pairwise_kernel<<<n_runs, 128, 0, s>>>(y, pred, run_start, run_len, order, corr, valid, ticket, st,
+                                                losses);
     check(cudaGetLastError(), "loss_pairwise launch");
 }
 

@@ -275,12 +275,14 @@ __device__ __forceinline__ double leaf_value(double G, double H, double l2) { re
 __global__ void __launch_bounds__(1024)
     finalize_tree_kernel(PostParams pp, DevTreeState* __restrict__ st, unsigned long long* __restrict__ seg_sums,
                          const int* __restrict__ bucket_seg_end, const int* __restrict__ cuts, AllScale* __restrict__ sc,
-                         double* __restrict__ values, int* __restrict__ cover, double* __restrict__ prefix,
-                         const DevNode* __restrict__ nodes, DevNode* __restrict__ nodes_out,
-                         DevTreeState* __restrict__ st_out, int max_nodes) {
+                         const DevNode* __restrict__ nodes, TreeOut out) {
     pdl_wait();
     pdl_trigger();
-    const int nn = st->n_nodes;
+    const int nn = st->n_nodes, t = st->tree, max_nodes = out.max_nodes;
+    double* values = out.values + static_cast<size_t>(t) * max_nodes;
+    int* cover = out.cover + static_cast<size_t>(t) * max_nodes;
+    double* prefix = out.prefix + static_cast<size_t>(t) * out.n_buckets * max_nodes;
+    DevNode* nodes_out = out.nodes + static_cast<size_t>(t) * max_nodes;
     const double ig = sc->inv_gscale, ih = sc->inv_hscale;
     for (int k = threadIdx.x; k < nn; k += blockDim.x) {
         unsigned long long G = 0, H = 0, Cn = 0;
@@ -305,7 +307,7 @@ __global__ void __launch_bounds__(1024)
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        *st_out = *st;
+        out.st[t] = *st;
         sc->maxg_bits = sc->maxh_bits = 0ull;
         st->max_abs_g_bits = st->max_h_bits = 0ull;
     }
@@ -334,11 +336,15 @@ __global__ void __launch_bounds__(1024)
     }
 }
 
-__global__ void pred_update_kernel(PostParams pp, const int16_t* __restrict__ nid,
-                                   const double* __restrict__ prefix, const DevTreeState* __restrict__ st,
-                                   double* __restrict__ pred) {
+__device__ __forceinline__ const double* tree_prefix(const TreeOut& out, int t) {
+    return out.prefix + static_cast<size_t>(t) * out.n_buckets * out.max_nodes;
+}
+
+__global__ void pred_update_kernel(PostParams pp, const int16_t* __restrict__ nid, TreeOut out,
+                                   const DevTreeState* __restrict__ st, double* __restrict__ pred) {
     pdl_wait();
     pdl_trigger();
+    const double* __restrict__ prefix = tree_prefix(out, st->tree);
     const int nn = st->n_nodes;
     const int n = pp.n;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -354,17 +360,18 @@ __global__ void pred_update_kernel(PostParams pp, const int16_t* __restrict__ ni
 
 // pred update fused with the MSE training loss on the updated predictions
 // (booster.cpp:655-664 then 704-706): per-block partial sums of (pred - y)^2.
-// g != nullptr: also the next tree's mse gradient g = 1 * (pred - y) (objective.cpp:105-118,
+// Also the next tree's mse gradient g = 1 * (pred - y) (objective.cpp:105-118,
 // the same double the gradient kernel computes) and its largest |g| into sc (reset by
 // finalize_tree), so that the next tree needs no separate pass over pred and y.  The last CTA to
 // finish adds the partial sums up, in a fixed order, and writes the loss.
-__global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict__ nid,
-                                        const double* __restrict__ prefix, const DevTreeState* __restrict__ st,
-                                        double* __restrict__ pred, const double* __restrict__ y,
-                                        double* __restrict__ partials, double* __restrict__ g,
-                                        AllScale* __restrict__ sc, int* __restrict__ ticket, double* __restrict__ loss) {
+__global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict__ nid, TreeOut out,
+                                        DevTreeState* __restrict__ st, double* __restrict__ pred,
+                                        const double* __restrict__ y, double* __restrict__ partials,
+                                        double* __restrict__ g, AllScale* __restrict__ sc, int* __restrict__ ticket) {
     pdl_wait();
     pdl_trigger();
+    const int t = st->tree;
+    const double* __restrict__ prefix = tree_prefix(out, t);
     const int nn = st->n_nodes;
     const int n = pp.n;
     double acc = 0.0, mg = 0.0;
@@ -378,13 +385,11 @@ __global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict
         pred[i] = p;
         const double d = p - y[i];
         acc += 1.0 * d * d;
-        if (g != nullptr) {
-            const double gv = 1.0 * d;
-            g[i] = gv;
-            mg = fmax(mg, fabs(gv));
-        }
+        const double gv = 1.0 * d;
+        g[i] = gv;
+        mg = fmax(mg, fabs(gv));
     }
-    if (g != nullptr) block_max_into(mg, 1.0, sc);
+    block_max_into(mg, 1.0, sc);
     __shared__ double ws[32];
     __shared__ int s_last;
     auto block_sum = [&](double v) {
@@ -409,8 +414,9 @@ __global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict
     for (int k = threadIdx.x; k < static_cast<int>(gridDim.x); k += blockDim.x) all += __ldcg(partials + k);
     all = block_sum(all);
     if (threadIdx.x == 0) {
-        *loss = n > 0 ? all / static_cast<double>(n) : 0.0;
+        out.losses[t] = n > 0 ? all / static_cast<double>(n) : 0.0;
         *ticket = 0;
+        st->tree = t + 1;  // every CTA has read it
     }
 }
 
@@ -596,11 +602,11 @@ void launch_predict_trees(const uint8_t* codes, int stride, int n, const Predict
 
 int pred_update_parts(int n) { return std::max(1, std::min(2368, (n + 255) / 256)); }
 
-void launch_pred_update_loss(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
+void launch_pred_update_loss(const PostParams& pp, const int16_t* nid, const TreeOut& out, DevTreeState* st,
                              double* pred, const double* y, double* partials, double* g, AllScale* sc, int* ticket,
-                             double* loss, cudaStream_t s) {
+                             cudaStream_t s) {
     launch_pdl(pred_update_loss_kernel, dim3(pred_update_parts(pp.n)), dim3(256), 0, s, "pred_update_loss launch", pp, nid,
-               prefix, st, pred, y, partials, g, sc, ticket, loss);
+               out, st, pred, y, partials, g, sc, ticket);
 }
 
 void launch_all_scale_finalize(AllScale* sc, int n, cudaStream_t s) {
@@ -637,17 +643,16 @@ void launch_apply_accum(const uint8_t* col, long long pitch, int n_f, const DevN
 }
 
 void launch_finalize_tree(const PostParams& pp, DevTreeState* st, unsigned long long* seg_sums,
-                          const int* bucket_seg_end, const int* cuts, AllScale* sc, double* values, int* cover,
-                          double* prefix, const DevNode* nodes, DevNode* nodes_out, DevTreeState* st_out, int max_nodes,
-                          cudaStream_t s) {
+                          const int* bucket_seg_end, const int* cuts, AllScale* sc, const DevNode* nodes,
+                          const TreeOut& out, cudaStream_t s) {
     launch_pdl(finalize_tree_kernel, dim3(1), dim3(1024), 0, s, "finalize_tree launch", pp, st, seg_sums, bucket_seg_end,
-               cuts, sc, values, cover, prefix, nodes, nodes_out, st_out, max_nodes);
+               cuts, sc, nodes, out);
 }
 
-void launch_pred_update(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
+void launch_pred_update(const PostParams& pp, const int16_t* nid, const TreeOut& out, const DevTreeState* st,
                         double* pred, cudaStream_t s) {
-    launch_pdl(pred_update_kernel, dim3(pred_update_parts(pp.n)), dim3(256), 0, s, "pred_update launch", pp, nid, prefix,
-               st, pred);
+    launch_pdl(pred_update_kernel, dim3(pred_update_parts(pp.n)), dim3(256), 0, s, "pred_update launch", pp, nid, out, st,
+               pred);
 }
 
 }  // namespace tgb

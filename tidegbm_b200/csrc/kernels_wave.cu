@@ -1352,8 +1352,9 @@ template <int kMode>
 __global__ void wave_quantize_kernel(const int32_t* __restrict__ rows, const double* __restrict__ g,
                                      const double* __restrict__ h, const uint8_t* __restrict__ goss_flag,
                                      double goss_scale, const DevTreeState* __restrict__ st,
-                                     unsigned long long seed, void* __restrict__ gq, void* __restrict__ hq,
-                                     unsigned long long* __restrict__ energy) {
+                                     unsigned long long seed, bool per_tree, void* __restrict__ gq,
+                                     void* __restrict__ hq, unsigned long long* __restrict__ energy) {
+    if (per_tree) seed = splitmix64(seed + static_cast<unsigned long long>(st->tree));
     const int count = st->n_sample;
     const double escale = energy != nullptr ? ldexp(1.0, energy_shift(st)) : 0.0;
     unsigned long long en = 0;
@@ -1422,8 +1423,7 @@ void set_smem(K kern, size_t bytes) {
           "wave hist smem attr");
 }
 
-// The shared-memory opt-in of each histogram instantiation, set once per device (never
-// inside a stream capture: the first launches of a fit run before its graph is captured).
+// The shared-memory opt-in of each histogram instantiation, set once per device.
 template <int kMode>
 void ensure_smem() {
     static std::atomic<bool> done[64] = {};
@@ -1445,22 +1445,22 @@ void hist_launch(const WaveCtx* ctxs, int n_ctx, int src, HistTune tune, unsigne
     cfg.dynamicSmemBytes = SmemLayout<kMode>::bytes;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = 1;
-    attr[1].val.clusterDim.y = tune.cluster;
-    attr[1].val.clusterDim.z = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = tune.cluster;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 2;
+    cfg.numAttrs = src == 0 && n_ctx > 1 ? 1 : 2;  // (the roots follow several streams' kernels)
     check(cudaLaunchKernelEx(&cfg, kern, ctxs, n_ctx, src, rows_counter), "wave_hist launch");
 }
 
 template <int kMode>
 void quantize_launch(const int32_t* rows, const double* g, const double* h, const uint8_t* flag, double gs,
-                     const DevTreeState* st, unsigned long long seed, void* gq, void* hq, unsigned long long* energy,
-                     int blocks, cudaStream_t s) {
-    wave_quantize_kernel<kMode><<<blocks, 256, 0, s>>>(rows, g, h, flag, gs, st, seed, gq, hq, energy);
+                     const DevTreeState* st, unsigned long long seed, bool per_tree, void* gq, void* hq,
+                     unsigned long long* energy, int blocks, cudaStream_t s) {
+    wave_quantize_kernel<kMode><<<blocks, 256, 0, s>>>(rows, g, h, flag, gs, st, seed, per_tree, gq, hq, energy);
 }
 
 }  // namespace
@@ -1565,16 +1565,16 @@ void launch_wave_scales(DevTreeState* st, const AllScale* all, int mode, cudaStr
 }
 
 void launch_wave_quantize(int mode, const int32_t* rows, const double* g, const double* h, const uint8_t* goss_flag,
-                          double goss_scale, const DevTreeState* st, unsigned long long seed, void* gq, void* hq,
-                          unsigned long long* energy, int max_rows, cudaStream_t s) {
+                          double goss_scale, const DevTreeState* st, unsigned long long seed, bool per_tree, void* gq,
+                          void* hq, unsigned long long* energy, int max_rows, cudaStream_t s) {
     const int blocks = std::max(1, std::min(1184, (max_rows + 255) / 256));
     switch (mode) {
-        case kHistExactConst: quantize_launch<kHistExactConst>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
-        case kHistExactVar: quantize_launch<kHistExactVar>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
-        case kHistQ16Const: quantize_launch<kHistQ16Const>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
-        case kHistQ16Var: quantize_launch<kHistQ16Var>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
-        case kHistQ8Const: quantize_launch<kHistQ8Const>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
-        default: quantize_launch<kHistQ8Var>(rows, g, h, goss_flag, goss_scale, st, seed, gq, hq, energy, blocks, s); break;
+        case kHistExactConst: quantize_launch<kHistExactConst>(rows, g, h, goss_flag, goss_scale, st, seed, per_tree, gq, hq, energy, blocks, s); break;
+        case kHistExactVar: quantize_launch<kHistExactVar>(rows, g, h, goss_flag, goss_scale, st, seed, per_tree, gq, hq, energy, blocks, s); break;
+        case kHistQ16Const: quantize_launch<kHistQ16Const>(rows, g, h, goss_flag, goss_scale, st, seed, per_tree, gq, hq, energy, blocks, s); break;
+        case kHistQ16Var: quantize_launch<kHistQ16Var>(rows, g, h, goss_flag, goss_scale, st, seed, per_tree, gq, hq, energy, blocks, s); break;
+        case kHistQ8Const: quantize_launch<kHistQ8Const>(rows, g, h, goss_flag, goss_scale, st, seed, per_tree, gq, hq, energy, blocks, s); break;
+        default: quantize_launch<kHistQ8Var>(rows, g, h, goss_flag, goss_scale, st, seed, per_tree, gq, hq, energy, blocks, s); break;
     }
     check(cudaGetLastError(), "wave_quantize launch");
 }

@@ -77,7 +77,7 @@ struct DevTreeState {
     double gscale, hscale, inv_gscale, inv_hscale;
     unsigned long long max_abs_g_bits, max_h_bits;  // reductions for the scales
     int n_sample;
-    int pad;
+    int tree;  // trees finished so far: the slot of every per-tree input and output
 };
 
 // Fixed-point scale for sums over all rows (post-tree leaf values).
@@ -359,29 +359,42 @@ void launch_grad_mse_fused(const double* y, const double* pred, int n, double* g
 // sc (may be null): the largest |g| and h are reduced into it (reset by the caller).
 void launch_grad_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len,
                           const int* order, int n_runs, int n, double* g, double* h, AllScale* sc, cudaStream_t s);
-// The ranking loss: corr / valid are per-run scratch, ticket a zero that is left at zero.
+// The ranking loss into losses[st->tree], then st->tree + 1; corr / valid are per-run scratch,
+// ticket a zero that is left at zero.
 void launch_loss_pairwise(const double* y, const double* pred, const int* run_start, const int* run_len,
-                          const int* order, int n_runs, double* corr, int* valid, int* ticket, double* loss,
-                          cudaStream_t s);
+                          const int* order, int n_runs, double* corr, int* valid, int* ticket, DevTreeState* st,
+                          double* losses, cudaStream_t s);
 
 // GOSS (kernels_goss.cu)
 size_t goss_cub_bytes(int n, bool exact);
 void launch_goss_iota(int32_t* vals, int n, cudaStream_t s);  // w.vals_in, once per fit
-// all: the all-row maxima of the tree's gradients (the 32-bit sort keys are relative to max |g|);
-// min_rest: the smallest of rest_pos[0..n_other).
-void launch_goss_select(const double* g, const double* h, int n, int n_top, int n_other, const int32_t* rest_pos,
-                        int min_rest, GossWork& w, const AllScale* all, double goss_scale, uint8_t* goss_flag,
-                        int32_t* rows0, int* tile_counts, DevTreeState* st, cudaStream_t s);
+// all: the all-row maxima of the tree's gradients (the 32-bit sort keys are relative to max |g|).
+// rest: two buffers of goss_rest_words(n_other) words, used by turns (st->tree): n_other
+// positions, then, as the last word, the smallest of them.
+inline int goss_rest_words(int n_other) { return (n_other > 1 ? n_other : 1) + 1; }
+void launch_goss_select(const double* g, const double* h, int n, int n_top, int n_other, const int32_t* rest,
+                        GossWork& w, const AllScale* all, double goss_scale, uint8_t* goss_flag, int32_t* rows0,
+                        int* tile_counts, DevTreeState* st, cudaStream_t s);
 
 // post-tree sweep (kernels_post.cu)
 void launch_all_scale_finalize(AllScale* sc, int n, cudaStream_t s);
-// pred += lr * prefix[bucket][leaf] and the mean of (pred - y)^2 into *loss (partials:
-// pred_update_parts(n) doubles of scratch, ticket: a zero that is left at zero).  g, sc (mse
-// only, may be null): the next tree's gradient and its maxima from the same pass.
+// A fit's per-tree outputs, a slot per tree (max_nodes nodes, n_buckets x max_nodes prefixes).
+struct TreeOut {
+    double* values;
+    int* cover;
+    double* prefix;
+    DevNode* nodes;
+    DevTreeState* st;
+    double* losses;
+    int max_nodes, n_buckets;
+};
+// pred += lr * prefix[bucket][leaf] and the mean of (pred - y)^2 into out.losses (partials:
+// pred_update_parts(n) doubles of scratch, ticket: a zero that is left at zero), then st->tree
+// + 1.  g, sc: the next tree's mse gradient and its maxima from the same pass.
 int pred_update_parts(int n);
-void launch_pred_update_loss(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
+void launch_pred_update_loss(const PostParams& pp, const int16_t* nid, const TreeOut& out, DevTreeState* st,
                              double* pred, const double* y, double* partials, double* g, AllScale* sc, int* ticket,
-                             double* loss, cudaStream_t s);
+                             cudaStream_t s);
 // col: column-major codes (col[f * pitch + r], launch_codes_transpose); seg_sums: zeroed by the caller
 void launch_apply_accum(const uint8_t* col, long long pitch, int n_f, const DevNode* nodes, const DevTreeState* st,
                         const double* g, const double* h, const int4* chunks, int n_chunks, const AllScale* sc,
@@ -389,10 +402,9 @@ void launch_apply_accum(const uint8_t* col, long long pitch, int n_f, const DevN
 // seg_sums is used up (turned into prefixes); the maxima in sc and st are reset for the next
 // tree; nodes and st are copied to the tree's slots.
 void launch_finalize_tree(const PostParams& pp, DevTreeState* st, unsigned long long* seg_sums,
-                          const int* bucket_seg_end, const int* cuts, AllScale* sc, double* values, int* cover,
-                          double* prefix, const DevNode* nodes, DevNode* nodes_out, DevTreeState* st_out, int max_nodes,
-                          cudaStream_t s);
-void launch_pred_update(const PostParams& pp, const int16_t* nid, const double* prefix, const DevTreeState* st,
+                          const int* bucket_seg_end, const int* cuts, AllScale* sc, const DevNode* nodes,
+                          const TreeOut& out, cudaStream_t s);
+void launch_pred_update(const PostParams& pp, const int16_t* nid, const TreeOut& out, const DevTreeState* st,
                         double* pred, cudaStream_t s);
 void launch_fill_pred(const double* init_prefix, int n, int n_buckets, int iid_mode, double* pred,
                       cudaStream_t s);

@@ -229,10 +229,11 @@ void launch_wave_begin(const WaveBegin& a, cudaStream_t s);
 // sample is every row, the all-row maxima (all).
 void launch_wave_scales(DevTreeState* st, const AllScale* all, int mode, cudaStream_t s);
 // Payload of the sampled rows for `mode` (rows0[0 .. st->n_sample)), by position in rows0.
+// The stochastic rounding's stream is `seed`, or with per_tree SplitMix64 of seed + st->tree.
 // energy (PAIR, else nullptr; zeroed by the caller): the root's gradient energy.
 void launch_wave_quantize(int mode, const int32_t* rows, const double* g, const double* h, const uint8_t* goss_flag,
-                          double goss_scale, const DevTreeState* st, unsigned long long seed, void* gq, void* hq,
-                          unsigned long long* energy, int max_rows, cudaStream_t s);
+                          double goss_scale, const DevTreeState* st, unsigned long long seed, bool per_tree, void* gq,
+                          void* hq, unsigned long long* energy, int max_rows, cudaStream_t s);
 
 // Wave launches over n_ctx contexts (ctxs: device array).  src 0: the roots, src 1: the
 // expansions planned by the last select.
