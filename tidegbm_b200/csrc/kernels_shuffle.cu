@@ -25,9 +25,18 @@
 // Word q of a block serves draw t + q.  Lemire's method (the one libstdc++'s
 // uniform_int_distribution uses for a 32-bit generator) rejects a word when the low
 // half of w * (t + 1) is below 2^32 mod (t + 1); that draw then takes the next word,
-// shifting the later ones by one.  The block tests all its words at once; at the first
-// rejected word the draws before it are committed and the rest are re-tested with the
-// shift.  Rejections happen with probability below (t + 1) / 2^32.
+// shifting the later ones by one.  Rejections happen with probability below
+// (t + 1) / 2^32: one block in three has one at ten million values.  A round tests the words
+// that are left for their draws as they stand; the draws before the first rejected word are
+// committed, and the words behind it go round again.
+// The draws are a chain of blocks on one SM, bound by the latency of its steps.  So ten warps
+// run the generator, four blocks ahead of the ten that test and commit; a round covers those
+// four blocks and has one barrier; indexes are 32 bits wide; only a warp with a word that may
+// be rejected (low half below t + 1) divides; hits on kept slots are predicated reductions; and
+// the state and the recurrence's terms are padded with zeros where a word lacks one.  10M draws
+// into 200,000 slots: 12.2 -> 7.7 ms (20 warps doing both, four barriers a rejection before).
+// A round takes about 1,400 cycles whatever its words, hence four blocks: two take 12.8 ms,
+// three 7.4, six 9.3, eight 9.2.
 #include "tgb_internal.h"
 
 #include <cub/block/block_scan.cuh>
@@ -37,7 +46,11 @@ namespace tgb {
 namespace {
 
 constexpr int kMtN = 624;
-constexpr int kDrawThreads = 640;
+constexpr int kMtHalf = kMtN / 2;
+constexpr int kDrawRole = 320;     // threads of a role, two words of a block each
+constexpr int kDrawThreads = 2 * kDrawRole;
+constexpr int kDrawBlocks = 4;     // blocks a round
+constexpr int kDrawWords = kDrawBlocks * kMtN;
 constexpr int kScanThreads = 1024;
 constexpr int kScanItems = 4;
 
@@ -54,95 +67,142 @@ __device__ __forceinline__ uint32_t mt_temper(uint32_t v) {
     return v;
 }
 
+// The threads of one role.
+__device__ __forceinline__ void role_sync(int id) {
+    asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDrawRole) : "memory");
+}
+
 // Range r: std::mt19937(seeds[r]) and draws t = 1 .. ms[r]-1 (ms[r] = 0: the range is
-// not handled here).  last/head hold keep entries per range, cnt keep + 1.  A range
+// not handled here; ms[r] < 2^31).  last/head hold keep entries per range, cnt keep + 1.  A range
 // whose refills exceed twice the expected count sets *err and stops.
 __global__ void __launch_bounds__(kDrawThreads)
     shuffle_draw_kernel(const uint32_t* __restrict__ seeds, const long long* __restrict__ ms, int keep,
                         int32_t* __restrict__ last, int32_t* __restrict__ head, int32_t* __restrict__ cnt,
                         int* __restrict__ err) {
-    __shared__ uint32_t st[kMtN];
-    __shared__ uint32_t a[kMtN];
-    __shared__ int first;
+    __shared__ uint32_t st[kMtN + 96];   // zeros after the state: word k >= 227 has no old[k + 397]
+    __shared__ uint32_t az[227 + kMtN];  // zeros before a[]: word k < 227 has no a[k - 227], ...
+    __shared__ uint32_t words[2][kDrawWords];
+    // The first rejected word, by turns: round k posts in slot k % 3, reads it after the barrier,
+    // and clears slot (k + 2) % 3, which every thread had read before that barrier and uses
+    // after the next.
+    __shared__ int first[3];
+    __shared__ int stop[2];  // of even and odd rounds: set in a round for the next, read after its barrier
     const int r = blockIdx.x;
-    const long long m = ms[r];
-    if (m < 2 || keep <= 0) return;
-    const int t = threadIdx.x;
-    if (t == 0) {  // std::mt19937's seeding recurrence
+    const long long m64 = ms[r];
+    if (m64 < 2 || keep <= 0) return;
+    const uint32_t m = static_cast<uint32_t>(m64);
+    const bool draws = threadIdx.x < kDrawRole;
+    const int t = draws ? threadIdx.x : threadIdx.x - kDrawRole;
+    const bool has = t < kMtHalf;  // the words t and t + 312 of a block
+    const int t0 = has ? t : 0;    // (the last eight threads of a role only wait)
+    for (int k = threadIdx.x; k < 227; k += kDrawThreads) az[k] = 0u;
+    for (int k = kMtN + threadIdx.x; k < kMtN + 96; k += kDrawThreads) st[k] = 0u;
+    if (threadIdx.x == 0) {  // std::mt19937's seeding recurrence
         uint32_t x = seeds[r];
         st[0] = x;
         for (int k = 1; k < kMtN; ++k) {
             x = 1812433253u * (x ^ (x >> 30)) + static_cast<uint32_t>(k);
             st[k] = x;
         }
+        stop[0] = stop[1] = 0;
     }
+    if (threadIdx.x < 3) first[threadIdx.x] = kDrawWords;
     __syncthreads();
+    uint32_t* a = az + 227;
+    auto refill = [&](uint32_t* out) {
+        for (int b = 0; b < kDrawBlocks; ++b, out += kMtN) {
+            uint32_t a0 = mt_mix(st[t0], st[t0 + 1]) ^ st[t0 + 397];
+            const uint32_t hi = st[t0 + kMtHalf];
+            uint32_t a1 = mt_mix(hi, st[t0 + kMtHalf + 1]);
+            if (has) {
+                a[t] = a0;
+                a[t + kMtHalf] = a1;
+            }
+            role_sync(2);
+            if (t == kMtHalf - 1) a1 = mt_mix(hi, a[0]);  // word 623 mixes with the new word 0
+            a0 ^= a[t0 - 227];
+            a1 ^= a[t0 + kMtHalf - 227] ^ a[t0 + kMtHalf - 454];
+            if (has) {
+                st[t] = a0;
+                st[t + kMtHalf] = a1;
+            }
+            role_sync(2);
+            if (has) {
+                out[t] = mt_temper(a0);
+                out[t + kMtHalf] = mt_temper(a1);
+            }
+        }
+    };
+    if (!draws) {
+        refill(words[0]);
+        for (int buf = 1;; buf ^= 1) {
+            __syncthreads();  // words[buf ^ 1] are there, words[buf] used up
+            if (stop[buf ^ 1] != 0) return;
+            refill(words[buf]);
+        }
+    }
     int32_t* lst = last + static_cast<size_t>(r) * keep;
     int32_t* hd = head + static_cast<size_t>(r) * keep;
     int32_t* ct = cnt + static_cast<size_t>(r) * (keep + 1);
     const uint32_t K = static_cast<uint32_t>(keep);
-    long long i = 1;  // the next draw
-    int pos = kMtN;   // the next unused word of the block
-    uint32_t w = 0;
-    long long refills_left = 2 * (m / kMtN) + 16;
-    while (i < m) {
-        if (pos >= kMtN) {
-            if (--refills_left < 0) {
-                if (t == 0) atomicExch(err, 1);
-                return;
+    uint32_t i = 1;  // the next draw
+    int slot = 0;
+    uint32_t refills_left = 2 * (m / kDrawWords) + 16;
+    for (int buf = 0;; buf ^= 1) {
+        __syncthreads();
+        if (stop[buf] != 0) return;
+        uint32_t w[2 * kDrawBlocks];
+#pragma unroll
+        for (int q = 0; q < 2 * kDrawBlocks; ++q) w[q] = words[buf][t0 + q * kMtHalf];
+        for (int pos = 0; pos < kDrawWords && i < m;) {  // words before pos are settled
+            const uint32_t off = has ? static_cast<uint32_t>(t0 - pos) : 0x80000000u;
+            const uint32_t left = static_cast<uint32_t>(kDrawWords - pos);
+            unsigned near = 0;
+#pragma unroll
+            for (int q = 0; q < 2 * kDrawBlocks; ++q) {
+                const uint32_t o = off + q * kMtHalf, d = i + o;
+                if (w[q] * (d + 1u) <= d && o < left) near |= 1u << q;
             }
-            uint32_t ak = 0;
-            if (t < kMtN - 1) {
-                ak = mt_mix(st[t], st[t + 1]);
-                if (t < 227) ak ^= st[t + 397];
-            } else if (t == kMtN - 1) {
-                ak = mt_mix(st[kMtN - 1], st[397] ^ mt_mix(st[0], st[1]));
-            }
-            if (t < kMtN) a[t] = ak;
-            __syncthreads();
-            if (t < kMtN) {
-                uint32_t nk = ak;
-                if (t >= 227) nk ^= a[t - 227];
-                if (t >= 454) nk ^= a[t - 454];
-                st[t] = nk;  // read again only after the barrier of the draw loop
-                w = mt_temper(nk);
-            }
-            pos = 0;
-        }
-        while (true) {
-            const long long d = i + (t - pos);
-            const bool live = t >= pos && t < kMtN && d < m;
-            const uint32_t range = static_cast<uint32_t>(d + 1);
-            const uint64_t p = static_cast<uint64_t>(w) * range;
-            const uint32_t low = static_cast<uint32_t>(p);
-            const bool rej = live && low < range && low < (0u - range) % range;
-            const bool any = __syncthreads_or(rej);
-            int fr = kMtN;
-            if (any) {
-                if (t == 0) first = kMtN;
-                __syncthreads();
-                if (rej) atomicMin(&first, t);
-                __syncthreads();
-                fr = first;
-            }
-            const uint32_t j = static_cast<uint32_t>(p >> 32);
-            if (live && t < fr && j < K) {
-                atomicMax(lst + j, static_cast<int>(d));
-                if (d < keep) {
-                    hd[d] = static_cast<int32_t>(j);
-                    atomicAdd(ct + j, 1);
+            for (; near != 0; near &= near - 1) {
+                const uint32_t o = off + (__ffs(near) - 1) * kMtHalf, range = i + o + 1u;
+                const uint32_t low = words[buf][pos + o] * range;
+                if (low < (0u - range) % range) {
+                    atomicMin(&first[slot], pos + static_cast<int>(o));
+                    break;
                 }
             }
-            if (!any) {
-                const long long used = min(static_cast<long long>(kMtN - pos), m - i);
-                i += used;
-                pos += static_cast<int>(used);
-                break;
+            role_sync(1);
+            const int f = first[slot];
+            if (t == 0) first[slot == 0 ? 2 : slot - 1] = kDrawWords;
+            slot = slot == 2 ? 0 : slot + 1;
+            const uint32_t span = min(static_cast<uint32_t>(f - pos), m - i);  // draws settled
+#pragma unroll
+            for (int q = 0; q < 2 * kDrawBlocks; ++q) {
+                const uint32_t o = off + q * kMtHalf, d = i + o, j = __umulhi(w[q], d + 1u);
+                asm volatile(
+                    "{\n .reg .pred p;\n setp.ne.u32 p, %0, 0;\n @p red.global.max.s32 [%1], %2;\n}" ::"r"(
+                        static_cast<uint32_t>(j < K && o < span)),
+                    "l"(lst + j), "r"(d)
+                    : "memory");
             }
-            i += fr - pos;  // the rejected word is consumed; draw i + (fr - pos) takes the next word
-            pos = fr + 1;
-            if (pos >= kMtN) break;
+            if (i < K) {  // some are draws of the prefix itself
+#pragma unroll
+                for (int q = 0; q < 2 * kDrawBlocks; ++q) {
+                    const uint32_t o = off + q * kMtHalf, d = i + o, j = __umulhi(w[q], d + 1u);
+                    if (j < K && o < span && d < K) {
+                        hd[d] = static_cast<int32_t>(j);
+                        atomicAdd(ct + j, 1);
+                    }
+                }
+            }
+            i += static_cast<uint32_t>(f - pos);
+            pos = f + 1;  // a rejected word is consumed; its draw takes the next word
         }
+        if (t == 0 && (i >= m || refills_left == 0)) {
+            if (i < m) atomicExch(err, 1);
+            stop[buf ^ 1] = 1;
+        }
+        --refills_left;
     }
 }
 
