@@ -594,6 +594,8 @@ void FitRun::prepare(const void* X_in, int x_dtype, const double* y_in, int n_in
         // (bit-identical to the host binner's) and the vocabularies (binning.cpp:47-84) from the
         // host's X.
         const int* cats = any_cat ? B.is_cat.data() : nullptr;
+        // Edges from the device leave the host idle: the first trees' draws run meanwhile.
+        if (sampler && !cats && binner_fits_device(n, n_f, c.bin_sample)) sampler->start_workers();
         if (binner_fits_device(n, n_f, c.bin_sample))
             B.n_bins = binner_fit_device(Xd.p, x_dtype, n, n_f, c.max_bin, c.bin_sample,
                                          static_cast<uint32_t>(c.random_state), B.edges, B.n_edges, n_threads, s,
