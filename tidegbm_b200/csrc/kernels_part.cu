@@ -10,6 +10,9 @@
 //            from ballots, rows written to the other ping-pong buffer.  Block 0 also
 //            records n_left and, in tree mode, fills the children's segments and picks
 //            the smaller child (left on ties, cpp/src/tree.cpp:423).
+// Row-major codes cost a memory line a row, so they are read with load_sparse, 64 bytes of the
+// line, and the scatter finds them in the L2; the scatter of a given job also starts its first
+// tile's loads under the count.  1.2M of 4M rows x 128: 54.7 -> 42.3 -> 38.4 us.
 // A thread owns 8 rows of a tile (rows base + i*256 + tid), so each of the kernels
 // issues all its row-id loads, then all its code loads, before it waits: two memory
 // round trips per tile rather than one per 256 rows.
@@ -63,7 +66,7 @@ __device__ __forceinline__ void load_tile(const uint8_t* __restrict__ codes, int
         if (row[i] < 0) continue;
         if (j.flag) b[i] = j.flag[row[i]];
         else if (j.col) b[i] = j.col[static_cast<size_t>(j.feature) * j.col_n + row[i]];
-        else b[i] = codes[static_cast<size_t>(row[i]) * stride + j.feature];
+        else b[i] = static_cast<int>(load_sparse(codes + static_cast<size_t>(row[i]) * stride + j.feature));
     }
 #pragma unroll
     for (int i = 0; i < kPartPer; ++i) {
@@ -114,9 +117,18 @@ __global__ void __launch_bounds__(kPartThreads)
     part_scatter_kernel(const uint8_t* __restrict__ codes, int stride, PartJob given, DevNode* __restrict__ nodes,
                         DevTreeState* __restrict__ st, int32_t* rows0, int32_t* rows1,
                         const int* __restrict__ tile_counts) {
+    PartJob j = given;
+    int32_t row[kPartPer];
+    bool left[kPartPer];
+    // A given job's rows and codes are inputs of the count too, which started after all that was
+    // before it: the first tile's loads go out while the count still runs.
+    const bool early = st == nullptr && static_cast<int>(blockIdx.x) * kPartTile < j.count;
+    if (early) {
+        const int base = static_cast<int>(blockIdx.x) * kPartTile;
+        load_tile(codes, stride, j, base, base + min(kPartTile, j.count - base), row, left);
+    }
     pdl_wait();
     pdl_trigger();
-    PartJob j;
     if (!resolve_job(given, nodes, st, rows0, rows1, j)) return;
     __shared__ int red[kPartWarps];
     __shared__ int wc[kPartPer * kPartWarps];
@@ -152,9 +164,7 @@ __global__ void __launch_bounds__(kPartThreads)
         prev_tiles = t;
         const int base = t * kPartTile;
         const int end = min(base + kPartTile, j.count);
-        int32_t row[kPartPer];
-        bool left[kPartPer];
-        load_tile(codes, stride, j, base, end, row, left);
+        if (!early || t != static_cast<int>(blockIdx.x)) load_tile(codes, stride, j, base, end, row, left);
         unsigned bal[kPartPer];
 #pragma unroll
         for (int i = 0; i < kPartPer; ++i) {
