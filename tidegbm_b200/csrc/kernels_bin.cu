@@ -17,7 +17,10 @@
 // banks, 3.4 deep on average, one row at a time: 2,513 us for 4M x 128 float32.)  Eight rows
 // are searched together while the next eight load, and the first two of the eight steps
 // compare with edges held in registers, so a value costs six shared loads, compares and
-// predicated adds: 805 us there, bound by instruction issue (its bytes take 396 us).
+// predicated adds: 805 us there.  Edges past the last are NaN, which no value counts, and rows
+// are addressed by uniform pointers and a lane's 32-bit offset: 37 instructions a value instead
+// of 41, and registers for a fifth CTA on every SM: 750 us, with issue slots 73% busy and
+// waits for X the rest (its bytes take 396 us; four CTAs 805, six of six rows 862).
 #include "tgb_internal.h"
 
 #include <atomic>
@@ -30,8 +33,8 @@ namespace {
 constexpr int kBinWarps = 8;
 constexpr int kBinThreads = kBinWarps * 32;
 constexpr int kBinRows = 8;  // rows a lane searches together
-// CTAs per SM: 64 registers a thread, or 64 KB of double edges
-constexpr int kBinCtas32 = 4, kBinCtas64 = 3;
+// CTAs per SM: 51 registers a thread, or 64 KB of double edges
+constexpr int kBinCtas32 = 5, kBinCtas64 = 3;
 
 // std::upper_bound's own bisection (libstdc++ __upper_bound) over edge k at e[32 k]: the same
 // probes and the same answer as the reference, also when NaN edges break the order.
@@ -82,14 +85,14 @@ __device__ __forceinline__ double edge_at(unsigned p, double) {
     asm volatile("ld.shared.f64 %0, [%1 + %2];" : "=d"(v) : "r"(p), "n"(k * 256));
     return v;
 }
-// p += k unless v < e, as one compare and one predicated add.
+// p += k if v >= e (never with a NaN), as one compare and one predicated add.
 template <unsigned k>
 __device__ __forceinline__ void advance(unsigned& p, float v, float e) {
-    asm("{ .reg .pred t; setp.geu.f32 t, %1, %2; @t add.u32 %0, %0, %3; }" : "+r"(p) : "f"(v), "f"(e), "n"(k));
+    asm("{ .reg .pred t; setp.ge.f32 t, %1, %2; @t add.u32 %0, %0, %3; }" : "+r"(p) : "f"(v), "f"(e), "n"(k));
 }
 template <unsigned k>
 __device__ __forceinline__ void advance(unsigned& p, double v, double e) {
-    asm("{ .reg .pred t; setp.geu.f64 t, %1, %2; @t add.u32 %0, %0, %3; }" : "+r"(p) : "d"(v), "d"(e), "n"(k));
+    asm("{ .reg .pred t; setp.ge.f64 t, %1, %2; @t add.u32 %0, %0, %3; }" : "+r"(p) : "d"(v), "d"(e), "n"(k));
 }
 // One halving step of kBinRows searches: p is the shared address of the first edge not yet
 // known to be <= v.
@@ -124,7 +127,7 @@ __global__ void __launch_bounds__(kBinThreads, sizeof(T) == 4 ? kBinCtas32 : kBi
         for (int b0 = warp; b0 < 256; b0 += 16 * kBinWarps) {
             T v[16];
 #pragma unroll
-            for (int q = 0; q < 16; ++q) v[q] = b0 + q * kBinWarps < ne ? ef[b0 + q * kBinWarps] : T(INFINITY);
+            for (int q = 0; q < 16; ++q) v[q] = b0 + q * kBinWarps < ne ? ef[b0 + q * kBinWarps] : T(NAN);
 #pragma unroll
             for (int q = 0; q < 16; ++q) se[(b0 + q * kBinWarps) * 32 + lane] = v[q];
         }
@@ -135,7 +138,7 @@ __global__ void __launch_bounds__(kBinThreads, sizeof(T) == 4 ? kBinCtas32 : kBi
     // ascending edges without NaN: counting the edges <= v by halving steps is upper_bound
     bool plain = true;
 #pragma unroll 8
-    for (int b = warp; b < 255; b += kBinWarps) {  // past ne the staged edges are infinite
+    for (int b = warp; b < 255; b += kBinWarps) {  // past ne the staged edges are NaN: no value counts them
         const T lo = e[32 * b], hi = e[32 * (b + 1)];
         plain &= b >= ne || (b + 1 < ne ? lo <= hi : lo == lo);
     }
@@ -147,31 +150,37 @@ __global__ void __launch_bounds__(kBinThreads, sizeof(T) == 4 ? kBinCtas32 : kBi
     const int r1 = min(n, r0 + rows_per_cta);
     const T e127 = e[32 * 127], e63 = e[32 * 63], e191 = e[32 * 191];
     const int step = kBinWarps * rpw;
-    int r = r0 + warp * rpw + sub;
     constexpr unsigned kRow = 32 * sizeof(T);  // bytes from one edge to the next
     const unsigned base = static_cast<unsigned>(__cvta_generic_to_shared(e));
     const size_t x_step = static_cast<size_t>(step) * n_f, c_step = static_cast<size_t>(step) * stride;
-    const T* x = X + static_cast<size_t>(r) * n_f + f;
-    uint8_t* out = codes + static_cast<size_t>(r) * stride + f;
+    int r = r0 + warp * rpw + sub;
     if (active && plain && !cat) {
+        // the CTA's rows by uniform pointers, a lane's place in them by a 32-bit offset
+        const T* xb = X + static_cast<size_t>(r0) * n_f;
+        uint8_t* ob = codes + static_cast<size_t>(r0) * stride;
+        const unsigned xo = static_cast<unsigned>(warp * rpw + sub) * n_f + f;
+        const unsigned oo = static_cast<unsigned>(warp * rpw + sub) * stride + f;
+        const unsigned first = (base / kRow) - 1u;  // code = p / kRow - first
         T nv[kBinRows];  // the next rows' values, loaded while these are searched
-        const bool any = r + (kBinRows - 1) * step < r1;
+        int left = (r1 - r0) / (kBinRows * step);
 #pragma unroll
-        for (int q = 0; q < kBinRows; ++q) nv[q] = any ? __ldcs(x + q * x_step) : T(0);
-        for (; r + (kBinRows - 1) * step < r1; r += kBinRows * step, out += kBinRows * c_step) {
+        for (int q = 0; q < kBinRows; ++q) nv[q] = left > 0 ? __ldcs(xb + q * x_step + xo) : T(0);
+        r += left * kBinRows * step;
+        for (; left > 0; --left, ob += kBinRows * c_step) {
             T v[kBinRows];
             unsigned p[kBinRows];
 #pragma unroll
             for (int q = 0; q < kBinRows; ++q) v[q] = nv[q];
-            x += kBinRows * x_step;
-            const bool more = r + (2 * kBinRows - 1) * step < r1;
+            xb += kBinRows * x_step;
+            if (left > 1) {
 #pragma unroll
-            for (int q = 0; q < kBinRows; ++q) nv[q] = more ? __ldcs(x + q * x_step) : T(0);
+                for (int q = 0; q < kBinRows; ++q) nv[q] = __ldcs(xb + q * x_step + xo);
+            }
 #pragma unroll
             for (int q = 0; q < kBinRows; ++q) {
                 p[q] = base;
                 advance<128 * kRow>(p[q], v[q], e127);
-                advance<64 * kRow>(p[q], v[q], v[q] < e127 ? e63 : e191);
+                advance<64 * kRow>(p[q], v[q], v[q] >= e127 ? e191 : e63);
             }
             halve<32>(p, v);
             halve<16>(p, v);
@@ -180,12 +189,12 @@ __global__ void __launch_bounds__(kBinThreads, sizeof(T) == 4 ? kBinCtas32 : kBi
             halve<2>(p, v);
             halve<1>(p, v);
 #pragma unroll
-            for (int q = 0; q < kBinRows; ++q) {
-                const int code = min(static_cast<int>((p[q] - base) / kRow), ne) + 1;
-                out[q * c_step] = static_cast<uint8_t>(v[q] != v[q] ? 0 : code);  // NaN -> 0
-            }
+            for (int q = 0; q < kBinRows; ++q)
+                (ob + q * c_step)[oo] = static_cast<uint8_t>(v[q] != v[q] ? 0u : p[q] / kRow - first);  // NaN -> 0
         }
     }
+    const T* x = X + static_cast<size_t>(r) * n_f + f;
+    uint8_t* out = codes + static_cast<size_t>(r) * stride + f;
     if (active) {  // the last rows of a plain feature, all rows of the others
         for (; r < r1; r += step, x += x_step, out += c_step) {
             const T v = *x;
