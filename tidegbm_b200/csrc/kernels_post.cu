@@ -382,21 +382,49 @@ __device__ __forceinline__ const double* tree_prefix(const TreeOut& out, int t) 
     return out.prefix + static_cast<size_t>(t) * out.n_buckets * out.max_nodes;
 }
 
-__global__ void pred_update_kernel(PostParams pp, const int16_t* __restrict__ nid, TreeOut out,
-                                   const DevTreeState* __restrict__ st, double* __restrict__ pred) {
+// time_buckets on time-sorted rows (cpp/src/booster.cpp:60-72): rank = row.
+__device__ __forceinline__ int row_bucket(const PostParams& pp, int i) {
+    if (pp.iid_mode) return 0;
+    const int b = static_cast<int>(static_cast<double>(i) / max(pp.n, 1) * pp.n_buckets);
+    return min(b, pp.n_buckets - 1);
+}
+
+// The prediction updates go over steps of kUpdRows rows a thread (256 apart), whose loads go out
+// together.  The bucket is monotone in the row, so a step that starts and ends in one bucket, as
+// nearly all do, divides twice and not once a row.  With the loss, 10M rows: 78 -> 52 us of a
+// tree (its bytes take 52 at the copy rate), 1.2M: 20 -> 11.
+constexpr int kUpdThreads = 256;
+constexpr int kUpdRows = 4;
+constexpr int kUpdStep = kUpdThreads * kUpdRows;
+
+__global__ void __launch_bounds__(kUpdThreads)
+    pred_update_kernel(PostParams pp, const int16_t* __restrict__ nid, TreeOut out,
+                       const DevTreeState* __restrict__ st, double* __restrict__ pred) {
     pdl_wait();
     pdl_trigger();
     const double* __restrict__ prefix = tree_prefix(out, st->tree);
     const int nn = st->n_nodes;
     const int n = pp.n;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int b = 0;
-        if (!pp.iid_mode) {
-            // time_buckets on time-sorted rows (cpp/src/booster.cpp:60-72): rank = row.
-            b = static_cast<int>(static_cast<double>(i) / max(n, 1) * pp.n_buckets);
-            if (b >= pp.n_buckets) b = pp.n_buckets - 1;
+    for (long long base = static_cast<long long>(blockIdx.x) * kUpdStep; base < n;
+         base += static_cast<long long>(gridDim.x) * kUpdStep) {
+        const int i0 = static_cast<int>(base) + threadIdx.x;
+        const int end = static_cast<int>(min(base + kUpdStep, static_cast<long long>(n)));
+        double p[kUpdRows];
+        int k[kUpdRows];
+#pragma unroll
+        for (int q = 0; q < kUpdRows; ++q) {
+            const int i = i0 + q * kUpdThreads;
+            p[q] = i < end ? pred[i] : 0.0;
+            k[q] = i < end ? nid[i] : 0;
         }
-        pred[i] += pp.learning_rate * prefix[static_cast<size_t>(b) * nn + nid[i]];
+        const int b0 = row_bucket(pp, static_cast<int>(base)), b1 = row_bucket(pp, end - 1);
+#pragma unroll
+        for (int q = 0; q < kUpdRows; ++q) {
+            const int i = i0 + q * kUpdThreads;
+            if (i >= end) continue;
+            const int b = b0 == b1 ? b0 : row_bucket(pp, i);
+            pred[i] = p[q] + pp.learning_rate * prefix[static_cast<size_t>(b) * nn + k[q]];
+        }
     }
 }
 
@@ -406,10 +434,10 @@ __global__ void pred_update_kernel(PostParams pp, const int16_t* __restrict__ ni
 // the same double the gradient kernel computes) and its largest |g| into sc (reset by
 // finalize_tree), so that the next tree needs no separate pass over pred and y.  The last CTA to
 // finish adds the partial sums up, in a fixed order, and writes the loss.
-__global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict__ nid, TreeOut out,
-                                        DevTreeState* __restrict__ st, double* __restrict__ pred,
-                                        const double* __restrict__ y, double* __restrict__ partials,
-                                        double* __restrict__ g, AllScale* __restrict__ sc, int* __restrict__ ticket) {
+__global__ void __launch_bounds__(kUpdThreads)
+    pred_update_loss_kernel(PostParams pp, const int16_t* __restrict__ nid, TreeOut out, DevTreeState* __restrict__ st,
+                            double* __restrict__ pred, const double* __restrict__ y, double* __restrict__ partials,
+                            double* __restrict__ g, AllScale* __restrict__ sc, int* __restrict__ ticket) {
     pdl_wait();
     pdl_trigger();
     const int t = st->tree;
@@ -417,19 +445,33 @@ __global__ void pred_update_loss_kernel(PostParams pp, const int16_t* __restrict
     const int nn = st->n_nodes;
     const int n = pp.n;
     double acc = 0.0, mg = 0.0;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        int b = 0;
-        if (!pp.iid_mode) {
-            b = static_cast<int>(static_cast<double>(i) / max(n, 1) * pp.n_buckets);
-            if (b >= pp.n_buckets) b = pp.n_buckets - 1;
+    for (long long base = static_cast<long long>(blockIdx.x) * kUpdStep; base < n;
+         base += static_cast<long long>(gridDim.x) * kUpdStep) {
+        const int i0 = static_cast<int>(base) + threadIdx.x;
+        const int end = static_cast<int>(min(base + kUpdStep, static_cast<long long>(n)));
+        double p[kUpdRows], yv[kUpdRows];
+        int k[kUpdRows];
+#pragma unroll
+        for (int q = 0; q < kUpdRows; ++q) {
+            const int i = i0 + q * kUpdThreads;
+            p[q] = i < end ? pred[i] : 0.0;
+            yv[q] = i < end ? y[i] : 0.0;
+            k[q] = i < end ? nid[i] : 0;
         }
-        const double p = pred[i] + pp.learning_rate * prefix[static_cast<size_t>(b) * nn + nid[i]];
-        pred[i] = p;
-        const double d = p - y[i];
-        acc += 1.0 * d * d;
-        const double gv = 1.0 * d;
-        g[i] = gv;
-        mg = fmax(mg, fabs(gv));
+        const int b0 = row_bucket(pp, static_cast<int>(base)), b1 = row_bucket(pp, end - 1);
+#pragma unroll
+        for (int q = 0; q < kUpdRows; ++q) {
+            const int i = i0 + q * kUpdThreads;
+            if (i >= end) continue;
+            const int b = b0 == b1 ? b0 : row_bucket(pp, i);
+            const double pn = p[q] + pp.learning_rate * prefix[static_cast<size_t>(b) * nn + k[q]];
+            pred[i] = pn;
+            const double d = pn - yv[q];
+            acc += 1.0 * d * d;
+            const double gv = 1.0 * d;
+            g[i] = gv;
+            mg = fmax(mg, fabs(gv));
+        }
     }
     block_max_into(mg, 1.0, sc);
     __shared__ double ws[32];
@@ -642,12 +684,15 @@ void launch_predict_trees(const uint8_t* codes, int stride, int n, const Predict
     else predict_launch<1>(variant, bytes, codes, stride, n, m, base, lr, out, s);
 }
 
-int pred_update_parts(int n) { return std::max(1, std::min(2368, (n + 255) / 256)); }
+// Four CTAs an SM at most: a CTA's reductions cost more than its rows on small data.
+int pred_update_parts(int n) {
+    return static_cast<int>(std::max(1ll, std::min(592ll, (static_cast<long long>(n) + kUpdStep - 1) / kUpdStep)));
+}
 
 void launch_pred_update_loss(const PostParams& pp, const int16_t* nid, const TreeOut& out, DevTreeState* st,
                              double* pred, const double* y, double* partials, double* g, AllScale* sc, int* ticket,
                              cudaStream_t s) {
-    launch_pdl(pred_update_loss_kernel, dim3(pred_update_parts(pp.n)), dim3(256), 0, s, "pred_update_loss launch", pp, nid,
+    launch_pdl(pred_update_loss_kernel, dim3(pred_update_parts(pp.n)), dim3(kUpdThreads), 0, s, "pred_update_loss launch", pp, nid,
                out, st, pred, y, partials, g, sc, ticket);
 }
 
@@ -693,7 +738,7 @@ void launch_finalize_tree(const PostParams& pp, DevTreeState* st, unsigned long 
 
 void launch_pred_update(const PostParams& pp, const int16_t* nid, const TreeOut& out, const DevTreeState* st,
                         double* pred, cudaStream_t s) {
-    launch_pdl(pred_update_kernel, dim3(pred_update_parts(pp.n)), dim3(256), 0, s, "pred_update launch", pp, nid, out, st,
+    launch_pdl(pred_update_kernel, dim3(pred_update_parts(pp.n)), dim3(kUpdThreads), 0, s, "pred_update launch", pp, nid, out, st,
                pred);
 }
 
