@@ -18,8 +18,7 @@
 // round trips per tile rather than one per 256 rows.
 // In tree mode the job (row segment, feature, threshold, missing direction) is read
 // from the node table at st->parent, so the sequence runs without host
-// synchronisation; grids are sized for the largest node and exit early.  The same
-// kernels compact flagged rows (GOSS sample) in index order.
+// synchronisation; grids are sized for the largest node and exit early.
 #include "tgb_internal.h"
 
 #include <stdexcept>
@@ -64,14 +63,12 @@ __device__ __forceinline__ void load_tile(const uint8_t* __restrict__ codes, int
     for (int i = 0; i < kPartPer; ++i) {
         b[i] = 0;
         if (row[i] < 0) continue;
-        if (j.flag) b[i] = j.flag[row[i]];
-        else if (j.col) b[i] = j.col[static_cast<size_t>(j.feature) * j.col_n + row[i]];
+        if (j.col) b[i] = j.col[static_cast<size_t>(j.feature) * j.col_n + row[i]];
         else b[i] = static_cast<int>(load_sparse(codes + static_cast<size_t>(row[i]) * stride + j.feature));
     }
 #pragma unroll
     for (int i = 0; i < kPartPer; ++i) {
         if (row[i] < 0) left[i] = false;
-        else if (j.flag) left[i] = b[i] != 0;
         else left[i] = b[i] == 0 ? j.missing_left != 0 : b[i] <= j.threshold;
     }
 }
@@ -192,7 +189,7 @@ __global__ void __launch_bounds__(kPartThreads)
             const int lrank = excl[i] + __popc(bal[i] & lt_mask);  // lefts before k in the tile
             if (left[i]) {
                 j.out[left0 + lrank] = row[i];
-            } else if (!j.left_only) {
+            } else {
                 const int rrank = (k - base) - lrank;
                 j.out[n_left + (base - left0) + rrank] = row[i];
             }
@@ -238,18 +235,6 @@ void launch_partition_rows(const uint8_t* codes, int stride, const int32_t* rows
     }
     run_partition(codes, stride, j, nullptr, nullptr, nullptr, nullptr, tile_counts,
                   (n_rows + kPartTile - 1) / kPartTile, s);
-}
-
-void launch_compact_flagged(const uint8_t* flag, int n, int32_t* out, int* n_out_dev, int* tile_counts,
-                            cudaStream_t s) {
-    PartJob j{};
-    j.in = nullptr;  // rows are 0..n-1
-    j.out = out;
-    j.count = n;
-    j.flag = flag;
-    j.left_only = 1;
-    j.n_left_out = n_out_dev;
-    run_partition(nullptr, 0, j, nullptr, nullptr, nullptr, nullptr, tile_counts, (n + kPartTile - 1) / kPartTile, s);
 }
 
 // ---- partition without caller-provided scratch -------------------------------------

@@ -90,14 +90,11 @@ struct AllScale {
 struct PartJob {
     const int32_t* in;    // row list (nullptr: rows 0..count-1)
     int32_t* out;
-    const uint8_t* flag;  // compaction mode: keep rows with flag != 0
     int* n_left_out;      // optional copy of n_left
     const uint8_t* col;   // column-major codes [F][col_n] (nullptr: read the row-major codes)
     long long col_n;
     int count;
     int feature, threshold, missing_left;
-    int left_only;
-    int pad;
 };
 
 struct GrowParams {
@@ -354,8 +351,6 @@ void launch_codes_transpose(const uint8_t* codes, int stride, int n, int n_f, ui
 void launch_partition_rows(const uint8_t* codes, int stride, const int32_t* rows, int n_rows, int feature,
                            int threshold, int missing_left, int32_t* out, int* n_left_dev, int* tile_counts,
                            cudaStream_t s);
-void launch_compact_flagged(const uint8_t* flag, int n, int32_t* out, int* n_out_dev, int* tile_counts,
-                            cudaStream_t s);
 // Same partition with its scratch in a fixed device array of kernels_part.cu (no allocation).
 int partition_noalloc_max_rows();
 void launch_partition_rows_noalloc(const uint8_t* codes, int stride, const int32_t* rows, int n_rows, int feature,
