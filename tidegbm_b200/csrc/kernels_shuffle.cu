@@ -17,11 +17,11 @@
 //   shuffle_resolve_kernel  every slot: last[p], else the walk above, answered from the
 //                           buckets; written over last[p]
 // The generator is MT19937 (Matsumoto & Nishimura, ACM TOMACS 8(1), 1998), seeded as
-// std::mt19937(seed) is, with the 624-word state in shared memory, one thread per word.
+// std::mt19937(seed) is, with the 624-word state in shared memory, two words a thread.
 // A refill is the recurrence x[k+624] = x[k+397] ^ mix(x[k], x[k+1]); with
 // a[k] = mix(old[k], old[k+1]) (^ old[k+397] for k < 227) the new words are
 // a[k] ^ a[k-227] ^ a[k-454] (terms with negative index omitted), and word 623 mixes
-// with the new word 0: one shared-memory pass and one barrier per 624 words.
+// with the new word 0: one shared-memory pass and two barriers per 624 words.
 // Word q of a block serves draw t + q.  Lemire's method (the one libstdc++'s
 // uniform_int_distribution uses for a 32-bit generator) rejects a word when the low
 // half of w * (t + 1) is below 2^32 mod (t + 1); that draw then takes the next word,
@@ -67,8 +67,9 @@ __device__ __forceinline__ uint32_t mt_temper(uint32_t v) {
     return v;
 }
 
-// The threads of one role.
+// The threads of one role (the barrier wants whole warps).
 __device__ __forceinline__ void role_sync(int id) {
+    __syncwarp();
     asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kDrawRole) : "memory");
 }
 
