@@ -52,8 +52,8 @@ TGB_API void tgb_booster_free(tgb_booster* b);
  * stochastically rounded to int16 / int8 per tree, summed exactly in 32-bit words: fewer
  * shared reductions per code, an approximate split search; leaf values stay exact);
  * "grow" = 1 (default: batched waves, many leaves per launch) or 0 (one split per
- * launch sequence; hist_bits 0, or 8 with objective mse); "graph" = 1 (default: a tree's
- * waves run as one CUDA graph with a device-side loop) or 0 (enqueued by the host);
+ * launch sequence; hist_bits 0, or 8 with objective mse); "graph" = 1 (default: a tree
+ * runs as one CUDA graph, its waves a device-side loop) or 0 (enqueued by the host);
  * "hist_tune" = 1 (default: the histogram's launch shape is tuned on the first tree and
  * kept for the process) or 0; "wave_expand" = 8 (default: a wave plans the 8 best leaves
  * ranked within the splits left), k > 0 (the k best) or 0 (all of them; the same trees
@@ -127,7 +127,7 @@ TGB_API int tgb_fit_stats(tgb_booster* b, double* out18);
  * "transpose", "trees", "pre_upload" / "prep" (host set-up before the upload / before
  * the tree loop), "goss_refits" (1 when the fit was repeated with the full 64-bit GOSS
  * sort), "timed_selects" (wave selects run in the timed range: with batched growth a tree
- * runs 3 + 4 x (selects - 1) kernels in its waves), "graph_used" (1 when the waves ran as
+ * runs 3 + 4 x (selects - 1) kernels in its waves), "graph_used" (1 when trees ran as
  * a CUDA graph), "hist_cluster" / "hist_clusters" (the tuned launch shape of the
  * histogram: CTAs per cluster, clusters launched), "driver" (set-up of the batched
  * growth), "driver_free" (its release after the tree loop), "finish_sync" (from the tree

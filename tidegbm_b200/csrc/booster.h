@@ -68,8 +68,8 @@ struct Config {
     // search, exact leaf values).  With grow = 0 only 8 with a constant hessian (mse).
     int hist_bits = 0;
     // Tree growth: 1 = batched waves (many leaves, and many fits, per launch; wave.h),
-    // 0 = one split per iteration.  Both grow the reference's tree.  graph: the waves of a
-    // tree run as one CUDA graph with a device-side loop (1) or are enqueued by the host (0).
+    // 0 = one split per iteration.  Both grow the reference's tree.  graph: a tree runs
+    // as one CUDA graph, its waves a device-side loop (1), or is enqueued by the host (0).
     int grow = 1;
     int graph = 1;
     // Batched growth: tune the histogram's launch shape on the first tree (1), or use the
@@ -128,7 +128,7 @@ struct FitStats {
     int hist_launches = 0;
     long long hist_rows = 0;  // rows histogrammed in the timed range
     long long timed_selects = 0;  // wave selects run in the timed range (batched growth)
-    int graph_used = 0;           // the waves ran as a CUDA graph with a device-side loop
+    int graph_used = 0;           // trees ran as a CUDA graph with a device-side loop
     int hist_cluster = 0, hist_clusters = 0;  // the histogram's launch shape (autotuned)
 };
 
