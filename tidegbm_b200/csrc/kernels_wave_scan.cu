@@ -647,8 +647,9 @@ __global__ void __launch_bounds__(kPairThreads, 2)
                 const bool weak = t.eligible && X.gp.n_features >= 2 && X.pair_top_k >= 2 &&
                                   ((axis_gain < X.pair_trigger * fmax(energy * 0.01, 1e-12)) || axis_gain <= 0);
                 if (weak) cnt = N->count;
-                else if (j % static_cast<int>(gridDim.x) == static_cast<int>(blockIdx.x))
-                    *(src == 0 ? X.splits_pair : X.spec_split_pair + t.ci) = *axis;  // no pair search
+                // no pair search: also for a weak child without rows (min_samples_leaf 0), which no chunk finishes
+                if (cnt == 0 && j % static_cast<int>(gridDim.x) == static_cast<int>(blockIdx.x))
+                    *(src == 0 ? X.splits_pair : X.spec_split_pair + t.ci) = *axis;
             }
         }
         // chunks of the batch's weak children
