@@ -430,7 +430,7 @@ __device__ __noinline__ unsigned int accumulate_const_tma(unsigned int* __restri
                     phase ^= 1u << s;
                     pending &= ~(1u << s);
                 } else if (lane == 0) {
-                    atomicExch(err, kErrStaging);
+                    set_error(err, kErrStaging);
                 }
             }
             const unsigned int rp = slot0 + s * kSlotStride + lane * 32;
@@ -1252,7 +1252,6 @@ __device__ __forceinline__ void init_tree(DevNode* nodes, DevSplit* splits, DevT
     ctl->tiles_total = 0;
     ctl->active = 1;
     ctl->slot0 = 1;
-    ctl->error = 0;
     ctl->waves = 0;
     ctl->pair_used = 0;
     ctl->expanded[0] = 0;

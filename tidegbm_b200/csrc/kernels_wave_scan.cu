@@ -494,12 +494,12 @@ __global__ void __launch_bounds__(kSelectThreads)
                 ctl->slot0 = slot_first;
                 ctl->exp_counter += n_exp;
                 ctl->exp_total += n_exp;
-                if (slot_first + 2 * n_exp > X.n_slots || base_tiles > X.max_tiles) ctl->error = 1;
+                if (slot_first + 2 * n_exp > X.n_slots || base_tiles > X.max_tiles) set_error(&ctl->error, 1);
             }
             active = n_exp > 0 && slot_first + 2 * n_exp <= X.n_slots && base_tiles <= X.max_tiles;
         }
         if (lane == 0) {
-            if (runaway) ctl->error = 1;
+            if (runaway) set_error(&ctl->error, 1);
             st->n_nodes = nn;
             ctl->splits_done = done_splits;
             ctl->pair_used = pair_used;

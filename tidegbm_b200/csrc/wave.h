@@ -92,7 +92,9 @@ struct WaveCtl {
     int tiles_total;  // partition tiles of the planned expansions
     int active;       // 1 while the tree grows
     int slot0;        // first histogram slot of the planned expansions
-    int error;        // a slot, buffer or wave-count bound was hit (never expected)
+    // a slot, buffer or wave-count bound was hit, or a staging wait gave up (never expected): the
+    // first such code of the fit, zeroed with the fit's buffers and read after its last tree
+    int error;
     int waves;        // selects run for this tree (bounded: a tree needs at most max_leaves)
     int pair_used;    // PAIR splits committed in this tree
     int exp_total;    // expansions planned over all trees of the fit (not reset per tree)
@@ -186,6 +188,9 @@ __device__ __forceinline__ int energy_shift(const DevTreeState* st) {
     const int clog = n > 1 ? 32 - __clz(n - 1) : 0;
     return max(-1000, min(1000, 61 - (ilogb(e2) + 1) - clog));
 }
+
+// Notes an error of the fit; a later one does not replace it.
+__device__ __forceinline__ void set_error(int* error, int code) { atomicCAS(error, 0, code); }
 
 // Copies the first context into shared memory (the caller synchronises the CTA).  The
 // contexts are written before the fit's first tree and do not change, so a wave kernel does
