@@ -262,84 +262,80 @@ __global__ void __launch_bounds__(kGradWarps * 32)
     if (sc != nullptr) block_max_into(mg, mh, sc);
 }
 
-// A CTA takes runs in turn, so that a panel of many dates costs one ticket a resident CTA (a
-// ticket a run took 0.6 ms a tree at 100,000 runs; a CTA a run without tickets 0.11).
+// A CTA a run; the last one to finish adds the correlations up, all loads of a step before the
+// first use: 100,000 runs of 3 rows 311 us (611 with a load of the correlation behind each load
+// of its flag, 128 threads over all of them; 353 with resident CTAs that walk the runs).
 constexpr int kLossThreads = 128;
-constexpr int kLossCtas = 148 * 12;  // resident at once (40 registers a thread)
-constexpr int kLossSums = 8;         // partial sums a thread of the last CTA: 1,024 in all
+constexpr int kLossSums = 8;  // partial sums a thread of the last CTA: 1,024 in all
 
 __global__ void __launch_bounds__(kLossThreads)
     loss_pairwise_kernel(const double* __restrict__ y, const double* __restrict__ pred,
                          const int* __restrict__ run_start, const int* __restrict__ run_len,
-                         const int* __restrict__ order, int n_runs, double* __restrict__ corr,
+                         const int* __restrict__ order, double* __restrict__ corr,
                          int* __restrict__ valid, int* __restrict__ ticket, DevTreeState* __restrict__ st,
                          double* __restrict__ losses) {
+    const int n_runs = gridDim.x, r = blockIdx.x;
+    const int s0 = run_start[r], m = run_len[r];
     __shared__ double red[3][32];
     __shared__ double mean[2];
     __shared__ int s_last, s_ok[32];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5, nw = kLossThreads / 32;
-    for (int r = blockIdx.x; r < n_runs; r += gridDim.x) {
-        const int s0 = run_start[r], m = run_len[r];
-        double sy = 0, sp = 0;
-        for (int k = threadIdx.x; k < m; k += kLossThreads) {
-            const int i = row_at(order, s0 + k);
-            sy += y[i];
-            sp += pred[i];
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            sy += __shfl_xor_sync(0xffffffffu, sy, o);
-            sp += __shfl_xor_sync(0xffffffffu, sp, o);
-        }
-        __syncthreads();  // the run before is done
-        if (lane == 0) {
-            red[0][w] = sy;
-            red[1][w] = sp;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0, b = 0;
-            for (int k = 0; k < nw; ++k) {
-                a += red[0][k];
-                b += red[1][k];
-            }
-            mean[0] = a / m;
-            mean[1] = b / m;
-        }
-        __syncthreads();
-        double vy = 0, vp = 0, c = 0;
-        for (int k = threadIdx.x; k < m; k += kLossThreads) {
-            const int i = row_at(order, s0 + k);
-            const double dy = y[i] - mean[0], dp = pred[i] - mean[1];
-            vy += dy * dy;
-            vp += dp * dp;
-            c += dy * dp;
-        }
-        for (int o = 16; o > 0; o >>= 1) {
-            vy += __shfl_xor_sync(0xffffffffu, vy, o);
-            vp += __shfl_xor_sync(0xffffffffu, vp, o);
-            c += __shfl_xor_sync(0xffffffffu, c, o);
-        }
-        if (lane == 0) {  // (the sums of y and pred were read before the last barrier)
-            red[0][w] = vy;
-            red[1][w] = vp;
-            red[2][w] = c;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            double a = 0, b = 0, cc = 0;
-            for (int k = 0; k < nw; ++k) {
-                a += red[0][k];
-                b += red[1][k];
-                cc += red[2][k];
-            }
-            const bool ok = m >= 3 && a > 1e-18 && b > 1e-18;
-            corr[r] = ok ? cc / sqrt(a * b) : 0.0;
-            valid[r] = ok ? 1 : 0;
-        }
+    double sy = 0, sp = 0;
+    for (int k = threadIdx.x; k < m; k += kLossThreads) {
+        const int i = row_at(order, s0 + k);
+        sy += y[i];
+        sp += pred[i];
     }
+    for (int o = 16; o > 0; o >>= 1) {
+        sy += __shfl_xor_sync(0xffffffffu, sy, o);
+        sp += __shfl_xor_sync(0xffffffffu, sp, o);
+    }
+    if (lane == 0) {
+        red[0][w] = sy;
+        red[1][w] = sp;
+    }
+    __syncthreads();
     if (threadIdx.x == 0) {
+        double a = 0, b = 0;
+        for (int k = 0; k < nw; ++k) {
+            a += red[0][k];
+            b += red[1][k];
+        }
+        mean[0] = a / m;
+        mean[1] = b / m;
+    }
+    __syncthreads();
+    double vy = 0, vp = 0, c = 0;
+    for (int k = threadIdx.x; k < m; k += kLossThreads) {
+        const int i = row_at(order, s0 + k);
+        const double dy = y[i] - mean[0], dp = pred[i] - mean[1];
+        vy += dy * dy;
+        vp += dp * dp;
+        c += dy * dp;
+    }
+    for (int o = 16; o > 0; o >>= 1) {
+        vy += __shfl_xor_sync(0xffffffffu, vy, o);
+        vp += __shfl_xor_sync(0xffffffffu, vp, o);
+        c += __shfl_xor_sync(0xffffffffu, c, o);
+    }
+    if (lane == 0) {  // (the sums of y and pred were read before the last barrier)
+        red[0][w] = vy;
+        red[1][w] = vp;
+        red[2][w] = c;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        double a = 0, b = 0, cc = 0;
+        for (int k = 0; k < nw; ++k) {
+            a += red[0][k];
+            b += red[1][k];
+            cc += red[2][k];
+        }
+        const bool ok = m >= 3 && a > 1e-18 && b > 1e-18;
+        corr[r] = ok ? cc / sqrt(a * b) : 0.0;
+        valid[r] = ok ? 1 : 0;
         __threadfence();
-        s_last = atomicAdd(ticket, 1) == static_cast<int>(gridDim.x) - 1;
+        s_last = atomicAdd(ticket, 1) == n_runs - 1;
         __threadfence();
     }
     __syncthreads();
@@ -348,14 +344,20 @@ __global__ void __launch_bounds__(kLossThreads)
     // threads over the runs and then their 32 warps would.
     double t[kLossSums] = {};
     int n_ok[kLossSums] = {};
-    for (int k0 = 0; k0 < n_runs; k0 += kLossThreads * kLossSums) {
+#pragma unroll 2
+    for (int k0 = threadIdx.x; k0 < n_runs; k0 += kLossThreads * kLossSums) {
+        double c[kLossSums];
+        int ok[kLossSums];
+#pragma unroll
+        for (int q = 0; q < kLossSums; ++q) {  // a run that is not valid has left a zero
+            const int k = k0 + q * kLossThreads;
+            c[q] = k < n_runs ? __ldcg(corr + k) : 0.0;
+            ok[q] = k < n_runs ? __ldcg(valid + k) : 0;
+        }
 #pragma unroll
         for (int q = 0; q < kLossSums; ++q) {
-            const int k = k0 + q * kLossThreads + static_cast<int>(threadIdx.x);
-            if (k < n_runs && __ldcg(valid + k)) {
-                t[q] += __ldcg(corr + k);
-                n_ok[q] += 1;
-            }
+            t[q] += c[q];
+            n_ok[q] += ok[q];
         }
     }
 #pragma unroll
@@ -424,8 +426,7 @@ void launch_loss_pairwise(const double* y, const double* pred, const int* run_st
                           const int* order, int n_runs, double* corr, int* valid, int* ticket, DevTreeState* st,
                           double* losses, cudaStream_t s) {
     if (n_runs <= 0) return;
-    loss_pairwise_kernel<<<std::min(n_runs, kLossCtas), kLossThreads, 0, s>>>(y, pred, run_start, run_len, order, n_runs, corr,
-                                                                             valid, ticket, st, losses);
+    loss_pairwise_kernel<<<n_runs, kLossThreads, 0, s>>>(y, pred, run_start, run_len, order, corr, valid, ticket, st, losses);
     check(cudaGetLastError(), "loss_pairwise launch");
 }
 
