@@ -1021,10 +1021,11 @@ bool FitRun::finish() {
 //
 // The wave sequence of one tree of every context: roots (histogram, scan, select), then
 // waves (partition, histogram of the smaller children, scan, select) until no context
-// grows.  With `graph`, the whole sequence is one CUDA graph per fit: a conditional WHILE
-// node repeats the wave body while select leaves the loop condition at 1, so a tree costs
-// one graph launch and no host round trip.  Without it the host enqueues waves ahead of
-// the device and stops two waves after a mapped flag says every tree is done.
+// grows.  With `graph`, a tree, its set-up and its sweep included, is one launch of a CUDA
+// graph made once a fit: some waves in a row, more in IF nodes, the rest in a conditional WHILE
+// node whose condition the select sets (build_graph).  Without it the host enqueues waves ahead
+// of the device and stops two waves after a mapped flag says every tree is done.
+
 // Mapped host flags of the host-driven wave loop, kept for the process: allocating and
 // freeing mapped pinned memory can take tens to hundreds of milliseconds, which every fit
 // would otherwise pay.  Portable, so any device may use a flag.
@@ -1257,6 +1258,10 @@ private:
         }
     }
 
+    // Waves after which a tree that has ended skips the rest (build_graph).
+    static constexpr int kWaveStepCount = 3;
+    static constexpr int kWaveSteps[kWaveStepCount] = {3, 8, 16};
+
     void zero_roots() {
         for (auto* r : runs_) {
             const size_t slot = static_cast<size_t>(r->n_f) * kBins;
@@ -1286,66 +1291,85 @@ private:
         return least;
     }
 
+    // A whole tree of every context: each context's set-up on a branch of its own, the root
+    // stage, the waves that every full tree takes, then a WHILE node whose body is one wave,
+    // and each context's sweep on its branch.  The host then makes one launch a tree (and
+    // the copies of the draw positions): enqueueing six folds' set-ups and sweeps took it
+    // 0.55 ms of a 2.66 ms tree, in which the device waited, and they ran one after another.
+    // An iteration of the node costs about 4 us more than the next kernels of a stream.  A full
+    // tree takes at least straight_waves() and, in best-first order, a third more (9 to 12 for
+    // 31 leaves): 8 straight waves there took fits of 100k x 32, 0.85M x 64 and 10M x 128 from
+    // 69.7, 74.6 and 391 ms to 67.4, 72.8 and 386.  But a straight wave after the tree's end costs
+    // its five empty kernels (8 us), and trees end early where no split is left worth taking: so
+    // only the first kWaveSteps[0] waves run in any case, the further ones as bodies of IF nodes,
+    // in steps about as long as what came before.  Fits of 80 trees of one or two leaves, 5,000 rows:
+    // 14.2 -> 9.8 ms with 31 leaves allowed, 23.7 -> 13.3 with 255 (12.3 and 15.2 with every wave
+    // an iteration of the loop); an IF node costs a full tree 5 us (fit of 100k x 32: 60.0 -> 60.5 ms).
     void build_graph() {
-        // A whole tree of every context: each context's set-up on a branch of its own, the root
-        // stage, the waves that every full tree takes, then a WHILE node whose body is one wave,
-        // and each context's sweep on its branch.  The host then makes one launch a tree (and
-        // the copies of the draw positions): enqueueing six folds' set-ups and sweeps took it
-        // 0.55 ms of a 2.66 ms tree, in which the device waited, and they ran one after another.
-        // An iteration of the node costs about 4 us more than the next kernels of a stream; a
-        // straight wave after the tree's end costs its five empty kernels.  A full tree takes at
-        // least straight_waves() and, in best-first order, a third more (9 to 12 for 31 leaves):
-        // 8 straight waves there took fits of 100k x 32, 0.85M x 64 and 10M x 128 from 69.7, 74.6
-        // and 391 ms to 67.4, 72.8 and 386.
         check(cudaGraphCreate(&graph_, 0), "graph create");
-        cudaGraphConditionalHandle handle;
-        check(cudaGraphConditionalHandleCreate(&handle, graph_, 1, cudaGraphCondAssignDefault),
-              "graph conditional handle");
         std::vector<OwnedStream>(n_ctx_ - 1).swap(side_);
         for (auto& q : side_) check(cudaStreamCreateWithFlags(&q.s, cudaStreamNonBlocking), "cudaStreamCreate");
         std::vector<OwnedEvent>(n_ctx_).swap(side_ev_);
         for (auto& e : side_ev_) e.get();
+        // the waves before the WHILE node, cut at kWaveSteps, and every conditional node's handle:
+        // 0 unless the last select before the node finds a tree that still grows
+        const int straight = std::min(kWaveSteps[kWaveStepCount - 1], straight_waves() * 4 / 3);
+        std::vector<int> steps;
+        for (int k = 0, done = 0; k < kWaveStepCount && done < straight; ++k) {
+            steps.push_back(std::min(kWaveSteps[k], straight) - done);
+            done += steps.back();
+        }
+        std::vector<cudaGraphConditionalHandle> handles(std::max<size_t>(1, steps.size()));
+        for (auto& h : handles)
+            check(cudaGraphConditionalHandleCreate(&h, graph_, 0, cudaGraphCondAssignDefault), "graph conditional handle");
         const long long before = t_kernel_launches;
+        // n waves; the last select sets the condition `next`
+        auto waves = [&](int n, cudaGraphConditionalHandle next) {
+            for (int k = 0; k < n; ++k) {
+                launch_wave_partition(ctx_.p, n_ctx_, part_grid_, pair_, s_);
+                launch_wave_hist(mode_, ctx_.p, n_ctx_, 1, tune_, rows_counter_, s_);
+                launch_wave_scan(ctx_.p, n_ctx_, 1, max_f_, scan_ys_, cat_, s_);
+                if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 1, (mode_ & 1) != 0, s_);
+                launch_wave_select(ctx_.p, n_ctx_, gsync_.p, nullptr, next, k == n - 1 ? 1 : 0, s_);
+            }
+        };
         check(cudaStreamBeginCaptureToGraph(s_, graph_, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
               "graph capture");
         branch([](FitRun* r, cudaStream_t q) { r->tree_begin(0, q); });
         launch_wave_hist(mode_, ctx_.p, n_ctx_, 0, tune_, rows_counter_, s_);
         launch_wave_scan(ctx_.p, n_ctx_, 0, max_f_, scan_ys_, cat_, s_);
         if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 0, (mode_ & 1) != 0, s_);
-        launch_wave_select(ctx_.p, n_ctx_, gsync_.p, nullptr, handle, 1, s_);
-        auto wave = [&] {
-            launch_wave_partition(ctx_.p, n_ctx_, part_grid_, pair_, s_);
-            launch_wave_hist(mode_, ctx_.p, n_ctx_, 1, tune_, rows_counter_, s_);
-            launch_wave_scan(ctx_.p, n_ctx_, 1, max_f_, scan_ys_, cat_, s_);
-            if (pair_) launch_wave_pair(ctx_.p, n_ctx_, 1, (mode_ & 1) != 0, s_);
-            launch_wave_select(ctx_.p, n_ctx_, gsync_.p, nullptr, handle, 1, s_);
-        };
-        const int straight = std::min(16, straight_waves() * 4 / 3);
-        for (int k = 0; k < straight; ++k) wave();
-        cudaStreamCaptureStatus cs;
-        const cudaGraphNode_t* deps = nullptr;
-        size_t n_deps = 0;
-        check(cudaStreamGetCaptureInfo(s_, &cs, nullptr, nullptr, &deps, &n_deps), "capture info");
-        cudaGraphNodeParams cp = {};
-        cp.type = cudaGraphNodeTypeConditional;
-        cp.conditional.handle = handle;
-        cp.conditional.type = cudaGraphCondTypeWhile;
-        cp.conditional.size = 1;
-        cudaGraphNode_t cond_node;
-        check(cudaGraphAddNode(&cond_node, graph_, deps, n_deps, &cp), "graph conditional node");
-        cudaGraph_t body = cp.conditional.phGraph_out[0];
-        check(cudaStreamUpdateCaptureDependencies(s_, &cond_node, 1, cudaStreamSetCaptureDependencies),
-              "capture dependencies");
+        launch_wave_select(ctx_.p, n_ctx_, gsync_.p, nullptr, handles[0], steps.empty() ? 1 : 0, s_);
+        if (!steps.empty()) waves(steps[0], handles[0]);
+        // the conditional nodes, one after another: an IF a further step, then the WHILE
+        std::vector<cudaGraph_t> bodies;
+        for (size_t k = 0; k < handles.size(); ++k) {
+            cudaStreamCaptureStatus cs;
+            const cudaGraphNode_t* deps = nullptr;
+            size_t n_deps = 0;
+            check(cudaStreamGetCaptureInfo_v2(s_, &cs, nullptr, nullptr, &deps, &n_deps), "capture info");
+            cudaGraphNodeParams cp = {};
+            cp.type = cudaGraphNodeTypeConditional;
+            cp.conditional.handle = handles[k];
+            cp.conditional.type = k + 1 < handles.size() ? cudaGraphCondTypeIf : cudaGraphCondTypeWhile;
+            cp.conditional.size = 1;
+            cudaGraphNode_t node = nullptr;
+            check(cudaGraphAddNode(&node, graph_, deps, n_deps, &cp), "conditional node");
+            bodies.push_back(cp.conditional.phGraph_out[0]);
+            check(cudaStreamUpdateCaptureDependencies(s_, &node, 1, cudaStreamSetCaptureDependencies), "capture dependencies");
+        }
         branch([](FitRun* r, cudaStream_t q) { r->tree_end(q); });
         graph_kernels_ = t_kernel_launches - before;
         cudaGraph_t top = nullptr;
         check(cudaStreamEndCapture(s_, &top), "graph capture end");
-        // the body: one wave
-        check(cudaStreamBeginCaptureToGraph(s_, body, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
-              "body capture");
-        wave();
-        cudaGraph_t body_out = nullptr;
-        check(cudaStreamEndCapture(s_, &body_out), "body capture end");
+        for (size_t k = 0; k < bodies.size(); ++k) {
+            const bool last = k + 1 == bodies.size();
+            check(cudaStreamBeginCaptureToGraph(s_, bodies[k], nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal),
+                  "body capture");
+            waves(last ? 1 : steps[k + 1], last ? handles[k] : handles[k + 1]);
+            cudaGraph_t body_out = nullptr;
+            check(cudaStreamEndCapture(s_, &body_out), "body capture end");
+        }
         check(cudaGraphInstantiate(&exec_, graph_, 0), "graph instantiate");
         // captured, not launched: tree() counts the kernels of the top graph
         g_kernel_launches.fetch_sub(t_kernel_launches - before);
