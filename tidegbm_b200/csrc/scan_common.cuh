@@ -146,8 +146,8 @@ __device__ __forceinline__ double near_rcp(double d) {
 // candidates side by side; the second evaluates the reference's expression for those within
 // 2^-34 of the warp's best estimate, usually one.  The others cannot win or tie: the gain is
 // a monotone function of that sum, the parent's term is at most twice it (hessian sums are
-// not negative), and where a gamma could absorb the difference, or a denominator lies
-// outside the range of the reciprocal, every candidate is evaluated.
+// not negative), and where a gamma could absorb the difference, a denominator lies outside
+// the range of the reciprocal, or a term near the ends of a double's, every candidate is evaluated.
 __device__ __forceinline__ Cand scan_feature_warp(long long* __restrict__ Gf, long long* __restrict__ Hf,
                                                   int* __restrict__ Cf, const long long* __restrict__ PGf,
                                                   const long long* __restrict__ PHf, const int* __restrict__ PCf,
@@ -271,9 +271,15 @@ __device__ __forceinline__ Cand scan_feature_warp(long long* __restrict__ Gf, lo
             __reduce_max_sync(0xffffffffu, static_cast<unsigned>(tb >> 32) == hi ? static_cast<unsigned>(tb) : 0u);
         top = __longlong_as_double(static_cast<long long>((static_cast<unsigned long long>(hi) << 32) | lo));
     }
-    // every denominator lies in [l2 + min_child_weight, H + l2]
-    const bool exact_all = !(lam + fmax(min_hess, 0.0) >= 1e-30) || !(dHt + lam < 1e30) || !(top > 0.0) ||
-                           !(fabs(gamma) <= top * inv_gs * inv_gs * 1048576.0);
+    // When to evaluate every candidate.  Every denominator lies in [l2 + min_child_weight, H + l2],
+    // which must lie in the reciprocal's range.  A candidate left out is more than 2^-35.1 of
+    // sum = top * inv_gs^2 below the best in the gain; its gain then rounds below the best's as
+    // long as one ulp of the gain, at most 2^-52 (|gamma| + 1.5 sum), is less: |gamma| <= 2^16 sum
+    // (at 2^20, the bound before, two gains could round alike and the lower bin be lost).  And
+    // no term may overflow or fall among the denormals.
+    const double sum = top * inv_gs * inv_gs;
+    const bool exact_all = !(lam + fmax(min_hess, 0.0) >= 1e-30) || !(dHt + lam < 1e30) || !(sum > 1e-270) ||
+                           !(sum < 1e270) || !(fabs(gamma) <= sum * 65536.0);
     if (!exact_all) {
         const double least = top * (1.0 - 0x1p-34);
 #pragma unroll
@@ -311,7 +317,8 @@ __device__ __forceinline__ Cand scan_feature_warp(long long* __restrict__ Gf, lo
 // sort past 2 * floor(log2 n) levels, then insertion sort), restated step for step so
 // that elements the comparator ties end in the order the reference's std::sort leaves
 // them (best_categorical sorts bins by a ratio that ties for bins of equal sums).  One
-// thread, at most 256 elements in shared memory; less(a, b) compares two elements.
+// thread, at most 1,024 elements (the PAIR ranking's features) in shared memory; less(a, b)
+// compares two elements.
 template <typename Less>
 __device__ void libstdcxx_sort(short* v, int n, Less less) {
     struct Sorter {
