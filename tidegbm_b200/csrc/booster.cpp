@@ -35,7 +35,12 @@ std::atomic<long long> g_kernel_launches{0};
 static thread_local long long t_kernel_launches = 0;  // this thread's share of them
 
 void check(cudaError_t e, const char* what) {
-    if (e != cudaSuccess) throw TideError(std::string("CUDA ") + what + ": " + cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // the next launch's check is not to find this one
+        const std::string msg = std::string("CUDA ") + what + ": " + cudaGetErrorString(e);
+        if (e == cudaErrorMemoryAllocation) throw OutOfMemory(msg);
+        throw TideError(msg);
+    }
     const size_t L = std::strlen(what);
     if (L > 7 && std::strcmp(what + L - 7, " launch") == 0) {
         g_kernel_launches.fetch_add(1);

@@ -13,6 +13,9 @@ namespace tgb {
 struct TideError : std::runtime_error {
     explicit TideError(const std::string& m) : std::runtime_error(m) {}
 };
+struct OutOfMemory : TideError {  // of the device
+    using TideError::TideError;
+};
 
 // The Config fields (cpp/include/tidegbm/config.hpp:12-97) the GPU path reads.  Every
 // other option keeps its default; options the GPU path does not implement are
