@@ -15,7 +15,6 @@
 #include <atomic>
 #include <chrono>
 #include <cmath>
-#include <condition_variable>
 #include <cstring>
 #include <exception>
 #include <mutex>
@@ -24,6 +23,7 @@
 
 #include <memory>
 
+#include "batch_setup.h"
 #include "goss_sampler.h"
 #include "sampling.h"
 #include "tgb_internal.h"
@@ -1543,76 +1543,52 @@ void GpuBooster::fit_batch(const std::vector<GpuBooster*>& bs, const std::vector
     for (auto* b : bs)
         if (b->device != b0.device) throw TideError("fit_batch: boosters must share one device");
     cudaStream_t s = b0.ds_->stream;
-    // The buffers belong to the boosters' own streams, the trees run on s: nothing goes back
-    // before s is done with it, however the call ends.
+    std::vector<std::unique_ptr<FitRun>> own(bs.size());
+    std::vector<FitRun*> runs(bs.size());
+    // The buffers belong to the boosters' own streams, the trees run on s: the runs do not go
+    // before s is done with what they hold, however the call ends.
     struct SyncOnExit {
         cudaStream_t s;
         ~SyncOnExit() { cudaStreamSynchronize(s); }
     } sync_on_exit{s};
-    std::vector<std::unique_ptr<FitRun>> own;
-    std::vector<FitRun*> runs;
-    for (size_t k = 0; k < bs.size(); ++k) {
+    auto reset = [&](int k) {
         bs[k]->stats = FitStats();
         Config ck = bs[k]->cfg;
         if (k > 0) {  // one timing range for the whole batch
             ck.timing_from = -1;
             ck.profile_hist = false;
         }
-        own.push_back(std::make_unique<FitRun>(*bs[k], ck, *bs[k]->ds_, s, false));
-        runs.push_back(own.back().get());
-    }
+        own[k] = std::make_unique<FitRun>(*bs[k], ck, *bs[k]->ds_, s, false);
+        runs[k] = own[k].get();
+    };
+    for (size_t k = 0; k < bs.size(); ++k) reset(static_cast<int>(k));
     // Set-ups overlap, each on its booster's stream: one fit's upload runs under the binning
     // of others, whose shuffles and sorts (a CTA per feature) leave most of the chip idle.  Three
     // at a time, as long as their uploaded X together stay within kBatchUpload; a larger one goes
     // alone, as when they ran one after another (6 folds of 0.4M to 0.85M x 64: 57 ms of 141).
+    // Where the device has no room for them together they run one after another after all.
     constexpr size_t kBatchUpload = 8ull << 30;
     constexpr int kBatchThreads = 3;
-    std::mutex mu;
-    std::condition_variable cv;
-    size_t next = 0, uploading = 0;
-    int running = 0;
-    std::vector<std::exception_ptr> failed(bs.size());
-    bool stop = false;
-    auto work = [&] {
-        while (true) {
-            size_t k, bytes;
-            {
-                std::unique_lock<std::mutex> lk(mu);
-                cv.wait(lk, [&] {
-                    if (stop || next >= bs.size()) return true;
-                    const size_t b = static_cast<size_t>(std::max(in[next].n, 0)) * std::max(in[next].n_f, 0) *
-                                     (in[next].x_dtype == 0 ? 4 : 8);
-                    return running == 0 || uploading + b <= kBatchUpload;
-                });
-                if (stop || next >= bs.size()) return;
-                k = next++;
-                bytes = static_cast<size_t>(std::max(in[k].n, 0)) * std::max(in[k].n_f, 0) * (in[k].x_dtype == 0 ? 4 : 8);
-                uploading += bytes;
-                ++running;
-            }
+    run_setups(
+        static_cast<int>(bs.size()), kBatchThreads, kBatchUpload,
+        [&](int k) {
+            return static_cast<size_t>(std::max(in[k].n, 0)) * std::max(in[k].n_f, 0) * (in[k].x_dtype == 0 ? 4 : 8);
+        },
+        [&](int k) { runs[k]->prepare(in[k].X, in[k].x_dtype, in[k].y, in[k].n, in[k].n_f, in[k].ts, in[k].entity); },
+        [&](int k) {
+            reset(k);
+            bs[k]->ds_->release_fit_buffers();
+            check(cudaStreamSynchronize(bs[k]->ds_->stream), "set-up taken back");  // the pool has its memory again
+        },
+        [](const std::exception_ptr& e) {
             try {
-                runs[k]->prepare(in[k].X, in[k].x_dtype, in[k].y, in[k].n, in[k].n_f, in[k].ts, in[k].entity);
+                std::rethrow_exception(e);
+            } catch (const OutOfMemory&) {
+                return true;
             } catch (...) {
-                failed[k] = std::current_exception();
+                return false;
             }
-            {
-                std::lock_guard<std::mutex> lk(mu);
-                uploading -= bytes;
-                --running;
-                if (failed[k]) stop = true;  // as when they ran in order: no later one starts
-            }
-            cv.notify_all();
-        }
-    };
-    {
-        std::vector<std::thread> th;
-        const size_t n_th = std::min<size_t>(kBatchThreads, bs.size());
-        for (size_t t = 1; t < n_th; ++t) th.emplace_back(work);
-        work();
-        for (auto& t : th) t.join();
-    }
-    for (auto& f : failed)
-        if (f) std::rethrow_exception(f);
+        });
     fit_runs(runs, s);
     std::vector<size_t> refit;
     for (size_t k = 0; k < bs.size(); ++k) {
