@@ -1706,7 +1706,48 @@ struct PinnedBlock {
 // a number of rows, which bounds the pinned block of the results (2 MB).
 constexpr size_t kPredictChunkBytes = 16u << 20;
 constexpr size_t kPredictChunkRows = 131072;
+int predict_chunk_rows(int n, size_t row_bytes) {
+    return static_cast<int>(std::min({static_cast<size_t>(n), kPredictChunkRows,
+                                      std::max<size_t>(1024, kPredictChunkBytes / row_bytes / 1024 * 1024)}));
+}
+// What the pool rounds up, the context's share of a launch, small arrays.
+constexpr size_t kWorkingSetSlack = 64u << 20;
 }  // namespace
+
+size_t predict_working_set(const Config& c, int n, int n_f, int x_dtype) {
+    const size_t xsz = x_dtype == 0 ? 4 : 8, stride = (static_cast<size_t>(n_f) + 15) / 16 * 16;
+    const size_t nodes = static_cast<size_t>(c.n_estimators) * (2 * static_cast<size_t>(c.max_leaves) - 1);
+    const size_t chunk = static_cast<size_t>(predict_chunk_rows(n, n_f * xsz)), slots = chunk < static_cast<size_t>(n) ? 2 : 1;
+    return chunk * (slots * (n_f * xsz + 8) + stride) +            // X, results, codes
+           nodes * (8 + 8 + 32 + 2) + n_f * 256 * xsz +           // the model's layout and its edges
+           kWorkingSetSlack;
+}
+
+// The buffers of FitRun::prepare and of the binner, all at once (X and the binner's go before the GOSS
+// buffers come).
+size_t fit_working_set(const Config& c, int n_in, int n_f_in, int x_dtype) {
+    const size_t n = n_in, n_f = n_f_in, xsz = x_dtype == 0 ? 4 : 8;
+    const bool const_h = c.objective == 0, wave = c.grow != 0;
+    const int mode = hist_mode(c.hist_bits, const_h);
+    const size_t max_nodes = 2 * static_cast<size_t>(c.max_leaves) - 1, T = c.n_estimators;
+    const size_t col = n_f * static_cast<size_t>(codes_col_pitch(n_in));
+    size_t per_row = 3 * 8 + (const_h ? 0 : 8 + 4)  // y, pred, g, h, order
+                     + 2 * 4 + 2                    // row lists, leaf ids
+                     + (wave ? 2 * hist_pay_bytes(mode) + (mode == kHistExactVar ? 16 : 0) : 8);
+    if ((c.goss > 0 || (c.goss < 0 && n >= 250000)) && c.goss_top < 1.0)
+        per_row += 2 * 8 + 2 * 4 + 1 + 12                                                  // keys, values, flags, the sort's
+                   + static_cast<size_t>(std::ceil(8.0 * std::min(1.0, std::max(0.0, c.goss_other))));  // positions
+    const size_t slots = wave ? 1 + 2 * max_nodes : max_nodes;
+    size_t bytes = n * (n_f * xsz + (n_f + 15) / 16 * 16 + per_row) + col + slots * n_f * kBins * 20;
+    bytes += T * max_nodes * (sizeof(DevNode) + 8 + 4 + 8 * static_cast<size_t>(std::max(64, c.n_time_buckets)));  // the trees
+    bytes += (2 * kMaxNodes + 1) * n_f * (8 + 4 + 32);                                                        // scan candidates
+    if (c.pair_splits && n < 1000000)
+        bytes += static_cast<size_t>(wave_children(c.max_leaves, c.wave_expand)) * kMaxPairs * kBins * 20;
+    // the binner's samples, draws and kept bits, as far as they do not fit the column-major codes
+    const size_t sample = std::min(n, static_cast<size_t>(std::max(0, c.bin_sample)));
+    const size_t scratch = n_f * (sample * (3 * xsz + 8) + n / 8 + 256 * 8);
+    return bytes + (scratch > col ? scratch - col : 0) + kWorkingSetSlack;
+}
 
 // X in chunks: the copy stream brings chunk c + 1 while the booster's stream transforms and
 // walks chunk c, and the host moves the results of chunk c - 1 from pinned memory to `out`.
@@ -1726,9 +1767,7 @@ void GpuBooster::predict_raw(const void* X, int x_dtype, int n, int n_f, double*
     if (D.edges_dtype != dtype) upload_edges(dtype);
     const PredictTrees m{D.t_word.p,    D.t_val.p, D.t_trees.p, D.t_batches.p, D.n_batches, D.t_cat.p,
                          D.t_feat2.p, n_bins,    D.any_kind};
-    const int chunk = static_cast<int>(
-        std::min({static_cast<size_t>(n), kPredictChunkRows,
-                  std::max<size_t>(1024, kPredictChunkBytes / row_bytes / 1024 * 1024)}));
+    const int chunk = predict_chunk_rows(n, row_bytes);
     const int n_chunks = (n + chunk - 1) / chunk, slots = std::min(2, n_chunks);
     DBuf<unsigned char> Xd;
     DBuf<uint8_t> codes;

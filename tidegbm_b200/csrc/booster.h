@@ -192,6 +192,11 @@ private:
     DeviceState* ds_ = nullptr;
 };
 
+// Upper estimates of the device memory that a fit or a prediction of this configuration holds, from
+// the sizes its buffers are allocated with, and an allowance for scratch.
+size_t fit_working_set(const Config& c, int n, int n_f, int x_dtype);
+size_t predict_working_set(const Config& c, int n, int n_f, int x_dtype);
+
 // Host part of Binner::fit (cpp/src/binning.cpp:14-102) for numeric features: the
 // sampled values per feature and their quantile edges.  Returns max_bins().
 int binner_fit(const void* X, int x_dtype, int n, int n_f, int max_bin, int bin_sample, uint32_t seed,

@@ -55,23 +55,9 @@ namespace {
 
 thread_local std::string g_err;
 
-// Device working set of a fit or predict request, the serving loop's admission figure:
-// the buffers of one fit context (X during binning, row-major and column-major codes,
-// per-row f64 state, row lists, GOSS keys, the node histograms) or of one prediction
-// (X, codes, output), plus a fixed allowance for scratch and the CUDA context's share.
-size_t working_set_bytes(const tgb::Config& c, int kind, long long n, long long n_f, int x_dtype) {
-    const long long xsz = x_dtype == 0 ? 4 : 8;
-    const long long stride = (n_f + 15) / 16 * 16;
-    const long long pitch = (n + 15) / 16 * 16;
-    const long long slack = 64ll << 20;
-    if (kind == 1) return static_cast<size_t>(n * n_f * xsz + n * stride + 8 * n + slack);
-    const long long per_row = 8 * 3              // y, pred, g
-                              + (c.objective == 0 ? 16 : 40)  // payloads in both row buffers (+ h)
-                              + 8 + 2            // row lists, leaf ids
-                              + 26;              // GOSS keys, values and flags
-    const long long nodes = 2ll * c.max_leaves - 1;
-    const long long hist = n_f * 256 * 20 * nodes;
-    return static_cast<size_t>(n * n_f * xsz + n * stride + n_f * pitch + per_row * n + hist + slack);
+// Device working set of a fit (kind 0) or predict request, the serving loop's admission figure.
+size_t working_set_bytes(const tgb::Config& c, int kind, int n, int n_f, int x_dtype) {
+    return kind == 1 ? tgb::predict_working_set(c, n, n_f, x_dtype) : tgb::fit_working_set(c, n, n_f, x_dtype);
 }
 
 template <class F>
