@@ -23,7 +23,6 @@
 // waits for X the rest (its bytes take 396 us; four CTAs 805, six of six rows 862).
 #include "tgb_internal.h"
 
-#include <atomic>
 #include <cmath>
 
 namespace tgb {
@@ -257,16 +256,8 @@ void launch_bin(const T* X, int n, int n_f, const T* edges, const int* n_edges, 
     const int ctas = std::max(1, 148 * (sizeof(T) == 4 ? kBinCtas32 : kBinCtas64) / groups);
     const int min_rows = kBinWarps * kBinRows;
     const int rows_per_cta = std::max(min_rows, (n + ctas - 1) / ctas);
-    {
-        static std::atomic<bool> done[64] = {};
-        int dev = 0;
-        check(cudaGetDevice(&dev), "cudaGetDevice");
-        if (dev < 0 || dev >= 64 || !done[dev]) {
-            check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)),
-                  "bin smem attr");
-            if (dev >= 0 && dev < 64) done[dev] = true;
-        }
-    }
+    // on every call (under 1 us), so that it holds after a cudaDeviceReset too
+    check(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)), "bin smem attr");
     dim3 grid((n + rows_per_cta - 1) / rows_per_cta, groups);
     kern<<<grid, kBinThreads, smem, s>>>(X, n, n_f, edges, n_edges, codes, stride, rows_per_cta, is_cat);
     check(cudaGetLastError(), "bin_transform launch");
