@@ -127,8 +127,8 @@ TGB_API int tgb_fit_stats(tgb_booster* b, double* out18);
  * "transpose", "trees", "pre_upload" / "prep" (host set-up before the upload / before
  * the tree loop), "goss_refits" (1 when the fit was repeated with the full 64-bit GOSS
  * sort), "timed_selects" (wave selects run in the timed range: with batched growth a tree
- * runs 3 + 4 x (selects - 1) kernels in its waves), "graph_used" (1 when trees ran as
- * a CUDA graph), "hist_cluster" / "hist_clusters" (the tuned launch shape of the
+ * runs 3 + 4 x (selects - 1) kernels in its waves, one more for each select with categorical
+ * columns and with PAIR splits), "graph_used" (1 when trees ran as a CUDA graph), "hist_cluster" / "hist_clusters" (the tuned launch shape of the
  * histogram: CTAs per cluster, clusters launched), "driver" (set-up of the batched
  * growth), "driver_free" (its release after the tree loop), "finish_sync" (from the tree
  * loop's end to the GOSS sampler's stop), "release" (the fit's buffers back to the pool),

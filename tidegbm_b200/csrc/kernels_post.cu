@@ -37,7 +37,7 @@ __device__ __forceinline__ void add64s(unsigned int* lo, unsigned int* hi, int k
     if (up != 0u) atomicAdd(&hi[k], up);
 }
 
-constexpr int kApplyRows = 8;  // rows a thread walks together
+constexpr int kApplyRows = 8;  // rows a thread walks together in the gather walk (two in the staged one)
 
 // Staged walk: a block stages, per tile of kStageRows rows, only the columns the tree
 // splits on (each distinct split feature once, 16-byte copies of whole tile runs) in shared

@@ -1,16 +1,17 @@
 // Wave scan and select (wave.h describes the scheme).  Compiled with -fmad=false: the
 // gain arithmetic follows the reference's statement order (scan_common.cuh).
 //
-// scan: one CTA of 256 threads (thread = bin) per (child, feature), grid-stride over the
-// children of all planned leaves of all contexts (or over the roots).  The larger child's
-// histogram is derived as parent - smaller child on the way (subtract_hist_inplace,
-// cpp/src/histogram.cpp:108-117, exact in fixed point).  The last CTA of a child to
-// finish (ticket counter, nothing waits) reduces the per-feature candidates, lowest
-// feature on ties (best_for_leaf, cpp/src/tree.cpp:120-166).
+// scan: one warp per (child, numeric feature), grid-stride over the children of all planned
+// leaves of all contexts (or over the roots), one CTA of 256 threads (thread = bin) per
+// categorical feature.  The larger child's histogram is derived as parent - smaller child on
+// the way (subtract_hist_inplace, cpp/src/histogram.cpp:108-117, exact in fixed point).  The
+// last feature of a child to finish (ticket counter, nothing waits) reduces the per-feature
+// candidates, lowest feature on ties (best_for_leaf, cpp/src/tree.cpp:120-166).
 //
 // select: one warp per context.  It commits expanded best leaves in the reference's
 // best-first order (grow_tree, cpp/src/tree.cpp:343-383) and plans the next wave's
-// expansions; the last context to finish sets the launch-loop condition.
+// expansions; the last context to finish sets the condition of the tree graph's next
+// conditional node.
 #include "scan_common.cuh"
 #include "wave.h"
 
@@ -453,7 +454,6 @@ __global__ void __launch_bounds__(kSelectThreads)
                     const bool pr = X.pair_on && pair_used < X.max_pair;
                     const DevSplit S = pr ? X.splits_pair[L] : splits[L];
                     tiles = (N.count + kPartTile - 1) / kPartTile;
-                    ctl->exp_leaf[e] = L;
                     ctl->part_cur[e] = 0ull;
                     ctl->expanded[L] = pr ? 2 : 1;
                     ctl->exp[e] = WaveExp{L, N.start, N.count, N.buf, S.feature, S.threshold, S.missing_left, S.type,
@@ -511,7 +511,7 @@ __global__ void __launch_bounds__(kSelectThreads)
             }
         }
     }
-    // launch-loop condition: any context still growing (the last context to finish sets it)
+    // the condition: any context still growing (the last context to finish sets it)
     if (threadIdx.x == 0) {
         unsigned v = active ? 1u : 0u;
         bool last = true;

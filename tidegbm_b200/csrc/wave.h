@@ -21,7 +21,8 @@
 //             child is free: everything computed from a row list is an exact integer sum.
 //   histogram the smaller child of every planned leaf, one persistent cluster launch
 //             over all (context, leaf) jobs: rows x feature groups cut into one
-//             contiguous range per cluster.
+//             contiguous range per cluster, or, where there are clusters enough, clusters
+//             of its own for every (job, group).
 //   scan      both children of every planned leaf (the larger by parent - smaller,
 //             histogram.cpp:108-117) for their best split and their totals.
 //
@@ -99,7 +100,6 @@ struct WaveCtl {
     int pair_used;    // PAIR splits committed in this tree
     int exp_total;    // expansions planned over all trees of the fit (not reset per tree)
     int pad[2];
-    int exp_leaf[kMaxLeavesCap];
     int exp_tile0[kMaxLeavesCap + 1];
     // rows of the planned leaf placed so far by its partition tiles: left in the low word,
     // right in the high word (zeroed by the select that plans the expansion)
@@ -257,8 +257,9 @@ bool encode_codes_map(CUtensorMap* map, const uint8_t* codes, long long n_rows, 
 void launch_wave_hist(int mode, const WaveCtx* ctxs, int n_ctx, int src, HistTune tune,
                       unsigned long long* rows_counter, cudaStream_t s);
 void launch_wave_scan(const WaveCtx* ctxs, int n_ctx, int src, int max_f, int ys, bool any_cat, cudaStream_t s);
-// gsync: 2 device ints (flag, ticket), zero.  host_flag: mapped host word or nullptr;
-// cond / use_cond: the graph's loop condition (set to "any context still growing").
+// gsync: 3 device ints (flag, ticket, selects run so far), zeroed before the first select.
+// host_flag: mapped host word or nullptr; cond / use_cond: the condition of a node of the graph,
+// set to "any context still growing".
 void launch_wave_select(const WaveCtx* ctxs, int n_ctx, int* gsync, unsigned* host_flag,
                         unsigned long long cond, int use_cond, cudaStream_t s);
 void launch_wave_partition(const WaveCtx* ctxs, int n_ctx, int grid, bool pair, cudaStream_t s);
