@@ -710,8 +710,14 @@ __device__ __forceinline__ void flush_piece(const WaveCtx& X, const unsigned lon
 //
 // The plan and each piece's parameters are worked out by one warp and left in shared memory:
 // 32 warps doing the same scalar work (64-bit divisions above all) took 8,000 cycles a piece.
+//
+// kPieceRows 0 (equal ranges only, nearly) / 500 / 1,500 / 5,000: 1.2M x 96 int8 73.8 / 64.5 / 64.8 /
+// 64.7 ms, 0.85M x 64 pairwise 67.6 / 61.5 / 62 / 61.6, 20k x 16 35.8 / 32.8 / 32.3 / 31.4 (0.5 apart
+// from run to run): anything but 0.  kMinCtaRows, below which a pair is not split further (a
+// CTA's fold and flush cost more than its rows), 32 / 128 / 512: 64.4 / 64.8 / 64.4 and 31.5 / 32.3 /
+// 32.4 ms, within the noise.
 constexpr int kPieceRows = 1500;
-constexpr int kMinCtaRows = 128;  // no finer split of a pair: a CTA's fold and flush cost more
+constexpr int kMinCtaRows = 128;
 constexpr int kWarpJobs = 32;
 
 template <int kMode>

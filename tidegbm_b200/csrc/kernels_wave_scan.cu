@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(kSelectThreads)
 constexpr int kPairThreads = 256;
 constexpr int kPairWarps = kPairThreads / 32;
 constexpr int kPairChunk = 8192;   // the 19-bit low sums stay below 2^32, the counts in 16 bits
-constexpr int kPairMinChunk = 512;
+constexpr int kPairMinChunk = 512;  // 256 / 512 / 2,048: 100k x 32 60.1 / 60.3 / 62.2 ms, 20k x 32 40.7 / 40.9 / 41.7
 constexpr int kPairLo = 19;
 constexpr int kPairTop = 6;        // pair_top_k (host-checked)
 
