@@ -19,3 +19,22 @@ def test_a_fit_after_one_out_of_memory(native):
     got = native.Booster(**params)
     got.fit(X, y, timestamps=ts)
     assert np.array_equal(got.raw_predict(X), want.raw_predict(X))
+
+
+def test_a_batch_after_one_whose_set_up_fails(native):
+    rng = np.random.default_rng(1)
+    data = []
+    for n in (3000, 200, 5000, 700):
+        X = rng.standard_normal((n, 6)).astype(np.float32)
+        data.append((X, X[:, 0] + 0.1 * rng.standard_normal(n), np.arange(n) // 10))
+    params = dict(n_estimators=3, horizon=1, pair_splits=False, goss=1, min_samples_leaf=5)
+    bs = [native.Booster(**params) for _ in data]
+    bs[1].set_config(max_leaves=1)
+    with pytest.raises(native.TideError, match="max_leaves"):
+        native.Booster.fit_batch(bs, *[list(c) for c in zip(*data)])
+    bs[1].set_config(max_leaves=31)
+    native.Booster.fit_batch(bs, *[list(c) for c in zip(*data)])
+    for b, (X, y, ts) in zip(bs, data):
+        own = native.Booster(**params)
+        own.fit(X, y, timestamps=ts)
+        assert np.array_equal(b.raw_predict(X), own.raw_predict(X))
