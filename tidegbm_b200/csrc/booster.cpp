@@ -1309,7 +1309,10 @@ private:
     // only the first kWaveSteps[0] waves run in any case, the further ones as bodies of IF nodes,
     // in steps about as long as what came before.  Fits of 80 trees of one or two leaves, 5,000 rows:
     // 14.2 -> 9.8 ms with 31 leaves allowed, 23.7 -> 13.3 with 255 (12.3 and 15.2 with every wave
-    // an iteration of the loop); an IF node costs a full tree 5 us (fit of 100k x 32: 60.0 -> 60.5 ms).
+    // an iteration of the loop); an IF node costs a full tree 5 to 10 us.  Fits of 100k x 32, 1.2M x 96
+    // int8 and 20k x 16 by steps, ms: 16 (no IF) 60.5, 64.2, 31.3; 3, 8, 16 60.4, 64.9, 31.5; 4, 8, 16
+    // 61.0, 64.8, 32.2; 3, 5, 8, 16 62.2, 66.3, 32.4; 6 alone 59.4, 64.3, 31.9, but 40 us of empty
+    // waves for a tree of one leaf.
     void build_graph() {
         check(cudaGraphCreate(&graph_, 0), "graph create");
         std::vector<OwnedStream>(n_ctx_ - 1).swap(side_);
