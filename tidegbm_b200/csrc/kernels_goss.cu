@@ -74,8 +74,9 @@ __global__ void goss_fixup_kernel(const unsigned int* __restrict__ k32, const in
         int e = p + 1;
         while (e < n && e - a < kMaxRun && k32[e] == k) ++e;
         const unsigned long long km = abs_bits(g, me);
-        if ((a > 0 && k32[a - 1] == k) || (e < n && k32[e] == k)) {
-            // long run: in order as it is only if every pattern in it is equal
+        if (e - a > kMaxRun || (a > 0 && k32[a - 1] == k) || (e < n && k32[e] == k)) {
+            // long run (of kMaxRun + 1 the last element sees the whole): in order as it is only if
+            // every pattern in it is equal
             if (p > 0 && k32[p - 1] == k && abs_bits(g, order[p - 1]) != km) atomicExch(overflow, 1);
             fixed[p] = me;
             continue;
